@@ -129,7 +129,7 @@ struct FourierLayout {
 };
 
 // op codes
-enum { OP_SP2FC = 0, OP_SP2FCDMU = 1, OP_DV2UV = 2, OP_SP2FC_GPMT = 3 };
+enum { OP_SP2FC = 0, OP_SP2FCDMU = 1, OP_DV2UV = 2 };
 enum { OP_FC2SP = 0, OP_UV2DV = 1, OP_QTEND = 2, OP_MKTEND = 3 };
 
 // SIMT Legendre launchers (legendre_simt.cu)
@@ -139,6 +139,12 @@ exotx_status leg_inverse_l(exotx_plan p, int op, const T *a, const T *b, T *oa, 
 template <typename T>
 exotx_status leg_forward_l(exotx_plan p, int op, const T *const *in, T *const *out, int nlev,
                            FourierLayout L, long long o_fs, cudaStream_t s);
+// the Legendre half of a whole set in one launch, on the m-major intermediate W
+// of ninst states (dset = 0 gridpointa, 1 gridpointd)
+template <typename T>
+exotx_status leg_inverse_set(exotx_plan p, int dset, const T *spin, T *W, int L, int ninst, cudaStream_t s);
+template <typename T>
+exotx_status leg_forward_set(exotx_plan p, int dset, const T *W, T *spout, int L, int ninst, cudaStream_t s);
 
 // FFT launchers (fft.cu).  kf = Fourier coefficients read (inverse) or
 // written (forward) per row; the rest are zero.  Fourier side addressed as

@@ -104,33 +104,9 @@ static exotx_status forward_set_static(exotx_plan p, const T *gpin, T *spout, in
             g_tw_esz[dev] = (int)sizeof(T);
         }
     }
-    const long long nrsp = 2LL * p->ncsp;
     const long long nrows = (9LL * L + 1) * p->nlat;
     EXOTX_TRY(fft_forward_tw<T>(gpin, W, p->nlon, nrows, p->ntp1, 1, nrows, dw, dr, s));
-    const FourierLayout F{p->nlat, 1, nrows, p->ntp1};
-    auto fld = [&](long long f) -> const T * { return W + 2 * f * p->nlat; };
-    // gtn[L] gqn[L] gut[L] gvt[L] guz[L] gvz[L] gke[L] gvpp guq[L] gvq[L]
-    const T *gtn = fld(0), *gqn = fld(L), *gut = fld(2 * L), *gvt = fld(3 * L), *guz = fld(4 * L),
-            *gvz = fld(5 * L), *gke = fld(6 * L), *gvpp = fld(7 * L), *guq = fld(7 * L + 1),
-            *gvq = fld(8 * L + 1);
-    T *sdf = spout, *stf = spout + L * nrsp, *szf = spout + 2 * L * nrsp, *sqf = spout + 3 * L * nrsp,
-      *spf = spout + 4 * L * nrsp;
-    {
-        const T *in[1] = {gvpp};
-        T *out[1] = {spf};
-        EXOTX_TRY(leg_forward_l<T>(p, OP_FC2SP, in, out, 1, F, nrsp, s));
-    }
-    {
-        const T *in[6] = {gtn, gvz, guz, gke, gut, gvt};
-        T *out[3] = {sdf, stf, szf};
-        EXOTX_TRY(leg_forward_l<T>(p, OP_MKTEND, in, out, L, F, nrsp, s));
-    }
-    {
-        const T *in[3] = {gqn, guq, gvq};
-        T *out[1] = {sqf};
-        EXOTX_TRY(leg_forward_l<T>(p, OP_QTEND, in, out, L, F, nrsp, s));
-    }
-    return EXOTX_OK;
+    return leg_forward_set<T>(p, 0, W, spout, L, 1, s);
 }
 
 }  // namespace exotx
