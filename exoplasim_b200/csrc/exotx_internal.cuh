@@ -91,12 +91,13 @@ struct exotx_plan_s {
     int *d_woff = nullptr;        // first mode index of each m, [ntp1+1]
     double *d_sid = nullptr, *d_gwd = nullptr;
     double *d_qref = nullptr;     // 8 tables, reference layout q(NCSP,NLAT) [t][lat][w]
-    // inverse tables qi,qj,qu,qv for northern latitudes, [t][w][j] (j fastest)
+    // inverse tables qi,qj,qu,qv for northern latitudes, [t][w][j] (j fastest), then 8 rows of zeros
     double *d_inv64 = nullptr;
-    float *d_inv32 = nullptr;
-    // forward tables qc,qe,qm,qq for northern latitudes, per m block [t][woff*nlath + j*K + (n-m)]
+    // forward tables qc,qe,qm,qq for northern latitudes: fwd_tsz entries each, the block
+    // (m, parity p of n-m) at d_foff[2m + p] holding [j][(n-m-p)/2, padded to 8]
     double *d_fwd64 = nullptr;
-    float *d_fwd32 = nullptr;
+    long long *d_foff = nullptr;
+    size_t fwd_tsz = 0;
     double *d_fs64 = nullptr, *d_fg64 = nullptr;  // skspgp, skgpsp [ntp1]
     float *d_fs32 = nullptr, *d_fg32 = nullptr;
     // work buffer for the forward transform set (Fourier rows of gpin)

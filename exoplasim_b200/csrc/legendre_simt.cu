@@ -1,4 +1,6 @@
-// Folded SIMT Legendre transforms (FP64 parity path and FP32 path).
+// Folded Legendre transforms of the FP64 and FP32 paths on the FP64 tensor
+// cores (mma.sync m8n8k4.f64: fused multiply-adds in FP64, no split or rounding
+// of the operands; tcgen05 has no FP64 form).
 //
 // Every spectral->Fourier operation of legmod.f90 is, per zonal wavenumber m,
 //     F(lat, m) = sum_n c * T(m,n,lat) * X(m,n)      c in {1,-1,i,-i}
@@ -15,26 +17,45 @@
 //
 // A transform set is one launch per direction: the blocks of one launch cover
 // every field, level and state of the set, so a small set fills the GPU and
-// pays one launch.  Each thread keeps a register tile of the contraction
-// (inverse: latitudes x columns, forward: modes x the outputs of a level) and
-// reads its table entries straight from global memory (coalesced, shared by
-// the block's warps through L1) one step ahead of their use; the other operand
-// is staged in shared memory and read as broadcasts.
+// pays one launch.  A warp owns 8-row tiles of the table (latitudes inverse,
+// modes forward) by groups of 8 real columns (4 complex fields or levels).  Its
+// table fragments come straight from global memory (64-byte runs, shared by the
+// block's warps through L1), one step ahead of their use; the other operand is
+// staged in shared memory as FP64, also for the FP32 path, whose arrays are
+// float but whose sums run in FP64 with the FP64 tables and are rounded once.
+// Factors i and -i read the partner column (re <-> im) and flip its sign.
+//
+// One T127 L20 state, FP64: INV_A_US inverse and FWD_A_US forward against 147
+// and 180 us for register-tiled FP64 FMA kernels (4 x 4 tiles: 240 registers,
+// 6 warps per SM, the FP64 pipe 16% busy: two of three instructions were loads
+// and addresses).  Eight DMMAs need six loads here, and the FP64 tensor cores
+// were measured at 36.7 TFLOP/s (FMA: 30.8).
 //
 // Fourier-side addressing of the single operations is general: complex
 // element (field f, latitude l, wavenumber m) lives at base + f*fs + l*ls +
 // m*ms (complex units).  The sets work on the plan's m-major intermediate,
 // complex (field, l, m) at m*nrows + field*nlat + l.
 #include <algorithm>
+#include <type_traits>
 #include "exotx_internal.cuh"
 
 namespace exotx {
 
 template <typename T> struct __align__(2 * sizeof(T)) C2 { T x, y; };
+using Z2 = C2<double>;
 // a caller's array is aligned to its reals only
-template <typename T> __device__ __forceinline__ C2<T> ld2(const T *p) { return C2<T>{p[0], p[1]}; }
-__device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
-__device__ __forceinline__ float mad(float a, float b, float c) { return fmaf(a, b, c); }
+template <typename T> __device__ __forceinline__ Z2 ld2(const T *p) { return Z2{(double)p[0], (double)p[1]}; }
+
+// d (8x8, lane: row lane/4, columns 2(lane%4) and +1) += a (8x4, lane: row
+// lane/4, column lane%4) * b (4x8, lane: row lane%4, column lane/4)
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
+}
+// row stride (doubles) of staged operands of nc real columns (a multiple of 8):
+// 4 or 12 mod 16, so the four rows of a fragment fall on distinct banks
+__host__ __device__ constexpr int leg_stride(int nc) { return nc + 4; }
 
 constexpr int LEG_MAXSMEM = 200 * 1024;
 
@@ -45,17 +66,18 @@ constexpr int LEG_MAXSMEM = 200 * 1024;
 //   2  qu and qv: a unit is a (divergence, vorticity) pair -> (u, v)
 template <typename T>
 struct LegInv {
-    const T *tab;        // 4 inverse tables [t][w][j]
+    const double *tab;   // 4 inverse tables [t][w][j]
     const int *woff;
-    const T *filt;       // skspgp(n)
+    const double *filt;  // skspgp(n)
     const T *a, *b;      // spectral inputs (re, im pairs); single op: fields a (and b) at stride a_fs (b_fs)
     long long a_fs, b_fs;
     T *oa, *ob;          // Fourier outputs (set: oa is the intermediate)
     long long fs, ls, ms, nrows;
     int nu[3], nt[3];    // units and column tiles of each group
-    int ntiles, ty, tx;  // tiles per wavenumber; threads along columns and latitudes
+    int ntiles, nlb;     // tiles per wavenumber; latitude blocks
+    int wm, wn, kc;      // warps along latitudes and columns; modes staged at a time
     int L, nlat, nlath, ntp1, ncsp, nrsp, dset, mz;  // single op: wavenumbers ntp1 <= m < mz are zeroed
-    T plavor;
+    double plavor;
 };
 
 // field maps of the sets: gridpointa takes sd[L] st[L] sz[L] sq[L] sp to
@@ -74,26 +96,22 @@ __device__ __forceinline__ void inv_field(int L, int dset, int u, int *inst, int
     }
 }
 
-// Tile: JT latitudes x CC complex columns per thread (a column pair's two
-// parities in separate sums).  Bound by the FP64 / FP32 pipe once the tile is
-// 4 x 4 and by latency at the small resolutions, where 1 x 1 tiles spread the
-// outputs over more threads (see inv_tile).
-template <typename T, int JT, int CC, bool SET>
+// A warp: MT tiles of 8 latitudes x NT groups of 4 complex columns (group 2:
+// x 4 (D, Z) pairs), both parities of n-m in separate accumulators.
+template <typename T, int MT, int NT, bool SET>
 __global__ void __launch_bounds__(256) k_leg_inv(const __grid_constant__ LegInv<T> A) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    constexpr int LT = CC > 1 ? CC / 2 : 1;            // (D, Z) pairs per thread in group 2
-    constexpr int U = JT * CC >= 8 ? 2 : 4;            // modes whose table entries are fetched together (even)
-    C2<T> *xs = reinterpret_cast<C2<T> *>(smraw);
-    const int m = blockIdx.x / A.ntiles;
-    int ti = blockIdx.x - m * A.ntiles, g = 0;
+    double *xs = reinterpret_cast<double *>(smraw);
+    int ti = blockIdx.x % A.ntiles, g = 0;
+    const int mb = blockIdx.x / A.ntiles, m = mb / A.nlb, lb = mb - m * A.nlb;
     while (ti >= A.nt[g]) ti -= A.nt[g++];
-    const int cpt = g == 2 ? LT : CC, cb = A.ty * cpt, u0 = ti * cb, n = min(cb, A.nu[g] - u0);
+    const int cb = (g == 2 ? 4 : 4 * NT) * A.wn, u0 = ti * cb, n = min(cb, A.nu[g] - u0);
     const int nlat = A.nlat, nlath = A.nlath;
     pdl_trigger();
     pdl_wait();
     if (!SET && m >= A.ntp1) {   // the zero tail of the Fourier rows, wavenumbers fastest
         const int nz = A.mz - A.ntp1;
-        for (int i = threadIdx.x; i < n * nlat * nz; i += blockDim.x) {
+        for (int i = threadIdx.x + lb * blockDim.x; i < n * nlat * nz; i += A.nlb * blockDim.x) {
             const int z = i % nz, r = i / nz, lat = r % nlat, c = r / nlat;
             const size_t o = 2 * ((u0 + c) * A.fs + lat * A.ls + (long long)(A.ntp1 + z) * A.ms);
             A.oa[o] = 0; A.oa[o + 1] = 0;
@@ -101,97 +119,146 @@ __global__ void __launch_bounds__(256) k_leg_inv(const __grid_constant__ LegInv<
         }
         return;
     }
-    const int K = A.ntp1 - m, w0 = A.woff[m], Kp = (K + U - 1) / U * U;
-    const int cs = cb + 1;       // odd row stride in complex units: staging writes spread over the banks
-    C2<T> *xz = xs + (size_t)Kp * cs;
-    // stage the filtered coefficients as [k][column], zeros past the last mode and column
-    for (int i = threadIdx.x; i < cb * Kp; i += blockDim.x) {
-        const int c = i / Kp, k = i - c * Kp;
-        C2<T> va{0, 0}, vb{0, 0};
-        if (c < n && k < K) {
-            const T f = A.filt[m + k];
-            const T *pa, *pb = nullptr;
-            if constexpr (SET) {
-                int inst, fin, fout;
-                if (g == 0) inv_field(A.L, A.dset, u0 + c, &inst, &fin, &fout);
-                else if (g == 1) { inst = u0 + c; fin = 4 * A.L; }
-                else { inst = (u0 + c) / A.L; fin = (u0 + c) - inst * A.L; }
-                pa = A.a + ((size_t)inst * (4 * A.L + 1) + fin) * A.nrsp;
-                pb = pa + (size_t)2 * A.L * A.nrsp;
-            } else {
-                pa = A.a + (u0 + c) * A.a_fs;
-                if (g == 2) pb = A.b + (u0 + c) * A.b_fs;
+    const int K = A.ntp1 - m, w0 = A.woff[m];
+    const int rs = leg_stride(2 * cb);
+    double *xz = xs + (size_t)A.kc * rs;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
+    const int wn = warp / A.wm, wm = warp - wn * A.wm;
+    const int cw = wn * (g == 2 ? 4 : 4 * NT);                       // the warp's first column of the block
+    const int j0 = (lb * A.wm + wm) * 8 * MT;
+    const bool active = wn < A.wn && cw < n && j0 < nlath;
+    const size_t tsz = (size_t)A.ncsp * nlath;
+    int jc[MT];
+#pragma unroll
+    for (int i = 0; i < MT; i++) jc[i] = min(j0 + 8 * i + r, nlath - 1);
+    const double *t0 = A.tab + (g == 0 ? INV_QI : g == 1 ? INV_QJ : INV_QU) * tsz + (size_t)w0 * nlath;
+    const double *t1 = A.tab + INV_QV * tsz + (size_t)w0 * nlath;    // group 2
+    // accumulators by parity: [p][tile][column group] (group 2: symmetric and
+    // antisymmetric sums of u, then of v)
+    double acc[2][MT][NT < 2 ? 2 : NT][2];
+#pragma unroll
+    for (int p = 0; p < 2; p++)
+#pragma unroll
+        for (int i = 0; i < MT; i++)
+#pragma unroll
+            for (int c = 0; c < (NT < 2 ? 2 : NT); c++) acc[p][i][c][0] = acc[p][i][c][1] = 0.0;
+    for (int kb = 0; kb < K; kb += A.kc) {
+        const int kn = min(A.kc, K - kb), kp = (kn + 7) & ~7, kh = kp >> 1;
+        if (kb) __syncthreads();
+        // stage the filtered coefficients, even modes then odd ones, zeros past the last mode and column
+        for (int i = threadIdx.x; i < cb * kp; i += blockDim.x) {
+            const int c = i / kp, k = i - c * kp, mode = kb + k;
+            Z2 va{0, 0}, vb{0, 0};
+            if (c < n && mode < K) {
+                const double f = A.filt[m + mode];
+                const T *pa, *pb = nullptr;
+                if constexpr (SET) {
+                    int inst, fin, fout;
+                    if (g == 0) inv_field(A.L, A.dset, u0 + c, &inst, &fin, &fout);
+                    else if (g == 1) { inst = u0 + c; fin = 4 * A.L; }
+                    else { inst = (u0 + c) / A.L; fin = (u0 + c) - inst * A.L; }
+                    pa = A.a + ((size_t)inst * (4 * A.L + 1) + fin) * A.nrsp;
+                    pb = pa + (size_t)2 * A.L * A.nrsp;
+                } else {
+                    pa = A.a + (u0 + c) * A.a_fs;
+                    if (g == 2) pb = A.b + (u0 + c) * A.b_fs;
+                }
+                va = ld2(pa + 2 * (w0 + mode));
+                va.x *= f; va.y *= f;
+                if (g == 2) {
+                    // vorticity; plavor leaves mode (0,1) (legmod.f90:332)
+                    vb = ld2(pb + 2 * (w0 + mode));
+                    if (m == 0 && mode == 1) vb.x -= A.plavor;
+                    vb.x *= f; vb.y *= f;
+                }
             }
-            va = ld2(pa + 2 * (w0 + k));
-            va.x *= f; va.y *= f;
-            if (g == 2) {
-                // vorticity; plavor leaves mode (0,1) (legmod.f90:332)
-                vb = ld2(pb + 2 * (w0 + k));
-                if (m == 0 && k == 1) vb.x -= A.plavor;
-                vb.x *= f; vb.y *= f;
+            const size_t o = (size_t)((k & 1) * kh + (k >> 1)) * rs + 2 * c;
+            *reinterpret_cast<Z2 *>(xs + o) = va;
+            if (g == 2) *reinterpret_cast<Z2 *>(xz + o) = vb;
+        }
+        __syncthreads();
+        if (!active) continue;
+        const double *tk = t0 + (size_t)(kb + 2 * q) * nlath, *uk = t1 + (size_t)(kb + 2 * q) * nlath;
+        const int nst = kp >> 3;
+        if (g < 2) {
+            const double *xb = xs + q * rs + 2 * cw + r;
+            double fa[2][MT], fb[2][MT];   // table fragments of two steps (8 modes: 4 of each parity)
+            auto fetch = [&](double (&t)[2][MT], int st) {
+                const double *tp = tk + (size_t)(8 * st) * nlath;
+#pragma unroll
+                for (int p = 0; p < 2; p++)
+#pragma unroll
+                    for (int i = 0; i < MT; i++) t[p][i] = tp[p * nlath + jc[i]];
+            };
+            auto step = [&](const double (&t)[2][MT], int st) {
+#pragma unroll
+                for (int p = 0; p < 2; p++) {
+                    const double *xp = xb + (size_t)(p * kh + 4 * st) * rs;
+#pragma unroll
+                    for (int c = 0; c < NT; c++) {
+                        const double b = xp[8 * c];
+#pragma unroll
+                        for (int i = 0; i < MT; i++) dmma(acc[p][i][c], t[p][i], b);
+                    }
+                }
+            };
+            fetch(fa, 0);
+            for (int st = 0; st < nst; st += 2) {
+                if (st + 1 < nst) fetch(fb, st + 1);
+                step(fa, st);
+                if (st + 1 >= nst) break;
+                if (st + 2 < nst) fetch(fa, st + 2);
+                step(fb, st + 1);
+            }
+        } else {
+            // u = sum qv*Z - i*qu*D ; v = sum -i*qu*Z - qv*D  (legmod.f90:338-341)
+            const int rx = r ^ 1;
+            const double *xd = xs + q * rs + 2 * cw, *xv = xz + q * rs + 2 * cw;
+            double fa[2][MT], fb[2][MT];   // (qu, qv) fragments of one half step (4 modes of one parity)
+            auto fetch = [&](double (&t)[2][MT], int hs) {
+                const size_t o = (size_t)(8 * (hs >> 1) + (hs & 1)) * nlath;
+#pragma unroll
+                for (int i = 0; i < MT; i++) { t[0][i] = tk[o + jc[i]]; t[1][i] = uk[o + jc[i]]; }
+            };
+            auto half = [&](const double (&t)[2][MT], int st, auto par) {
+                constexpr int p = decltype(par)::value;
+                const size_t o = (size_t)(p * kh + 4 * st) * rs;
+                const double d = xd[o + r], z = xv[o + r];
+                double di = xd[o + rx], zi = xv[o + rx];   // -i*x: re <- im, im <- -re
+                if (r & 1) { di = -di; zi = -zi; }
+                // qu terms (P-type) and qv terms (Q-type) fall on opposite parities
+#pragma unroll
+                for (int i = 0; i < MT; i++) {
+                    dmma(acc[p][i][0], t[0][i], di);
+                    dmma(acc[1 - p][i][0], t[1][i], z);
+                    dmma(acc[p][i][1], t[0][i], zi);
+                    dmma(acc[1 - p][i][1], t[1][i], -d);
+                }
+            };
+            fetch(fa, 0);
+            for (int st = 0; st < nst; st++) {
+                fetch(fb, 2 * st + 1);
+                half(fa, st, std::integral_constant<int, 0>{});
+                if (st + 1 < nst) fetch(fa, 2 * st + 2);
+                half(fb, st, std::integral_constant<int, 1>{});
             }
         }
-        xs[(size_t)k * cs + c] = va;
-        if (g == 2) xz[(size_t)k * cs + c] = vb;
     }
-    __syncthreads();
-    const int ty = threadIdx.x / A.tx, tx = threadIdx.x - ty * A.tx;
-    if (ty >= A.ty) return;
-    const size_t tsz = (size_t)A.ncsp * nlath;
-    int jc[JT];
-#pragma unroll
-    for (int i = 0; i < JT; i++) jc[i] = min(tx + i * A.tx, nlath - 1);
-    const C2<T> *xr = xs + ty * cpt;
-    auto put = [&](T *o, long long f, int lat, C2<T> v) {
-        if constexpr (SET) reinterpret_cast<C2<T> *>(o)[(size_t)m * A.nrows + f * nlat + lat] = v;
-        else {
+    if (!active) return;
+    auto put = [&](T *o, long long f, int lat, double x, double y) {
+        if constexpr (SET) {
+            reinterpret_cast<C2<T> *>(o)[(size_t)m * A.nrows + f * nlat + lat] = C2<T>{(T)x, (T)y};
+        } else {
             const size_t e = 2 * (f * A.fs + lat * A.ls + (long long)m * A.ms);
-            o[e] = v.x; o[e + 1] = v.y;
+            o[e] = (T)x; o[e + 1] = (T)y;
         }
     };
     if (g < 2) {
-        // qi is P-type (even n-m symmetric), qj Q-type: its two sums swap roles
-        const T *tp = A.tab + (g == 0 ? INV_QI : INV_QJ) * tsz + (size_t)w0 * nlath;
-        C2<T> s[JT][CC], a[JT][CC];
-        T t0[U][JT], t1[U][JT];
+        // qi is P-type (even n-m symmetric); qj is Q-type: its two sums swap roles
 #pragma unroll
-        for (int i = 0; i < JT; i++)
-#pragma unroll
-            for (int c = 0; c < CC; c++) s[i][c] = a[i][c] = C2<T>{0, 0};
-        auto fetch = [&](T (&t)[U][JT], int k) {
-#pragma unroll
-            for (int e = 0; e < U; e++)
-#pragma unroll
-                for (int i = 0; i < JT; i++) t[e][i] = k + e < K ? tp[(size_t)(k + e) * nlath + jc[i]] : (T)0;
-        };
-        auto step = [&](const T (&t)[U][JT], int k) {
-#pragma unroll
-            for (int e = 0; e < U; e++) {
-                C2<T> x[CC];
-#pragma unroll
-                for (int c = 0; c < CC; c++) x[c] = xr[(size_t)(k + e) * cs + c];
-#pragma unroll
-                for (int i = 0; i < JT; i++)
-#pragma unroll
-                    for (int c = 0; c < CC; c++) {
-                        C2<T> &o = (e & 1) ? a[i][c] : s[i][c];
-                        o.x = mad(t[e][i], x[c].x, o.x);
-                        o.y = mad(t[e][i], x[c].y, o.y);
-                    }
-            }
-        };
-        fetch(t0, 0);
-        for (int k = 0; k < Kp; k += 2 * U) {
-            fetch(t1, k + U);
-            step(t0, k);
-            if (k + U >= Kp) break;
-            fetch(t0, k + 2 * U);
-            step(t1, k + U);
-        }
-#pragma unroll
-        for (int c = 0; c < CC; c++) {
-            const int u = u0 + ty * CC + c;
-            if (ty * CC + c >= n) continue;
+        for (int c = 0; c < NT; c++) {
+            const int u = u0 + cw + 4 * c + q;
+            if (cw + 4 * c + q >= n) continue;
             long long f = u;
             bool gpmt = false;
             if constexpr (SET) {
@@ -202,91 +269,40 @@ __global__ void __launch_bounds__(256) k_leg_inv(const __grid_constant__ LegInv<
                 gpmt = g == 0 && !A.dset && fout == 6 * A.L + 2;
             }
 #pragma unroll
-            for (int i = 0; i < JT; i++) {
-                const int j = tx + i * A.tx;
+            for (int i = 0; i < MT; i++) {
+                const int j = j0 + 8 * i + r;
                 if (j >= nlath) continue;
-                const C2<T> e = s[i][c], o = a[i][c];
-                const C2<T> vn{e.x + o.x, e.y + o.y};
-                const C2<T> vs = g == 0 ? C2<T>{e.x - o.x, e.y - o.y} : C2<T>{o.x - e.x, o.y - e.y};
-                put(A.oa, f, j, vn);
-                put(A.oa, f, nlat - 1 - j, vs);
+                const double *e = acc[0][i][c], *o = acc[1][i][c];
+                const double nx = e[0] + o[0], ny = e[1] + o[1];
+                const double sx = g == 0 ? e[0] - o[0] : o[0] - e[0], sy = g == 0 ? e[1] - o[1] : o[1] - e[1];
+                put(A.oa, f, j, nx, ny);
+                put(A.oa, f, nlat - 1 - j, sx, sy);
                 if (gpmt) {   // gpmt = i*m*gp (plasim.f90:2425-2430), the field before gp
-                    const T mm = (T)m;
-                    put(A.oa, f - 1, j, C2<T>{-vn.y * mm, vn.x * mm});
-                    put(A.oa, f - 1, nlat - 1 - j, C2<T>{-vs.y * mm, vs.x * mm});
+                    const double mm = (double)m;
+                    put(A.oa, f - 1, j, -ny * mm, nx * mm);
+                    put(A.oa, f - 1, nlat - 1 - j, -sy * mm, sx * mm);
                 }
             }
         }
-    } else {
-        // u = sum qv*Z - i*qu*D ; v = sum -i*qu*Z - qv*D  (legmod.f90:338-341)
-        const T *tu = A.tab + INV_QU * tsz + (size_t)w0 * nlath, *tv = A.tab + INV_QV * tsz + (size_t)w0 * nlath;
-        const C2<T> *zr = xz + ty * cpt;
-        C2<T> us[JT][LT], ua[JT][LT], vs[JT][LT], va[JT][LT];   // symmetric and antisymmetric sums of u and v
-        T p0[U][JT], q0[U][JT], p1[U][JT], q1[U][JT];
-#pragma unroll
-        for (int i = 0; i < JT; i++)
-#pragma unroll
-            for (int c = 0; c < LT; c++) us[i][c] = ua[i][c] = vs[i][c] = va[i][c] = C2<T>{0, 0};
-        auto fetch = [&](T (&p)[U][JT], T (&q)[U][JT], int k) {
-#pragma unroll
-            for (int e = 0; e < U; e++)
-#pragma unroll
-                for (int i = 0; i < JT; i++) {
-                    const size_t o = (size_t)(k + e) * nlath + jc[i];
-                    p[e][i] = k + e < K ? tu[o] : (T)0;
-                    q[e][i] = k + e < K ? tv[o] : (T)0;
-                }
-        };
-        auto step = [&](const T (&p)[U][JT], const T (&q)[U][JT], int k) {
-#pragma unroll
-            for (int e = 0; e < U; e++)
-#pragma unroll
-                for (int c = 0; c < LT; c++) {
-                    const C2<T> D = xr[(size_t)(k + e) * cs + c], Z = zr[(size_t)(k + e) * cs + c];
-#pragma unroll
-                    for (int i = 0; i < JT; i++) {
-                        // qu terms (P-type) and qv terms (Q-type) fall on opposite parities
-                        C2<T> &uP = (e & 1) ? ua[i][c] : us[i][c], &uQ = (e & 1) ? us[i][c] : ua[i][c];
-                        C2<T> &vP = (e & 1) ? va[i][c] : vs[i][c], &vQ = (e & 1) ? vs[i][c] : va[i][c];
-                        uP.x = mad(p[e][i], D.y, uP.x);
-                        uP.y = mad(-p[e][i], D.x, uP.y);
-                        uQ.x = mad(q[e][i], Z.x, uQ.x);
-                        uQ.y = mad(q[e][i], Z.y, uQ.y);
-                        vP.x = mad(p[e][i], Z.y, vP.x);
-                        vP.y = mad(-p[e][i], Z.x, vP.y);
-                        vQ.x = mad(-q[e][i], D.x, vQ.x);
-                        vQ.y = mad(-q[e][i], D.y, vQ.y);
-                    }
-                }
-        };
-        fetch(p0, q0, 0);
-        for (int k = 0; k < Kp; k += 2 * U) {
-            fetch(p1, q1, k + U);
-            step(p0, q0, k);
-            if (k + U >= Kp) break;
-            fetch(p0, q0, k + 2 * U);
-            step(p1, q1, k + U);
+    } else if (cw + q < n) {
+        const int u = u0 + cw + q;
+        long long fu = u, fv = u;
+        T *ov = A.ob;
+        if constexpr (SET) {
+            const int inst = u / A.L;
+            fu = (long long)inst * (A.dset ? 4 * A.L + 1 : 6 * A.L + 3) + (u - inst * A.L);
+            fv = fu + A.L;
+            ov = A.oa;
         }
 #pragma unroll
-        for (int c = 0; c < LT; c++) {
-            const int u = u0 + ty * LT + c;
-            if (ty * LT + c >= n) continue;
-            long long fu = u, fv = u;
-            T *ov = A.ob;
-            if constexpr (SET) {
-                const int inst = u / A.L;
-                fu = (long long)inst * (A.dset ? 4 * A.L + 1 : 6 * A.L + 3) + (u - inst * A.L);
-                fv = fu + A.L;
-                ov = A.oa;
-            }
+        for (int i = 0; i < MT; i++) {
+            const int j = j0 + 8 * i + r;
+            if (j >= nlath) continue;
 #pragma unroll
-            for (int i = 0; i < JT; i++) {
-                const int j = tx + i * A.tx;
-                if (j >= nlath) continue;
-                put(A.oa, fu, j, C2<T>{us[i][c].x + ua[i][c].x, us[i][c].y + ua[i][c].y});
-                put(A.oa, fu, nlat - 1 - j, C2<T>{us[i][c].x - ua[i][c].x, us[i][c].y - ua[i][c].y});
-                put(ov, fv, j, C2<T>{vs[i][c].x + va[i][c].x, vs[i][c].y + va[i][c].y});
-                put(ov, fv, nlat - 1 - j, C2<T>{vs[i][c].x - va[i][c].x, vs[i][c].y - va[i][c].y});
+            for (int x = 0; x < 2; x++) {
+                const double *s = acc[0][i][x], *a = acc[1][i][x];
+                put(x ? ov : A.oa, x ? fv : fu, j, s[0] + a[0], s[1] + a[1]);
+                put(x ? ov : A.oa, x ? fv : fu, nlat - 1 - j, s[0] - a[0], s[1] - a[1]);
             }
         }
     }
@@ -297,19 +313,25 @@ __global__ void __launch_bounds__(256) k_leg_inv(const __grid_constant__ LegInv<
 // gridpointd's fc2sp of the temperature and humidity tendencies and uv2dv
 enum { OP_LEVEL_A = 4, OP_LEVEL_D = 5 };
 
+constexpr int FWD_THREADS = 192;   // least threads of a block; chunks hold at most 3 x 192 staged values
+constexpr int FWD_ITEMS = 3;
+
 template <typename T>
 struct LegFwd {
-    const T *tab;        // 4 forward tables, per-m blocks [t][woff*nlath + j*K + k]
+    const double *tab;       // 4 forward tables of tsz entries, blocks (m, parity) [j][mode of the parity, padded to 8]
+    const long long *foff;   // block offsets [m*2 + p]
+    size_t tsz;
     const int *woff;
-    const T *filt;       // skgpsp(n)
-    const T *in[6];      // single op: Fourier inputs; set: in[0] is the intermediate
+    const double *filt;      // skgpsp(n)
+    const T *in[6];          // single op: Fourier inputs; set: in[0] is the intermediate
     long long fs, ls, ms, nrows;
-    T *out[3];           // single op: spectral outputs; set: out[0] is the set's output
-    long long o_fs;      // spectral field stride (reals)
-    int nu, nt;          // units (levels x states) and unit tiles per wavenumber
-    int nu1, nt1;        // gridpointa: ln ps tendencies (fc2sp) and their tiles
-    int lb, jc;          // units per block, latitude pairs per staged chunk
-    int L, nlat, nlath, ntp1, ncsp;
+    T *out[3];               // single op: spectral outputs; set: out[0] is the set's output
+    long long o_fs;          // spectral field stride (reals)
+    int nu, nt;              // units (levels x states) and unit tiles per wavenumber
+    int nu1, nt1;            // gridpointa: ln ps tendencies (fc2sp) and their tiles
+    int ng, jc;              // groups of 4 units per block, latitude pairs per staged chunk
+    int wb, nmb;             // warps along the modes of a block; mode blocks per wavenumber
+    int L, nlat, nlath, ntp1;
 };
 
 template <int OP> struct FwdShape;
@@ -320,102 +342,92 @@ template <> struct FwdShape<OP_MKTEND> { static constexpr int nin = 6, nout = 3;
 template <> struct FwdShape<OP_LEVEL_A> { static constexpr int nin = 9, nout = 4; static constexpr bool c = 1, e = 1, m = 1, q = 1; };
 template <> struct FwdShape<OP_LEVEL_D> { static constexpr int nin = 4, nout = 4; static constexpr bool c = 1, e = 1, m = 1, q = 0; };
 
-// o += t * x, o += i * t * x, o -= i * t * x
-template <typename T> __device__ __forceinline__ void acc(C2<T> &o, T t, C2<T> x) { o.x = mad(t, x.x, o.x); o.y = mad(t, x.y, o.y); }
-template <typename T> __device__ __forceinline__ void acc_i(C2<T> &o, T t, C2<T> x) { o.x = mad(-t, x.y, o.x); o.y = mad(t, x.x, o.y); }
-template <typename T> __device__ __forceinline__ void acc_mi(C2<T> &o, T t, C2<T> x) { o.x = mad(t, x.y, o.x); o.y = mad(-t, x.x, o.y); }
+template <int MT> struct FwdFrag { double c[MT], e[MT], m[MT], q[MT]; };
 
-// One latitude pair's terms of one mode; P(i), Q(i) are input i's folded value
-// of the parity that P- and Q-type tables pair with.  In FP32 a latitude
-// pair's terms are summed before they join the running sum: one rounding of the
-// long sum per latitude pair instead of three (relative error against FP64 at
-// T85 2.2e-7 instead of 3.2e-7); in FP64 the tables' own rounding dominates.
-template <typename T, int OP, typename FP, typename FQ>
-__device__ __forceinline__ void fwd_terms(C2<T> *sum, T c, T e, T mm, T qq, FP P, FQ Q) {
-    constexpr int NOUT = FwdShape<OP>::nout;
-    constexpr bool GROUP = sizeof(T) == 4;
-    C2<T> part[NOUT];
-    C2<T> *o = GROUP ? part : sum;
-    if constexpr (GROUP) {
+// Four latitude pairs' terms.  V(i, type, rot) is input i's fragment of the
+// parity that P-type (0) or Q-type (1) tables pair with, or (rot) i times it
+template <int OP, int MT, typename Val>
+__device__ __forceinline__ void fwd_terms(double (*o)[FwdShape<OP>::nout][2], const FwdFrag<MT> &t, Val V) {
+    auto add = [&](int x, const double (&a)[MT], double b) {
 #pragma unroll
-        for (int x = 0; x < NOUT; x++) part[x] = C2<T>{0, 0};
-    }
+        for (int i = 0; i < MT; i++) dmma(o[i][x], a[i], b);
+    };
     if constexpr (OP == OP_FC2SP) {          // sp = sum qc*f  (legmod.f90:203-220)
-        acc(o[0], c, P(0));
+        add(0, t.c, V(0, 0, 0));
     } else if constexpr (OP == OP_UV2DV) {   // d = -qe*v + i*qm*u, z = qe*u + i*qm*v  (:391-424)
-        acc(o[0], -e, Q(1)); acc_i(o[0], mm, P(0));
-        acc(o[1], e, Q(0));  acc_i(o[1], mm, P(1));
+        add(0, t.e, -V(1, 1, 0)); add(0, t.m, V(0, 0, 1));
+        add(1, t.e, V(0, 1, 0));  add(1, t.m, V(1, 0, 1));
     } else if constexpr (OP == OP_QTEND) {   // q = qe*vq + qc*qn - i*qm*uq; in qn, uq, vq  (:466-497)
-        acc(o[0], e, Q(2)); acc(o[0], c, P(0)); acc_mi(o[0], mm, P(1));
+        add(0, t.e, V(2, 1, 0)); add(0, t.c, V(0, 0, 0)); add(0, t.m, -V(1, 0, 1));
     } else if constexpr (OP == OP_MKTEND || OP == OP_LEVEL_A) {
         // mktend (:555-602): d = qq*ke - qe*fv + i*qm*fu, t = qe*vt + qc*tn - i*qm*ut, z = qe*fu + i*qm*fv.
         // Inputs: mktend tn, fu, fv, ke, ut, vt; the level's tn, qn, ut, vt, fv (guz), fu (gvz), ke, uq, vq
         constexpr bool A = OP == OP_LEVEL_A;
         constexpr int TN = 0, FU = A ? 5 : 1, FV = A ? 4 : 2, KE = A ? 6 : 3, UT = A ? 2 : 4, VT = A ? 3 : 5;
-        acc(o[0], qq, P(KE)); acc(o[0], -e, Q(FV)); acc_i(o[0], mm, P(FU));
-        acc(o[1], e, Q(VT)); acc(o[1], c, P(TN)); acc_mi(o[1], mm, P(UT));
-        acc(o[2], e, Q(FU)); acc_i(o[2], mm, P(FV));
-        if constexpr (A) { acc(o[3], e, Q(8)); acc(o[3], c, P(1)); acc_mi(o[3], mm, P(7)); }   // qtend
+        add(0, t.q, V(KE, 0, 0)); add(1, t.e, V(VT, 1, 0)); add(2, t.e, V(FU, 1, 0));
+        if constexpr (A) add(3, t.e, V(8, 1, 0));                                        // qtend
+        add(0, t.e, -V(FV, 1, 0)); add(1, t.c, V(TN, 0, 0)); add(2, t.m, V(FV, 0, 1));
+        if constexpr (A) add(3, t.c, V(1, 0, 0));
+        add(0, t.m, V(FU, 0, 1)); add(1, t.m, -V(UT, 0, 1));
+        if constexpr (A) add(3, t.m, -V(7, 0, 1));
     } else {                                 // gridpointd: in t, u, v, q
-        acc(o[0], -e, Q(2)); acc_i(o[0], mm, P(1));
-        acc(o[1], c, P(0));
-        acc(o[2], e, Q(1)); acc_i(o[2], mm, P(2));
-        acc(o[3], c, P(3));
-    }
-    if constexpr (GROUP) {
-#pragma unroll
-        for (int x = 0; x < NOUT; x++) { sum[x].x += part[x].x; sum[x].y += part[x].y; }
+        add(0, t.e, -V(2, 1, 0)); add(2, t.e, V(1, 1, 0));
+        add(1, t.c, V(0, 0, 0)); add(3, t.c, V(3, 0, 0));
+        add(0, t.m, V(1, 0, 1)); add(2, t.m, V(2, 0, 1));
     }
 }
 
-// Tile: KT modes of one parity x every output of one unit per thread; the
-// lanes of a warp take consecutive modes of both parities.  The units' folded
-// values (N+S, N-S) are staged jc latitude pairs at a time and read as
-// broadcasts, eleven complex values for the 22 products of a gridpointa level,
-// so with KT = 4 the kernel is near the FP64 / FP32 pipe's rate; small sets
-// take KT = 1 for more threads (see fwd_tile).
-template <typename T, int OP, int KT, bool SET>
-__device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, C2<T> *sm, int m, int u0, int n, int lb) {
+// A warp: MT tiles of 8 modes of one parity x one group of 4 units, every
+// output.  The units' folded values (N+S, N-S) are staged jc latitude pairs at
+// a time into one of two buffers while the other is read.
+template <typename T, int OP, int MT, bool SET>
+__device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, double *sm, int m, int mblk, int u0, int n) {
     using S = FwdShape<OP>;
     constexpr int NIN = S::nin, NOUT = S::nout;
-    const int nlath = A.nlath, nlat = A.nlat, L = A.L;
-    const int K = A.ntp1 - m, w0 = A.woff[m];
-    const int K0 = (K + 1) >> 1, K1 = K >> 1, q0 = (K0 + KT - 1) / KT, q1 = (K1 + KT - 1) / KT, qn = q0 + q1;
-    const int us = 2 * A.jc + 1;          // a unit's staged values of one input: {sum, difference} per latitude pair
-    // this thread's unit and modes
-    const int l = threadIdx.x / qn, r = threadIdx.x - l * qn;
-    const bool odd = r >= q0, active = l < n;
-    const int kq = odd ? r - q0 : r, kst = odd ? q1 : q0, kcnt = odd ? K1 : K0;
-    int k[KT];
+    const int nlath = A.nlath, nlat = A.nlat, L = A.L, jcn = A.jc, lbu = 4 * A.ng;
+    const int K = A.ntp1 - m, K0 = (K + 1) >> 1, K1 = K >> 1;
+    const int n0 = (K0 + 8 * MT - 1) / (8 * MT), n1 = (K1 + 8 * MT - 1) / (8 * MT);   // warps per parity
+    if (mblk * A.wb >= n0 + n1) return;   // block-uniform
+    const int rs = leg_stride(8 * A.ng), bufsz = NIN * 2 * jcn * rs;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
+    const int g = warp / A.wb, wl = mblk * A.wb + warp - g * A.wb;
+    const bool active = g < A.ng && wl < n0 + n1 && 4 * g < n;
+    const int p = wl >= n0 ? 1 : 0, kq = p ? K1 : K0, k8 = (kq + 7) & ~7;
+    const int kk0 = (p ? wl - n0 : wl) * 8 * MT;
+    double o[MT][NOUT][2];
 #pragma unroll
-    for (int i = 0; i < KT; i++) k[i] = 2 * min(kq + i * kst, kcnt - 1) + odd;
-    const size_t tsz = (size_t)A.ncsp * nlath;
-    const T *tb = A.tab + (size_t)w0 * nlath;
-    C2<T> o[KT][NOUT];
+    for (int i = 0; i < MT; i++)
 #pragma unroll
-    for (int i = 0; i < KT; i++)
+        for (int x = 0; x < NOUT; x++) o[i][x][0] = o[i][x][1] = 0.0;
+    // this warp's table fragments: rows kk0 + 8i + r, latitude pairs j + q
+    const double *tb = nullptr;
+    int ko[MT];
+    if (active) {
+        tb = A.tab + A.foff[2 * m + p] + (size_t)q * k8;
 #pragma unroll
-        for (int x = 0; x < NOUT; x++) o[i][x] = C2<T>{0, 0};
-    const C2<T> *sp = sm + (size_t)l * us + (odd ? 1 : 0), *sq = sm + (size_t)l * us + (odd ? 0 : 1);
-    struct Tab { T c, e, m, q; };
-    auto fetch = [&](Tab (&t)[KT], int j) {
-        const size_t jo = (size_t)j * K;
+        for (int i = 0; i < MT; i++) ko[i] = min(kk0 + 8 * i, k8 - 8) + r;
+    }
+    auto fetch = [&](FwdFrag<MT> &t, int j) {
+        const double *tj = tb + (size_t)j * k8;
 #pragma unroll
-        for (int i = 0; i < KT; i++) {
-            if constexpr (S::c) t[i].c = tb[FWD_QC * tsz + jo + k[i]];
-            if constexpr (S::e) t[i].e = tb[FWD_QE * tsz + jo + k[i]];
-            if constexpr (S::m) t[i].m = tb[FWD_QM * tsz + jo + k[i]];
-            if constexpr (S::q) t[i].q = tb[FWD_QQ * tsz + jo + k[i]];
+        for (int i = 0; i < MT; i++) {
+            if constexpr (S::c) t.c[i] = tj[FWD_QC * A.tsz + ko[i]];
+            if constexpr (S::e) t.e[i] = tj[FWD_QE * A.tsz + ko[i]];
+            if constexpr (S::m) t.m[i] = tj[FWD_QM * A.tsz + ko[i]];
+            if constexpr (S::q) t.q[i] = tj[FWD_QQ * A.tsz + ko[i]];
         }
     };
-    Tab ta[KT], tn[KT];
-    if (active) fetch(ta, 0);
-    for (int j0 = 0; j0 < nlath; j0 += A.jc) {
-        const int nj = min(A.jc, nlath - j0);
-        if (j0) __syncthreads();
-        for (int idx = threadIdx.x; idx < NIN * n * nj; idx += blockDim.x) {
-            const int jj = idx % nj, rr = idx / nj, ul = rr % n, i = rr / n, u = u0 + ul, j = j0 + jj;
-            C2<T> vn, vs;
+    // staged values: item (input i, unit, latitude pair), latitude pairs fastest
+    Z2 vn[FWD_ITEMS], vs[FWD_ITEMS];
+    const int nitem = NIN * lbu * jcn;
+    auto load = [&](int j0) {
+#pragma unroll
+        for (int e = 0; e < FWD_ITEMS; e++) {
+            const int idx = threadIdx.x + e * blockDim.x;
+            vn[e] = vs[e] = Z2{0, 0};
+            if (idx >= nitem) continue;
+            const int jj = idx % jcn, rr = idx / jcn, ul = rr % lbu, i = rr / lbu, u = u0 + ul, j = j0 + jj;
+            if (ul >= n || j >= nlath) continue;
             if constexpr (SET) {
                 long long f;
                 if constexpr (OP == OP_FC2SP) f = (long long)u * (9 * L + 1) + 7 * L;   // gvpp of state u
@@ -425,36 +437,59 @@ __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, C2<T> *sm, int
                     f = (long long)inst * (OP == OP_LEVEL_A ? 9 * L + 1 : 4 * L) + i * L + lev + (OP == OP_LEVEL_A && i >= 7);
                 }
                 const C2<T> *w = reinterpret_cast<const C2<T> *>(A.in[0]) + (size_t)m * A.nrows + f * nlat;
-                vn = w[j];
-                vs = w[nlat - 1 - j];
+                const C2<T> a = w[j], b = w[nlat - 1 - j];
+                vn[e] = Z2{(double)a.x, (double)a.y};
+                vs[e] = Z2{(double)b.x, (double)b.y};
             } else {
                 const T *w = A.in[i] + 2 * (u * A.fs + (long long)m * A.ms);
-                vn = ld2(w + 2 * (j * A.ls));
-                vs = ld2(w + 2 * ((nlat - 1 - j) * A.ls));
+                vn[e] = ld2(w + 2 * (j * A.ls));
+                vs[e] = ld2(w + 2 * ((nlat - 1 - j) * A.ls));
             }
-            C2<T> *d = sm + ((size_t)i * lb + ul) * us + 2 * jj;
-            d[0] = C2<T>{vn.x + vs.x, vn.y + vs.y};
-            d[1] = C2<T>{vn.x - vs.x, vn.y - vs.y};
         }
+    };
+    auto store = [&](double *buf) {
+#pragma unroll
+        for (int e = 0; e < FWD_ITEMS; e++) {
+            const int idx = threadIdx.x + e * blockDim.x;
+            if (idx >= nitem) continue;
+            const int jj = idx % jcn, rr = idx / jcn, ul = rr % lbu, i = rr / lbu;
+            double *d = buf + (size_t)(2 * i * jcn + jj) * rs + 2 * ul;
+            *reinterpret_cast<Z2 *>(d) = Z2{vn[e].x + vs[e].x, vn[e].y + vs[e].y};
+            *reinterpret_cast<Z2 *>(d + (size_t)jcn * rs) = Z2{vn[e].x - vs[e].x, vn[e].y - vs[e].y};
+        }
+    };
+    FwdFrag<MT> ta, tn;
+    if (active) fetch(ta, 0);
+    load(0);
+    store(sm);
+    __syncthreads();
+    const int nl4 = (nlath + 3) & ~3, nch = (nlath + jcn - 1) / jcn;
+    for (int c = 0; c < nch; c++) {
+        const int j0 = c * jcn;
+        if (c + 1 < nch) load(j0 + jcn);
+        if (active) {
+            const double *xb = sm + (size_t)(c & 1) * bufsz + q * rs + 8 * g;
+            const int je = min(jcn, nl4 - j0);
+            for (int jj = 0; jj < je; jj += 4) {
+                if (j0 + jj + 4 < nl4) fetch(tn, j0 + jj + 4);
+                fwd_terms<OP, MT>(o, ta, [&](int i, int type, int rot) {
+                    // P-type tables see the sum on even n-m and the difference on odd, Q-type the reverse
+                    const double v = xb[(size_t)((2 * i + (type ^ p)) * jcn + jj) * rs + (r ^ rot)];
+                    return rot && !(r & 1) ? -v : v;   // i*x: re <- -im, im <- re
+                });
+                ta = tn;
+            }
+        }
+        if (c + 1 < nch) store(sm + (size_t)((c + 1) & 1) * bufsz);
         __syncthreads();
-        if (!active) continue;
-        const size_t is = (size_t)lb * us;
-        for (int jj = 0; jj < nj; jj++) {
-            fetch(tn, min(j0 + jj + 1, nlath - 1));
-#pragma unroll
-            for (int i = 0; i < KT; i++)
-                fwd_terms<T, OP>(o[i], ta[i].c, ta[i].e, ta[i].m, ta[i].q,
-                                 [&](int f) { return sp[f * is + 2 * jj]; }, [&](int f) { return sq[f * is + 2 * jj]; });
-#pragma unroll
-            for (int i = 0; i < KT; i++) ta[i] = tn[i];
-        }
     }
-    if (!active) return;
-    const int u = u0 + l;
+    if (!active || 4 * g + q >= n) return;
+    const int u = u0 + 4 * g + q, w0 = A.woff[m];
 #pragma unroll
-    for (int i = 0; i < KT; i++) {
-        if (kq + i * kst >= kcnt) continue;
-        const T f = A.filt[m + k[i]];
+    for (int i = 0; i < MT; i++) {
+        const int kk = kk0 + 8 * i + r, k = 2 * kk + p;
+        if (kk >= kq) continue;
+        const double f = A.filt[m + k];
 #pragma unroll
         for (int x = 0; x < NOUT; x++) {
             T *d;
@@ -466,96 +501,70 @@ __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, C2<T> *sm, int
                     d = A.out[0] + ((size_t)inst * (OP == OP_LEVEL_A ? 4 * L + 1 : 4 * L) + x * L + lev) * A.o_fs;
                 }
             } else d = A.out[x] + (size_t)u * A.o_fs;
-            d[2 * (w0 + k[i])] = o[i][x].x * f;
-            d[2 * (w0 + k[i]) + 1] = o[i][x].y * f;
+            d[2 * (w0 + k)] = (T)(o[i][x][0] * f);
+            d[2 * (w0 + k) + 1] = (T)(o[i][x][1] * f);
         }
     }
 }
 
-template <typename T, int OP, int KT, bool SET>
-__global__ void __launch_bounds__(KT == 4 ? 384 : 512) k_leg_fwd(const __grid_constant__ LegFwd<T> A) {
+template <typename T, int OP, int MT, bool SET>
+__global__ void __launch_bounds__(512) k_leg_fwd(const __grid_constant__ LegFwd<T> A) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    C2<T> *sm = reinterpret_cast<C2<T> *>(smraw);
-    const int nt = A.nt + A.nt1, m = blockIdx.x / nt, ti = blockIdx.x - m * nt;
+    double *sm = reinterpret_cast<double *>(smraw);
+    const int nt = A.nt + A.nt1, mb = blockIdx.x / nt, ti = blockIdx.x - mb * nt;
+    const int m = mb / A.nmb, mblk = mb - m * A.nmb, lbu = 4 * A.ng;
     pdl_trigger();
     pdl_wait();
     if (ti < A.nt) {
-        const int u0 = ti * A.lb;
-        leg_fwd_block<T, OP, KT, SET>(A, sm, m, u0, min(A.lb, A.nu - u0), A.lb);
+        const int u0 = ti * lbu;
+        leg_fwd_block<T, OP, MT, SET>(A, sm, m, mblk, u0, min(lbu, A.nu - u0));
     } else if constexpr (OP == OP_LEVEL_A) {
-        const int u0 = (ti - A.nt) * A.lb;
-        leg_fwd_block<T, OP_FC2SP, KT, SET>(A, sm, m, u0, min(A.lb, A.nu1 - u0), A.lb);
+        const int u0 = (ti - A.nt) * lbu;
+        leg_fwd_block<T, OP_FC2SP, MT, SET>(A, sm, m, mblk, u0, min(lbu, A.nu1 - u0));
     }
 }
 
-template <typename T> static const T *inv_tab(exotx_plan p);
-template <> const double *inv_tab<double>(exotx_plan p) { return p->d_inv64; }
-template <> const float *inv_tab<float>(exotx_plan p) { return p->d_inv32; }
-template <typename T> static const T *fwd_tab(exotx_plan p);
-template <> const double *fwd_tab<double>(exotx_plan p) { return p->d_fwd64; }
-template <> const float *fwd_tab<float>(exotx_plan p) { return p->d_fwd32; }
-template <typename T> static const T *filt_s(exotx_plan p);
-template <> const double *filt_s<double>(exotx_plan p) { return p->d_fs64; }
-template <> const float *filt_s<float>(exotx_plan p) { return p->d_fs32; }
-template <typename T> static const T *filt_g(exotx_plan p);
-template <> const double *filt_g<double>(exotx_plan p) { return p->d_fg64; }
-template <> const float *filt_g<float>(exotx_plan p) { return p->d_fg32; }
-
 // ------------------------------------------------------------ host launchers
-// the inverse tile (0: 1 x 1, 1: 2 x 2, 2: 4 x 4 outputs per thread): the
-// largest that still leaves LEG_THREADS threads.  cols: complex columns, a
-// (D, Z) pair counting as two
-constexpr long long LEG_THREADS = 40000;   // about 270 per SM
-static int inv_tile(exotx_plan p, long long cols) {
-    const long long outs = (long long)p->ntp1 * p->nlath * cols;
-    return outs / 16 >= LEG_THREADS || p->nlath > 512 ? 2 : outs / 4 >= LEG_THREADS || p->nlath > 256 ? 1 : 0;
-}
-// modes per thread of the forward kernels, by the same rule
-static int fwd_tile(exotx_plan p, long long units) {
-    const long long outs = units * p->ncsp;
-    return outs / 4 >= LEG_THREADS || p->ntp1 > 512 ? 4 : outs / 2 >= LEG_THREADS ? 2 : 1;
-}
+// Both directions take the larger warp tile where that still leaves LEG_WARPS
+// warps (about 8 per SM), and the smaller one otherwise.
+constexpr long long LEG_WARPS = 1200;
 
-template <typename T, int JT, int CC, bool SET>
+template <typename T, int MT, int NT, bool SET>
 static exotx_status inv_launch_t(exotx_plan p, LegInv<T> &A, cudaStream_t s) {
-    constexpr int LT = CC > 1 ? CC / 2 : 1;
-    A.tx = (p->nlath + JT - 1) / JT;
-    const int want = JT == 4 ? 192 : 128;
-    A.ty = std::max(1, want / A.tx);
-    // the staged columns of a block (modes x columns, twice for (D, Z) pairs) within the budget
-    auto smem_of = [&](int ty) {
-        const size_t Kp = (p->ntp1 + 3) & ~3;
-        const size_t one = Kp * (ty * CC + 1), two = A.nu[2] ? 2 * Kp * (ty * LT + 1) : 0;
-        return std::max(one, two) * 2 * sizeof(T);
+    const int lt = (p->nlath + 8 * MT - 1) / (8 * MT);   // latitude warps
+    A.wm = std::min(lt, 4);
+    A.nlb = (lt + A.wm - 1) / A.wm;
+    A.wn = std::max(1, 6 / A.wm);
+    // the staged columns of a block: all modes at once where they fit the budget
+    auto smem_of = [&](int kc, int wn) {
+        const size_t one = (size_t)kc * leg_stride(8 * NT * wn), two = A.nu[2] ? 2 * (size_t)kc * leg_stride(8 * wn) : 0;
+        return std::max(one, two) * sizeof(double);
     };
-    while (A.ty > 1 && smem_of(A.ty) > 72 * 1024) A.ty--;
-    const size_t smem = smem_of(A.ty);
-    if (smem > LEG_MAXSMEM) return EXOTX_BAD_DIM;
-    const int cb[3] = {A.ty * CC, A.ty * CC, A.ty * LT};
+    A.kc = (p->ntp1 + 7) & ~7;
+    while (A.wn > 1 && smem_of(A.kc, A.wn) > 72 * 1024) A.wn--;
+    if (smem_of(A.kc, A.wn) > 96 * 1024) A.kc = 256;
+    const size_t smem = smem_of(A.kc, A.wn);
+    const int cb[3] = {4 * NT * A.wn, 4 * NT * A.wn, 4 * A.wn};
     A.ntiles = 0;
     for (int g = 0; g < 3; g++) A.ntiles += A.nt[g] = (A.nu[g] + cb[g] - 1) / cb[g];
     const int nm = p->ntp1 + (!SET && A.mz > p->ntp1 ? 1 : 0);
-    const long long blocks = (long long)nm * A.ntiles;
-    if (blocks > 0x7fffffffLL) return EXOTX_BAD_DIM;
-    const int threads = (A.tx * A.ty + 31) / 32 * 32;
-    auto kern = k_leg_inv<T, JT, CC, SET>;
+    const long long blocks = (long long)nm * A.nlb * A.ntiles;
+    if (blocks > 0x7fffffffLL || smem > LEG_MAXSMEM) return EXOTX_BAD_DIM;
+    auto kern = k_leg_inv<T, MT, NT, SET>;
     if (smem > 48 * 1024) EXOTX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LEG_MAXSMEM));
     cudaEvent_t ev = ktimer_start(EXOTX_K_LEG_INVERSE, s);
-    EXOTX_CUDA(launch_pdl(kern, dim3((unsigned)blocks), dim3(threads), smem, s, A));
+    EXOTX_CUDA(launch_pdl(kern, dim3((unsigned)blocks), dim3(32 * A.wm * A.wn), smem, s, A));
     EXOTX_CHECK_LAUNCH();
     ktimer_stop(EXOTX_K_LEG_INVERSE, s, ev);
     return EXOTX_OK;
 }
 template <typename T, bool SET>
 static exotx_status inv_launch(exotx_plan p, LegInv<T> &A, cudaStream_t s) {
-    A.tab = inv_tab<T>(p); A.woff = p->d_woff; A.filt = filt_s<T>(p);
+    A.tab = p->d_inv64; A.woff = p->d_woff; A.filt = p->d_fs64;
     A.nlat = p->nlat; A.nlath = p->nlath; A.ntp1 = p->ntp1; A.ncsp = p->ncsp; A.nrsp = 2 * p->ncsp;
-    A.plavor = (T)p->desc.plavor;
-    switch (inv_tile(p, (long long)A.nu[0] + A.nu[1] + 2LL * A.nu[2])) {
-        case 0: return inv_launch_t<T, 1, 1, SET>(p, A, s);
-        case 1: return inv_launch_t<T, 2, 2, SET>(p, A, s);
-        default: return inv_launch_t<T, 4, 4, SET>(p, A, s);
-    }
+    A.plavor = p->desc.plavor;
+    const long long tiles = (long long)p->ntp1 * ((p->nlath + 7) / 8) * ((A.nu[0] + A.nu[1]) / 4 + A.nu[2] / 2 + 1);
+    return tiles / 8 >= LEG_WARPS ? inv_launch_t<T, 4, 2, SET>(p, A, s) : inv_launch_t<T, 2, 1, SET>(p, A, s);
 }
 
 template <typename T>
@@ -583,22 +592,23 @@ exotx_status leg_inverse_set(exotx_plan p, int dset, const T *spin, T *W, int L,
     return inv_launch<T, true>(p, A, s);
 }
 
-template <typename T, int OP, int KT, bool SET>
+template <typename T, int OP, int MT, bool SET>
 static exotx_status fwd_launch_t(exotx_plan p, LegFwd<T> &A, cudaStream_t s) {
     const int K0 = (p->ntp1 + 1) / 2, K1 = p->ntp1 / 2;
-    const int qn = (K0 + KT - 1) / KT + (K1 + KT - 1) / KT;   // threads per unit at m = 0
-    A.lb = std::min(std::max(1, 160 / qn), std::max(A.nu, 1));
-    A.jc = std::min(p->nlath, 32);
-    auto smem_of = [&] { return (size_t)FwdShape<OP>::nin * A.lb * (2 * A.jc + 1) * 2 * sizeof(T); };
-    while (A.jc > 8 && smem_of() > 48 * 1024) A.jc = (A.jc + 1) / 2;
-    const size_t smem = smem_of();
-    const int threads = (qn * A.lb + 31) / 32 * 32;
-    if (smem > LEG_MAXSMEM || threads > (KT == 4 ? 384 : 512)) return EXOTX_BAD_DIM;
-    A.nt = (A.nu + A.lb - 1) / A.lb;
-    A.nt1 = (A.nu1 + A.lb - 1) / A.lb;
-    const long long blocks = (long long)p->ntp1 * (A.nt + A.nt1);
-    if (blocks > 0x7fffffffLL) return EXOTX_BAD_DIM;
-    auto kern = k_leg_fwd<T, OP, KT, SET>;
+    const int nw = (K0 + 8 * MT - 1) / (8 * MT) + (K1 + 8 * MT - 1) / (8 * MT);   // mode warps at m = 0
+    A.ng = nw <= 8 && A.nu > 4 ? 2 : 1;
+    A.wb = std::min(nw, 16 / A.ng);
+    A.nmb = (nw + A.wb - 1) / A.wb;
+    const int threads = std::max(FWD_THREADS, 32 * A.wb * A.ng);
+    // latitude pairs per chunk: 16, fewer where a chunk's values do not fit FWD_ITEMS per thread
+    A.jc = 16;
+    while (A.jc > 4 && FwdShape<OP>::nin * 4 * A.ng * A.jc > FWD_ITEMS * threads) A.jc /= 2;
+    const size_t smem = (size_t)FwdShape<OP>::nin * 2 * A.jc * leg_stride(8 * A.ng) * 2 * sizeof(double);
+    A.nt = (A.nu + 4 * A.ng - 1) / (4 * A.ng);
+    A.nt1 = (A.nu1 + 4 * A.ng - 1) / (4 * A.ng);
+    const long long blocks = (long long)p->ntp1 * A.nmb * (A.nt + A.nt1);
+    if (blocks > 0x7fffffffLL || smem > LEG_MAXSMEM) return EXOTX_BAD_DIM;
+    auto kern = k_leg_fwd<T, OP, MT, SET>;
     if (smem > 48 * 1024) EXOTX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LEG_MAXSMEM));
     cudaEvent_t ev = ktimer_start(EXOTX_K_LEG_FORWARD, s);
     EXOTX_CUDA(launch_pdl(kern, dim3((unsigned)blocks), dim3(threads), smem, s, A));
@@ -608,13 +618,10 @@ static exotx_status fwd_launch_t(exotx_plan p, LegFwd<T> &A, cudaStream_t s) {
 }
 template <typename T, int OP, bool SET>
 static exotx_status fwd_launch(exotx_plan p, LegFwd<T> &A, cudaStream_t s) {
-    A.tab = fwd_tab<T>(p); A.woff = p->d_woff; A.filt = filt_g<T>(p);
-    A.nlat = p->nlat; A.nlath = p->nlath; A.ntp1 = p->ntp1; A.ncsp = p->ncsp;
-    switch (fwd_tile(p, A.nu)) {
-        case 1: return fwd_launch_t<T, OP, 1, SET>(p, A, s);
-        case 2: return fwd_launch_t<T, OP, 2, SET>(p, A, s);
-        default: return fwd_launch_t<T, OP, 4, SET>(p, A, s);
-    }
+    A.tab = p->d_fwd64; A.foff = p->d_foff; A.tsz = p->fwd_tsz; A.woff = p->d_woff; A.filt = p->d_fg64;
+    A.nlat = p->nlat; A.nlath = p->nlath; A.ntp1 = p->ntp1;
+    const long long tiles = (long long)(p->ncsp / 8 + p->ntp1) * ((A.nu + 3) / 4);
+    return tiles / 2 >= LEG_WARPS ? fwd_launch_t<T, OP, 2, SET>(p, A, s) : fwd_launch_t<T, OP, 1, SET>(p, A, s);
 }
 
 template <typename T>

@@ -137,8 +137,7 @@ __global__ void k_legini(int nlat, int ntru, int ncsp, const int *woff, const do
 }
 
 // inverse layout [t][w][j] for qi,qj,qu,qv (reference tables 0,1,6,7)
-__global__ void k_layout_inv(int nlat, int ncsp, int nlath, const double *qref, double *inv64,
-                             float *inv32) {
+__global__ void k_layout_inv(int nlat, int ncsp, int nlath, const double *qref, double *inv64) {
     size_t tsz = (size_t)ncsp * nlat;
     size_t total = (size_t)4 * ncsp * nlath;
     const int src[4] = {0, 1, 6, 7};
@@ -148,33 +147,23 @@ __global__ void k_layout_inv(int nlat, int ncsp, int nlath, const double *qref, 
         size_t r = i / nlath;
         int w = (int)(r % ncsp);
         int t = (int)(r / ncsp);
-        double v = qref[src[t] * tsz + (size_t)j * ncsp + w];
-        inv64[i] = v;
-        inv32[i] = (float)v;
+        inv64[i] = qref[src[t] * tsz + (size_t)j * ncsp + w];
     }
 }
 
-// forward layout per m block [t][woff(m)*nlath + j*K_m + (n-m)] for qc,qe,qm,qq (2,3,4,5)
-__global__ void k_layout_fwd(int nlat, int ntru, int ncsp, int nlath, const int *woff,
-                             const double *qref, double *fwd64, float *fwd32) {
-    size_t tsz = (size_t)ncsp * nlat;
-    size_t total = (size_t)4 * ncsp * nlath;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
-         i += (size_t)gridDim.x * blockDim.x) {
-        int t = (int)(i / ((size_t)ncsp * nlath));
-        size_t r = i % ((size_t)ncsp * nlath);
-        // find m: woff[m]*nlath <= r < woff[m+1]*nlath (binary search)
-        int lo = 0, hi = ntru;
-        while (lo < hi) {
-            int mid = (lo + hi + 1) / 2;
-            if ((size_t)woff[mid] * nlath <= r) lo = mid; else hi = mid - 1;
-        }
-        int m = lo, K = ntru + 1 - m;
-        size_t rr = r - (size_t)woff[m] * nlath;
-        int j = (int)(rr / K), k = (int)(rr % K);
-        double v = qref[(2 + t) * tsz + (size_t)j * ncsp + woff[m] + k];
-        fwd64[i] = v;
-        fwd32[i] = (float)v;
+// forward layout for qc,qe,qm,qq (2,3,4,5): block (m, parity p of n-m) at
+// foff[2m + p] holds [j][kk] for the modes n-m = 2kk + p, kk padded to 8 and the
+// latitude pairs to 4 with zeros.  One block per (m, p)
+__global__ void k_layout_fwd(int nlat, int ntru, int ncsp, int nlath, const int *woff, const long long *foff,
+                             size_t ftsz, const double *qref, double *fwd64) {
+    const int m = blockIdx.x >> 1, p = blockIdx.x & 1, K = ntru + 1 - m, kq = (K + 1 - p) >> 1, k8 = (kq + 7) & ~7;
+    const int nl4 = (nlath + 3) & ~3;
+    const size_t tsz = (size_t)ncsp * nlat;
+    for (int i = threadIdx.x; i < nl4 * k8; i += blockDim.x) {
+        const int j = i / k8, kk = i - j * k8;
+        for (int t = 0; t < 4; t++)
+            fwd64[t * ftsz + foff[blockIdx.x] + i] =
+                (j < nlath && kk < kq) ? qref[(2 + t) * tsz + (size_t)j * ncsp + woff[m] + 2 * kk + p] : 0.0;
     }
 }
 
@@ -235,9 +224,8 @@ static void plan_free(exotx_plan p) {
     cudaFree(p->d_gwd);
     cudaFree(p->d_qref);
     cudaFree(p->d_inv64);
-    cudaFree(p->d_inv32);
     cudaFree(p->d_fwd64);
-    cudaFree(p->d_fwd32);
+    cudaFree(p->d_foff);
     cudaFree(p->d_fs64);
     cudaFree(p->d_fg64);
     cudaFree(p->d_fs32);
@@ -315,6 +303,13 @@ EXOTX_API exotx_status exotx_plan_create(const exotx_grid_desc *d, exotx_plan *o
     std::vector<float> g32(g.begin(), g.end()), s32(sv.begin(), sv.end());
     size_t tsz = (size_t)ncsp * nlat;
     size_t half = (size_t)4 * ncsp * nlath;
+    // the inverse kernel reads whole steps of 8 modes: up to 7 rows past the last one, times zero
+    const size_t inv_pad = (size_t)8 * nlath;
+    std::vector<long long> foff(2 * ntp1);
+    for (int i = 0; i < 2 * ntp1; i++) {
+        foff[i] = (long long)p->fwd_tsz;
+        p->fwd_tsz += (size_t)((nlath + 3) & ~3) * ((((ntp1 - i / 2 + 1 - i % 2) >> 1) + 7) & ~7);
+    }
     exotx_status st = EXOTX_OK;
 #define PALLOC(ptr, bytes)                                           \
     do {                                                             \
@@ -327,10 +322,9 @@ EXOTX_API exotx_status exotx_plan_create(const exotx_grid_desc *d, exotx_plan *o
     PALLOC(p->d_sid, sizeof(double) * nlat);
     PALLOC(p->d_gwd, sizeof(double) * nlat);
     PALLOC(p->d_qref, sizeof(double) * 8 * tsz);
-    PALLOC(p->d_inv64, sizeof(double) * half);
-    PALLOC(p->d_inv32, sizeof(float) * half);
-    PALLOC(p->d_fwd64, sizeof(double) * half);
-    PALLOC(p->d_fwd32, sizeof(float) * half);
+    PALLOC(p->d_inv64, sizeof(double) * (half + inv_pad));
+    PALLOC(p->d_fwd64, sizeof(double) * 4 * p->fwd_tsz);
+    PALLOC(p->d_foff, sizeof(long long) * 2 * ntp1);
     PALLOC(p->d_fs64, sizeof(double) * ntp1);
     PALLOC(p->d_fg64, sizeof(double) * ntp1);
     PALLOC(p->d_fs32, sizeof(float) * ntp1);
@@ -338,7 +332,9 @@ EXOTX_API exotx_status exotx_plan_create(const exotx_grid_desc *d, exotx_plan *o
 #undef PALLOC
     {
         cudaStream_t s = 0;
-        if (cudaMemcpy(p->d_woff, woff.data(), sizeof(int) * (ntp1 + 1), cudaMemcpyHostToDevice) ||
+        if (cudaMemset(p->d_inv64 + half, 0, sizeof(double) * inv_pad) ||
+            cudaMemcpy(p->d_foff, foff.data(), sizeof(long long) * 2 * ntp1, cudaMemcpyHostToDevice) ||
+            cudaMemcpy(p->d_woff, woff.data(), sizeof(int) * (ntp1 + 1), cudaMemcpyHostToDevice) ||
             cudaMemcpy(p->d_fg64, g.data(), sizeof(double) * ntp1, cudaMemcpyHostToDevice) ||
             cudaMemcpy(p->d_fs64, sv.data(), sizeof(double) * ntp1, cudaMemcpyHostToDevice) ||
             cudaMemcpy(p->d_fg32, g32.data(), sizeof(float) * ntp1, cudaMemcpyHostToDevice) ||
@@ -352,10 +348,10 @@ EXOTX_API exotx_status exotx_plan_create(const exotx_grid_desc *d, exotx_plan *o
                                                               p->d_gwd, p->d_qref);
         note_launch();
         int blocks = (int)std::min<size_t>((half + 255) / 256, 148 * 16);
-        k_layout_inv<<<blocks, 256, 0, s>>>(nlat, ncsp, nlath, p->d_qref, p->d_inv64, p->d_inv32);
+        k_layout_inv<<<blocks, 256, 0, s>>>(nlat, ncsp, nlath, p->d_qref, p->d_inv64);
         note_launch();
-        k_layout_fwd<<<blocks, 256, 0, s>>>(nlat, p->ntru, ncsp, nlath, p->d_woff, p->d_qref, p->d_fwd64,
-                                            p->d_fwd32);
+        k_layout_fwd<<<2 * ntp1, 256, 0, s>>>(nlat, p->ntru, ncsp, nlath, p->d_woff, p->d_foff, p->fwd_tsz, p->d_qref,
+                                              p->d_fwd64);
         note_launch();
         if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) {
             st = EXOTX_CUDA_ERR;
