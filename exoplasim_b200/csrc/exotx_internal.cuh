@@ -91,13 +91,11 @@ struct exotx_plan_s {
     int *d_woff = nullptr;        // first mode index of each m, [ntp1+1]
     double *d_sid = nullptr, *d_gwd = nullptr;
     double *d_qref = nullptr;     // 8 tables, reference layout q(NCSP,NLAT) [t][lat][w]
-    // inverse tables qi,qj,qu,qv for northern latitudes, [t][w][j] (j fastest), then 8 rows of zeros
-    double *d_inv64 = nullptr;
-    // forward tables qc,qe,qm,qq for northern latitudes: fwd_tsz entries each, the block
-    // (m, parity p of n-m) at d_foff[2m + p] holding [j][(n-m-p)/2, padded to 8]
-    double *d_fwd64 = nullptr;
-    long long *d_foff = nullptr;
-    size_t fwd_tsz = 0;
+    // tables for northern latitudes as tensor-core operand fragments (plan.cu):
+    // inverse qi,qj,qu,qv of inv_tsz fragment pairs (16 bytes) each, forward qc,qe,qm,qq
+    double *d_inv64 = nullptr, *d_fwd64 = nullptr;
+    int *d_ioff = nullptr, *d_foff = nullptr;  // first inverse step of m; first forward fragment of (m, parity)
+    size_t inv_tsz = 0;
     double *d_fs64 = nullptr, *d_fg64 = nullptr;  // skspgp, skgpsp [ntp1]
     float *d_fs32 = nullptr, *d_fg32 = nullptr;
     // work buffer for the forward transform set (Fourier rows of gpin)

@@ -53,6 +53,19 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
                  : "+d"(d[0]), "+d"(d[1])
                  : "d"(a), "d"(b));
 }
+// asynchronous copy of one complex value to shared memory (zeros where !ok);
+// WIDE: source aligned to its size, otherwise to its reals only
+template <bool WIDE, typename T>
+__device__ __forceinline__ void cp_complex(C2<T> *dst, const T *src, bool ok) {
+    constexpr int B = sizeof(T);
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if constexpr (WIDE) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(2 * B), "r"(ok ? 2 * B : 0) : "memory");
+    } else {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(B), "r"(ok ? B : 0) : "memory");
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d + B), "l"(src + 1), "n"(B), "r"(ok ? B : 0) : "memory");
+    }
+}
 // row stride (doubles) of staged operands of nc real columns (a multiple of 8):
 // 4 or 12 mod 16, so the four rows of a fragment fall on distinct banks
 __host__ __device__ constexpr int leg_stride(int nc) { return nc + 4; }
@@ -66,7 +79,9 @@ constexpr int LEG_MAXSMEM = 200 * 1024;
 //   2  qu and qv: a unit is a (divergence, vorticity) pair -> (u, v)
 template <typename T>
 struct LegInv {
-    const double *tab;   // 4 inverse tables [t][w][j]
+    const double2 *tab;  // 4 inverse tables of tsz fragment pairs (plan.cu k_layout_inv)
+    const int *ioff;     // first step of each wavenumber
+    size_t tsz;
     const int *woff;
     const double *filt;  // skspgp(n)
     const T *a, *b;      // spectral inputs (re, im pairs); single op: fields a (and b) at stride a_fs (b_fs)
@@ -76,7 +91,7 @@ struct LegInv {
     int nu[3], nt[3];    // units and column tiles of each group
     int ntiles, nlb;     // tiles per wavenumber; latitude blocks
     int wm, wn, kc;      // warps along latitudes and columns; modes staged at a time
-    int L, nlat, nlath, ntp1, ncsp, nrsp, dset, mz;  // single op: wavenumbers ntp1 <= m < mz are zeroed
+    int L, nlat, nlath, ntl, ntp1, nrsp, dset, mz;  // ntl: tiles of 8 latitudes; single op: wavenumbers ntp1 <= m < mz are zeroed
     double plavor;
 };
 
@@ -97,9 +112,11 @@ __device__ __forceinline__ void inv_field(int L, int dset, int u, int *inst, int
 }
 
 // A warp: MT tiles of 8 latitudes x NT groups of 4 complex columns (group 2:
-// x 4 (D, Z) pairs), both parities of n-m in separate accumulators.
+// x 4 (D, Z) pairs), both parities of n-m in separate accumulators.  A step is
+// 8 modes: a tile's fragments of both parities are one 16-byte load per lane.
 template <typename T, int MT, int NT, bool SET>
-__global__ void __launch_bounds__(256) k_leg_inv(const __grid_constant__ LegInv<T> A) {
+__global__ void __launch_bounds__(192, NT == 1 ? 2 : 4) k_leg_inv(const __grid_constant__ LegInv<T> A) {
+    constexpr bool PF = NT == 1;   // fetch a step ahead: few warps to hide the latency
     extern __shared__ __align__(16) unsigned char smraw[];
     double *xs = reinterpret_cast<double *>(smraw);
     int ti = blockIdx.x % A.ntiles, g = 0;
@@ -126,13 +143,13 @@ __global__ void __launch_bounds__(256) k_leg_inv(const __grid_constant__ LegInv<
     const int wn = warp / A.wm, wm = warp - wn * A.wm;
     const int cw = wn * (g == 2 ? 4 : 4 * NT);                       // the warp's first column of the block
     const int j0 = (lb * A.wm + wm) * 8 * MT;
-    const bool active = wn < A.wn && cw < n && j0 < nlath;
-    const size_t tsz = (size_t)A.ncsp * nlath;
-    int jc[MT];
+    const bool active = cw < n && j0 < nlath;
+    // fragment pairs of the warp's tiles, step by step (tiles past the last repeat it)
+    const size_t sstr = (size_t)A.ntl * 32;
+    const double2 *t0 = A.tab + (g == 0 ? INV_QI : g == 1 ? INV_QJ : INV_QU) * A.tsz + A.ioff[m] * sstr + lane;
+    int to[MT];
 #pragma unroll
-    for (int i = 0; i < MT; i++) jc[i] = min(j0 + 8 * i + r, nlath - 1);
-    const double *t0 = A.tab + (g == 0 ? INV_QI : g == 1 ? INV_QJ : INV_QU) * tsz + (size_t)w0 * nlath;
-    const double *t1 = A.tab + INV_QV * tsz + (size_t)w0 * nlath;    // group 2
+    for (int i = 0; i < MT; i++) to[i] = min((j0 >> 3) + i, A.ntl - 1) * 32;
     // accumulators by parity: [p][tile][column group] (group 2: symmetric and
     // antisymmetric sums of u, then of v)
     double acc[2][MT][NT < 2 ? 2 : NT][2];
@@ -145,13 +162,11 @@ __global__ void __launch_bounds__(256) k_leg_inv(const __grid_constant__ LegInv<
     for (int kb = 0; kb < K; kb += A.kc) {
         const int kn = min(A.kc, K - kb), kp = (kn + 7) & ~7, kh = kp >> 1;
         if (kb) __syncthreads();
-        // stage the filtered coefficients, even modes then odd ones, zeros past the last mode and column
-        for (int i = threadIdx.x; i < cb * kp; i += blockDim.x) {
-            const int c = i / kp, k = i - c * kp, mode = kb + k;
-            Z2 va{0, 0}, vb{0, 0};
-            if (c < n && mode < K) {
-                const double f = A.filt[m + mode];
-                const T *pa, *pb = nullptr;
+        // stage the filtered coefficients, even modes then odd ones, zeros past the
+        // last mode and column; a warp takes a column, lanes along its modes
+        for (int c = warp; c < cb; c += blockDim.x >> 5) {
+            const T *pa = nullptr, *pb = nullptr;
+            if (c < n) {
                 if constexpr (SET) {
                     int inst, fin, fout;
                     if (g == 0) inv_field(A.L, A.dset, u0 + c, &inst, &fin, &fout);
@@ -163,84 +178,108 @@ __global__ void __launch_bounds__(256) k_leg_inv(const __grid_constant__ LegInv<
                     pa = A.a + (u0 + c) * A.a_fs;
                     if (g == 2) pb = A.b + (u0 + c) * A.b_fs;
                 }
-                va = ld2(pa + 2 * (w0 + mode));
-                va.x *= f; va.y *= f;
-                if (g == 2) {
-                    // vorticity; plavor leaves mode (0,1) (legmod.f90:332)
-                    vb = ld2(pb + 2 * (w0 + mode));
-                    if (m == 0 && mode == 1) vb.x -= A.plavor;
-                    vb.x *= f; vb.y *= f;
-                }
+                pa += 2 * (w0 + kb);
+                pb += 2 * (w0 + kb);
             }
-            const size_t o = (size_t)((k & 1) * kh + (k >> 1)) * rs + 2 * c;
-            *reinterpret_cast<Z2 *>(xs + o) = va;
-            if (g == 2) *reinterpret_cast<Z2 *>(xz + o) = vb;
+            const double *fl = A.filt + m + kb;
+#pragma unroll 2
+            for (int k = lane; k < kp; k += 32) {
+                Z2 va{0, 0}, vb{0, 0};
+                if (c < n && k < kn) {
+                    const double f = fl[k];
+                    va = ld2(pa + 2 * k);
+                    va.x *= f; va.y *= f;
+                    if (g == 2) {
+                        // vorticity; plavor leaves mode (0,1) (legmod.f90:332)
+                        vb = ld2(pb + 2 * k);
+                        if (m == 0 && kb + k == 1) vb.x -= A.plavor;
+                        vb.x *= f; vb.y *= f;
+                    }
+                }
+                const int o = ((k & 1) * kh + (k >> 1)) * rs + 2 * c;
+                *reinterpret_cast<Z2 *>(xs + o) = va;
+                if (g == 2) *reinterpret_cast<Z2 *>(xz + o) = vb;
+            }
         }
         __syncthreads();
         if (!active) continue;
-        const double *tk = t0 + (size_t)(kb + 2 * q) * nlath, *uk = t1 + (size_t)(kb + 2 * q) * nlath;
         const int nst = kp >> 3;
+        const double2 *tk = t0 + (kb >> 3) * sstr;
+        const double *x0 = xs + q * rs + 2 * cw + r, *x1 = x0 + kh * rs;   // the two parities' rows
+        const int dx = 4 * rs;
         if (g < 2) {
-            const double *xb = xs + q * rs + 2 * cw + r;
-            double fa[2][MT], fb[2][MT];   // table fragments of two steps (8 modes: 4 of each parity)
-            auto fetch = [&](double (&t)[2][MT], int st) {
-                const double *tp = tk + (size_t)(8 * st) * nlath;
+            double2 fa[MT], fb[MT];
+            auto fetch = [&](double2 (&t)[MT]) {
 #pragma unroll
-                for (int p = 0; p < 2; p++)
-#pragma unroll
-                    for (int i = 0; i < MT; i++) t[p][i] = tp[p * nlath + jc[i]];
+                for (int i = 0; i < MT; i++) t[i] = tk[to[i]];
+                tk += sstr;
             };
-            auto step = [&](const double (&t)[2][MT], int st) {
+            auto step = [&](const double2 (&t)[MT]) {
 #pragma unroll
-                for (int p = 0; p < 2; p++) {
-                    const double *xp = xb + (size_t)(p * kh + 4 * st) * rs;
+                for (int c = 0; c < NT; c++) {
+                    const double b0 = x0[8 * c], b1 = x1[8 * c];
 #pragma unroll
-                    for (int c = 0; c < NT; c++) {
-                        const double b = xp[8 * c];
-#pragma unroll
-                        for (int i = 0; i < MT; i++) dmma(acc[p][i][c], t[p][i], b);
+                    for (int i = 0; i < MT; i++) {
+                        dmma(acc[0][i][c], t[i].x, b0);
+                        dmma(acc[1][i][c], t[i].y, b1);
                     }
                 }
+                x0 += dx;
+                x1 += dx;
             };
-            fetch(fa, 0);
-            for (int st = 0; st < nst; st += 2) {
-                if (st + 1 < nst) fetch(fb, st + 1);
-                step(fa, st);
-                if (st + 1 >= nst) break;
-                if (st + 2 < nst) fetch(fa, st + 2);
-                step(fb, st + 1);
+            if constexpr (PF) {
+                fetch(fa);
+                for (int st = 0; st < nst; st += 2) {
+                    if (st + 1 < nst) fetch(fb);
+                    step(fa);
+                    if (st + 1 >= nst) break;
+                    if (st + 2 < nst) fetch(fa);
+                    step(fb);
+                }
+            } else {
+                for (int st = 0; st < nst; st++) { fetch(fa); step(fa); }
             }
         } else {
             // u = sum qv*Z - i*qu*D ; v = sum -i*qu*Z - qv*D  (legmod.f90:338-341)
-            const int rx = r ^ 1;
-            const double *xd = xs + q * rs + 2 * cw, *xv = xz + q * rs + 2 * cw;
-            double fa[2][MT], fb[2][MT];   // (qu, qv) fragments of one half step (4 modes of one parity)
-            auto fetch = [&](double (&t)[2][MT], int hs) {
-                const size_t o = (size_t)(8 * (hs >> 1) + (hs & 1)) * nlath;
+            const int sw = (r ^ 1) - r, dz = A.kc * rs;   // the partner column, and Z behind D
+            const double sg = (r & 1) ? -1.0 : 1.0;       // -i*x: re <- im, im <- -re
+            const double2 *uk = tk + (INV_QV - INV_QU) * A.tsz;
+            double2 pa[MT], qa[MT], pb[MT], qb[MT];
+            auto fetch = [&](double2 (&t)[MT], double2 (&u)[MT]) {
 #pragma unroll
-                for (int i = 0; i < MT; i++) { t[0][i] = tk[o + jc[i]]; t[1][i] = uk[o + jc[i]]; }
+                for (int i = 0; i < MT; i++) { t[i] = tk[to[i]]; u[i] = uk[to[i]]; }
+                tk += sstr;
+                uk += sstr;
             };
-            auto half = [&](const double (&t)[2][MT], int st, auto par) {
-                constexpr int p = decltype(par)::value;
-                const size_t o = (size_t)(p * kh + 4 * st) * rs;
-                const double d = xd[o + r], z = xv[o + r];
-                double di = xd[o + rx], zi = xv[o + rx];   // -i*x: re <- im, im <- -re
-                if (r & 1) { di = -di; zi = -zi; }
-                // qu terms (P-type) and qv terms (Q-type) fall on opposite parities
+            auto step = [&](const double2 (&t)[MT], const double2 (&u)[MT]) {
 #pragma unroll
-                for (int i = 0; i < MT; i++) {
-                    dmma(acc[p][i][0], t[0][i], di);
-                    dmma(acc[1 - p][i][0], t[1][i], z);
-                    dmma(acc[p][i][1], t[0][i], zi);
-                    dmma(acc[1 - p][i][1], t[1][i], -d);
+                for (int p = 0; p < 2; p++) {
+                    const double *x = p ? x1 : x0;
+                    const double d = -x[0], z = x[dz], di = sg * x[sw], zi = sg * x[dz + sw];
+                    // qu terms (P-type) and qv terms (Q-type) fall on opposite parities
+#pragma unroll
+                    for (int i = 0; i < MT; i++) {
+                        const double tu = p ? t[i].y : t[i].x, tv = p ? u[i].y : u[i].x;
+                        dmma(acc[p][i][0], tu, di);
+                        dmma(acc[1 - p][i][0], tv, z);
+                        dmma(acc[p][i][1], tu, zi);
+                        dmma(acc[1 - p][i][1], tv, d);
+                    }
                 }
+                x0 += dx;
+                x1 += dx;
             };
-            fetch(fa, 0);
-            for (int st = 0; st < nst; st++) {
-                fetch(fb, 2 * st + 1);
-                half(fa, st, std::integral_constant<int, 0>{});
-                if (st + 1 < nst) fetch(fa, 2 * st + 2);
-                half(fb, st, std::integral_constant<int, 1>{});
+            if constexpr (PF) {
+                fetch(pa, qa);
+                for (int st = 0; st < nst; st += 2) {
+                    if (st + 1 < nst) fetch(pb, qb);
+                    step(pa, qa);
+                    if (st + 1 >= nst) break;
+                    if (st + 2 < nst) fetch(pa, qa);
+                    step(pb, qb);
+                }
+            } else {
+                for (int st = 0; st < nst; st++) { fetch(pa, qa); step(pa, qa); }
             }
         }
     }
@@ -313,14 +352,15 @@ __global__ void __launch_bounds__(256) k_leg_inv(const __grid_constant__ LegInv<
 // gridpointd's fc2sp of the temperature and humidity tendencies and uv2dv
 enum { OP_LEVEL_A = 4, OP_LEVEL_D = 5 };
 
-constexpr int FWD_THREADS = 192;   // least threads of a block; chunks hold at most 3 x 192 staged values
+constexpr int FWD_THREADS = 192;   // least threads of a block
+constexpr int FWD_JC = 16;         // latitude pairs per staged chunk
+// staged (north, south) values per thread and chunk: 9 inputs x 4 units x 16 pairs over 192 threads
 constexpr int FWD_ITEMS = 3;
 
 template <typename T>
 struct LegFwd {
-    const double *tab;       // 4 forward tables of tsz entries, blocks (m, parity) [j][mode of the parity, padded to 8]
-    const long long *foff;   // block offsets [m*2 + p]
-    size_t tsz;
+    const double4 *tab;      // forward fragments, the four tables side by side (plan.cu k_layout_fwd)
+    const int *foff;         // first fragment of each (m, parity)
     const int *woff;
     const double *filt;      // skgpsp(n)
     const T *in[6];          // single op: Fourier inputs; set: in[0] is the intermediate
@@ -329,165 +369,182 @@ struct LegFwd {
     long long o_fs;          // spectral field stride (reals)
     int nu, nt;              // units (levels x states) and unit tiles per wavenumber
     int nu1, nt1;            // gridpointa: ln ps tendencies (fc2sp) and their tiles
-    int ng, jc;              // groups of 4 units per block, latitude pairs per staged chunk
     int wb, nmb;             // warps along the modes of a block; mode blocks per wavenumber
     int L, nlat, nlath, ntp1;
 };
 
 template <int OP> struct FwdShape;
-template <> struct FwdShape<OP_FC2SP> { static constexpr int nin = 1, nout = 1; static constexpr bool c = 1, e = 0, m = 0, q = 0; };
-template <> struct FwdShape<OP_UV2DV> { static constexpr int nin = 2, nout = 2; static constexpr bool c = 0, e = 1, m = 1, q = 0; };
-template <> struct FwdShape<OP_QTEND> { static constexpr int nin = 3, nout = 1; static constexpr bool c = 1, e = 1, m = 1, q = 0; };
-template <> struct FwdShape<OP_MKTEND> { static constexpr int nin = 6, nout = 3; static constexpr bool c = 1, e = 1, m = 1, q = 1; };
-template <> struct FwdShape<OP_LEVEL_A> { static constexpr int nin = 9, nout = 4; static constexpr bool c = 1, e = 1, m = 1, q = 1; };
-template <> struct FwdShape<OP_LEVEL_D> { static constexpr int nin = 4, nout = 4; static constexpr bool c = 1, e = 1, m = 1, q = 0; };
+template <> struct FwdShape<OP_FC2SP> { static constexpr int nin = 1, nout = 1; static constexpr bool m = 0, q = 0; };
+template <> struct FwdShape<OP_UV2DV> { static constexpr int nin = 2, nout = 2; static constexpr bool m = 1, q = 0; };
+template <> struct FwdShape<OP_QTEND> { static constexpr int nin = 3, nout = 1; static constexpr bool m = 1, q = 0; };
+template <> struct FwdShape<OP_MKTEND> { static constexpr int nin = 6, nout = 3; static constexpr bool m = 1, q = 1; };
+template <> struct FwdShape<OP_LEVEL_A> { static constexpr int nin = 9, nout = 4; static constexpr bool m = 1, q = 1; };
+template <> struct FwdShape<OP_LEVEL_D> { static constexpr int nin = 4, nout = 4; static constexpr bool m = 1, q = 0; };
 
-template <int MT> struct FwdFrag { double c[MT], e[MT], m[MT], q[MT]; };
+// The four tables' fragments (qc, qe, qm, qq) of one tile
+struct __align__(32) FwdFrag { double c, e, m, q; };
 
 // Four latitude pairs' terms.  V(i, type, rot) is input i's fragment of the
 // parity that P-type (0) or Q-type (1) tables pair with, or (rot) i times it
 template <int OP, int MT, typename Val>
-__device__ __forceinline__ void fwd_terms(double (*o)[FwdShape<OP>::nout][2], const FwdFrag<MT> &t, Val V) {
-    auto add = [&](int x, const double (&a)[MT], double b) {
+__device__ __forceinline__ void fwd_terms(double (*o)[FwdShape<OP>::nout][2], const FwdFrag (&t)[MT], Val V) {
+    auto add = [&](int x, double FwdFrag::*a, double b) {
 #pragma unroll
-        for (int i = 0; i < MT; i++) dmma(o[i][x], a[i], b);
+        for (int i = 0; i < MT; i++) dmma(o[i][x], t[i].*a, b);
     };
     if constexpr (OP == OP_FC2SP) {          // sp = sum qc*f  (legmod.f90:203-220)
-        add(0, t.c, V(0, 0, 0));
+        add(0, &FwdFrag::c, V(0, 0, 0));
     } else if constexpr (OP == OP_UV2DV) {   // d = -qe*v + i*qm*u, z = qe*u + i*qm*v  (:391-424)
-        add(0, t.e, -V(1, 1, 0)); add(0, t.m, V(0, 0, 1));
-        add(1, t.e, V(0, 1, 0));  add(1, t.m, V(1, 0, 1));
+        add(0, &FwdFrag::e, -V(1, 1, 0)); add(0, &FwdFrag::m, V(0, 0, 1));
+        add(1, &FwdFrag::e, V(0, 1, 0));  add(1, &FwdFrag::m, V(1, 0, 1));
     } else if constexpr (OP == OP_QTEND) {   // q = qe*vq + qc*qn - i*qm*uq; in qn, uq, vq  (:466-497)
-        add(0, t.e, V(2, 1, 0)); add(0, t.c, V(0, 0, 0)); add(0, t.m, -V(1, 0, 1));
+        add(0, &FwdFrag::e, V(2, 1, 0)); add(0, &FwdFrag::c, V(0, 0, 0)); add(0, &FwdFrag::m, -V(1, 0, 1));
     } else if constexpr (OP == OP_MKTEND || OP == OP_LEVEL_A) {
         // mktend (:555-602): d = qq*ke - qe*fv + i*qm*fu, t = qe*vt + qc*tn - i*qm*ut, z = qe*fu + i*qm*fv.
         // Inputs: mktend tn, fu, fv, ke, ut, vt; the level's tn, qn, ut, vt, fv (guz), fu (gvz), ke, uq, vq
         constexpr bool A = OP == OP_LEVEL_A;
         constexpr int TN = 0, FU = A ? 5 : 1, FV = A ? 4 : 2, KE = A ? 6 : 3, UT = A ? 2 : 4, VT = A ? 3 : 5;
-        add(0, t.q, V(KE, 0, 0)); add(1, t.e, V(VT, 1, 0)); add(2, t.e, V(FU, 1, 0));
-        if constexpr (A) add(3, t.e, V(8, 1, 0));                                        // qtend
-        add(0, t.e, -V(FV, 1, 0)); add(1, t.c, V(TN, 0, 0)); add(2, t.m, V(FV, 0, 1));
-        if constexpr (A) add(3, t.c, V(1, 0, 0));
-        add(0, t.m, V(FU, 0, 1)); add(1, t.m, -V(UT, 0, 1));
-        if constexpr (A) add(3, t.m, -V(7, 0, 1));
+        add(0, &FwdFrag::q, V(KE, 0, 0)); add(1, &FwdFrag::e, V(VT, 1, 0)); add(2, &FwdFrag::e, V(FU, 1, 0));
+        if constexpr (A) add(3, &FwdFrag::e, V(8, 1, 0));                                        // qtend
+        add(0, &FwdFrag::e, -V(FV, 1, 0)); add(1, &FwdFrag::c, V(TN, 0, 0)); add(2, &FwdFrag::m, V(FV, 0, 1));
+        if constexpr (A) add(3, &FwdFrag::c, V(1, 0, 0));
+        add(0, &FwdFrag::m, V(FU, 0, 1)); add(1, &FwdFrag::m, -V(UT, 0, 1));
+        if constexpr (A) add(3, &FwdFrag::m, -V(7, 0, 1));
     } else {                                 // gridpointd: in t, u, v, q
-        add(0, t.e, -V(2, 1, 0)); add(2, t.e, V(1, 1, 0));
-        add(1, t.c, V(0, 0, 0)); add(3, t.c, V(3, 0, 0));
-        add(0, t.m, V(1, 0, 1)); add(2, t.m, V(2, 0, 1));
+        add(0, &FwdFrag::e, -V(2, 1, 0)); add(2, &FwdFrag::e, V(1, 1, 0));
+        add(1, &FwdFrag::c, V(0, 0, 0)); add(3, &FwdFrag::c, V(3, 0, 0));
+        add(0, &FwdFrag::m, V(1, 0, 1)); add(2, &FwdFrag::m, V(2, 0, 1));
     }
 }
 
-// A warp: MT tiles of 8 modes of one parity x one group of 4 units, every
-// output.  The units' folded values (N+S, N-S) are staged jc latitude pairs at
-// a time into one of two buffers while the other is read.
+// A warp: MT tiles of 8 modes of one parity x the block's group of 4 units,
+// every output.  The units' folded values (N+S, N-S) are staged jc latitude
+// pairs at a time into one of two buffers while the other is read.
 template <typename T, int OP, int MT, bool SET>
 __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, double *sm, int m, int mblk, int u0, int n) {
     using S = FwdShape<OP>;
-    constexpr int NIN = S::nin, NOUT = S::nout;
-    const int nlath = A.nlath, nlat = A.nlat, L = A.L, jcn = A.jc, lbu = 4 * A.ng;
+    constexpr int NIN = S::nin, NOUT = S::nout, rs = leg_stride(8), SEL = FWD_JC * rs, BUF = NIN * 2 * SEL;
+    static_assert(NIN * 4 * FWD_JC <= FWD_ITEMS * FWD_THREADS, "a chunk's values fit the threads' items");
+    const int nlath = A.nlath, nlat = A.nlat, L = A.L;
     const int K = A.ntp1 - m, K0 = (K + 1) >> 1, K1 = K >> 1;
     const int n0 = (K0 + 8 * MT - 1) / (8 * MT), n1 = (K1 + 8 * MT - 1) / (8 * MT);   // warps per parity
     if (mblk * A.wb >= n0 + n1) return;   // block-uniform
-    const int rs = leg_stride(8 * A.ng), bufsz = NIN * 2 * jcn * rs;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
-    const int g = warp / A.wb, wl = mblk * A.wb + warp - g * A.wb;
-    const bool active = g < A.ng && wl < n0 + n1 && 4 * g < n;
-    const int p = wl >= n0 ? 1 : 0, kq = p ? K1 : K0, k8 = (kq + 7) & ~7;
-    const int kk0 = (p ? wl - n0 : wl) * 8 * MT;
+    const int wl = mblk * A.wb + warp;
+    const bool active = warp < A.wb && wl < n0 + n1;
+    const int p = wl >= n0 ? 1 : 0, kq = p ? K1 : K0, kt = (kq + 7) >> 3;   // tiles of this parity
+    const int kt0 = (p ? wl - n0 : wl) * MT;
     double o[MT][NOUT][2];
 #pragma unroll
     for (int i = 0; i < MT; i++)
 #pragma unroll
         for (int x = 0; x < NOUT; x++) o[i][x][0] = o[i][x][1] = 0.0;
-    // this warp's table fragments: rows kk0 + 8i + r, latitude pairs j + q
-    const double *tb = nullptr;
-    int ko[MT];
-    if (active) {
-        tb = A.tab + A.foff[2 * m + p] + (size_t)q * k8;
+    // this warp's table fragments, four latitude pairs a step (tiles past the last repeat it)
+    const FwdFrag *tb = reinterpret_cast<const FwdFrag *>(A.tab);
+    int to[MT];
 #pragma unroll
-        for (int i = 0; i < MT; i++) ko[i] = min(kk0 + 8 * i, k8 - 8) + r;
-    }
-    auto fetch = [&](FwdFrag<MT> &t, int j) {
-        const double *tj = tb + (size_t)j * k8;
+    for (int i = 0; i < MT; i++) to[i] = active ? min(kt0 + i, kt - 1) * 32 : 0;
+    if (active) tb += (size_t)A.foff[2 * m + p] * 32 + lane;
+    const int tstr = kt * 32;
+    auto fetch = [&](FwdFrag (&t)[MT]) {
 #pragma unroll
         for (int i = 0; i < MT; i++) {
-            if constexpr (S::c) t.c[i] = tj[FWD_QC * A.tsz + ko[i]];
-            if constexpr (S::e) t.e[i] = tj[FWD_QE * A.tsz + ko[i]];
-            if constexpr (S::m) t.m[i] = tj[FWD_QM * A.tsz + ko[i]];
-            if constexpr (S::q) t.q[i] = tj[FWD_QQ * A.tsz + ko[i]];
+            const double2 *f = reinterpret_cast<const double2 *>(tb + to[i]);
+            const double2 ce = f[0];
+            t[i].c = ce.x; t[i].e = ce.y;
+            if constexpr (S::m || S::q) { const double2 mq = f[1]; t[i].m = mq.x; t[i].q = mq.y; }
         }
+        tb += tstr;
     };
-    // staged values: item (input i, unit, latitude pair), latitude pairs fastest
-    Z2 vn[FWD_ITEMS], vs[FWD_ITEMS];
-    const int nitem = NIN * lbu * jcn;
+    // this thread's staged items (latitude pair jj of a chunk, unit, input i):
+    // the chunk's northern and southern values arrive in `raw` by asynchronous
+    // copies and the same thread folds them into the operand buffer
+    C2<T> *raw = reinterpret_cast<C2<T> *>(sm + BUF) + threadIdx.x;
+    const T *pn[FWD_ITEMS];
+    int so[FWD_ITEMS], je[FWD_ITEMS];
+    const long long ls = SET ? 1 : A.ls;
+#pragma unroll
+    for (int e = 0; e < FWD_ITEMS; e++) {
+        const int idx = threadIdx.x + e * blockDim.x, jj = idx % FWD_JC, rr = idx / FWD_JC, ul = rr & 3, i = rr >> 2, u = u0 + ul;
+        so[e] = i < NIN ? 2 * i * SEL + jj * rs + 2 * ul : -1;
+        je[e] = i < NIN && ul < n ? jj : nlath;   // the chunk from j0 holds this pair while j0 + je < nlath
+        pn[e] = A.in[0];
+        if (je[e] >= nlath) continue;
+        if constexpr (SET) {
+            long long f;
+            if constexpr (OP == OP_FC2SP) f = (long long)u * (9 * L + 1) + 7 * L;   // gvpp of state u
+            else {
+                const int inst = u / L, lev = u - inst * L;
+                // gridpointa: tn qn ut vt uz vz ke [vpp] uq vq; gridpointd: t u v q
+                f = (long long)inst * (OP == OP_LEVEL_A ? 9 * L + 1 : 4 * L) + i * L + lev + (OP == OP_LEVEL_A && i >= 7);
+            }
+            pn[e] = A.in[0] + 2 * ((size_t)m * A.nrows + f * nlat);
+        } else {
+            pn[e] = A.in[i] + 2 * (u * A.fs + (long long)m * A.ms);
+        }
+    }
     auto load = [&](int j0) {
 #pragma unroll
         for (int e = 0; e < FWD_ITEMS; e++) {
-            const int idx = threadIdx.x + e * blockDim.x;
-            vn[e] = vs[e] = Z2{0, 0};
-            if (idx >= nitem) continue;
-            const int jj = idx % jcn, rr = idx / jcn, ul = rr % lbu, i = rr / lbu, u = u0 + ul, j = j0 + jj;
-            if (ul >= n || j >= nlath) continue;
-            if constexpr (SET) {
-                long long f;
-                if constexpr (OP == OP_FC2SP) f = (long long)u * (9 * L + 1) + 7 * L;   // gvpp of state u
-                else {
-                    const int inst = u / L, lev = u - inst * L;
-                    // gridpointa: tn qn ut vt uz vz ke [vpp] uq vq; gridpointd: t u v q
-                    f = (long long)inst * (OP == OP_LEVEL_A ? 9 * L + 1 : 4 * L) + i * L + lev + (OP == OP_LEVEL_A && i >= 7);
-                }
-                const C2<T> *w = reinterpret_cast<const C2<T> *>(A.in[0]) + (size_t)m * A.nrows + f * nlat;
-                const C2<T> a = w[j], b = w[nlat - 1 - j];
-                vn[e] = Z2{(double)a.x, (double)a.y};
-                vs[e] = Z2{(double)b.x, (double)b.y};
-            } else {
-                const T *w = A.in[i] + 2 * (u * A.fs + (long long)m * A.ms);
-                vn[e] = ld2(w + 2 * (j * A.ls));
-                vs[e] = ld2(w + 2 * ((nlat - 1 - j) * A.ls));
-            }
+            const int j = j0 + je[e];
+            C2<T> *d = raw + 2 * e * blockDim.x;
+            const bool ok = j < nlath;   // zeros otherwise
+            cp_complex<SET>(d, pn[e] + (ok ? 2 * (j * ls) : 0), ok);
+            cp_complex<SET>(d + blockDim.x, pn[e] + (ok ? 2 * ((nlat - 1 - j) * ls) : 0), ok);
         }
     };
-    auto store = [&](double *buf) {
+    auto fold = [&] {
+        asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
         for (int e = 0; e < FWD_ITEMS; e++) {
-            const int idx = threadIdx.x + e * blockDim.x;
-            if (idx >= nitem) continue;
-            const int jj = idx % jcn, rr = idx / jcn, ul = rr % lbu, i = rr / lbu;
-            double *d = buf + (size_t)(2 * i * jcn + jj) * rs + 2 * ul;
-            *reinterpret_cast<Z2 *>(d) = Z2{vn[e].x + vs[e].x, vn[e].y + vs[e].y};
-            *reinterpret_cast<Z2 *>(d + (size_t)jcn * rs) = Z2{vn[e].x - vs[e].x, vn[e].y - vs[e].y};
+            if (so[e] < 0) continue;
+            const C2<T> vn = raw[2 * e * blockDim.x], vs = raw[(2 * e + 1) * blockDim.x];
+            const double nx = vn.x, ny = vn.y, sx = vs.x, sy = vs.y;
+            *reinterpret_cast<Z2 *>(sm + so[e]) = Z2{nx + sx, ny + sy};
+            *reinterpret_cast<Z2 *>(sm + so[e] + SEL) = Z2{nx - sx, ny - sy};
         }
     };
-    FwdFrag<MT> ta, tn;
-    if (active) fetch(ta, 0);
+    const int nl4 = (nlath + 3) & ~3;
+    constexpr bool PF = MT == 1;   // fetch a step ahead: few warps to hide the latency
+    FwdFrag ta[MT], tn[MT];
     load(0);
-    store(sm);
-    __syncthreads();
-    const int nl4 = (nlath + 3) & ~3, nch = (nlath + jcn - 1) / jcn;
-    for (int c = 0; c < nch; c++) {
-        const int j0 = c * jcn;
-        if (c + 1 < nch) load(j0 + jcn);
+    if (PF && active) fetch(tn);
+    // P-type tables see the sum on even n-m and the difference on odd, Q-type
+    // the reverse; the partner column (re <-> im) for i*x: re <- -im, im <- re
+    const double *bp = sm + q * rs + r + (p ? SEL : 0), *bq = sm + q * rs + r + (p ? 0 : SEL);
+    const int sw = (r ^ 1) - r;
+    const double sg = (r & 1) ? 1.0 : -1.0;
+    for (int j0 = 0; j0 < nlath; j0 += FWD_JC) {
+        fold();
+        __syncthreads();
+        if (j0 + FWD_JC < nlath) load(j0 + FWD_JC);
         if (active) {
-            const double *xb = sm + (size_t)(c & 1) * bufsz + q * rs + 8 * g;
-            const int je = min(jcn, nl4 - j0);
-            for (int jj = 0; jj < je; jj += 4) {
-                if (j0 + jj + 4 < nl4) fetch(tn, j0 + jj + 4);
+            const double *xp = bp, *xq = bq;
+            const int jn = min(FWD_JC, nl4 - j0);
+#pragma unroll 1
+            for (int jj = 0; jj < jn; jj += 4) {
+                if constexpr (PF) {
+#pragma unroll
+                    for (int i = 0; i < MT; i++) ta[i] = tn[i];
+                    if (j0 + jj + 4 < nl4) fetch(tn);
+                } else {
+                    fetch(ta);
+                }
                 fwd_terms<OP, MT>(o, ta, [&](int i, int type, int rot) {
-                    // P-type tables see the sum on even n-m and the difference on odd, Q-type the reverse
-                    const double v = xb[(size_t)((2 * i + (type ^ p)) * jcn + jj) * rs + (r ^ rot)];
-                    return rot && !(r & 1) ? -v : v;   // i*x: re <- -im, im <- re
+                    const double *x = (type ? xq : xp) + 2 * i * SEL;
+                    return rot ? sg * x[sw] : x[0];
                 });
-                ta = tn;
+                xp += 4 * rs;
+                xq += 4 * rs;
             }
         }
-        if (c + 1 < nch) store(sm + (size_t)((c + 1) & 1) * bufsz);
         __syncthreads();
     }
-    if (!active || 4 * g + q >= n) return;
-    const int u = u0 + 4 * g + q, w0 = A.woff[m];
+    if (!active || q >= n) return;
+    const int u = u0 + q, w0 = A.woff[m];
 #pragma unroll
     for (int i = 0; i < MT; i++) {
-        const int kk = kk0 + 8 * i + r, k = 2 * kk + p;
+        const int kk = (kt0 + i) * 8 + r, k = 2 * kk + p;
         if (kk >= kq) continue;
         const double f = A.filt[m + k];
 #pragma unroll
@@ -508,19 +565,18 @@ __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, double *sm, in
 }
 
 template <typename T, int OP, int MT, bool SET>
-__global__ void __launch_bounds__(512) k_leg_fwd(const __grid_constant__ LegFwd<T> A) {
+__global__ void __launch_bounds__(384, MT == 1 ? 1 : 2) k_leg_fwd(const __grid_constant__ LegFwd<T> A) {
     extern __shared__ __align__(16) unsigned char smraw[];
     double *sm = reinterpret_cast<double *>(smraw);
     const int nt = A.nt + A.nt1, mb = blockIdx.x / nt, ti = blockIdx.x - mb * nt;
-    const int m = mb / A.nmb, mblk = mb - m * A.nmb, lbu = 4 * A.ng;
+    const int m = mb / A.nmb, mblk = mb - m * A.nmb;
     pdl_trigger();
     pdl_wait();
     if (ti < A.nt) {
-        const int u0 = ti * lbu;
-        leg_fwd_block<T, OP, MT, SET>(A, sm, m, mblk, u0, min(lbu, A.nu - u0));
+        leg_fwd_block<T, OP, MT, SET>(A, sm, m, mblk, 4 * ti, min(4, A.nu - 4 * ti));
     } else if constexpr (OP == OP_LEVEL_A) {
-        const int u0 = (ti - A.nt) * lbu;
-        leg_fwd_block<T, OP_FC2SP, MT, SET>(A, sm, m, mblk, u0, min(lbu, A.nu1 - u0));
+        const int u0 = 4 * (ti - A.nt);
+        leg_fwd_block<T, OP_FC2SP, MT, SET>(A, sm, m, mblk, u0, min(4, A.nu1 - u0));
     }
 }
 
@@ -532,9 +588,9 @@ constexpr long long LEG_WARPS = 1200;
 template <typename T, int MT, int NT, bool SET>
 static exotx_status inv_launch_t(exotx_plan p, LegInv<T> &A, cudaStream_t s) {
     const int lt = (p->nlath + 8 * MT - 1) / (8 * MT);   // latitude warps
-    A.wm = std::min(lt, 4);
-    A.nlb = (lt + A.wm - 1) / A.wm;
-    A.wn = std::max(1, 6 / A.wm);
+    A.nlb = (lt + 3) / 4;
+    A.wm = (lt + A.nlb - 1) / A.nlb;
+    A.wn = 6 / A.wm;
     // the staged columns of a block: all modes at once where they fit the budget
     auto smem_of = [&](int kc, int wn) {
         const size_t one = (size_t)kc * leg_stride(8 * NT * wn), two = A.nu[2] ? 2 * (size_t)kc * leg_stride(8 * wn) : 0;
@@ -560,11 +616,12 @@ static exotx_status inv_launch_t(exotx_plan p, LegInv<T> &A, cudaStream_t s) {
 }
 template <typename T, bool SET>
 static exotx_status inv_launch(exotx_plan p, LegInv<T> &A, cudaStream_t s) {
-    A.tab = p->d_inv64; A.woff = p->d_woff; A.filt = p->d_fs64;
-    A.nlat = p->nlat; A.nlath = p->nlath; A.ntp1 = p->ntp1; A.ncsp = p->ncsp; A.nrsp = 2 * p->ncsp;
+    A.tab = reinterpret_cast<const double2 *>(p->d_inv64); A.ioff = p->d_ioff; A.tsz = p->inv_tsz;
+    A.woff = p->d_woff; A.filt = p->d_fs64;
+    A.nlat = p->nlat; A.nlath = p->nlath; A.ntl = (p->nlath + 7) / 8; A.ntp1 = p->ntp1; A.nrsp = 2 * p->ncsp;
     A.plavor = p->desc.plavor;
-    const long long tiles = (long long)p->ntp1 * ((p->nlath + 7) / 8) * ((A.nu[0] + A.nu[1]) / 4 + A.nu[2] / 2 + 1);
-    return tiles / 8 >= LEG_WARPS ? inv_launch_t<T, 4, 2, SET>(p, A, s) : inv_launch_t<T, 2, 1, SET>(p, A, s);
+    const long long tiles = (long long)p->ntp1 * A.ntl * ((A.nu[0] + A.nu[1]) / 4 + A.nu[2] / 2 + 1);
+    return tiles / 4 >= LEG_WARPS ? inv_launch_t<T, 2, 2, SET>(p, A, s) : inv_launch_t<T, 2, 1, SET>(p, A, s);
 }
 
 template <typename T>
@@ -596,16 +653,14 @@ template <typename T, int OP, int MT, bool SET>
 static exotx_status fwd_launch_t(exotx_plan p, LegFwd<T> &A, cudaStream_t s) {
     const int K0 = (p->ntp1 + 1) / 2, K1 = p->ntp1 / 2;
     const int nw = (K0 + 8 * MT - 1) / (8 * MT) + (K1 + 8 * MT - 1) / (8 * MT);   // mode warps at m = 0
-    A.ng = nw <= 8 && A.nu > 4 ? 2 : 1;
-    A.wb = std::min(nw, 16 / A.ng);
-    A.nmb = (nw + A.wb - 1) / A.wb;
-    const int threads = std::max(FWD_THREADS, 32 * A.wb * A.ng);
-    // latitude pairs per chunk: 16, fewer where a chunk's values do not fit FWD_ITEMS per thread
-    A.jc = 16;
-    while (A.jc > 4 && FwdShape<OP>::nin * 4 * A.ng * A.jc > FWD_ITEMS * threads) A.jc /= 2;
-    const size_t smem = (size_t)FwdShape<OP>::nin * 2 * A.jc * leg_stride(8 * A.ng) * 2 * sizeof(double);
-    A.nt = (A.nu + 4 * A.ng - 1) / (4 * A.ng);
-    A.nt1 = (A.nu1 + 4 * A.ng - 1) / (4 * A.ng);
+    A.nmb = (nw + 11) / 12;
+    A.wb = (nw + A.nmb - 1) / A.nmb;
+    const int threads = std::max(FWD_THREADS, 32 * A.wb);
+    // one operand chunk and the copies on their way
+    const size_t smem = (size_t)FwdShape<OP>::nin * 2 * FWD_JC * leg_stride(8) * sizeof(double) +
+                        (size_t)FWD_ITEMS * 2 * threads * sizeof(C2<T>);
+    A.nt = (A.nu + 3) / 4;
+    A.nt1 = (A.nu1 + 3) / 4;
     const long long blocks = (long long)p->ntp1 * A.nmb * (A.nt + A.nt1);
     if (blocks > 0x7fffffffLL || smem > LEG_MAXSMEM) return EXOTX_BAD_DIM;
     auto kern = k_leg_fwd<T, OP, MT, SET>;
@@ -618,7 +673,7 @@ static exotx_status fwd_launch_t(exotx_plan p, LegFwd<T> &A, cudaStream_t s) {
 }
 template <typename T, int OP, bool SET>
 static exotx_status fwd_launch(exotx_plan p, LegFwd<T> &A, cudaStream_t s) {
-    A.tab = p->d_fwd64; A.foff = p->d_foff; A.tsz = p->fwd_tsz; A.woff = p->d_woff; A.filt = p->d_fg64;
+    A.tab = reinterpret_cast<const double4 *>(p->d_fwd64); A.foff = p->d_foff; A.woff = p->d_woff; A.filt = p->d_fg64;
     A.nlat = p->nlat; A.nlath = p->nlath; A.ntp1 = p->ntp1;
     const long long tiles = (long long)(p->ncsp / 8 + p->ntp1) * ((A.nu + 3) / 4);
     return tiles / 2 >= LEG_WARPS ? fwd_launch_t<T, OP, 2, SET>(p, A, s) : fwd_launch_t<T, OP, 1, SET>(p, A, s);

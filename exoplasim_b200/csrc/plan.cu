@@ -136,34 +136,46 @@ __global__ void k_legini(int nlat, int ntru, int ncsp, const int *woff, const do
     }
 }
 
-// inverse layout [t][w][j] for qi,qj,qu,qv (reference tables 0,1,6,7)
-__global__ void k_layout_inv(int nlat, int ncsp, int nlath, const double *qref, double *inv64) {
-    size_t tsz = (size_t)ncsp * nlat;
-    size_t total = (size_t)4 * ncsp * nlath;
+// Both layouts hold the tables as the 8x4 operand fragments that the Legendre
+// kernels' FP64 tensor-core instructions read (legendre_simt.cu): 32 lanes,
+// lane = 4 r + q for row r and column q, zeros past the last latitude or mode.
+// One block per wavenumber (and parity).
+
+// inverse, qi,qj,qu,qv (reference tables 0,1,6,7): table t, step s of 8 modes,
+// latitude tile b: lane (r, q) holds latitude 8b + r of the modes n-m = 8s + 2q
+// and 8s + 2q + 1 side by side; ioff[m] steps precede wavenumber m
+__global__ void k_layout_inv(int nlat, int ntru, int ncsp, int nlath, const int *woff, const int *ioff, size_t tsz,
+                             const double *qref, double2 *inv64) {
+    const int m = blockIdx.x, K = ntru + 1 - m, ns = (K + 7) >> 3, ntl = (nlath + 7) >> 3;
+    const size_t rsz = (size_t)ncsp * nlat;
     const int src[4] = {0, 1, 6, 7};
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
-         i += (size_t)gridDim.x * blockDim.x) {
-        int j = (int)(i % nlath);
-        size_t r = i / nlath;
-        int w = (int)(r % ncsp);
-        int t = (int)(r / ncsp);
-        inv64[i] = qref[src[t] * tsz + (size_t)j * ncsp + w];
+    for (int i = threadIdx.x; i < ns * ntl * 32; i += blockDim.x) {
+        const int lane = i & 31, b = (i >> 5) % ntl, s = (i >> 5) / ntl;
+        const int j = 8 * b + (lane >> 2), k = 8 * s + 2 * (lane & 3);
+        for (int t = 0; t < 4; t++) {
+            const double *q = qref + src[t] * rsz + (size_t)j * ncsp + woff[m];
+            inv64[t * tsz + (size_t)ioff[m] * ntl * 32 + i] =
+                make_double2(j < nlath && k < K ? q[k] : 0.0, j < nlath && k + 1 < K ? q[k + 1] : 0.0);
+        }
     }
 }
 
-// forward layout for qc,qe,qm,qq (2,3,4,5): block (m, parity p of n-m) at
-// foff[2m + p] holds [j][kk] for the modes n-m = 2kk + p, kk padded to 8 and the
-// latitude pairs to 4 with zeros.  One block per (m, p)
-__global__ void k_layout_fwd(int nlat, int ntru, int ncsp, int nlath, const int *woff, const long long *foff,
-                             size_t ftsz, const double *qref, double *fwd64) {
-    const int m = blockIdx.x >> 1, p = blockIdx.x & 1, K = ntru + 1 - m, kq = (K + 1 - p) >> 1, k8 = (kq + 7) & ~7;
-    const int nl4 = (nlath + 3) & ~3;
-    const size_t tsz = (size_t)ncsp * nlat;
-    for (int i = threadIdx.x; i < nl4 * k8; i += blockDim.x) {
-        const int j = i / k8, kk = i - j * k8;
-        for (int t = 0; t < 4; t++)
-            fwd64[t * ftsz + foff[blockIdx.x] + i] =
-                (j < nlath && kk < kq) ? qref[(2 + t) * tsz + (size_t)j * ncsp + woff[m] + 2 * kk + p] : 0.0;
+// forward, qc,qe,qm,qq (2,3,4,5) side by side: block (m, parity p of n-m), step
+// s of 4 latitude pairs, tile b of 8 modes: lane (r, q) holds mode
+// n-m = 2 (8b + r) + p at latitude 4s + q; foff[2m + p] fragments precede a block
+__global__ void k_layout_fwd(int nlat, int ntru, int ncsp, int nlath, const int *woff, const int *foff,
+                             const double *qref, double4 *fwd64) {
+    const int m = blockIdx.x >> 1, p = blockIdx.x & 1, K = ntru + 1 - m, kq = (K + 1 - p) >> 1, kt = (kq + 7) >> 3;
+    const size_t rsz = (size_t)ncsp * nlat;
+    for (int i = threadIdx.x; i < ((nlath + 3) >> 2) * kt * 32; i += blockDim.x) {
+        const int lane = i & 31, b = (i >> 5) % kt, s = (i >> 5) / kt;
+        const int j = 4 * s + (lane & 3), kk = 8 * b + (lane >> 2);
+        double4 v = make_double4(0.0, 0.0, 0.0, 0.0);
+        if (j < nlath && kk < kq) {
+            const double *q = qref + 2 * rsz + (size_t)j * ncsp + woff[m] + 2 * kk + p;
+            v = make_double4(q[0], q[rsz], q[2 * rsz], q[3 * rsz]);
+        }
+        fwd64[(size_t)foff[blockIdx.x] * 32 + i] = v;
     }
 }
 
@@ -225,6 +237,7 @@ static void plan_free(exotx_plan p) {
     cudaFree(p->d_qref);
     cudaFree(p->d_inv64);
     cudaFree(p->d_fwd64);
+    cudaFree(p->d_ioff);
     cudaFree(p->d_foff);
     cudaFree(p->d_fs64);
     cudaFree(p->d_fg64);
@@ -302,14 +315,17 @@ EXOTX_API exotx_status exotx_plan_create(const exotx_grid_desc *d, exotx_plan *o
     host_filters(*d, p->ntru, g, sv);
     std::vector<float> g32(g.begin(), g.end()), s32(sv.begin(), sv.end());
     size_t tsz = (size_t)ncsp * nlat;
-    size_t half = (size_t)4 * ncsp * nlath;
-    // the inverse kernel reads whole steps of 8 modes: up to 7 rows past the last one, times zero
-    const size_t inv_pad = (size_t)8 * nlath;
-    std::vector<long long> foff(2 * ntp1);
-    for (int i = 0; i < 2 * ntp1; i++) {
-        foff[i] = (long long)p->fwd_tsz;
-        p->fwd_tsz += (size_t)((nlath + 3) & ~3) * ((((ntp1 - i / 2 + 1 - i % 2) >> 1) + 7) & ~7);
+    std::vector<int> ioff(ntp1), foff(2 * ntp1);
+    int nstep = 0, nfrag = 0;
+    for (int m = 0; m < ntp1; m++) {
+        ioff[m] = nstep;
+        nstep += (ntp1 - m + 7) / 8;
+        for (int q = 0; q < 2; q++) {
+            foff[2 * m + q] = nfrag;
+            nfrag += (nlath + 3) / 4 * (((ntp1 - m + 1 - q) / 2 + 7) / 8);
+        }
     }
+    p->inv_tsz = (size_t)nstep * ((nlath + 7) / 8) * 32;
     exotx_status st = EXOTX_OK;
 #define PALLOC(ptr, bytes)                                           \
     do {                                                             \
@@ -322,9 +338,10 @@ EXOTX_API exotx_status exotx_plan_create(const exotx_grid_desc *d, exotx_plan *o
     PALLOC(p->d_sid, sizeof(double) * nlat);
     PALLOC(p->d_gwd, sizeof(double) * nlat);
     PALLOC(p->d_qref, sizeof(double) * 8 * tsz);
-    PALLOC(p->d_inv64, sizeof(double) * (half + inv_pad));
-    PALLOC(p->d_fwd64, sizeof(double) * 4 * p->fwd_tsz);
-    PALLOC(p->d_foff, sizeof(long long) * 2 * ntp1);
+    PALLOC(p->d_inv64, sizeof(double2) * 4 * p->inv_tsz);
+    PALLOC(p->d_fwd64, sizeof(double4) * 32 * (size_t)nfrag);
+    PALLOC(p->d_ioff, sizeof(int) * ntp1);
+    PALLOC(p->d_foff, sizeof(int) * 2 * ntp1);
     PALLOC(p->d_fs64, sizeof(double) * ntp1);
     PALLOC(p->d_fg64, sizeof(double) * ntp1);
     PALLOC(p->d_fs32, sizeof(float) * ntp1);
@@ -332,8 +349,8 @@ EXOTX_API exotx_status exotx_plan_create(const exotx_grid_desc *d, exotx_plan *o
 #undef PALLOC
     {
         cudaStream_t s = 0;
-        if (cudaMemset(p->d_inv64 + half, 0, sizeof(double) * inv_pad) ||
-            cudaMemcpy(p->d_foff, foff.data(), sizeof(long long) * 2 * ntp1, cudaMemcpyHostToDevice) ||
+        if (cudaMemcpy(p->d_ioff, ioff.data(), sizeof(int) * ntp1, cudaMemcpyHostToDevice) ||
+            cudaMemcpy(p->d_foff, foff.data(), sizeof(int) * 2 * ntp1, cudaMemcpyHostToDevice) ||
             cudaMemcpy(p->d_woff, woff.data(), sizeof(int) * (ntp1 + 1), cudaMemcpyHostToDevice) ||
             cudaMemcpy(p->d_fg64, g.data(), sizeof(double) * ntp1, cudaMemcpyHostToDevice) ||
             cudaMemcpy(p->d_fs64, sv.data(), sizeof(double) * ntp1, cudaMemcpyHostToDevice) ||
@@ -347,11 +364,11 @@ EXOTX_API exotx_status exotx_plan_create(const exotx_grid_desc *d, exotx_plan *o
         k_legini<<<nlat, 128, sizeof(double) * 2 * ntp1, s>>>(nlat, p->ntru, ncsp, p->d_woff, p->d_sid,
                                                               p->d_gwd, p->d_qref);
         note_launch();
-        int blocks = (int)std::min<size_t>((half + 255) / 256, 148 * 16);
-        k_layout_inv<<<blocks, 256, 0, s>>>(nlat, ncsp, nlath, p->d_qref, p->d_inv64);
+        k_layout_inv<<<ntp1, 256, 0, s>>>(nlat, p->ntru, ncsp, nlath, p->d_woff, p->d_ioff, p->inv_tsz, p->d_qref,
+                                          reinterpret_cast<double2 *>(p->d_inv64));
         note_launch();
-        k_layout_fwd<<<2 * ntp1, 256, 0, s>>>(nlat, p->ntru, ncsp, nlath, p->d_woff, p->d_foff, p->fwd_tsz, p->d_qref,
-                                              p->d_fwd64);
+        k_layout_fwd<<<2 * ntp1, 256, 0, s>>>(nlat, p->ntru, ncsp, nlath, p->d_woff, p->d_foff, p->d_qref,
+                                              reinterpret_cast<double4 *>(p->d_fwd64));
         note_launch();
         if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) {
             st = EXOTX_CUDA_ERR;
