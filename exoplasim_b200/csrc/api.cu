@@ -12,30 +12,31 @@ static FourierLayout ref_layout(exotx_plan p) {
 static bool prec_ok(int prec) { return prec == EXOTX_FP64 || prec == EXOTX_FP32 || prec == EXOTX_MIXED; }
 
 // The FP64 and FP32 sets over ninst states: one Legendre and one FFT launch per
-// chunk of states.  A chunk's m-major intermediate is held to SIMT_CHUNK bytes
+// chunk of states.  A chunk's m-major intermediate is held to PLAIN_CHUNK bytes
 // (at least one state), so that it is still in L2 when the next kernel reads it
 // and the plan's work buffer stays small.
-constexpr size_t SIMT_CHUNK = (size_t)96 << 20;
-static int simt_chunk(size_t per_inst, int ninst) {
-    return (int)std::min<size_t>((size_t)ninst, std::max<size_t>(1, SIMT_CHUNK / per_inst));
+constexpr size_t PLAIN_CHUNK = (size_t)96 << 20;
+static int plain_chunk(size_t per_inst, int ninst) {
+    return (int)std::min<size_t>((size_t)ninst, std::max<size_t>(1, PLAIN_CHUNK / per_inst));
 }
 
 // invlega / invlegd (legmod.f90:635-677) and fc2gp of every field: gridpointa
 // (dset = 0, plasim.f90:2396-2440) spin (4L+1 fields) -> gpout (6L+3),
 // gridpointd (dset = 1, :3142-3149) -> 4L+1
 template <typename T>
-static exotx_status inverse_set_simt(exotx_plan p, const T *spin, T *gpout, int L, int ninst, int dset,
+static exotx_status inverse_set_plain(exotx_plan p, const T *spin, T *gpout, int L, int ninst, int dset,
                                      cudaStream_t s) {
     const size_t nrsp = 2 * (size_t)p->ncsp, nhor = (size_t)p->nlat * p->nlon;
     const int nfo = dset ? 4 * L + 1 : 6 * L + 3;
     const size_t per_inst = sizeof(T) * 2 * (size_t)nfo * p->nlat * p->ntp1;
-    const int chunk = simt_chunk(per_inst, ninst);
+    const int chunk = plain_chunk(per_inst, ninst);
     EXOTX_TRY(ensure_work(p, per_inst * chunk));
     T *w = (T *)p->d_work;
     for (int i0 = 0; i0 < ninst; i0 += chunk) {
         const int ni = std::min(chunk, ninst - i0);
         const long long nrows = (long long)ni * nfo * p->nlat;
-        EXOTX_TRY(leg_inverse_set<T>(p, dset, spin + i0 * (4 * L + 1) * nrsp, w, L, ni, s));
+        const LegSeg<T> g = {p, L, ni, spin + i0 * (4 * L + 1) * nrsp, w, false};
+        EXOTX_TRY(leg_inverse_set<T>(&g, 1, dset, s));
         EXOTX_TRY(fft_inverse_l<T>(w, gpout + i0 * nfo * nhor, p->nlon, nrows, p->ntp1, 1, nrows, s));
     }
     return EXOTX_OK;
@@ -44,19 +45,20 @@ static exotx_status inverse_set_simt(exotx_plan p, const T *spin, T *gpout, int 
 // gp2fc of every field, then mktend, qtend and fc2sp(gvpp) (gridpointa,
 // plasim.f90:2462-2486) or fc2sp and uv2dv (gridpointd, :3415-3428)
 template <typename T>
-static exotx_status forward_set_simt(exotx_plan p, const T *gpin, T *spout, int L, int ninst, int dset,
+static exotx_status forward_set_plain(exotx_plan p, const T *gpin, T *spout, int L, int ninst, int dset,
                                      cudaStream_t s) {
     const size_t nrsp = 2 * (size_t)p->ncsp, nhor = (size_t)p->nlat * p->nlon;
     const int nfi = dset ? 4 * L : 9 * L + 1, nfo = dset ? 4 * L : 4 * L + 1;
     const size_t per_inst = sizeof(T) * 2 * (size_t)nfi * p->nlat * p->ntp1;
-    const int chunk = simt_chunk(per_inst, ninst);
+    const int chunk = plain_chunk(per_inst, ninst);
     EXOTX_TRY(ensure_work(p, per_inst * chunk));
     T *w = (T *)p->d_work;
     for (int i0 = 0; i0 < ninst; i0 += chunk) {
         const int ni = std::min(chunk, ninst - i0);
         const long long nrows = (long long)ni * nfi * p->nlat;
         EXOTX_TRY(fft_forward_l<T>(gpin + i0 * nfi * nhor, w, p->nlon, nrows, p->ntp1, 1, nrows, s));
-        EXOTX_TRY(leg_forward_set<T>(p, dset, w, spout + i0 * nfo * nrsp, L, ni, s));
+        const LegSeg<T> g = {p, L, ni, w, spout + i0 * nfo * nrsp, false};
+        EXOTX_TRY(leg_forward_set<T>(&g, 1, dset, s));
     }
     return EXOTX_OK;
 }
@@ -176,7 +178,7 @@ static exotx_status inverse_set_api(exotx_plan p, int prec, const void *spin, vo
                                                                (cudaStream_t)s);
     return by_prec(prec, [&](auto tag) {
         using T = std::remove_pointer_t<decltype(tag)>;
-        return inverse_set_simt<T>(p, (const T *)spin, (T *)gpout, nlev, ninst, dset, (cudaStream_t)s);
+        return inverse_set_plain<T>(p, (const T *)spin, (T *)gpout, nlev, ninst, dset, (cudaStream_t)s);
     });
 }
 static exotx_status forward_set_api(exotx_plan p, int prec, const void *gpin, void *spout, int nlev, int ninst,
@@ -189,7 +191,7 @@ static exotx_status forward_set_api(exotx_plan p, int prec, const void *gpin, vo
                                                                (cudaStream_t)s);
     return by_prec(prec, [&](auto tag) {
         using T = std::remove_pointer_t<decltype(tag)>;
-        return forward_set_simt<T>(p, (const T *)gpin, (T *)spout, nlev, ninst, dset, (cudaStream_t)s);
+        return forward_set_plain<T>(p, (const T *)gpin, (T *)spout, nlev, ninst, dset, (cudaStream_t)s);
     });
 }
 

@@ -69,11 +69,10 @@ static exotx_status ens_inverse(exotx_ensemble e, const float *spin, float *gpou
 static exotx_status ens_forward(exotx_ensemble e, const float *gpin, float *spout, cudaStream_t s) {
     std::vector<EnsSeg> v = ens_segs(e, nullptr, spout);
     std::vector<FftEnsSeg> f(v.size());
-    const bool folded = tc_ens_fwd_folded(v.data(), (int)v.size());   // persistent kernel: folded intermediate
     for (size_t i = 0; i < v.size(); i++) {
         const exotx_plan p = v[i].p;
         const long long rows = (long long)v[i].ninst * (9 * v[i].L + 1) * p->nlat;
-        f[i] = FftEnsSeg{gpin + e->seg_gin[i], v[i].W, rows, 1, rows, p->nlon, p->ntp1, folded ? p->nlat : 0};
+        f[i] = FftEnsSeg{gpin + e->seg_gin[i], v[i].W, rows, 1, rows, p->nlon, p->ntp1, p->nlat};   // folded intermediate
     }
     EXOTX_TRY(fft_ens(true, f.data(), (int)f.size(), s));
     EXOTX_TRY(tc_ens_run(v.data(), (int)v.size(), 1, e->jobs[1], e->njobs[1], e->smem[1], e->nprod, s));
@@ -232,6 +231,10 @@ EXOTX_API exotx_status exotx_ensemble_tune(exotx_ensemble e, const float *spin, 
                 for (int d = 0; d < 2 && st == EXOTX_OK; d++) {
                     st = exotx_ensemble_configure(e, qi[a], uv[b], so[c], np[d]);
                     if (st != EXOTX_OK) break;
+                    // tiles, order and split belong to the tcgen05 kernels: without a job of
+                    // theirs every candidate is the same, and only the default is timed
+                    if (e->njobs[0] + e->njobs[1] == 0 && (qi[a] != best[0] || uv[b] != best[1] || !so[c] || np[d] != 6))
+                        continue;
                     // warm-up and accuracy against the reference (relative L2, both halves)
                     st = ens_inverse(e, spin, gpout, s);
                     if (st == EXOTX_OK) st = ens_forward(e, gpin, spout, s);

@@ -131,19 +131,29 @@ struct FourierLayout {
 enum { OP_SP2FC = 0, OP_SP2FCDMU = 1, OP_DV2UV = 2 };
 enum { OP_FC2SP = 0, OP_UV2DV = 1, OP_QTEND = 2, OP_MKTEND = 3 };
 
-// SIMT Legendre launchers (legendre_simt.cu)
+// FP64 tensor-core Legendre launchers (legendre_fp64mma.cu)
 template <typename T>
 exotx_status leg_inverse_l(exotx_plan p, int op, const T *a, const T *b, T *oa, T *ob, int nlev,
                            long long a_fs, long long b_fs, FourierLayout L, cudaStream_t s);
 template <typename T>
 exotx_status leg_forward_l(exotx_plan p, int op, const T *const *in, T *const *out, int nlev,
                            FourierLayout L, long long o_fs, cudaStream_t s);
-// the Legendre half of a whole set in one launch, on the m-major intermediate W
-// of ninst states (dset = 0 gridpointa, 1 gridpointd)
+// the Legendre half of a set in one launch over up to TC_MAXSEG segments, a
+// resolution, a level count and a run of states each (dset = 0 gridpointa, 1
+// gridpointd, one segment): inverse spectral states -> m-major intermediate,
+// forward the reverse.  folded: the intermediate holds N+S and N-S per field
+constexpr int TC_MAXSEG = 12;  // segments per Legendre launch
+template <typename T> struct LegSeg {
+    exotx_plan p;
+    int L, ninst;
+    const T *in;
+    T *out;
+    bool folded;
+};
 template <typename T>
-exotx_status leg_inverse_set(exotx_plan p, int dset, const T *spin, T *W, int L, int ninst, cudaStream_t s);
+exotx_status leg_inverse_set(const LegSeg<T> *segs, int n, int dset, cudaStream_t s);
 template <typename T>
-exotx_status leg_forward_set(exotx_plan p, int dset, const T *W, T *spout, int L, int ninst, cudaStream_t s);
+exotx_status leg_forward_set(const LegSeg<T> *segs, int n, int dset, cudaStream_t s);
 
 // FFT launchers (fft.cu).  kf = Fourier coefficients read (inverse) or
 // written (forward) per row; the rest are zero.  Fourier side addressed as
@@ -202,7 +212,6 @@ exotx_status tc_forward_batch(exotx_plan p, const float *gpin, float *spout, int
 exotx_status tc_inverse_batch_d(exotx_plan p, const float *spin, float *gpout, int L, int ninst, cudaStream_t s);
 exotx_status tc_forward_batch_d(exotx_plan p, const float *gpin, float *spout, int L, int ninst, cudaStream_t s);
 // uneven ensembles: a segment is a run of instances of one resolution and level count
-constexpr int TC_MAXSEG = 12;  // segments per tensor-core launch
 struct EnsSeg {
     exotx_plan p;
     int L, ninst;
@@ -214,7 +223,6 @@ exotx_status tc_ens_jobs(const EnsSeg *segs, int nseg, int dir, int nc_qi_cap, i
                          int4 **d_jobs, int *njobs, size_t *smem);
 exotx_status tc_ens_run(const EnsSeg *segs, int nseg, int dir, const int4 *d_jobs, int njobs, size_t smem,
                         int nprod, cudaStream_t s);
-bool tc_ens_fwd_folded(const EnsSeg *segs, int nseg);
 exotx_status tc_ens_n0(const EnsSeg *segs, const float *const *gpin, int nseg, cudaStream_t s);
 // FP32-accurate GEMM on the tensor cores (tc_gemm.cu): C = A B (+ bias), A(m,k) = A[m*am + k*ak],
 // B(k,n) = B[k*bk + n*bn]; work: tc_sgemm_work(M, N, K) floats (0: none needed)

@@ -95,6 +95,21 @@ struct LegInv {
     double plavor;
 };
 
+// One launch covers up to NSEG segments (a resolution, a level count and a run
+// of states each); segment i's blocks start at blk0[i]
+template <typename A, int NSEG>
+struct LegLaunch {
+    A seg[NSEG];
+    int blk0[NSEG];
+    int nseg;
+    __device__ __forceinline__ int find(int b) const {
+        int i = 0;
+        if constexpr (NSEG > 1)
+            while (i + 1 < nseg && b >= blk0[i + 1]) i++;
+        return i;
+    }
+};
+
 // field maps of the sets: gridpointa takes sd[L] st[L] sz[L] sq[L] sp to
 // gu gv gt gd gz gq gpj gpmt gp (6L+3 fields), gridpointd the same state to
 // gu gv gt gq gp (4L+1).  Unit u of group 0 -> instance, input and output field
@@ -114,13 +129,15 @@ __device__ __forceinline__ void inv_field(int L, int dset, int u, int *inst, int
 // A warp: MT tiles of 8 latitudes x NT groups of 4 complex columns (group 2:
 // x 4 (D, Z) pairs), both parities of n-m in separate accumulators.  A step is
 // 8 modes: a tile's fragments of both parities are one 16-byte load per lane.
-template <typename T, int MT, int NT, bool SET>
-__global__ void __launch_bounds__(192, NT == 1 ? 2 : 4) k_leg_inv(const __grid_constant__ LegInv<T> A) {
+template <typename T, int MT, int NT, bool SET, int NSEG>
+__global__ void __launch_bounds__(192, NT == 1 ? 2 : 4) k_leg_inv(const __grid_constant__ LegLaunch<LegInv<T>, NSEG> P) {
+    const int seg = P.find(blockIdx.x), blk = blockIdx.x - P.blk0[seg];
+    const LegInv<T> &A = P.seg[seg];
     constexpr bool PF = NT == 1;   // fetch a step ahead: few warps to hide the latency
     extern __shared__ __align__(16) unsigned char smraw[];
     double *xs = reinterpret_cast<double *>(smraw);
-    int ti = blockIdx.x % A.ntiles, g = 0;
-    const int mb = blockIdx.x / A.ntiles, m = mb / A.nlb, lb = mb - m * A.nlb;
+    int ti = blk % A.ntiles, g = 0;
+    const int mb = blk / A.ntiles, m = mb / A.nlb, lb = mb - m * A.nlb;
     while (ti >= A.nt[g]) ti -= A.nt[g++];
     const int cb = (g == 2 ? 4 : 4 * NT) * A.wn, u0 = ti * cb, n = min(cb, A.nu[g] - u0);
     const int nlat = A.nlat, nlath = A.nlath;
@@ -143,7 +160,7 @@ __global__ void __launch_bounds__(192, NT == 1 ? 2 : 4) k_leg_inv(const __grid_c
     const int wn = warp / A.wm, wm = warp - wn * A.wm;
     const int cw = wn * (g == 2 ? 4 : 4 * NT);                       // the warp's first column of the block
     const int j0 = (lb * A.wm + wm) * 8 * MT;
-    const bool active = cw < n && j0 < nlath;
+    const bool active = wn < A.wn && cw < n && j0 < nlath;
     // fragment pairs of the warp's tiles, step by step (tiles past the last repeat it)
     const size_t sstr = (size_t)A.ntl * 32;
     const double2 *t0 = A.tab + (g == 0 ? INV_QI : g == 1 ? INV_QJ : INV_QU) * A.tsz + A.ioff[m] * sstr + lane;
@@ -214,9 +231,9 @@ __global__ void __launch_bounds__(192, NT == 1 ? 2 : 4) k_leg_inv(const __grid_c
                 for (int i = 0; i < MT; i++) t[i] = tk[to[i]];
                 tk += sstr;
             };
-            auto step = [&](const double2 (&t)[MT]) {
+            auto step = [&](const double2 (&t)[MT], auto nc) {
 #pragma unroll
-                for (int c = 0; c < NT; c++) {
+                for (int c = 0; c < decltype(nc)::value; c++) {
                     const double b0 = x0[8 * c], b1 = x1[8 * c];
 #pragma unroll
                     for (int i = 0; i < MT; i++) {
@@ -231,13 +248,15 @@ __global__ void __launch_bounds__(192, NT == 1 ? 2 : 4) k_leg_inv(const __grid_c
                 fetch(fa);
                 for (int st = 0; st < nst; st += 2) {
                     if (st + 1 < nst) fetch(fb);
-                    step(fa);
+                    step(fa, std::integral_constant<int, NT>{});
                     if (st + 1 >= nst) break;
                     if (st + 2 < nst) fetch(fa);
-                    step(fb);
+                    step(fb, std::integral_constant<int, NT>{});
                 }
-            } else {
-                for (int st = 0; st < nst; st++) { fetch(fa); step(fa); }
+            } else if (cw + 4 < n) {
+                for (int st = 0; st < nst; st++) { fetch(fa); step(fa, std::integral_constant<int, NT>{}); }
+            } else {   // the block's last columns: one group
+                for (int st = 0; st < nst; st++) { fetch(fa); step(fa, std::integral_constant<int, 1>{}); }
             }
         } else {
             // u = sum qv*Z - i*qu*D ; v = sum -i*qu*Z - qv*D  (legmod.f90:338-341)
@@ -367,6 +386,7 @@ struct LegFwd {
     long long fs, ls, ms, nrows;
     T *out[3];               // single op: spectral outputs; set: out[0] is the set's output
     long long o_fs;          // spectral field stride (reals)
+    int folded;              // the intermediate holds N+S, then N-S per field (rfft_fwd_fold_body)
     int nu, nt;              // units (levels x states) and unit tiles per wavenumber
     int nu1, nt1;            // gridpointa: ln ps tendencies (fc2sp) and their tiles
     int wb, nmb;             // warps along the modes of a block; mode blocks per wavenumber
@@ -386,11 +406,11 @@ struct __align__(32) FwdFrag { double c, e, m, q; };
 
 // Four latitude pairs' terms.  V(i, type, rot) is input i's fragment of the
 // parity that P-type (0) or Q-type (1) tables pair with, or (rot) i times it
-template <int OP, int MT, typename Val>
+template <int OP, int NTILE, int MT, typename Val>
 __device__ __forceinline__ void fwd_terms(double (*o)[FwdShape<OP>::nout][2], const FwdFrag (&t)[MT], Val V) {
     auto add = [&](int x, double FwdFrag::*a, double b) {
 #pragma unroll
-        for (int i = 0; i < MT; i++) dmma(o[i][x], t[i].*a, b);
+        for (int i = 0; i < NTILE; i++) dmma(o[i][x], t[i].*a, b);
     };
     if constexpr (OP == OP_FC2SP) {          // sp = sum qc*f  (legmod.f90:203-220)
         add(0, &FwdFrag::c, V(0, 0, 0));
@@ -446,9 +466,10 @@ __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, double *sm, in
     for (int i = 0; i < MT; i++) to[i] = active ? min(kt0 + i, kt - 1) * 32 : 0;
     if (active) tb += (size_t)A.foff[2 * m + p] * 32 + lane;
     const int tstr = kt * 32;
-    auto fetch = [&](FwdFrag (&t)[MT]) {
+    auto fetch = [&](FwdFrag (&t)[MT], int ntile) {
 #pragma unroll
         for (int i = 0; i < MT; i++) {
+            if (i >= ntile) break;
             const double2 *f = reinterpret_cast<const double2 *>(tb + to[i]);
             const double2 ce = f[0];
             t[i].c = ce.x; t[i].e = ce.y;
@@ -463,6 +484,7 @@ __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, double *sm, in
     const T *pn[FWD_ITEMS];
     int so[FWD_ITEMS], je[FWD_ITEMS];
     const long long ls = SET ? 1 : A.ls;
+    const bool folded = SET && A.folded;
 #pragma unroll
     for (int e = 0; e < FWD_ITEMS; e++) {
         const int idx = threadIdx.x + e * blockDim.x, jj = idx % FWD_JC, rr = idx / FWD_JC, ul = rr & 3, i = rr >> 2, u = u0 + ul;
@@ -483,42 +505,48 @@ __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, double *sm, in
             pn[e] = A.in[i] + 2 * (u * A.fs + (long long)m * A.ms);
         }
     }
-    auto load = [&](int j0) {
+    auto load = [&](int j0, int ring) {
 #pragma unroll
         for (int e = 0; e < FWD_ITEMS; e++) {
+            if (so[e] < 0 || j0 >= nlath) continue;
             const int j = j0 + je[e];
-            C2<T> *d = raw + 2 * e * blockDim.x;
+            C2<T> *d = raw + 2 * (ring * FWD_ITEMS + e) * blockDim.x;
             const bool ok = j < nlath;   // zeros otherwise
             cp_complex<SET>(d, pn[e] + (ok ? 2 * (j * ls) : 0), ok);
-            cp_complex<SET>(d + blockDim.x, pn[e] + (ok ? 2 * ((nlat - 1 - j) * ls) : 0), ok);
+            cp_complex<SET>(d + blockDim.x, pn[e] + (ok ? 2 * ((folded ? nlath + j : nlat - 1 - j) * ls) : 0), ok);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto fold = [&] {
-        asm volatile("cp.async.wait_all;" ::: "memory");
+    auto fold = [&](int ring) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
 #pragma unroll
         for (int e = 0; e < FWD_ITEMS; e++) {
             if (so[e] < 0) continue;
-            const C2<T> vn = raw[2 * e * blockDim.x], vs = raw[(2 * e + 1) * blockDim.x];
+            const C2<T> *v = raw + 2 * (ring * FWD_ITEMS + e) * blockDim.x;
+            const C2<T> vn = v[0], vs = v[blockDim.x];
             const double nx = vn.x, ny = vn.y, sx = vs.x, sy = vs.y;
-            *reinterpret_cast<Z2 *>(sm + so[e]) = Z2{nx + sx, ny + sy};
-            *reinterpret_cast<Z2 *>(sm + so[e] + SEL) = Z2{nx - sx, ny - sy};
+            *reinterpret_cast<Z2 *>(sm + so[e]) = folded ? Z2{nx, ny} : Z2{nx + sx, ny + sy};
+            *reinterpret_cast<Z2 *>(sm + so[e] + SEL) = folded ? Z2{sx, sy} : Z2{nx - sx, ny - sy};
         }
     };
     const int nl4 = (nlath + 3) & ~3;
     constexpr bool PF = MT == 1;   // fetch a step ahead: few warps to hide the latency
     FwdFrag ta[MT], tn[MT];
-    load(0);
-    if (PF && active) fetch(tn);
+    load(0, 0);
+    load(FWD_JC, 1);
+    if (PF && active) fetch(tn, 1);
     // P-type tables see the sum on even n-m and the difference on odd, Q-type
     // the reverse; the partner column (re <-> im) for i*x: re <- -im, im <- re
     const double *bp = sm + q * rs + r + (p ? SEL : 0), *bq = sm + q * rs + r + (p ? 0 : SEL);
     const int sw = (r ^ 1) - r;
     const double sg = (r & 1) ? 1.0 : -1.0;
-    for (int j0 = 0; j0 < nlath; j0 += FWD_JC) {
-        fold();
+    for (int j0 = 0, ring = 0; j0 < nlath; j0 += FWD_JC, ring ^= 1) {
+        fold(ring);
         __syncthreads();
-        if (j0 + FWD_JC < nlath) load(j0 + FWD_JC);
-        if (active) {
+        load(j0 + 2 * FWD_JC, ring);   // two chunks ahead
+        // the chunk's steps over the warp's tiles (the last warp of a parity may hold one of MT = 2)
+        auto steps = [&](auto nt) {
+            constexpr int NTILE = decltype(nt)::value;
             const double *xp = bp, *xq = bq;
             const int jn = min(FWD_JC, nl4 - j0);
 #pragma unroll 1
@@ -526,17 +554,21 @@ __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, double *sm, in
                 if constexpr (PF) {
 #pragma unroll
                     for (int i = 0; i < MT; i++) ta[i] = tn[i];
-                    if (j0 + jj + 4 < nl4) fetch(tn);
+                    if (j0 + jj + 4 < nl4) fetch(tn, NTILE);
                 } else {
-                    fetch(ta);
+                    fetch(ta, NTILE);
                 }
-                fwd_terms<OP, MT>(o, ta, [&](int i, int type, int rot) {
+                fwd_terms<OP, NTILE>(o, ta, [&](int i, int type, int rot) {
                     const double *x = (type ? xq : xp) + 2 * i * SEL;
                     return rot ? sg * x[sw] : x[0];
                 });
                 xp += 4 * rs;
                 xq += 4 * rs;
             }
+        };
+        if (active) {
+            if (MT == 1 || kt0 + 1 >= kt) steps(std::integral_constant<int, 1>{});
+            else steps(std::integral_constant<int, MT>{});
         }
         __syncthreads();
     }
@@ -564,16 +596,21 @@ __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, double *sm, in
     }
 }
 
-template <typename T, int OP, int MT, bool SET>
-__global__ void __launch_bounds__(384, MT == 1 ? 1 : 2) k_leg_fwd(const __grid_constant__ LegFwd<T> A) {
+template <typename T, int OP, int MT, bool SET, int NSEG>
+__global__ void __launch_bounds__(384, MT == 1 ? 1 : 2) k_leg_fwd(const __grid_constant__ LegLaunch<LegFwd<T>, NSEG> P) {
+    const int seg = P.find(blockIdx.x), blk = blockIdx.x - P.blk0[seg];
+    const LegFwd<T> &A = P.seg[seg];
     extern __shared__ __align__(16) unsigned char smraw[];
     double *sm = reinterpret_cast<double *>(smraw);
-    const int nt = A.nt + A.nt1, mb = blockIdx.x / nt, ti = blockIdx.x - mb * nt;
+    const int nt = A.nt + A.nt1, mb = blk / nt, ti = blk - mb * nt;
     const int m = mb / A.nmb, mblk = mb - m * A.nmb;
     pdl_trigger();
     pdl_wait();
     if (ti < A.nt) {
-        leg_fwd_block<T, OP, MT, SET>(A, sm, m, mblk, 4 * ti, min(4, A.nu - 4 * ti));
+        // where one tile per warp suffices (the larger half of the wavenumbers) every warp of the block works
+        const int K = A.ntp1 - m, tiles = (((K + 1) >> 1) + 7) / 8 + ((K >> 1) + 7) / 8;
+        if (MT > 1 && tiles <= A.wb) leg_fwd_block<T, OP, 1, SET>(A, sm, m, mblk, 4 * ti, min(4, A.nu - 4 * ti));
+        else leg_fwd_block<T, OP, MT, SET>(A, sm, m, mblk, 4 * ti, min(4, A.nu - 4 * ti));
     } else if constexpr (OP == OP_LEVEL_A) {
         const int u0 = 4 * (ti - A.nt);
         leg_fwd_block<T, OP_FC2SP, MT, SET>(A, sm, m, mblk, u0, min(4, A.nu1 - u0));
@@ -582,46 +619,65 @@ __global__ void __launch_bounds__(384, MT == 1 ? 1 : 2) k_leg_fwd(const __grid_c
 
 // ------------------------------------------------------------ host launchers
 // Both directions take the larger warp tile where that still leaves LEG_WARPS
-// warps (about 8 per SM), and the smaller one otherwise.
+// warps (about 8 per SM; twice that for the inverse, whose larger tile does not
+// fetch ahead), and the smaller one otherwise.  T42 L20, one state: inverse
+// 13 us with the smaller tile, 16 with the larger; T85 L13 x3: 33 and 29.
 constexpr long long LEG_WARPS = 1200;
 
-template <typename T, int MT, int NT, bool SET>
-static exotx_status inv_launch_t(exotx_plan p, LegInv<T> &A, cudaStream_t s) {
-    const int lt = (p->nlath + 8 * MT - 1) / (8 * MT);   // latitude warps
-    A.nlb = (lt + 3) / 4;
-    A.wm = (lt + A.nlb - 1) / A.nlb;
-    A.wn = 6 / A.wm;
-    // the staged columns of a block: all modes at once where they fit the budget
-    auto smem_of = [&](int kc, int wn) {
-        const size_t one = (size_t)kc * leg_stride(8 * NT * wn), two = A.nu[2] ? 2 * (size_t)kc * leg_stride(8 * wn) : 0;
-        return std::max(one, two) * sizeof(double);
-    };
-    A.kc = (p->ntp1 + 7) & ~7;
-    while (A.wn > 1 && smem_of(A.kc, A.wn) > 72 * 1024) A.wn--;
-    if (smem_of(A.kc, A.wn) > 96 * 1024) A.kc = 256;
-    const size_t smem = smem_of(A.kc, A.wn);
-    const int cb[3] = {4 * NT * A.wn, 4 * NT * A.wn, 4 * A.wn};
-    A.ntiles = 0;
-    for (int g = 0; g < 3; g++) A.ntiles += A.nt[g] = (A.nu[g] + cb[g] - 1) / cb[g];
-    const int nm = p->ntp1 + (!SET && A.mz > p->ntp1 ? 1 : 0);
-    const long long blocks = (long long)nm * A.nlb * A.ntiles;
-    if (blocks > 0x7fffffffLL || smem > LEG_MAXSMEM) return EXOTX_BAD_DIM;
-    auto kern = k_leg_inv<T, MT, NT, SET>;
+// one segment to launch: its plan and its arguments, completed by the launcher
+template <typename A> struct LegItem { exotx_plan p; A a; };
+
+template <typename T, int MT, int NT, bool SET, int NSEG>
+static exotx_status inv_launch_t(LegItem<LegInv<T>> *it, int n, cudaStream_t s) {
+    LegLaunch<LegInv<T>, NSEG> P;
+    P.nseg = n;
+    size_t smem = 0;
+    int threads = 0;
+    long long blocks = 0;
+    for (int i = 0; i < n; i++) {
+        exotx_plan p = it[i].p;
+        LegInv<T> &A = P.seg[i] = it[i].a;
+        A.tab = reinterpret_cast<const double2 *>(p->d_inv64); A.ioff = p->d_ioff; A.tsz = p->inv_tsz;
+        A.woff = p->d_woff; A.filt = p->d_fs64;
+        A.nlat = p->nlat; A.nlath = p->nlath; A.ntl = (p->nlath + 7) / 8; A.ntp1 = p->ntp1; A.nrsp = 2 * p->ncsp;
+        A.plavor = p->desc.plavor;
+        const int lt = (p->nlath + 8 * MT - 1) / (8 * MT);   // latitude warps
+        A.nlb = (lt + 3) / 4;
+        A.wm = (lt + A.nlb - 1) / A.nlb;
+        A.wn = 6 / A.wm;
+        // the staged columns of a block: all modes at once where they fit the budget
+        auto smem_of = [&](int kc, int wn) {
+            const size_t one = (size_t)kc * leg_stride(8 * NT * wn), two = A.nu[2] ? 2 * (size_t)kc * leg_stride(8 * wn) : 0;
+            return std::max(one, two) * sizeof(double);
+        };
+        A.kc = (p->ntp1 + 7) & ~7;
+        while (A.wn > 1 && smem_of(A.kc, A.wn) > 72 * 1024) A.wn--;
+        if (smem_of(A.kc, A.wn) > 96 * 1024) A.kc = 256;
+        smem = std::max(smem, smem_of(A.kc, A.wn));
+        threads = std::max(threads, 32 * A.wm * A.wn);
+        const int cb[3] = {4 * NT * A.wn, 4 * NT * A.wn, 4 * A.wn};
+        A.ntiles = 0;
+        for (int g = 0; g < 3; g++) A.ntiles += A.nt[g] = (A.nu[g] + cb[g] - 1) / cb[g];
+        P.blk0[i] = (int)blocks;
+        blocks += (long long)(p->ntp1 + (!SET && A.mz > p->ntp1 ? 1 : 0)) * A.nlb * A.ntiles;
+        if (blocks > 0x7fffffffLL) return EXOTX_BAD_DIM;
+    }
+    if (smem > LEG_MAXSMEM) return EXOTX_BAD_DIM;
+    auto kern = k_leg_inv<T, MT, NT, SET, NSEG>;
     if (smem > 48 * 1024) EXOTX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LEG_MAXSMEM));
     cudaEvent_t ev = ktimer_start(EXOTX_K_LEG_INVERSE, s);
-    EXOTX_CUDA(launch_pdl(kern, dim3((unsigned)blocks), dim3(32 * A.wm * A.wn), smem, s, A));
+    EXOTX_CUDA(launch_pdl(kern, dim3((unsigned)blocks), dim3(threads), smem, s, P));
     EXOTX_CHECK_LAUNCH();
     ktimer_stop(EXOTX_K_LEG_INVERSE, s, ev);
     return EXOTX_OK;
 }
-template <typename T, bool SET>
-static exotx_status inv_launch(exotx_plan p, LegInv<T> &A, cudaStream_t s) {
-    A.tab = reinterpret_cast<const double2 *>(p->d_inv64); A.ioff = p->d_ioff; A.tsz = p->inv_tsz;
-    A.woff = p->d_woff; A.filt = p->d_fs64;
-    A.nlat = p->nlat; A.nlath = p->nlath; A.ntl = (p->nlath + 7) / 8; A.ntp1 = p->ntp1; A.nrsp = 2 * p->ncsp;
-    A.plavor = p->desc.plavor;
-    const long long tiles = (long long)p->ntp1 * A.ntl * ((A.nu[0] + A.nu[1]) / 4 + A.nu[2] / 2 + 1);
-    return tiles / 4 >= LEG_WARPS ? inv_launch_t<T, 2, 2, SET>(p, A, s) : inv_launch_t<T, 2, 1, SET>(p, A, s);
+template <typename T, bool SET, int NSEG>
+static exotx_status inv_launch(LegItem<LegInv<T>> *it, int n, cudaStream_t s) {
+    long long tiles = 0;
+    for (int i = 0; i < n; i++)
+        tiles += (long long)it[i].p->ntp1 * ((it[i].p->nlath + 7) / 8) *
+                 ((it[i].a.nu[0] + it[i].a.nu[1]) / 4 + it[i].a.nu[2] / 2 + 1);
+    return tiles / 4 >= 2 * LEG_WARPS ? inv_launch_t<T, 2, 2, SET, NSEG>(it, n, s) : inv_launch_t<T, 2, 1, SET, NSEG>(it, n, s);
 }
 
 template <typename T>
@@ -629,61 +685,82 @@ exotx_status leg_inverse_l(exotx_plan p, int op, const T *a, const T *b, T *oa, 
                            long long a_fs, long long b_fs, FourierLayout L, cudaStream_t s) {
     if (nlev <= 0) return EXOTX_OK;
     if (op != OP_SP2FC && op != OP_SP2FCDMU && op != OP_DV2UV) return EXOTX_BAD_ARG;
-    LegInv<T> A = {};
+    LegItem<LegInv<T>> it = {p, {}};
+    LegInv<T> &A = it.a;
     A.a = a; A.b = b; A.a_fs = a_fs; A.b_fs = b_fs;
     A.oa = oa; A.ob = ob; A.fs = L.fs; A.ls = L.ls; A.ms = L.ms; A.mz = L.mz;
     A.nu[op == OP_SP2FC ? 0 : op == OP_SP2FCDMU ? 1 : 2] = nlev;
-    return inv_launch<T, false>(p, A, s);
+    return inv_launch<T, false, 1>(&it, 1, s);
 }
 
 template <typename T>
-exotx_status leg_inverse_set(exotx_plan p, int dset, const T *spin, T *W, int L, int ninst, cudaStream_t s) {
-    LegInv<T> A = {};
-    A.a = spin;
-    A.oa = W;
-    A.L = L; A.dset = dset;
-    A.nrows = (long long)ninst * (dset ? 4 * L + 1 : 6 * L + 3) * p->nlat;
-    A.nu[0] = ninst * (dset ? 2 * L + 1 : 4 * L + 1);
-    A.nu[1] = dset ? 0 : ninst;
-    A.nu[2] = ninst * L;
-    return inv_launch<T, true>(p, A, s);
+exotx_status leg_inverse_set(const LegSeg<T> *segs, int n, int dset, cudaStream_t s) {
+    if (n < 1 || n > TC_MAXSEG) return EXOTX_BAD_ARG;
+    LegItem<LegInv<T>> it[TC_MAXSEG];
+    for (int i = 0; i < n; i++) {
+        const LegSeg<T> &g = segs[i];
+        it[i] = {g.p, {}};
+        LegInv<T> &A = it[i].a;
+        A.a = g.in;
+        A.oa = g.out;
+        A.L = g.L; A.dset = dset;
+        A.nrows = (long long)g.ninst * (dset ? 4 * g.L + 1 : 6 * g.L + 3) * g.p->nlat;
+        A.nu[0] = g.ninst * (dset ? 2 * g.L + 1 : 4 * g.L + 1);
+        A.nu[1] = dset ? 0 : g.ninst;
+        A.nu[2] = g.ninst * g.L;
+    }
+    if (n == 1) return inv_launch<T, true, 1>(it, n, s);
+    if constexpr (sizeof(T) == 4) return inv_launch<T, true, TC_MAXSEG>(it, n, s);   // ensembles are float
+    return EXOTX_BAD_ARG;
 }
 
-template <typename T, int OP, int MT, bool SET>
-static exotx_status fwd_launch_t(exotx_plan p, LegFwd<T> &A, cudaStream_t s) {
-    const int K0 = (p->ntp1 + 1) / 2, K1 = p->ntp1 / 2;
-    const int nw = (K0 + 8 * MT - 1) / (8 * MT) + (K1 + 8 * MT - 1) / (8 * MT);   // mode warps at m = 0
-    A.nmb = (nw + 11) / 12;
-    A.wb = (nw + A.nmb - 1) / A.nmb;
-    const int threads = std::max(FWD_THREADS, 32 * A.wb);
-    // one operand chunk and the copies on their way
+template <typename T, int OP, int MT, bool SET, int NSEG>
+static exotx_status fwd_launch_t(LegItem<LegFwd<T>> *it, int n, cudaStream_t s) {
+    LegLaunch<LegFwd<T>, NSEG> P;
+    P.nseg = n;
+    int threads = FWD_THREADS;
+    long long blocks = 0;
+    for (int i = 0; i < n; i++) {
+        exotx_plan p = it[i].p;
+        LegFwd<T> &A = P.seg[i] = it[i].a;
+        A.tab = reinterpret_cast<const double4 *>(p->d_fwd64); A.foff = p->d_foff; A.woff = p->d_woff; A.filt = p->d_fg64;
+        A.nlat = p->nlat; A.nlath = p->nlath; A.ntp1 = p->ntp1;
+        const int K0 = (p->ntp1 + 1) / 2, K1 = p->ntp1 / 2;
+        const int nw = (K0 + 8 * MT - 1) / (8 * MT) + (K1 + 8 * MT - 1) / (8 * MT);   // mode warps at m = 0
+        A.nmb = (nw + 11) / 12;
+        A.wb = (nw + A.nmb - 1) / A.nmb;
+        threads = std::max(threads, 32 * A.wb);
+        A.nt = (A.nu + 3) / 4;
+        A.nt1 = (A.nu1 + 3) / 4;
+        P.blk0[i] = (int)blocks;
+        blocks += (long long)p->ntp1 * A.nmb * (A.nt + A.nt1);
+        if (blocks > 0x7fffffffLL) return EXOTX_BAD_DIM;
+    }
+    // one operand chunk and two chunks of copies on their way
     const size_t smem = (size_t)FwdShape<OP>::nin * 2 * FWD_JC * leg_stride(8) * sizeof(double) +
-                        (size_t)FWD_ITEMS * 2 * threads * sizeof(C2<T>);
-    A.nt = (A.nu + 3) / 4;
-    A.nt1 = (A.nu1 + 3) / 4;
-    const long long blocks = (long long)p->ntp1 * A.nmb * (A.nt + A.nt1);
-    if (blocks > 0x7fffffffLL || smem > LEG_MAXSMEM) return EXOTX_BAD_DIM;
-    auto kern = k_leg_fwd<T, OP, MT, SET>;
+                        (size_t)FWD_ITEMS * 4 * threads * sizeof(C2<T>);
+    if (smem > LEG_MAXSMEM) return EXOTX_BAD_DIM;
+    auto kern = k_leg_fwd<T, OP, MT, SET, NSEG>;
     if (smem > 48 * 1024) EXOTX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LEG_MAXSMEM));
     cudaEvent_t ev = ktimer_start(EXOTX_K_LEG_FORWARD, s);
-    EXOTX_CUDA(launch_pdl(kern, dim3((unsigned)blocks), dim3(threads), smem, s, A));
+    EXOTX_CUDA(launch_pdl(kern, dim3((unsigned)blocks), dim3(threads), smem, s, P));
     EXOTX_CHECK_LAUNCH();
     ktimer_stop(EXOTX_K_LEG_FORWARD, s, ev);
     return EXOTX_OK;
 }
-template <typename T, int OP, bool SET>
-static exotx_status fwd_launch(exotx_plan p, LegFwd<T> &A, cudaStream_t s) {
-    A.tab = reinterpret_cast<const double4 *>(p->d_fwd64); A.foff = p->d_foff; A.woff = p->d_woff; A.filt = p->d_fg64;
-    A.nlat = p->nlat; A.nlath = p->nlath; A.ntp1 = p->ntp1;
-    const long long tiles = (long long)(p->ncsp / 8 + p->ntp1) * ((A.nu + 3) / 4);
-    return tiles / 2 >= LEG_WARPS ? fwd_launch_t<T, OP, 2, SET>(p, A, s) : fwd_launch_t<T, OP, 1, SET>(p, A, s);
+template <typename T, int OP, bool SET, int NSEG>
+static exotx_status fwd_launch(LegItem<LegFwd<T>> *it, int n, cudaStream_t s) {
+    long long tiles = 0;
+    for (int i = 0; i < n; i++) tiles += (long long)(it[i].p->ncsp / 8 + it[i].p->ntp1) * ((it[i].a.nu + 3) / 4);
+    return tiles / 2 >= LEG_WARPS ? fwd_launch_t<T, OP, 2, SET, NSEG>(it, n, s) : fwd_launch_t<T, OP, 1, SET, NSEG>(it, n, s);
 }
 
 template <typename T>
 exotx_status leg_forward_l(exotx_plan p, int op, const T *const *in, T *const *out, int nlev,
                            FourierLayout L, long long o_fs, cudaStream_t s) {
     if (nlev <= 0) return EXOTX_OK;
-    LegFwd<T> A = {};
+    LegItem<LegFwd<T>> it = {p, {}};
+    LegFwd<T> &A = it.a;
     const int nin = op == OP_FC2SP ? 1 : op == OP_UV2DV ? 2 : op == OP_QTEND ? 3 : 6;
     const int nout = op == OP_MKTEND ? 3 : op == OP_UV2DV ? 2 : 1;
     for (int i = 0; i < nin; i++) A.in[i] = in[i];
@@ -691,25 +768,37 @@ exotx_status leg_forward_l(exotx_plan p, int op, const T *const *in, T *const *o
     A.fs = L.fs; A.ls = L.ls; A.ms = L.ms; A.o_fs = o_fs;
     A.nu = nlev;
     switch (op) {
-        case OP_FC2SP: return fwd_launch<T, OP_FC2SP, false>(p, A, s);
-        case OP_UV2DV: return fwd_launch<T, OP_UV2DV, false>(p, A, s);
-        case OP_QTEND: return fwd_launch<T, OP_QTEND, false>(p, A, s);
-        case OP_MKTEND: return fwd_launch<T, OP_MKTEND, false>(p, A, s);
+        case OP_FC2SP: return fwd_launch<T, OP_FC2SP, false, 1>(&it, 1, s);
+        case OP_UV2DV: return fwd_launch<T, OP_UV2DV, false, 1>(&it, 1, s);
+        case OP_QTEND: return fwd_launch<T, OP_QTEND, false, 1>(&it, 1, s);
+        case OP_MKTEND: return fwd_launch<T, OP_MKTEND, false, 1>(&it, 1, s);
     }
     return EXOTX_BAD_ARG;
 }
 
 template <typename T>
-exotx_status leg_forward_set(exotx_plan p, int dset, const T *W, T *spout, int L, int ninst, cudaStream_t s) {
-    LegFwd<T> A = {};
-    A.in[0] = W;
-    A.out[0] = spout;
-    A.o_fs = 2LL * p->ncsp;
-    A.L = L;
-    A.nrows = (long long)ninst * (dset ? 4 * L : 9 * L + 1) * p->nlat;
-    A.nu = ninst * L;
-    A.nu1 = dset ? 0 : ninst;
-    return dset ? fwd_launch<T, OP_LEVEL_D, true>(p, A, s) : fwd_launch<T, OP_LEVEL_A, true>(p, A, s);
+exotx_status leg_forward_set(const LegSeg<T> *segs, int n, int dset, cudaStream_t s) {
+    if (n < 1 || n > TC_MAXSEG) return EXOTX_BAD_ARG;
+    LegItem<LegFwd<T>> it[TC_MAXSEG];
+    for (int i = 0; i < n; i++) {
+        const LegSeg<T> &g = segs[i];
+        it[i] = {g.p, {}};
+        LegFwd<T> &A = it[i].a;
+        A.in[0] = g.in;
+        A.out[0] = g.out;
+        A.o_fs = 2LL * g.p->ncsp;
+        A.L = g.L;
+        A.folded = g.folded;
+        A.nrows = (long long)g.ninst * (dset ? 4 * g.L : 9 * g.L + 1) * g.p->nlat;
+        A.nu = g.ninst * g.L;
+        A.nu1 = dset ? 0 : g.ninst;
+    }
+    if (n > 1) {
+        if constexpr (sizeof(T) == 4)
+            if (!dset) return fwd_launch<T, OP_LEVEL_A, true, TC_MAXSEG>(it, n, s);
+        return EXOTX_BAD_ARG;
+    }
+    return dset ? fwd_launch<T, OP_LEVEL_D, true, 1>(it, n, s) : fwd_launch<T, OP_LEVEL_A, true, 1>(it, n, s);
 }
 
 #define LEG_INSTANCES(T)                                                                                            \
@@ -717,8 +806,8 @@ exotx_status leg_forward_set(exotx_plan p, int dset, const T *W, T *spout, int L
                                            long long, FourierLayout, cudaStream_t);                                 \
     template exotx_status leg_forward_l<T>(exotx_plan, int, const T *const *, T *const *, int, FourierLayout,       \
                                            long long, cudaStream_t);                                                \
-    template exotx_status leg_inverse_set<T>(exotx_plan, int, const T *, T *, int, int, cudaStream_t);              \
-    template exotx_status leg_forward_set<T>(exotx_plan, int, const T *, T *, int, int, cudaStream_t);
+    template exotx_status leg_inverse_set<T>(const LegSeg<T> *, int, int, cudaStream_t);                            \
+    template exotx_status leg_forward_set<T>(const LegSeg<T> *, int, int, cudaStream_t);
 LEG_INSTANCES(double)
 LEG_INSTANCES(float)
 

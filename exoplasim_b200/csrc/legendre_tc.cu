@@ -104,25 +104,33 @@ __global__ void __launch_bounds__(128) k_tc_selftest(const float *A, const float
 static const int kInvRef[4] = {0, 1, 6, 7};
 static const int kFwdRef[4] = {2, 3, 4, 5};
 
+// Which kernels a mixed set's contractions run on.  The tcgen05 kernels work in
+// tiles of 128 rows and six split products per term, so they need long
+// contractions: at T42 their forward tile is 37% full.  The FP64 tensor cores
+// (legendre_fp64mma.cu, 8-row tiles, one product, the float arrays' values exact
+// in FP64) take the rest.  Microseconds per launch, tcgen05 / FP64, L20 (T170:
+// L25) with 8 states (T170: one):
+//            T42       T63       T85       T106      T127      T170
+//   inverse  54 / 27   77 / 58   108 / 93  142 / 218 180 / 299 73 / 95
+//   forward  85 / 29   131 / 62  172 / 121 244 / 224 312 / 365 541 / 147
+//   d-set    87 / 23   131 / 50  170 / 81  238 / 155 305 / 235 522 / 110
+// (d-set: the gridpointd forward half, whose tcgen05 jobs would carry empty
+// columns; T170 forward: another tcgen05 kernel, no longer built.)
+static bool tc_inv(exotx_plan p) { return p->ntp1 > 96; }
+static bool tc_fwd(exotx_plan p) { return p->ntp1 > 112 && p->ntp1 <= 128; }
+
 struct TcTables {
     int nj8;                          // inverse rows: latitude pairs rounded up to 8
     int njc;                          // forward K extent: latitude pairs rounded up to 16
-    std::vector<long long> inv_off;   // byte offset of block (m, t), [m*4+t]
-    std::vector<int> inv_bytes;
-    std::vector<long long> fwd_off;
-    std::vector<int> fwd_bytes;
-    unsigned char *inv = nullptr, *fwd = nullptr;
-    long long *d_inv_off = nullptr, *d_fwd_off = nullptr;
-    // stacked-split forward tables (NTRU+1 <= 128): block (m, t, p) at [(m*4+t)*2+p]
-    bool has3 = false;
-    std::vector<long long> fwd3_off;
-    unsigned char *fwd3 = nullptr;
+    unsigned char *inv = nullptr;     // inverse blocks (m, t) at inv_off[m*4 + t] (tc_inv)
+    long long *d_inv_off = nullptr;
+    unsigned char *fwd3 = nullptr;    // stacked-split forward blocks (m, t, p) at [(m*4+t)*2+p] (tc_fwd)
     long long *d_fwd3_off = nullptr;
     // cached job lists, keyed by (direction, nlev, ninst)
     struct Jobs { int dir, nlev, ninst, njobs, dset; int4 *d = nullptr; };
     std::vector<Jobs> jobs;
     ~TcTables() {
-        cudaFree(inv); cudaFree(fwd); cudaFree(d_inv_off); cudaFree(d_fwd_off);
+        cudaFree(inv); cudaFree(d_inv_off);
         cudaFree(fwd3); cudaFree(d_fwd3_off);
         for (auto &j : jobs) cudaFree(j.d);
     }
@@ -170,36 +178,6 @@ __global__ void k_build_tc_inv(const double *qref, const int *woff, const long l
     }
 }
 
-// forward block (m, t) = [p][j-chunk][split][rows pad8(Kq)][chunk width] (K-major, K = j)
-__global__ void k_build_tc_fwd(const double *qref, const int *woff, const long long *off, int nlat, int nlath,
-                               int ncsp, int ntp1, int njc, int t, int tref, unsigned char *base) {
-    const int m = blockIdx.x;
-    const int K = ntp1 - m;
-    unsigned char *blk = base + off[m * 4 + t];
-    const double *q = qref + (size_t)tref * ncsp * nlat;
-    size_t poff = 0;
-    for (int p = 0; p < 2; p++) {
-        const int Kq = kpar(K, p), R = pad8(Kq);
-        if (Kq == 0) break;
-        for (int j0 = 0; j0 < njc; j0 += 32) {
-            const int jw = min(32, njc - j0);
-            const size_t tile = (size_t)R * jw * 2;
-            for (int idx = threadIdx.x; idx < R * jw; idx += blockDim.x) {
-                const int r = idx / jw, jj = idx % jw, j = j0 + jj;
-                double v = 0.0;
-                if (r < Kq && j < nlath) v = q[(size_t)j * ncsp + woff[m] + 2 * r + p];
-                __nv_bfloat16 h, mm, l;
-                split3d(v, h, mm, l);
-                const uint32_t o = tc::kmajor_off(r, jj, jw);
-                *reinterpret_cast<__nv_bfloat16 *>(blk + poff + o) = h;
-                *reinterpret_cast<__nv_bfloat16 *>(blk + poff + tile + o) = mm;
-                *reinterpret_cast<__nv_bfloat16 *>(blk + poff + 2 * tile + o) = l;
-            }
-            poff += 3 * tile;
-        }
-    }
-}
-
 // stacked-split forward block (m, t, p) = per latitude chunk of 32:
 // [S01: 2R rows (a0 of modes 0..R-1, then a1)][S2: 2R rows (zeros, then a2)] x chunk width
 __global__ void k_build_tc_fwd3(const double *qref, const int *woff, const long long *off3, int nlat, int nlath,
@@ -228,6 +206,7 @@ __global__ void k_build_tc_fwd3(const double *qref, const int *woff, const long 
     }
 }
 
+// the tables of the kernels this plan uses (tc_inv, tc_fwd)
 static exotx_status tc_tables(exotx_plan p, TcTables **out) {
     if (p->tc) { *out = p->tc; return EXOTX_OK; }
     if (p->nlath > 128) return EXOTX_BAD_DIM;  // inverse M tile = 128 latitude pairs
@@ -235,62 +214,44 @@ static exotx_status tc_tables(exotx_plan p, TcTables **out) {
     T->nj8 = pad8(p->nlath);
     T->njc = pad16(p->nlath);
     const int ntp1 = p->ntp1;
-    T->inv_off.assign(ntp1 * 4, 0);
-    T->inv_bytes.assign(ntp1 * 4, 0);
-    T->fwd_off.assign(ntp1 * 4, 0);
-    T->fwd_bytes.assign(ntp1 * 4, 0);
-    long long io = 0, fo = 0;
-    for (int m = 0; m < ntp1; m++) {
-        const int K = ntp1 - m;
-        for (int t = 0; t < 4; t++) {
-            long long bi = 0, bf = 0;
-            for (int q = 0; q < 2; q++) {
-                const int Kq = kpar(K, q);
-                if (!Kq) continue;
-                bi += 3LL * T->nj8 * pad16(Kq) * 2;
-                bf += 3LL * pad8(Kq) * T->njc * 2;
+    auto upload = [&](const std::vector<long long> &off, long long bytes, long long **d_off, unsigned char **tab) {
+        return cudaMalloc(tab, bytes) == cudaSuccess && cudaMalloc(d_off, sizeof(long long) * off.size()) == cudaSuccess &&
+               cudaMemcpy(*d_off, off.data(), sizeof(long long) * off.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+    };
+    bool ok = true;
+    if (tc_inv(p)) {
+        std::vector<long long> off(ntp1 * 4);
+        long long o = 0;
+        for (int m = 0; m < ntp1; m++)
+            for (int t = 0; t < 4; t++) {
+                off[m * 4 + t] = o;
+                for (int q = 0; q < 2; q++)
+                    if (kpar(ntp1 - m, q)) o += 3LL * T->nj8 * pad16(kpar(ntp1 - m, q)) * 2;
             }
-            T->inv_off[m * 4 + t] = io; T->inv_bytes[m * 4 + t] = (int)bi; io += bi;
-            T->fwd_off[m * 4 + t] = fo; T->fwd_bytes[m * 4 + t] = (int)bf; fo += bf;
+        ok = upload(off, o, &T->d_inv_off, &T->inv);
+        for (int t = 0; t < 4 && ok; t++) {
+            k_build_tc_inv<<<ntp1, 256>>>(p->d_qref, p->d_woff, T->d_inv_off, p->d_fs64, p->nlat, p->nlath, p->ncsp,
+                                          ntp1, T->nj8, t, kInvRef[t], T->inv);
+            note_launch();
         }
     }
-    bool ok = cudaMalloc(&T->inv, io) == cudaSuccess && cudaMalloc(&T->fwd, fo) == cudaSuccess &&
-              cudaMalloc(&T->d_inv_off, sizeof(long long) * ntp1 * 4) == cudaSuccess &&
-              cudaMalloc(&T->d_fwd_off, sizeof(long long) * ntp1 * 4) == cudaSuccess;
-    ok = ok && cudaMemcpy(T->d_inv_off, T->inv_off.data(), sizeof(long long) * ntp1 * 4, cudaMemcpyHostToDevice) ==
-                   cudaSuccess &&
-         cudaMemcpy(T->d_fwd_off, T->fwd_off.data(), sizeof(long long) * ntp1 * 4, cudaMemcpyHostToDevice) ==
-             cudaSuccess;
-    if (!ok) { delete T; return EXOTX_NO_MEM; }
-    if (ntp1 <= 128) {
-        // every parity has at most 64 modes: the stacked-split forward tables
-        T->fwd3_off.assign(ntp1 * 8, 0);
-        long long o3 = 0;
+    if (ok && tc_fwd(p)) {
+        std::vector<long long> off(ntp1 * 8);
+        long long o = 0;
         for (int m = 0; m < ntp1; m++)
             for (int t = 0; t < 4; t++)
                 for (int q = 0; q < 2; q++) {
-                    T->fwd3_off[(m * 4 + t) * 2 + q] = o3;
-                    o3 += 8LL * pad8(kpar(ntp1 - m, q)) * T->njc;
+                    off[(m * 4 + t) * 2 + q] = o;
+                    o += 8LL * pad8(kpar(ntp1 - m, q)) * T->njc;
                 }
-        T->has3 = cudaMalloc(&T->fwd3, o3) == cudaSuccess &&
-                  cudaMalloc(&T->d_fwd3_off, sizeof(long long) * ntp1 * 8) == cudaSuccess &&
-                  cudaMemcpy(T->d_fwd3_off, T->fwd3_off.data(), sizeof(long long) * ntp1 * 8,
-                             cudaMemcpyHostToDevice) == cudaSuccess;
-        if (!T->has3) { delete T; return EXOTX_NO_MEM; }
-        for (int t = 0; t < 4; t++) {
+        ok = upload(off, o, &T->d_fwd3_off, &T->fwd3);
+        for (int t = 0; t < 4 && ok; t++) {
             k_build_tc_fwd3<<<dim3(ntp1, 2), 256>>>(p->d_qref, p->d_woff, T->d_fwd3_off, p->nlat, p->nlath, p->ncsp,
                                                     ntp1, T->njc, t, kFwdRef[t], T->fwd3);
             note_launch();
         }
     }
-    for (int t = 0; t < 4; t++) {
-        k_build_tc_inv<<<ntp1, 256>>>(p->d_qref, p->d_woff, T->d_inv_off, p->d_fs64, p->nlat, p->nlath, p->ncsp,
-                                      ntp1, T->nj8, t, kInvRef[t], T->inv);
-        note_launch();
-        k_build_tc_fwd<<<ntp1, 256>>>(p->d_qref, p->d_woff, T->d_fwd_off, p->nlat, p->nlath, p->ncsp, ntp1, T->njc,
-                                      t, kFwdRef[t], T->fwd);
-        note_launch();
-    }
+    if (!ok) { delete T; return EXOTX_NO_MEM; }
     if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
         delete T;
         return EXOTX_CUDA_ERR;
@@ -343,18 +304,6 @@ static void inv_tiles(exotx_plan p, int nj8, int *nc_qi, int *nc_uv) {
     inv_tiles_full(nj8, p->ntp1, nc_qi, nc_uv);
 }
 
-// forward kernel variants, tried in order until the widest job fits shared memory:
-// 4 levels per job with both table halves resident, 4 levels with one half
-// buffer, 2 levels with one half buffer
-static const int kFwdNlt[3] = {4, 4, 2};
-static const bool kFwdOne[3] = {false, true, true};
-static int fwd_level(exotx_plan p, const TcTables *T) {
-    for (int v = 0; v < 3; v++)
-        if (fwd_smem(p->ntp1, T->njc, kFwdNlt[v], kFwdOne[v]) <= TC_SMEM_MAX) return v;
-    return -1;
-}
-// the persistent stacked-split forward kernel runs wherever its tables exist and fit
-static bool use_fwd3(const TcTables *T) { return T->has3 && fpipe_smem(T->njc) <= TC_SMEM_MAX; }
 // SMs of the current device (the grid of the persistent kernels)
 static exotx_status sm_count(int *nsm) {
     int dev = 0;
@@ -364,14 +313,14 @@ static exotx_status sm_count(int *nsm) {
     return EXOTX_OK;
 }
 // the persistent stacked-split forward kernel: one CTA per SM walks the job list
-static exotx_status launch_fwd_pipe(TcFwd3Launch &P, int njobs, int njmax, bool folded, cudaStream_t s) {
+static exotx_status launch_fwd_pipe(TcFwd3Launch &P, int njobs, int njmax, cudaStream_t s) {
     int nsm = 0;
     EXOTX_TRY(sm_count(&nsm));
     const size_t smem = std::max(fpipe_smem(njmax), kPersistSmemMin);   // one CTA per SM
     if (smem > TC_SMEM_MAX) return EXOTX_BAD_DIM;
     P.njobs = njobs;
     P.njmax = njmax;
-    auto kern = folded ? k_tc_forward_pipe<F3_NLT, true> : k_tc_forward_pipe<F3_NLT, false>;
+    auto kern = k_tc_forward_pipe<F3_NLT>;
     EXOTX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX));
     const int grid = std::max(1, std::min(njobs, nsm));
     cudaEvent_t ev = ktimer_start(EXOTX_K_TC_FORWARD, s);
@@ -401,59 +350,31 @@ static void fwd3_jobs(exotx_plan p, const TcTables *T, int L, int ninst, int seg
         }
 }
 
-static exotx_status launch_fwd(const TcFwdLaunch &P, int level, int njobs, size_t smem, cudaStream_t s) {
-    cudaEvent_t ev = nullptr;
-    if (kFwdNlt[level] == 4) {
-        EXOTX_CUDA(cudaFuncSetAttribute(k_tc_forward<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX));
-        ev = ktimer_start(EXOTX_K_TC_FORWARD, s);
-        k_tc_forward<4><<<njobs, TCT2, smem, s>>>(P);
-    } else {
-        EXOTX_CUDA(cudaFuncSetAttribute(k_tc_forward<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX));
-        ev = ktimer_start(EXOTX_K_TC_FORWARD, s);
-        k_tc_forward<2><<<njobs, TCT2, smem, s>>>(P);
-    }
-    EXOTX_CHECK_LAUNCH();
-    ktimer_stop(EXOTX_K_TC_FORWARD, s, ev);
-    return EXOTX_OK;
-}
-
-// dset = 1: the gridpointd inverse set (qi on st, sq, sp; no qj job), whose
-// forward jobs are the gridpointa ones
+// dset = 1: the gridpointd inverse set (qi on st, sq, sp; no qj job)
 static exotx_status tc_jobs(exotx_plan p, TcTables *T, int dir, int L, int ninst, const int4 **d, int *njobs,
                             int dset = 0) {
-    if (dir == 1) dset = 0;
     for (auto &j : T->jobs)
         if (j.dir == dir && j.nlev == L && j.ninst == ninst && j.dset == dset) {
             *d = j.d; *njobs = j.njobs; return EXOTX_OK;
         }
     std::vector<int4> v;
-    int INV_NC_QI, INV_NC_UV;
-    inv_tiles(p, T->nj8, &INV_NC_QI, &INV_NC_UV);
-    for (int m = 0; m < p->ntp1; m++) {
-        if (dir == 0) {
+    if (dir == 0) {
+        int INV_NC_QI, INV_NC_UV;
+        inv_tiles(p, T->nj8, &INV_NC_QI, &INV_NC_UV);
+        for (int m = 0; m < p->ntp1; m++) {
             const int n0 = ninst * (dset ? 2 * L + 1 : 4 * L + 1) * 2, n1 = dset ? 0 : ninst * 2, n2 = ninst * L * 4;
             for (int c = 0; c < n0; c += INV_NC_QI) v.push_back(make_int4(m, 0, c, std::min(INV_NC_QI, n0 - c)));
             for (int c = 0; c < n1; c += INV_NC_QI) v.push_back(make_int4(m, 1, c, std::min(INV_NC_QI, n1 - c)));
             for (int c = 0; c < n2; c += INV_NC_UV) v.push_back(make_int4(m, 2, c, std::min(INV_NC_UV, n2 - c)));
-        } else {
-            // slabs of nlt levels of one instance; the level-independent gvpp rides with slab 0
-            if (use_fwd3(T)) {
-                if (m == 0) {
-                    std::vector<std::pair<long long, int4>> w;
-                    fwd3_jobs(p, T, L, ninst, 0, w);
-                    std::stable_sort(w.begin(), w.end(), [](const std::pair<long long, int4> &x,
-                                                            const std::pair<long long, int4> &y) {
-                        return x.first > y.first;
-                    });
-                    for (auto &e : w) v.push_back(e.second);
-                }
-                continue;
-            }
-            const int lv = fwd_level(p, T), nlt = lv < 0 ? 2 : kFwdNlt[lv];
-            for (int i = 0; i < ninst; i++)
-                for (int l0 = 0; l0 < L; l0 += nlt)
-                    v.push_back(make_int4(m, i, l0, std::min(nlt, L - l0)));
         }
+    } else {
+        // slabs of F3_NLT levels of one instance; the level-independent gvpp rides with slab 0
+        std::vector<std::pair<long long, int4>> w;
+        fwd3_jobs(p, T, L, ninst, 0, w);
+        std::stable_sort(w.begin(), w.end(), [](const std::pair<long long, int4> &x, const std::pair<long long, int4> &y) {
+            return x.first > y.first;
+        });
+        for (auto &e : w) v.push_back(e.second);
     }
     TcTables::Jobs J;
     J.dir = dir; J.nlev = L; J.ninst = ninst; J.njobs = (int)v.size(); J.dset = dset;
@@ -477,6 +398,17 @@ static exotx_status tc_inverse_run(exotx_plan p, const float *spin, float *gpout
     int chunk = (int)std::max<size_t>(1, p->chunk_inv / per_inst);
     chunk = std::min(chunk, ninst);
     EXOTX_TRY(ensure_work(p, per_inst * chunk));
+    if (!tc_inv(p)) {
+        for (int i0 = 0; i0 < ninst; i0 += chunk) {
+            const int ni = std::min(chunk, ninst - i0);
+            const long long nrows = (long long)ni * nfo * p->nlat;
+            const LegSeg<float> g = {p, L, ni, spin + (size_t)i0 * (4 * L + 1) * nrsp, (float *)p->d_work, false};
+            EXOTX_TRY(leg_inverse_set<float>(&g, 1, dset, s));
+            EXOTX_TRY(fft_inverse_l<float>((const float *)p->d_work, gpout + (size_t)i0 * nfo * nhor, p->nlon, nrows,
+                                           p->ntp1, 1, nrows, s));
+        }
+        return EXOTX_OK;
+    }
     const int4 *jobs;
     int njobs;
     EXOTX_TRY(tc_jobs(p, T, 0, L, chunk, &jobs, &njobs, dset));
@@ -583,11 +515,10 @@ __global__ void __launch_bounds__(256) k_n0_fp64(const __grid_constant__ N0Launc
             const int lat = lat0 + g;
             double a = 0.0;
             if (lat < S.nlat) {
-                const float2 *row = reinterpret_cast<const float2 *>(S.gpin + (size_t)(row0 + lat) * S.nlon);
+                const float *row = S.gpin + (size_t)(row0 + lat) * S.nlon;   // aligned to its reals only
                 for (int e = t; e < h; e += 8) {
-                    const float2 x = row[e];
-                    a += (double)x.x;
-                    a += (double)x.y;
+                    a += (double)row[2 * e];
+                    a += (double)row[2 * e + 1];
                 }
             }
             for (int o = 1; o < 8; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
@@ -671,58 +602,36 @@ static exotx_status tc_forward_run(exotx_plan p, const float *gpin, float *spout
     const bool with_rs = fft_fold_rowsum(p->nlon);
     const size_t rs_off = (per_inst * chunk + 255) & ~(size_t)255;
     EXOTX_TRY(ensure_work(p, with_rs ? rs_off + (size_t)chunk * nfi * p->nlat * sizeof(double) : per_inst * chunk));
-    const int4 *jobs;
-    int njobs;
-    EXOTX_TRY(tc_jobs(p, T, 1, L, chunk, &jobs, &njobs));
-    const bool v3 = use_fwd3(T);
-    const int lv = fwd_level(p, T);
-    if (!v3 && lv < 0) return EXOTX_BAD_DIM;
-    const size_t smem = v3 ? 0 : fwd_smem(p->ntp1, T->njc, kFwdNlt[lv], kFwdOne[lv]);
     for (int i0 = 0; i0 < ninst; i0 += chunk) {
         const int ni = std::min(chunk, ninst - i0);
-        const int4 *jl = jobs;
-        int nj = njobs;
-        if (ni != chunk) EXOTX_TRY(tc_jobs(p, T, 1, L, ni, &jl, &nj));
         const long long nrows = (long long)ni * nfi * p->nlat;
         const float *gsrc = gpin + (size_t)i0 * nfi * nhor;
-        // the persistent kernel reads the intermediate folded about the equator where
-        // the grid length has a specialised FFT; otherwise as north and south rows
-        bool folded = false;
-        double *rowsum = nullptr;
-        if (v3) {
-            double *rs = with_rs ? reinterpret_cast<double *>(static_cast<char *>(p->d_work) + rs_off) : nullptr;
-            const exotx_status sf = fft_forward_fold(gsrc, (float *)p->d_work, p->nlon, p->nlat, nrows, p->ntp1,
-                                                     nrows, rs, s);
-            if (sf != EXOTX_OK && sf != EXOTX_NOT_BUILT) return sf;
-            folded = sf == EXOTX_OK;
-            if (folded) rowsum = rs;
-        }
-        if (!folded)
+        float *sdst = spout + (size_t)i0 * nfo * nrsp;
+        // the intermediate is folded about the equator where the grid length has
+        // a specialised FFT (and the grid is 16-byte aligned); otherwise north and south rows
+        double *rowsum = with_rs ? reinterpret_cast<double *>(static_cast<char *>(p->d_work) + rs_off) : nullptr;
+        const exotx_status sf = fft_forward_fold(gsrc, (float *)p->d_work, p->nlon, p->nlat, nrows, p->ntp1, nrows,
+                                                 rowsum, s);
+        if (sf != EXOTX_OK && sf != EXOTX_NOT_BUILT) return sf;
+        const bool folded = sf == EXOTX_OK;
+        if (!folded) {
+            rowsum = nullptr;
             EXOTX_TRY(fft_forward_l<float>(gsrc, (float *)p->d_work, p->nlon, nrows, p->ntp1, 1, nrows, s));
-        if (v3) {
+        }
+        if (folded && !dset && tc_fwd(p)) {
+            const int4 *jl;
+            int nj;
+            EXOTX_TRY(tc_jobs(p, T, 1, L, ni, &jl, &nj));
             TcFwd3Launch P3;
             P3.jobs = jl;
             P3.nprod = 6;
-            fwd3_args(P3.seg[0], p, T, L, (const float2 *)p->d_work, nrows, spout + (size_t)i0 * nfo * nrsp);
-            P3.seg[0].dset = dset;
-            EXOTX_TRY(launch_fwd_pipe(P3, nj, T->njc, folded, s));
-            EXOTX_TRY(n0_fp64(p, gsrc, rowsum, spout + (size_t)i0 * nfo * nrsp, L, ni, dset, s));
-            continue;
+            fwd3_args(P3.seg[0], p, T, L, (const float2 *)p->d_work, nrows, sdst);
+            EXOTX_TRY(launch_fwd_pipe(P3, nj, T->njc, s));
+        } else {
+            const LegSeg<float> g = {p, L, ni, (const float *)p->d_work, sdst, folded};
+            EXOTX_TRY(leg_forward_set<float>(&g, 1, dset, s));
         }
-        TcFwdLaunch P;
-        P.jobs = jl;
-        P.nprod = 6;
-        P.onebuf = kFwdOne[lv];
-        TcFwdArgs &A = P.seg[0];
-        A.tab = T->fwd; A.off = T->d_fwd_off; A.woff = p->d_woff;
-        A.W = (const float2 *)p->d_work;
-        A.nrows = nrows;
-        A.filt = p->d_fg32;
-        A.spout = spout + (size_t)i0 * nfo * nrsp;
-        A.L = L; A.nlat = p->nlat; A.nlath = p->nlath; A.njc = T->njc; A.ntp1 = p->ntp1; A.nrsp = (int)nrsp;
-        A.dset = dset;
-        EXOTX_TRY(launch_fwd(P, lv, nj, smem, s));
-        EXOTX_TRY(n0_fp64(p, gsrc, nullptr, spout + (size_t)i0 * nfo * nrsp, L, ni, dset, s));
+        EXOTX_TRY(n0_fp64(p, gsrc, rowsum, sdst, L, ni, dset, s));
     }
     return EXOTX_OK;
 }
@@ -742,21 +651,12 @@ exotx_status tc_ens_jobs(const EnsSeg *segs, int nseg, int dir, int nc_qi_cap, i
     if (nseg < 1 || nseg > TC_MAXSEG) return EXOTX_BAD_ARG;
     std::vector<std::pair<long long, int4>> v;
     size_t smax = 0;
-    int lv = 0;       // forward variant shared by every segment of the launch
-    bool v3 = true;   // stacked-split forward kernel when every segment has its tables
-    for (int sgi = 0; sgi < nseg && dir == 1; sgi++) {
-        TcTables *T;
-        EXOTX_TRY(tc_tables(segs[sgi].p, &T));
-        v3 = v3 && use_fwd3(T);
-        const int l = fwd_level(segs[sgi].p, T);
-        if (l < 0) return EXOTX_BAD_DIM;
-        lv = std::max(lv, l);
-    }
     for (int sgi = 0; sgi < nseg; sgi++) {
         const EnsSeg &g = segs[sgi];
         exotx_plan p = g.p;
         TcTables *T;
         EXOTX_TRY(tc_tables(p, &T));
+        if (!(dir == 0 ? tc_inv(p) : tc_fwd(p))) continue;   // the FP64 kernels' segment
         const int L = g.L, ni = g.ninst;
         if (dir == 0) {
             int a, b;
@@ -775,19 +675,9 @@ exotx_status tc_ens_jobs(const EnsSeg *segs, int nseg, int dir, int nc_qi_cap, i
                 for (int c = 0; c < n2; c += b)
                     v.push_back({2 * kw * b, make_int4(m, 2 | (sgi << 2), c, std::min(b, n2 - c))});
             }
-        } else if (v3) {
+        } else {
             smax = std::max(smax, fpipe_smem(T->njc));
             fwd3_jobs(p, T, L, ni, sgi, v);
-        } else {
-            const int nlt = kFwdNlt[lv];
-            smax = std::max(smax, fwd_smem(p->ntp1, T->njc, nlt, kFwdOne[lv]));
-            for (int m = 0; m < p->ntp1; m++) {
-                const int K = p->ntp1 - m;
-                const long long kw = (long long)(pad8(kpar(K, 0)) + pad8(kpar(K, 1))) * T->njc;
-                for (int i = 0; i < ni; i++)
-                    for (int l0 = 0; l0 < L; l0 += nlt)
-                        v.push_back({kw, make_int4(m, i | (sgi << 16), l0, std::min(nlt, L - l0))});
-            }
         }
     }
     if (smax > TC_SMEM_MAX) return EXOTX_BAD_DIM;
@@ -797,8 +687,8 @@ exotx_status tc_ens_jobs(const EnsSeg *segs, int nseg, int dir, int nc_qi_cap, i
     std::vector<int4> jobs(v.size());
     for (size_t i = 0; i < v.size(); i++) jobs[i] = v[i].second;
     int4 *d = nullptr;
-    EXOTX_CUDA(cudaMalloc(&d, sizeof(int4) * jobs.size()));
-    if (cudaMemcpy(d, jobs.data(), sizeof(int4) * jobs.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    EXOTX_CUDA(cudaMalloc(&d, sizeof(int4) * std::max<size_t>(jobs.size(), 1)));
+    if (!jobs.empty() && cudaMemcpy(d, jobs.data(), sizeof(int4) * jobs.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaFree(d);
         return EXOTX_CUDA_ERR;
     }
@@ -808,20 +698,20 @@ exotx_status tc_ens_jobs(const EnsSeg *segs, int nseg, int dir, int nc_qi_cap, i
     return EXOTX_OK;
 }
 
-// whether the forward tensor-core launch over these segments is the persistent
-// kernel, which reads the intermediate folded about the equator
-bool tc_ens_fwd_folded(const EnsSeg *segs, int nseg) {
-    for (int i = 0; i < nseg; i++) {
-        TcTables *T;
-        if (tc_tables(segs[i].p, &T) != EXOTX_OK || !use_fwd3(T)) return false;
-    }
-    return nseg > 0;
-}
-
-// one tensor-core launch over every segment: inverse (spin -> W) or forward (W -> spout)
+// the Legendre half of every segment: inverse (spin -> W) or forward (folded W
+// -> spout); one launch over the FP64 kernels' segments and one over the tcgen05
+// kernels'
 exotx_status tc_ens_run(const EnsSeg *segs, int nseg, int dir, const int4 *d_jobs, int njobs, size_t smem,
                         int nprod, cudaStream_t s) {
     if (nseg < 1 || nseg > TC_MAXSEG || (nprod != 3 && nprod != 6)) return EXOTX_BAD_ARG;
+    LegSeg<float> f64[TC_MAXSEG];
+    int n64 = 0;
+    for (int i = nseg - 1; i >= 0; i--) {   // the longest contractions first
+        const EnsSeg &g = segs[i];
+        if (dir == 0 ? tc_inv(g.p) : tc_fwd(g.p)) continue;
+        f64[n64++] = {g.p, g.L, g.ninst, dir == 0 ? g.spin : g.W, dir == 0 ? g.W : g.spout, true};
+    }
+    if (n64) EXOTX_TRY(dir == 0 ? leg_inverse_set<float>(f64, n64, 0, s) : leg_forward_set<float>(f64, n64, 0, s));
     if (njobs == 0) return EXOTX_OK;
     if (dir == 0) {
         TcInvLaunch P;
@@ -830,6 +720,7 @@ exotx_status tc_ens_run(const EnsSeg *segs, int nseg, int dir, const int4 *d_job
         for (int i = 0; i < nseg; i++) {
             const EnsSeg &g = segs[i];
             exotx_plan p = g.p;
+            if (!tc_inv(p)) continue;
             TcTables *T;
             EXOTX_TRY(tc_tables(p, &T));
             TcInvArgs &A = P.seg[i];
@@ -850,49 +741,19 @@ exotx_status tc_ens_run(const EnsSeg *segs, int nseg, int dir, const int4 *d_job
         EXOTX_CHECK_LAUNCH();
         ktimer_stop(EXOTX_K_TC_INVERSE, s, ev);
     } else {
-        TcFwdLaunch P;
-        P.jobs = d_jobs;
-        P.nprod = nprod;
-        int lv = 0;
-        bool v3 = true;
-        for (int i = 0; i < nseg; i++) {
-            TcTables *T;
-            EXOTX_TRY(tc_tables(segs[i].p, &T));
-            v3 = v3 && use_fwd3(T);
-            const int l = fwd_level(segs[i].p, T);
-            if (l < 0) return EXOTX_BAD_DIM;
-            lv = std::max(lv, l);
-        }
-        if (v3) {
-            TcFwd3Launch P3;
-            P3.jobs = d_jobs;
-            P3.nprod = nprod;
-            int njmax = 16;
-            for (int i = 0; i < nseg; i++) {
-                const EnsSeg &g = segs[i];
-                TcTables *T;
-                EXOTX_TRY(tc_tables(g.p, &T));
-                fwd3_args(P3.seg[i], g.p, T, g.L, (const float2 *)g.W,
-                          (long long)g.ninst * (9 * g.L + 1) * g.p->nlat, g.spout);
-                njmax = std::max(njmax, T->njc);
-            }
-            return launch_fwd_pipe(P3, njobs, njmax, true, s);   // the ensemble FFT writes the folded form
-        }
-        P.onebuf = kFwdOne[lv];
+        TcFwd3Launch P3;
+        P3.jobs = d_jobs;
+        P3.nprod = nprod;
+        int njmax = 16;
         for (int i = 0; i < nseg; i++) {
             const EnsSeg &g = segs[i];
-            exotx_plan p = g.p;
+            if (!tc_fwd(g.p)) continue;
             TcTables *T;
-            EXOTX_TRY(tc_tables(p, &T));
-            TcFwdArgs &A = P.seg[i];
-            A.tab = T->fwd; A.off = T->d_fwd_off; A.woff = p->d_woff;
-            A.W = (const float2 *)g.W;
-            A.nrows = (long long)g.ninst * (9 * g.L + 1) * p->nlat;
-            A.filt = p->d_fg32; A.spout = g.spout;
-            A.L = g.L; A.nlat = p->nlat; A.nlath = p->nlath; A.njc = T->njc; A.ntp1 = p->ntp1;
-            A.nrsp = 2 * p->ncsp;
+            EXOTX_TRY(tc_tables(g.p, &T));
+            fwd3_args(P3.seg[i], g.p, T, g.L, (const float2 *)g.W, (long long)g.ninst * (9 * g.L + 1) * g.p->nlat, g.spout);
+            njmax = std::max(njmax, T->njc);
         }
-        EXOTX_TRY(launch_fwd(P, lv, njobs, smem, s));
+        EXOTX_TRY(launch_fwd_pipe(P3, njobs, njmax, s));
     }
     return EXOTX_OK;
 }

@@ -5,8 +5,6 @@
 // share TMEM lane quarter w % 4.
 #pragma once
 
-constexpr int TCT2 = 256;
-
 __device__ __forceinline__ void st_shared16(unsigned char *p, uint4 v) { *reinterpret_cast<uint4 *>(p) = v; }
 __device__ __forceinline__ void st_shared4(unsigned char *p, uint32_t v) { *reinterpret_cast<uint32_t *>(p) = v; }
 __device__ __forceinline__ void st_shared8(unsigned char *p, uint2 v) { *reinterpret_cast<uint2 *>(p) = v; }
@@ -532,25 +530,6 @@ static size_t inv_smem_half(int nj8, int K, int ncp) {
 }
 
 // ------------------------------------------------------------ forward
-struct TcFwdArgs {
-    const unsigned char *tab;
-    const long long *off;
-    const int *woff;
-    const float2 *W;        // [m][row], row = (inst*(9L+1) + field)*nlat + lat
-    long long nrows;
-    const float *filt;      // skgpsp
-    float *spout;           // [inst][4L+1][NRSP] (gridpointd: [inst][4L][NRSP])
-    int L, nlat, nlath, njc, ntp1, nrsp;
-    int dset = 0;           // 0: gridpointa forward set, 1: gridpointd
-};
-
-struct TcFwdLaunch {
-    TcFwdArgs seg[TC_MAXSEG];
-    const int4 *jobs;       // (m, inst | seg << 16, first level, levels)
-    int nprod;
-    int onebuf;             // 1: both parity halves of a table share one buffer (large grids)
-};
-
 // Columns of one forward job (levels l0..l0+nl-1 of one instance), per table,
 // laid out as if the slab always had NLT levels (fixed positions):
 //   column (fi, li, ri) = (fi*NLT + li)*2 + ri
@@ -563,339 +542,17 @@ template <int NLT> __host__ __device__ constexpr int fwd_ncol(int t) {
     return t == 0 ? 2 * NLT * 2 + 2 : (t == 3 ? NLT * 2 : 4 * NLT * 2);
 }
 template <int NLT> __host__ __device__ constexpr int fwd_ncp(int t) { return (fwd_ncol<NLT>(t) + 15) & ~15; }
-template <int NLT> __host__ __device__ constexpr int fwd_colbase(int t) {
-    return t == 0 ? 0 : fwd_colbase<NLT>(t - 1) + 4 * fwd_ncp<NLT>(t - 1);  // 2 parities x (main, correction)
-}
-// TMEM loads of 16 or 32 columns without the wait
-template <int NC> __device__ __forceinline__ void tmem_ld_nw(uint32_t taddr, uint32_t *r) {
-    if constexpr (NC >= 32) tc::tmem_ld32_nw(taddr, r);
-    else tc::tmem_ld16_nw(taddr, r);
-}
-
-// Fourier row of field kind `kind`, level l of an instance, or -1 for a kind
-// the set does not have.  gridpointa (9L+1 fields) has every kind; gridpointd
-// (4L fields gtdt, gudt, gvdt, gqdt, plasim.f90:3415-3428) feeds fc2sp of
-// gtdt and gqdt through the tn and qn columns and uv2dv(gudt, gvdt) through
-// the fu and fv columns: mktend's d and z with ke = 0 are uv2dv's
-// (legmod.f90:356-426, :555-602), its t with vt = ut = 0 and qtend's q with
-// vq = uq = 0 are fc2sp's.
-__device__ __forceinline__ long long fwd_row(int L, int inst, int kind, int l, int dset = 0) {
-    if (dset) {
-        int F;
-        if (kind == 0) F = l;               // tn <- gtdt
-        else if (kind == 5) F = L + l;      // fu <- gudt
-        else if (kind == 4) F = 2 * L + l;  // fv <- gvdt
-        else if (kind == 1) F = 3 * L + l;  // qn <- gqdt
-        else return -1;
-        return (long long)inst * (4 * L) + F;
-    }
-    const int nfi = 9 * L + 1;
+// Fourier row of field kind `kind`, level l of an instance (9L+1 fields)
+__device__ __forceinline__ long long fwd_row(int L, int inst, int kind, int l) {
     int F;
     if (kind == 7) F = 7 * L;
     else if (kind < 7) F = kind * L + l;
     else F = 7 * L + 1 + (kind - 8) * L + l;
-    return (long long)inst * nfi + F;
-}
-
-template <int NLT>
-__global__ void __launch_bounds__(TCT2) k_tc_forward(const __grid_constant__ TcFwdLaunch P) {
-    extern __shared__ __align__(128) unsigned char sm[];
-    const int4 jb = P.jobs[blockIdx.x];
-    const TcFwdArgs &A = P.seg[jb.y >> 16];
-    const int nprod = P.nprod;
-    const int m = jb.x, inst = jb.y & 0xffff, l0 = jb.z, nl = jb.w;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quarter = warp & 3, half = warp >> 2;
-    const int K = A.ntp1 - m;
-    const int Kq[2] = {kpar(K, 0), kpar(K, 1)};
-    const int R[2] = {pad8(Kq[0]), pad8(Kq[1])};
-    const int njc = A.njc, L = A.L, nlat = A.nlat;
-    const bool with_vpp = (l0 == 0) && !A.dset;
-    const bool onebuf = P.onebuf != 0;
-    // a table block is [parity 0: 3 splits x R0 rows][parity 1: 3 splits x R1 rows];
-    // the halves travel separately, into two buffers so the next table's half 0
-    // lands while half 1 computes, or (large grids) one after the other into one
-    const uint32_t hbytes[2] = {(uint32_t)(3 * R[0] * njc * 2), (uint32_t)(3 * R[1] * njc * 2)};
-    const uint32_t hoff[2] = {0u, hbytes[0]};                 // in the global block
-    const uint32_t soff[2] = {0u, onebuf ? 0u : hbytes[0]};   // in shared memory
-    const size_t tregion = onebuf ? hbytes[0] : (size_t)hbytes[0] + hbytes[1];
-    // rows >= R of the M=128 table tiles read past the block: keep a margin
-    // before the data so those reads (whose TMEM lanes are never used) stay in bounds
-    unsigned char *tab = sm;
-    unsigned char *dat = sm + tregion + 128 * 32 * 2;
-    size_t doffs[4], dbytes = 0;
-    for (int t = 0; t < 4; t++) { doffs[t] = dbytes; dbytes += 2 * 3 * (size_t)fwd_ncp<NLT>(t) * njc * 2; }
-    unsigned char *tail = dat + dbytes;
-    uint64_t *bars = reinterpret_cast<uint64_t *>((reinterpret_cast<uintptr_t>(tail) + 15) & ~(uintptr_t)15);
-    uint64_t *bar_tma = bars;       // [2] table half of parity p landed
-    uint64_t *bar_mma = bars + 2;   // [2] MMAs reading table half p completed
-    uint64_t *bar_done = bars + 4;  // every MMA completed
-    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 5);
-    if (warp == 0) tc::tmem_alloc(slot, 512);
-    if (tid == 0) {
-        for (int i = 0; i < 5; i++) tc::mbar_init(bars + i, 1);
-        tc::mbar_fence_init();
-        for (int p = 0; p < 2; p++)
-            if (Kq[p] && (p == 0 || !onebuf)) {
-                tc::mbar_arrive_expect_tx(bar_tma + p, hbytes[p]);
-                tc::bulk_g2s(tab + soff[p], A.tab + A.off[m * 4 + 0] + hoff[p], hbytes[p], bar_tma + p);
-            }
-    }
-    // stage folded Fourier columns: for each table, S (= N+S) and D (= N-S)
-    // versions.  A unit is one column pair (re, im of one field-level) and 8
-    // latitude pairs: 16-byte loads of the north and south rows, and one
-    // 16-byte core-matrix row per column, split term and version.
-    const int ng = njc >> 3;
-    for (int t = 0; t < 4; t++) {
-        const int nf = c_fwd_nf[t];
-        const int ncp = fwd_ncp<NLT>(t), npair = ncp >> 1;
-        const int nreal = nf * NLT + ((t == 0) ? 1 : 0);  // column pairs in use (incl. padding levels)
-        const uint32_t dt = (uint32_t)ncp * njc * 2;       // one split tile
-        unsigned char *bS = dat + doffs[t], *bD = bS + 3 * dt;
-        const int nunit = npair * ng;
-        for (int u = tid; u < nunit; u += TCT2) {
-            const int q = u % npair, g = u / npair;
-            long long rb = -1;
-            if (q < nreal) {
-                if (t == 0 && q == nf * NLT) { if (with_vpp) rb = fwd_row(L, inst, 7, 0); }
-                else {
-                    const int fi = q / NLT, li = q - fi * NLT;
-                    if (li < nl) rb = fwd_row(L, inst, c_fwd_fields[t][fi], l0 + li, A.dset);
-                }
-            }
-            const int j0 = 8 * g;
-            float sr[8], si[8], dr[8], di[8];
-            float2 vn[8], vs[8];
-#pragma unroll
-            for (int e = 0; e < 8; e++) vn[e] = vs[e] = make_float2(0.f, 0.f);
-            if (rb >= 0) {
-                const float2 *wr = A.W + (size_t)m * A.nrows + (size_t)rb * nlat;
-                if (j0 + 8 <= A.nlath) {
-                    // rows j0..j0+7 north, and nlat-8-j0..nlat-1-j0 south (reversed)
-                    const float4 *pn = reinterpret_cast<const float4 *>(wr + j0);
-                    const float4 *ps = reinterpret_cast<const float4 *>(wr + nlat - 8 - j0);
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const float4 x = __ldg(pn + i), y = __ldg(ps + i);
-                        vn[2 * i] = make_float2(x.x, x.y);
-                        vn[2 * i + 1] = make_float2(x.z, x.w);
-                        vs[7 - 2 * i] = make_float2(y.x, y.y);
-                        vs[6 - 2 * i] = make_float2(y.z, y.w);
-                    }
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 8; e++)
-                        if (j0 + e < A.nlath) {
-                            vn[e] = __ldg(wr + j0 + e);
-                            vs[e] = __ldg(wr + nlat - 1 - j0 - e);
-                        }
-                }
-            }
-#pragma unroll
-            for (int e = 0; e < 8; e++) {
-                sr[e] = vn[e].x + vs[e].x;
-                si[e] = vn[e].y + vs[e].y;
-                dr[e] = vn[e].x - vs[e].x;
-                di[e] = vn[e].y - vs[e].y;
-            }
-            const uint32_t o = tc::kmajor_off(2 * q, j0, njc);  // re row; the im row follows at +16
-            uint4 h, mm, l;
-            tc::split3x8(sr, h, mm, l);
-            st_shared16(bS + o, h); st_shared16(bS + dt + o, mm); st_shared16(bS + 2 * dt + o, l);
-            tc::split3x8(si, h, mm, l);
-            st_shared16(bS + o + 16, h); st_shared16(bS + dt + o + 16, mm); st_shared16(bS + 2 * dt + o + 16, l);
-            tc::split3x8(dr, h, mm, l);
-            st_shared16(bD + o, h); st_shared16(bD + dt + o, mm); st_shared16(bD + 2 * dt + o, l);
-            tc::split3x8(di, h, mm, l);
-            st_shared16(bD + o + 16, h); st_shared16(bD + dt + o + 16, mm); st_shared16(bD + 2 * dt + o + 16, l);
-        }
-    }
-    tc::fence_proxy_async();
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    const uint32_t tmem = *slot;
-    bool ok = true;
-    if (tid == 0) {
-        const uint32_t sbo_b = (uint32_t)(njc / 8) * 128;
-        int u = 0;  // table-half units issued (one-buffer mode)
-        for (int t = 0; t < 4 && ok; t++) {
-            const int ncp = fwd_ncp<NLT>(t);
-            const uint32_t idesc = tc::idesc_bf16(128, ncp);
-            const uint32_t dt = (uint32_t)ncp * njc * 2;
-            // P-type (qc, qm, qq) use N+S on even n-m and N-S on odd; Q-type (qe) the reverse
-            const bool ptype = (t != 1);
-            for (int p = 0; p < 2 && ok; p++) {
-                if (!Kq[p]) break;
-                ok = onebuf ? tc::mbar_wait(bar_tma, u & 1) : tc::mbar_wait(bar_tma + p, t & 1);
-                if (!ok) break;
-                tc::fence_after_sync();
-                const int sel = ptype ? p : 1 - p;  // 0 -> S, 1 -> D
-                const uint64_t db0 = tc::smem_desc(dat + doffs[t] + (size_t)sel * 3 * dt, 128, sbo_b);
-                const uint32_t dm = tmem + (uint32_t)(fwd_colbase<NLT>(t) + (2 * p + 0) * ncp);
-                const uint32_t dc = tmem + (uint32_t)(fwd_colbase<NLT>(t) + (2 * p + 1) * ncp);
-                uint32_t jo = 0;
-                for (int j0 = 0; j0 < njc; j0 += 32) {
-                    const int jw = njc - j0 < 32 ? njc - j0 : 32;
-                    const uint32_t tt = (uint32_t)R[p] * jw * 2;
-                    const uint64_t da0 = tc::smem_desc(tab + soff[p] + jo, 128, (uint32_t)(jw / 8) * 128);
-                    for (int kc = 0; kc < jw / 16; kc++) {
-#pragma unroll
-                        for (int pr = 0; pr < 6; pr++)
-                            if (pr < nprod)
-                                tc::mma_bf16(pr == 0 ? dm : dc, tc::desc_add(da0, tc::pair_a(pr) * tt + kc * 256),
-                                             tc::desc_add(db0, tc::pair_b(pr) * dt + (j0 / 8) * 128 + kc * 256),
-                                             idesc, j0 > 0 || kc > 0 || pr > 1);
-                    }
-                    jo += 3 * tt;
-                }
-                if (onebuf) {
-                    // the next half may overwrite the buffer once these MMAs have read it
-                    const bool last = t == 3 && (p == 1 || !Kq[1]);
-                    if (!last) {
-                        tc::mma_commit(bar_mma);
-                        ok = tc::mbar_wait(bar_mma, u & 1);
-                        if (ok) {
-                            const int tn = (p == 0 && Kq[1]) ? t : t + 1, pn = (p == 0 && Kq[1]) ? 1 : 0;
-                            tc::mbar_arrive_expect_tx(bar_tma, hbytes[pn]);
-                            tc::bulk_g2s(tab, A.tab + A.off[m * 4 + tn] + hoff[pn], hbytes[pn], bar_tma);
-                        }
-                    }
-                    u++;
-                } else if (t < 3) {
-                    tc::mma_commit(bar_mma + p);
-                }
-            }
-            // refill each half with the next table once its MMAs have drained
-            for (int p = 0; p < 2 && ok && t < 3 && !onebuf; p++) {
-                if (!Kq[p]) break;
-                ok = tc::mbar_wait(bar_mma + p, t & 1);
-                if (!ok) break;
-                tc::mbar_arrive_expect_tx(bar_tma + p, hbytes[p]);
-                tc::bulk_g2s(tab + hoff[p], A.tab + A.off[m * 4 + t + 1] + hoff[p], hbytes[p], bar_tma + p);
-            }
-        }
-        if (ok) tc::mma_commit(bar_done);  // arrives once every MMA issued above has completed
-        if (!ok) atomicExch(&g_tc_error, 3);
-    }
-    __syncthreads();
-    ok = __all_sync(0xffffffffu, tc::mbar_wait(bar_done, 0));  // warp-uniform for the .sync.aligned TMEM loads
-    if (!ok && lane == 0) atomicExch(&g_tc_error, 4);
-    tc::fence_after_sync();
-    // epilogue: warp half h drains parity h; TMEM lane = mode index k'
-    const int p = half;
-    if (ok && Kq[p]) {
-        const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-        const int kk = quarter * 32 + lane;
-        const bool valid = kk < Kq[p];
-        // outputs per level: d, t, z, q (re, im)
-        float od[NLT][2], ot[NLT][2], oz[NLT][2], oq[NLT][2], ov[2] = {0.f, 0.f};
-#pragma unroll
-        for (int li = 0; li < NLT; li++)
-            for (int ri = 0; ri < 2; ri++) od[li][ri] = ot[li][ri] = oz[li][ri] = oq[li][ri] = 0.f;
-        uint32_t rm[32], rc[32];
-        float v[32];
-        // table qc (t=0): tn -> t, qn -> q, gvpp -> spf
-        tmem_ld_nw<fwd_ncp<NLT>(0)>(tmem + lane_addr + (uint32_t)(fwd_colbase<NLT>(0) + (2 * p) * fwd_ncp<NLT>(0)), rm);
-        tmem_ld_nw<fwd_ncp<NLT>(0)>(tmem + lane_addr + (uint32_t)(fwd_colbase<NLT>(0) + (2 * p + 1) * fwd_ncp<NLT>(0)), rc);
-        tc::tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 32; i++) v[i] = i < fwd_ncp<NLT>(0) ? __uint_as_float(rm[i]) + __uint_as_float(rc[i]) : 0.f;
-#pragma unroll
-        for (int li = 0; li < NLT; li++) {
-            ot[li][0] += v[(0 * NLT + li) * 2]; ot[li][1] += v[(0 * NLT + li) * 2 + 1];
-            oq[li][0] += v[(1 * NLT + li) * 2]; oq[li][1] += v[(1 * NLT + li) * 2 + 1];
-        }
-        ov[0] = v[2 * NLT * 2]; ov[1] = v[2 * NLT * 2 + 1];
-        // table qe (t=1): fv -> d (-), vt -> t, fu -> z, vq -> q
-        tmem_ld_nw<fwd_ncp<NLT>(1)>(tmem + lane_addr + (uint32_t)(fwd_colbase<NLT>(1) + (2 * p) * fwd_ncp<NLT>(1)), rm);
-        tmem_ld_nw<fwd_ncp<NLT>(1)>(tmem + lane_addr + (uint32_t)(fwd_colbase<NLT>(1) + (2 * p + 1) * fwd_ncp<NLT>(1)), rc);
-        tc::tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 32; i++) v[i] = i < fwd_ncp<NLT>(1) ? __uint_as_float(rm[i]) + __uint_as_float(rc[i]) : 0.f;
-#pragma unroll
-        for (int li = 0; li < NLT; li++)
-#pragma unroll
-            for (int ri = 0; ri < 2; ri++) {
-                od[li][ri] -= v[(0 * NLT + li) * 2 + ri];
-                ot[li][ri] += v[(1 * NLT + li) * 2 + ri];
-                oz[li][ri] += v[(2 * NLT + li) * 2 + ri];
-                oq[li][ri] += v[(3 * NLT + li) * 2 + ri];
-            }
-        // table qm (t=2): i*fu -> d, -i*ut -> t, i*fv -> z, -i*uq -> q  (i*(a+ib) = -b + ia)
-        tmem_ld_nw<fwd_ncp<NLT>(2)>(tmem + lane_addr + (uint32_t)(fwd_colbase<NLT>(2) + (2 * p) * fwd_ncp<NLT>(2)), rm);
-        tmem_ld_nw<fwd_ncp<NLT>(2)>(tmem + lane_addr + (uint32_t)(fwd_colbase<NLT>(2) + (2 * p + 1) * fwd_ncp<NLT>(2)), rc);
-        tc::tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 32; i++) v[i] = i < fwd_ncp<NLT>(2) ? __uint_as_float(rm[i]) + __uint_as_float(rc[i]) : 0.f;
-#pragma unroll
-        for (int li = 0; li < NLT; li++) {
-            const float fur = v[(0 * NLT + li) * 2], fui = v[(0 * NLT + li) * 2 + 1];
-            const float utr = v[(1 * NLT + li) * 2], uti = v[(1 * NLT + li) * 2 + 1];
-            const float fvr = v[(2 * NLT + li) * 2], fvi = v[(2 * NLT + li) * 2 + 1];
-            const float uqr = v[(3 * NLT + li) * 2], uqi = v[(3 * NLT + li) * 2 + 1];
-            od[li][0] -= fui; od[li][1] += fur;
-            ot[li][0] += uti; ot[li][1] -= utr;
-            oz[li][0] -= fvi; oz[li][1] += fvr;
-            oq[li][0] += uqi; oq[li][1] -= uqr;
-        }
-        // table qq (t=3): ke -> d
-        tc::tmem_ld16_nw(tmem + lane_addr + (uint32_t)(fwd_colbase<NLT>(3) + (2 * p) * fwd_ncp<NLT>(3)), rm);
-        tc::tmem_ld16_nw(tmem + lane_addr + (uint32_t)(fwd_colbase<NLT>(3) + (2 * p + 1) * fwd_ncp<NLT>(3)), rc);
-        tc::tmem_wait_ld();
-#pragma unroll
-        for (int li = 0; li < NLT; li++) {
-            od[li][0] += __uint_as_float(rm[2 * li]) + __uint_as_float(rc[2 * li]);
-            od[li][1] += __uint_as_float(rm[2 * li + 1]) + __uint_as_float(rc[2 * li + 1]);
-        }
-        if (valid) {
-            const int k = 2 * kk + p;  // n - m
-            const float fl = A.filt[m + k];
-            const size_t wo = 2 * (size_t)(A.woff[m] + k);
-            const int nfo = A.dset ? 4 * L : 4 * L + 1;
-#pragma unroll
-            for (int li = 0; li < NLT; li++) {
-                if (li >= nl) break;
-                const int l = l0 + li;
-                float2 *sd = reinterpret_cast<float2 *>(A.spout + ((size_t)inst * nfo + l) * A.nrsp + wo);
-                float2 *st = reinterpret_cast<float2 *>(A.spout + ((size_t)inst * nfo + L + l) * A.nrsp + wo);
-                float2 *sz = reinterpret_cast<float2 *>(A.spout + ((size_t)inst * nfo + 2 * L + l) * A.nrsp + wo);
-                float2 *sq = reinterpret_cast<float2 *>(A.spout + ((size_t)inst * nfo + 3 * L + l) * A.nrsp + wo);
-                *sd = make_float2(od[li][0] * fl, od[li][1] * fl);
-                *st = make_float2(ot[li][0] * fl, ot[li][1] * fl);
-                *sz = make_float2(oz[li][0] * fl, oz[li][1] * fl);
-                *sq = make_float2(oq[li][0] * fl, oq[li][1] * fl);
-            }
-            if (with_vpp) {
-                float2 *sp = reinterpret_cast<float2 *>(A.spout + ((size_t)inst * nfo + 4 * L) * A.nrsp + wo);
-                *sp = make_float2(ov[0] * fl, ov[1] * fl);
-            }
-        }
-    }
-    tc::fence_before_sync();
-    __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, 512);
-}
-
-static int fwd_ncp_rt(int nlt, int t) {
-    const int c = t == 0 ? 4 * nlt + 2 : (t == 3 ? 2 * nlt : 8 * nlt);
-    return (c + 15) & ~15;
-}
-// shared memory of a forward job at the widest m (K = NTP1 modes)
-static size_t fwd_smem(int K, int njc, int nlt, bool onebuf) {
-    size_t h[2] = {0, 0};
-    for (int p = 0; p < 2; p++) {
-        const int Kq = kpar(K, p);
-        if (Kq) h[p] = 3 * (size_t)pad8(Kq) * njc * 2;
-    }
-    const size_t tblk = onebuf ? std::max(h[0], h[1]) : h[0] + h[1];
-    size_t d = 0;
-    for (int t = 0; t < 4; t++) d += 2 * 3 * (size_t)fwd_ncp_rt(nlt, t) * njc * 2;
-    return tblk + 128 * 32 * 2 + d + 80;
+    return (long long)inst * (9 * L + 1) + F;
 }
 
 // ------------------------------------------------------------ forward, stacked splits
-// Variant for NTRU+1 <= 128 (every parity has at most 64 modes): one parity per
-// job, and the table's split terms stacked in the M=128 tile so that two MMAs
+// For NTRU+1 <= 128 (every parity has at most 64 modes): one parity per job, and the table's split terms stacked in the M=128 tile so that two MMAs
 // per K-chunk cover all six split products.  Per (m, table, parity) and
 // latitude chunk the table holds two 2R-row K-major tiles:
 //   S01 = [a0 of modes 0..R-1 ; a1 of modes 0..R-1],   S2 = [0 ; a2]
@@ -914,7 +571,6 @@ struct TcFwd3Args {
     const float *filt;
     float *spout;
     int L, nlat, nlath, njc, ntp1, nrsp;
-    int dset = 0;           // 0: gridpointa forward set, 1: gridpointd (no gvpp; 4L outputs)
 };
 struct TcFwd3Launch {
     TcFwd3Args seg[TC_MAXSEG];
@@ -961,83 +617,21 @@ __device__ __forceinline__ long long f3_row(const TcFwd3Args &A, int inst, int l
                                             int q) {
     const int nf = c_fwd_nf[t];
     if (q >= nf * NLT + ((t == 0) ? 1 : 0)) return -1;
-    if (t == 0 && q == nf * NLT) return (with_vpp && !A.dset) ? fwd_row(A.L, inst, 7, 0) : -1;
+    if (t == 0 && q == nf * NLT) return with_vpp ? fwd_row(A.L, inst, 7, 0) : -1;
     const int fi = q / NLT, li = q - fi * NLT;
-    return li < nl ? fwd_row(A.L, inst, c_fwd_fields[t][fi], l0 + li, A.dset) : -1;
+    return li < nl ? fwd_row(A.L, inst, c_fwd_fields[t][fi], l0 + li) : -1;
 }
 
-// Operand staging works on slots: a slot is one column pair q (a field level,
-// re and im) and the four latitude pairs j = 4jq .. 4jq+3.  Consecutive threads
-// take consecutive jq of a pair, so a warp's loads read 1 KB of a Fourier row's
-// northern half and of its mirrored southern half, and its 8-byte stores fall
-// in distinct banks of the padded operand layout (one half-warp per wavefront).
+// Operand staging works on slots.  The intermediate is folded about the equator
+// (rfft_fwd_fold_body): each field row holds E = N + S for the latitude pairs,
+// then O = N - S, so a parity reads only the half it needs.  A slot is one
+// column pair q (a field level, re and im) and eight latitude pairs j = 8jg ..
+// 8jg+7 of one row (n[] the first four, s[] the next four), stored as one
+// 16-byte core-matrix row per split term of the padded operand layout, where a
+// warp's stores fall in distinct banks.
 struct F3Slot {
-    float2 n[4], s[4];  // north and south values at latitude pairs j .. j+3
+    float2 n[4], s[4];
 };
-
-template <int NLT>
-__device__ __forceinline__ void f3_load(const TcFwd3Args &A, int m, int inst, int l0, int nl, bool with_vpp, int t,
-                                        int sl, F3Slot &v) {
-    const int hj = A.njc >> 2;
-    const int q = sl / hj, jq = sl - q * hj;
-#pragma unroll
-    for (int e = 0; e < 4; e++) v.n[e] = v.s[e] = make_float2(0.f, 0.f);
-    if (q >= (fwd_ncp<NLT>(t) >> 1)) return;
-    const long long rb = f3_row<NLT>(A, inst, l0, nl, with_vpp, t, q);
-    if (rb < 0) return;
-    const int j = 4 * jq, nlat = A.nlat, nlath = A.nlath;
-    const float2 *wr = A.W + (size_t)m * A.nrows + (size_t)rb * nlat;
-    if (j + 4 <= nlath) {
-        // north rows j .. j+3; south rows nlat-4-j .. nlat-1-j (pairs j+3 .. j)
-        const float4 x0 = __ldg(reinterpret_cast<const float4 *>(wr + j));
-        const float4 x1 = __ldg(reinterpret_cast<const float4 *>(wr + j + 2));
-        const float4 y0 = __ldg(reinterpret_cast<const float4 *>(wr + nlat - 4 - j));
-        const float4 y1 = __ldg(reinterpret_cast<const float4 *>(wr + nlat - 2 - j));
-        v.n[0] = make_float2(x0.x, x0.y); v.n[1] = make_float2(x0.z, x0.w);
-        v.n[2] = make_float2(x1.x, x1.y); v.n[3] = make_float2(x1.z, x1.w);
-        v.s[3] = make_float2(y0.x, y0.y); v.s[2] = make_float2(y0.z, y0.w);
-        v.s[1] = make_float2(y1.x, y1.y); v.s[0] = make_float2(y1.z, y1.w);
-    } else {
-#pragma unroll
-        for (int e = 0; e < 4; e++)
-            if (j + e < nlath) {
-                v.n[e] = __ldg(wr + j + e);
-                v.s[e] = __ldg(wr + nlat - 1 - j - e);
-            }
-    }
-}
-
-// fold a slot for parity p, split it into three BF16 terms and store the re
-// and im words of every term
-template <int NLT>
-__device__ __forceinline__ void f3_store(int t, int p, int sl, int njc, unsigned char *bt, const F3Slot &v) {
-    const int hj = njc >> 2, ngk = njc >> 3;
-    const int q = sl / hj, jq = sl - q * hj;
-    const int ncp = fwd_ncp<NLT>(t);
-    if (q >= (ncp >> 1)) return;
-    const bool diff = (t != 1) ? (p == 1) : (p == 0);
-    float xr[4], xi[4];
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        xr[e] = diff ? v.n[e].x - v.s[e].x : v.n[e].x + v.s[e].x;
-        xi[e] = diff ? v.n[e].y - v.s[e].y : v.n[e].y + v.s[e].y;
-    }
-    uint2 hr, mr, lr, hi, mi, li;
-    tc::split3x2(xr[0], xr[1], hr.x, mr.x, lr.x);
-    tc::split3x2(xr[2], xr[3], hr.y, mr.y, lr.y);
-    tc::split3x2(xi[0], xi[1], hi.x, mi.x, li.x);
-    tc::split3x2(xi[2], xi[3], hi.y, mi.y, li.y);
-    const uint32_t dt = (uint32_t)(ncp >> 3) * ngk * tc::kPadLbo;  // one split term
-    const uint32_t o = tc::kpad_off(2 * q, 4 * jq, ngk);            // re row; the im row follows at +16
-    st_shared8(bt + o, hr); st_shared8(bt + dt + o, mr); st_shared8(bt + 2 * dt + o, lr);
-    st_shared8(bt + o + 16, hi); st_shared8(bt + dt + o + 16, mi); st_shared8(bt + 2 * dt + o + 16, li);
-}
-
-// The same staging from the equator-folded intermediate (rfft_fwd_fold_body):
-// each field row holds E = N + S for the latitude pairs, then O = N - S, so a
-// parity reads only the half it needs and a slot covers eight latitude pairs
-// j = 8jg .. 8jg+7 of one row (n[] the first four, s[] the next four), stored
-// as one 16-byte core-matrix row per split term.
 template <int NLT>
 __device__ __forceinline__ void f3_load_fold(const TcFwd3Args &A, int m, int inst, int l0, int nl, bool with_vpp,
                                              int t, int p, int sl, F3Slot &v) {
@@ -1102,7 +696,6 @@ __device__ __forceinline__ void f3_store_fold(int t, int sl, int njc, unsigned c
 constexpr int FP_THREADS = 512;
 constexpr int FP_NST = 320;              // staging threads
 constexpr int FP_ACC = 144;              // TMEM columns of a slot: 3 x the widest table's columns
-constexpr int FP_SLOTS = 2;              // staging slots per thread kept in flight for one tile
 constexpr int FP_FOLD_DEPTH = 2;         // tiles ahead whose folded-intermediate loads are in flight
 
 struct FpLayout {
@@ -1177,8 +770,7 @@ __device__ __forceinline__ void fp_drain(int t, uint32_t X, int nprod, float (*o
     else fp_drain_t<NLT, 3>(X, nprod, o, ov);
 }
 
-// FOLD: the intermediate is folded about the equator (rfft_fwd_fold_body)
-template <int NLT, bool FOLD>
+template <int NLT>
 __global__ void __launch_bounds__(FP_THREADS, 1) k_tc_forward_pipe(const __grid_constant__ TcFwd3Launch P) {
     extern __shared__ __align__(128) unsigned char sm[];
     const FpLayout LY = fp_layout(P.njmax);
@@ -1333,7 +925,7 @@ __global__ void __launch_bounds__(FP_THREADS, 1) k_tc_forward_pipe(const __grid_
             if (!ok) break;
             if (r < Kq) {
                 const float *e = E + (size_t)r * NO;
-                const int L = A.L, nfo = A.dset ? 4 * L : 4 * L + 1, k = 2 * r + p;   // k = n - m
+                const int L = A.L, nfo = 4 * L + 1, k = 2 * r + p;   // k = n - m
                 const size_t wo = (size_t)wom + k;
 #pragma unroll
                 for (int li = 0; li < NLT; li++) {
@@ -1345,7 +937,7 @@ __global__ void __launch_bounds__(FP_THREADS, 1) k_tc_forward_pipe(const __grid_
                                               (o[li][kk][1] + e[(li * 4 + kk) * 2 + 1]) * fl);
                     }
                 }
-                if (l0 == 0 && !A.dset) {
+                if (l0 == 0) {
                     float2 *dst = reinterpret_cast<float2 *>(A.spout + ((size_t)inst * nfo + 4 * L) * A.nrsp);
                     dst[wo] = make_float2((ov[0] + e[NLT * 8]) * fl, (ov[1] + e[NLT * 8 + 1]) * fl);
                 }
@@ -1356,58 +948,43 @@ __global__ void __launch_bounds__(FP_THREADS, 1) k_tc_forward_pipe(const __grid_
         // ------------------------------------------------------------- staging
         const int stid = (warp < 4 ? warp - 2 : warp - 6) * 32 + lane;
         pdl_wait();   // the intermediate comes from the previous kernel
-        // slots per thread kept in flight for a tile, and how many tiles ahead
-        // they are loaded: the folded intermediate needs one slot per thread
-        // per tile (eight latitude pairs), so its loads run FP_FOLD_DEPTH tiles
+        // one slot per thread per tile, its loads running FP_FOLD_DEPTH tiles
         // ahead (a ring of registers: q[d] holds tile i + d)
-        constexpr int SL = FOLD ? 1 : FP_SLOTS, DEPTH = FOLD ? FP_FOLD_DEPTH : 1;
-        F3Slot q[DEPTH + 1][SL];
+        constexpr int DEPTH = FP_FOLD_DEPTH;
+        F3Slot q[DEPTH + 1];
         auto load = [&](const TcFwd3Args &A, int4 jb, int t, int sl, F3Slot &v) {
-            if constexpr (FOLD)
-                f3_load_fold<NLT>(A, jb.x, jb.y & 0xffff, jb.z, jb.w & 0xff, jb.z == 0, t, jb.w >> 8, sl, v);
-            else
-                f3_load<NLT>(A, jb.x, jb.y & 0xffff, jb.z, jb.w & 0xff, jb.z == 0, t, sl, v);
-        };
-        auto store = [&](int t, int p, int sl, int njc, unsigned char *bt, const F3Slot &v) {
-            if constexpr (FOLD) f3_store_fold<NLT>(t, sl, njc, bt, v);
-            else f3_store<NLT>(t, p, sl, njc, bt, v);
+            f3_load_fold<NLT>(A, jb.x, jb.y & 0xffff, jb.z, jb.w & 0xff, jb.z == 0, t, jb.w >> 8, sl, v);
         };
 #pragma unroll
         for (int d = 0; d < DEPTH; d++) {
             if (d < ntile) {
                 const int4 jb = job(d);
-#pragma unroll
-                for (int k = 0; k < SL; k++) load(P.seg[jb.y >> 16], jb, d & 3, stid + k * FP_NST, q[d][k]);
+                load(P.seg[jb.y >> 16], jb, d & 3, stid, q[d]);
             }
         }
         for (int i = 0; i < ntile; i++) {
             const int b = i & 1, u = i >> 1, t = i & 3;
             const int4 jb = job(i);
             const TcFwd3Args &A = P.seg[jb.y >> 16];
-            const int njc = A.njc, p = jb.w >> 8;
+            const int njc = A.njc;
             if (i + DEPTH < ntile) {
                 // later tiles' loads are in flight while this one is stored
                 const int4 jn = job(i + DEPTH);
-#pragma unroll
-                for (int k = 0; k < SL; k++) load(P.seg[jn.y >> 16], jn, (i + DEPTH) & 3, stid + k * FP_NST, q[DEPTH][k]);
+                load(P.seg[jn.y >> 16], jn, (i + DEPTH) & 3, stid, q[DEPTH]);
             }
             if (!fp_wait(op_empty + b, (u & 1) ^ 1, abort)) break;
             unsigned char *bt = opr + b * LY.ob;
-            const int nslot = (fwd_ncp<NLT>(t) >> 1) * (FOLD ? (njc >> 3) : (njc >> 2));
-#pragma unroll
-            for (int k = 0; k < SL; k++)
-                if (stid + k * FP_NST < nslot) store(t, p, stid + k * FP_NST, njc, bt, q[0][k]);
-            for (int s = stid + SL * FP_NST; s < nslot; s += FP_NST) {   // beyond the slots in flight
+            const int nslot = (fwd_ncp<NLT>(t) >> 1) * (njc >> 3);
+            if (stid < nslot) f3_store_fold<NLT>(t, stid, njc, bt, q[0]);
+            for (int s = stid + FP_NST; s < nslot; s += FP_NST) {   // beyond the slots in flight
                 F3Slot v;
                 load(A, jb, t, s, v);
-                store(t, p, s, njc, bt, v);
+                f3_store_fold<NLT>(t, s, njc, bt, v);
             }
             tc::fence_proxy_async();   // these stores feed the tensor cores
             tc::mbar_arrive(op_full + b);
 #pragma unroll
-            for (int d = 0; d < DEPTH; d++)
-#pragma unroll
-                for (int k = 0; k < SL; k++) q[d][k] = q[d + 1][k];
+            for (int d = 0; d < DEPTH; d++) q[d] = q[d + 1];
         }
     }
     tc::fence_before_sync();

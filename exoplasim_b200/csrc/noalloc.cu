@@ -106,7 +106,8 @@ static exotx_status forward_set_static(exotx_plan p, const T *gpin, T *spout, in
     }
     const long long nrows = (9LL * L + 1) * p->nlat;
     EXOTX_TRY(fft_forward_tw<T>(gpin, W, p->nlon, nrows, p->ntp1, 1, nrows, dw, dr, s));
-    return leg_forward_set<T>(p, 0, W, spout, L, 1, s);
+    const LegSeg<T> g = {p, L, 1, W, spout, false};
+    return leg_forward_set<T>(&g, 1, 0, s);
 }
 
 }  // namespace exotx
