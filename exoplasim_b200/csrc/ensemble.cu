@@ -2,11 +2,11 @@
 // runs one model state per process, plasim.f90 gridpointa :2396-2486).
 // Instances of different truncations and level counts are grouped into
 // segments of one resolution and level count; each half of the round trip is
-// one tensor-core Legendre launch plus one FFT launch over all segments, and
-// the forward half one small launch more for the FP64 global means, so the
-// whole ensemble step is five kernels (and one CUDA graph when captured).
-// Segments whose rows have a register-resident FFT kernel (NLON 384) take one
-// FFT launch more per half when they are mixed with other lengths.
+// one Legendre launch plus one FFT launch over all segments, and the forward
+// half one small launch more for the FP64 global means, so the whole ensemble
+// step is five kernels (and one CUDA graph when captured).  Segments whose
+// contractions run on the tcgen05 kernels (legendre_tc.cu) take one Legendre
+// launch more per half when they are mixed with others.
 #include <algorithm>
 #include <cmath>
 #include <map>
@@ -21,6 +21,8 @@ struct exotx_ensemble_s {
     std::vector<long long> spec_off, gin_off, gout_off;          // per instance, caller order
     long long totals[3] = {0, 0, 0};
     float *W = nullptr;
+    double *rs = nullptr;                           // row sums of the forward half's grid rows
+    std::vector<long long> seg_rs;
     int4 *jobs[2] = {nullptr, nullptr};
     int njobs[2] = {0, 0};
     size_t smem[2] = {0, 0};
@@ -39,6 +41,7 @@ static std::vector<EnsSeg> ens_segs(exotx_ensemble e, const float *spin, float *
         v[s].spin = spin ? spin + e->seg_spec[s] : nullptr;
         v[s].spout = spout ? spout + e->seg_spec[s] : nullptr;
         v[s].W = e->W + e->seg_W[s];
+        v[s].rowsum = e->rs + e->seg_rs[s];
     }
     return v;
 }
@@ -72,7 +75,8 @@ static exotx_status ens_forward(exotx_ensemble e, const float *gpin, float *spou
     for (size_t i = 0; i < v.size(); i++) {
         const exotx_plan p = v[i].p;
         const long long rows = (long long)v[i].ninst * (9 * v[i].L + 1) * p->nlat;
-        f[i] = FftEnsSeg{gpin + e->seg_gin[i], v[i].W, rows, 1, rows, p->nlon, p->ntp1, p->nlat};   // folded intermediate
+        f[i] = FftEnsSeg{gpin + e->seg_gin[i], v[i].W, rows, 1, rows, p->nlon, p->ntp1, p->nlat, v[i].rowsum,
+                         v[i].L};   // folded intermediate
     }
     EXOTX_TRY(fft_ens(true, f.data(), (int)f.size(), s));
     EXOTX_TRY(tc_ens_run(v.data(), (int)v.size(), 1, e->jobs[1], e->njobs[1], e->smem[1], e->nprod, s));
@@ -130,7 +134,7 @@ EXOTX_API exotx_status exotx_ensemble_create(int ninst, const int *nlat, const i
     e->spec_off.assign(ninst, 0);
     e->gin_off.assign(ninst, 0);
     e->gout_off.assign(ninst, 0);
-    long long so = 0, gi = 0, go = 0, wo = 0;
+    long long so = 0, gi = 0, go = 0, wo = 0, ro = 0;
     exotx_status st = EXOTX_OK;
     for (auto &kv : groups) {
         const int nl = kv.first.first, L = kv.first.second;
@@ -152,14 +156,18 @@ EXOTX_API exotx_status exotx_ensemble_create(int ninst, const int *nlat, const i
         e->seg_gin.push_back(gi);
         e->seg_gout.push_back(go);
         e->seg_W.push_back(wo);
+        e->seg_rs.push_back(ro);
         for (int i : kv.second) {
             e->spec_off[i] = so; so += (4LL * L + 1) * nrsp;
             e->gin_off[i] = gi; gi += (9LL * L + 1) * nhor;
             e->gout_off[i] = go; go += (6LL * L + 3) * nhor;
         }
         wo += (long long)kv.second.size() * (9LL * L + 1) * p->nlat * p->ntp1 * 2;
+        ro += (long long)kv.second.size() * (9LL * L + 1) * p->nlat;
     }
-    if (st == EXOTX_OK && cudaMalloc(&e->W, sizeof(float) * wo) != cudaSuccess) st = EXOTX_NO_MEM;
+    if (st == EXOTX_OK && (cudaMalloc(&e->W, sizeof(float) * wo) != cudaSuccess ||
+                           cudaMalloc(&e->rs, sizeof(double) * ro) != cudaSuccess))
+        st = EXOTX_NO_MEM;
     e->totals[0] = so; e->totals[1] = gi; e->totals[2] = go;
     if (st == EXOTX_OK) st = ens_build_jobs(e);
     if (st != EXOTX_OK) { exotx_ensemble_destroy(e); return st; }
@@ -170,6 +178,7 @@ EXOTX_API exotx_status exotx_ensemble_create(int ninst, const int *nlat, const i
 EXOTX_API exotx_status exotx_ensemble_destroy(exotx_ensemble e) {
     if (!e) return EXOTX_BAD_ARG;
     cudaFree(e->W);
+    cudaFree(e->rs);
     cudaFree(e->jobs[0]);
     cudaFree(e->jobs[1]);
     for (exotx_plan p : e->plans) exotx_plan_destroy(p);

@@ -181,14 +181,16 @@ struct FftEnsSeg {
     long long lot, f_rs, f_ms;
     int n, kf;
     int fold_nlat = 0;  // forward: > 0 writes the equator-folded layout for nlat-row fields
+    double *rowsum = nullptr;  // forward, folded: also the row sums of the gridpointa set of L levels
+    int L = 0;
 };
-// forward FFT into the equator-folded m-major layout of the tensor-core forward
-// kernel (E = north + south rows, then O = north - south, per field) (fft.cu).
-// rowsum (may be null): also the FP64 sum of every grid row, in the order of
-// row_sum_fp64 (register-resident lengths only; EXOTX_NOT_BUILT otherwise)
+// forward FFT into the equator-folded m-major layout of the Legendre kernels
+// (E = north + south rows, then O = north - south, per field) (fft.cu).
+// rowsum (may be null): also the FP64 sums, one per grid row, of the fields whose
+// n = 0 coefficient k_n0_fp64 forms, for a set of L levels (dset: gridpointd)
 exotx_status fft_forward_fold(const float *in, float *out, int n, int nlat, long long lot, int kf, long long f_ms,
-                              double *rowsum, cudaStream_t s);
-bool fft_fold_rowsum(int n);   // whether fft_forward_fold forms row sums for grid length n
+                              double *rowsum, int L, int dset, cudaStream_t s);
+bool fft_fold_rowsum(int n);   // whether fft_forward_fold is built for grid length n
 exotx_status fft_ens(bool fwd, const FftEnsSeg *segs, int nseg, cudaStream_t s);
 
 // element-wise FP64 <-> FP32 conversion of n device reals (fortran_abi.cu)
@@ -218,6 +220,7 @@ struct EnsSeg {
     const float *spin;  // inverse input, (4L+1) x NRSP per instance
     float *spout;       // forward output, (4L+1) x NRSP per instance
     float *W;           // m-major Fourier intermediate of the segment
+    double *rowsum;     // forward: FP64 row sums of the grid input
 };
 exotx_status tc_ens_jobs(const EnsSeg *segs, int nseg, int dir, int nc_qi_cap, int nc_uv_cap, bool sort,
                          int4 **d_jobs, int *njobs, size_t *smem);

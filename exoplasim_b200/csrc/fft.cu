@@ -13,6 +13,7 @@
 #include <cmath>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 #include "exotx_internal.cuh"
 #include "tc_prims.cuh"
@@ -230,351 +231,391 @@ __global__ void __launch_bounds__(256) k_rfft_inverse(const T *fc, T *gp, FftLau
     for (int i = threadIdx.x; i < rows * n; i += blockDim.x) dst[i] = zr[i];
 }
 
-// ------------------------------------------- length-specialised kernels
-// For the model's grid lengths the radix schedule, loop trip counts and
-// index divisions are compile-time constants and the twiddles live in
-// shared memory; one block transforms ROWS rows.
-__host__ __device__ constexpr int radix_count(int h) {
-    int r = h, k = 0;
-    while (r % 8 == 0 && r > 8) { k++; r /= 8; }
-    while (r % 4 == 0) { k++; r /= 4; }
-    while (r % 2 == 0) { k++; r /= 2; }
-    while (r % 3 == 0) { k++; r /= 3; }
-    while (r % 5 == 0) { k++; r /= 5; }
-    if (r == 8) k++;
-    return k;
-}
-__host__ __device__ constexpr int radix_at(int h, int idx) {
-    int r = h, k = 0;
-    while (r % 8 == 0 && r > 8) { if (k++ == idx) return 8; r /= 8; }
-    while (r % 4 == 0) { if (k++ == idx) return 4; r /= 4; }
-    while (r % 2 == 0) { if (k++ == idx) return 2; r /= 2; }
-    while (r % 3 == 0) { if (k++ == idx) return 3; r /= 3; }
-    while (r % 5 == 0) { if (k++ == idx) return 5; r /= 5; }
-    return 8;
-}
+// ------------------------------------------------ register-resident transforms
+// For the model's grid lengths (h = n/2 = P*Q complex points) P threads of a
+// warp work a row:
+//   Z[q + Q m] = sum_t W_P^{t m} W_h^{t q} sum_j z[t + P j] W_Q^{j q}   (W = e^{-2 pi i/.})
+// Thread t loads its column z[t + P j] straight from the grid row, takes the
+// Q-point DFT in registers and applies W_h^{t q}; one transposition through
+// shared memory within the warp then hands it the P-point DFTs q = t + P i.
+// The inverse runs the same steps in the other order.  A block of RR_THREADS
+// works RB = RR_THREADS/P rows.  The m-major Fourier side is reached rows
+// fastest: through the spectra in shared memory (forward) or the staged
+// coefficients (inverse), which take the transposition's place in turn.
+// T42 L20 FP64, one state (181 fields): forward RRF64 us, inverse RRI64 us,
+// against 11.3 and 10.1 us for the three-pass shared-memory (Stockham) kernels
+// before, which moved every value through shared memory six times and were
+// bound by instruction issue; T85 L13 x3 FP32 RRF32 and RRI32 against 39.8 and 32.9.
+constexpr int RR_THREADS = 128;
+// P: 16 where Q would need over 64 registers in FP64 (n = 384 with P = 8: 132
+// registers, 3 blocks per SM, forward 67 us per T127 L20 state)
+template <int N> constexpr int rr_p() { return N == 64 ? 4 : N < 384 ? 8 : 16; }
 
-// Rows in shared memory keep 2 spare complex slots after every 16 elements:
-// the passes' strided reads and writes then spread over the banks (about half
-// the wavefronts of a dense row), and even indices stay 16-byte aligned for the
-// vector copies.  H is a multiple of 16 for every specialised length.
-__host__ __device__ constexpr int fpad(int j) { return j + 2 * (j >> 4); }
-template <int H> __host__ __device__ constexpr int fpad_row() { return H + 2 * (H / 16); }
-
-template <typename T, int S, int H, int ROWS, int R, int NS>
-__device__ __forceinline__ void pass_ct(const cpx<T> *src, cpx<T> *dst, const cpx<T> *tw) {
-    constexpr int NQ = H / R, STEP = H / (NS * R), NIT = ROWS * NQ, HP = fpad_row<H>();
-    for (int it = threadIdx.x; it < NIT; it += blockDim.x) {
-        const int row = it / NQ, t = it - row * NQ, k = t % NS;
-        const cpx<T> *s = src + row * HP;
-        cpx<T> *d = dst + row * HP;
-        cpx<T> v[R];
-#pragma unroll
-        for (int r = 0; r < R; r++) v[r] = s[fpad(t + r * NQ)];
-        if constexpr (NS > 1) {  // the first pass has unit twiddles only
-#pragma unroll
-            for (int r = 1; r < R; r++) {
-                cpx<T> w = tw[r * k * STEP];
-                if (S > 0) w.y = -w.y;
-                v[r] = cmul(v[r], w);
-            }
-        }
-        dftR<T, S, R>(v);
-        const int base = (t / NS) * NS * R + k;
-#pragma unroll
-        for (int r = 0; r < R; r++) d[fpad(base + r * NS)] = v[r];
+// least stride >= x congruent to c modulo m
+__host__ __device__ constexpr int rr_pad(int x, int c, int m) { return x + ((c - x) % m + m) % m; }
+// Strides in complex values, for conflict-free accesses (a conflict group is a
+// half-warp of 8-byte values or a quarter-warp of 16-byte ones, G lanes):
+//   transposition: q-th DFT's P values at q*(P+1); rows a multiple of P apart
+//   in the banks (G/P rows of a group side by side)
+//   spectra: odd row stride; coefficients: k-major, the k step one group's rows wide
+template <typename T, int N> struct RrLayout {
+    static constexpr int P = rr_p<N>(), H = N / 2, Q = H / P, RB = RR_THREADS / P;
+    static constexpr int G = sizeof(T) == 4 ? 16 : 8, GR = G / P > 1 ? G / P : 1;   // rows of one row's threads per group
+    static constexpr int RS = rr_pad(Q * (P + 1), GR > 1 ? P : 0, G);
+    static constexpr int RZ = (H + 1) | 1;
+    static constexpr int RC = GR > 1 ? rr_pad(RB, GR, G) : RB + 1;
+    static constexpr int QP = (Q + P - 1) / P;
+    static_assert(P * Q == H && 32 % P == 0, "a row's threads are in one warp");
+    static constexpr size_t fwd_smem() { return (size_t)RB * (RS > RZ ? RS : RZ) * 2 * sizeof(T); }
+    static size_t inv_smem(int kf) {
+        const size_t c = (size_t)kf * RC, x = (size_t)RB * RS;
+        return (c > x ? c : x) * 2 * sizeof(T);
     }
-}
+};
 
-template <typename T, int S, int H, int ROWS, int IDX, int NS>
-__device__ __forceinline__ const cpx<T> *passes_ct(cpx<T> *src, cpx<T> *dst, const cpx<T> *tw) {
-    if constexpr (IDX >= radix_count(H)) {
-        return src;
+// cos(2 pi a / n) for n = 12, 16, 20, 24
+template <int LEN> __host__ __device__ constexpr double cos_len(int a) {
+    a = ((a % LEN) + LEN) % LEN;
+    if (2 * a > LEN) a = LEN - a;
+    if constexpr (LEN == 12 || LEN == 24) {
+        switch (24 / LEN * a) {
+            case 0: return 1.0;
+            case 1: return 0.96592582628906828675;
+            case 2: return 0.86602540378443864676;
+            case 3: return 0.70710678118654752440;
+            case 4: return 0.5;
+            case 5: return 0.25881904510252076235;
+            case 6: return 0.0;
+            case 7: return -0.25881904510252076235;
+            case 8: return -0.5;
+            case 9: return -0.70710678118654752440;
+            case 10: return -0.86602540378443864676;
+            case 11: return -0.96592582628906828675;
+            default: return -1.0;
+        }
+    } else if constexpr (LEN == 16) {
+        switch (a) {
+            case 0: return 1.0;
+            case 1: return 0.92387953251128675613;
+            case 2: return 0.70710678118654752440;
+            case 3: return 0.38268343236508977173;
+            case 4: return 0.0;
+            case 5: return -0.38268343236508977173;
+            case 6: return -0.70710678118654752440;
+            case 7: return -0.92387953251128675613;
+            default: return -1.0;
+        }
     } else {
-        constexpr int R = radix_at(H, IDX);
-        pass_ct<T, S, H, ROWS, R, NS>(src, dst, tw);
-        __syncthreads();
-        return passes_ct<T, S, H, ROWS, IDX + 1, NS * R>(dst, src, tw);
-    }
-}
-
-// First pass of a forward transform (unit twiddles), reading its inputs straight
-// from the grid rows in global memory: consecutive threads take consecutive
-// butterflies of a row, so each of the R loads is a contiguous run per row.
-template <typename T, int H, int ROWS, int R>
-__device__ __forceinline__ void pass_ct_first_global(const cpx<T> *__restrict__ g, int rows, cpx<T> *dst) {
-    constexpr int NQ = H / R, NIT = ROWS * NQ, HP = fpad_row<H>();
-    for (int it = threadIdx.x; it < NIT; it += blockDim.x) {
-        const int row = it / NQ, t = it - row * NQ;
-        cpx<T> v[R];
-        if (row < rows) {
-            const cpx<T> *s = g + (size_t)row * H;
-#pragma unroll
-            for (int r = 0; r < R; r++) v[r] = s[t + r * NQ];
-        } else {
-#pragma unroll
-            for (int r = 0; r < R; r++) v[r] = cpx<T>{0, 0};
+        static_assert(LEN == 20, "twiddle table");
+        switch (a) {
+            case 0: return 1.0;
+            case 1: return 0.95105651629515357212;
+            case 2: return 0.80901699437494742410;
+            case 3: return 0.58778525229247312917;
+            case 4: return 0.30901699437494742410;
+            case 5: return 0.0;
+            case 6: return -0.30901699437494742410;
+            case 7: return -0.58778525229247312917;
+            case 8: return -0.80901699437494742410;
+            case 9: return -0.95105651629515357212;
+            default: return -1.0;
         }
-        dftR<T, -1, R>(v);
-        cpx<T> *d = dst + row * HP;
-#pragma unroll
-        for (int r = 0; r < R; r++) d[fpad(t * R + r)] = v[r];
     }
 }
-
-// The same first pass for rows at arbitrary places: row r of the block is grid
-// row rowg[r] (in units of rows), or zeros where rowg[r] < 0.
-template <typename T, int H, int ROWS, int R>
-__device__ __forceinline__ void pass_ct_first_rows(const cpx<T> *__restrict__ g, const long long *rowg,
-                                                   cpx<T> *dst) {
-    constexpr int NQ = H / R, NIT = ROWS * NQ, HP = fpad_row<H>();
-    for (int it = threadIdx.x; it < NIT; it += blockDim.x) {
-        const int row = it / NQ, t = it - row * NQ;
-        const long long gr = rowg[row];
-        cpx<T> v[R];
-        if (gr >= 0) {
-            const cpx<T> *s = g + gr * H;
+// v * e^{S 2 pi i a / LEN} for a constant a
+template <typename T, int S, int LEN>
+__device__ __forceinline__ cpx<T> cmul_len(cpx<T> v, int a) {
+    a %= LEN;
+    if (a == 0) return v;
+    if (4 * a == LEN) return rot90<T, S>(v);
+    if (2 * a == LEN) return cpx<T>{-v.x, -v.y};
+    if (4 * a == 3 * LEN) return rot90<T, -S>(v);
+    const T c = (T)cos_len<LEN>(a), s = (T)(S * cos_len<LEN>(a - LEN / 4));   // sin(x) = cos(x - pi/2)
+    return cpx<T>{v.x * c - v.y * s, v.x * s + v.y * c};
+}
+// A*B-point DFT in registers, V[k] = sum_n v[n] e^{S 2 pi i nk/(AB)}:
+// n = B n1 + n2, k = k1 + A k2; A-point DFTs over n1, twiddles W^{n2 k1},
+// B-point DFTs over n2
+template <typename T, int S, int A, int B>
+__device__ __forceinline__ void dft_ab(cpx<T> *v) {
+    cpx<T> a[A * B];
 #pragma unroll
-            for (int r = 0; r < R; r++) v[r] = s[t + r * NQ];
-        } else {
+    for (int n2 = 0; n2 < B; n2++) {
+        cpx<T> t[A];
 #pragma unroll
-            for (int r = 0; r < R; r++) v[r] = cpx<T>{0, 0};
-        }
-        dftR<T, -1, R>(v);
-        cpx<T> *d = dst + row * HP;
+        for (int n1 = 0; n1 < A; n1++) t[n1] = v[B * n1 + n2];
+        dftR<T, S, A>(t);
 #pragma unroll
-        for (int r = 0; r < R; r++) d[fpad(t * R + r)] = v[r];
+        for (int k1 = 0; k1 < A; k1++) a[A * n2 + k1] = cmul_len<T, S, A * B>(t[k1], n2 * k1);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < A; k1++) {
+        cpx<T> t[B];
+#pragma unroll
+        for (int n2 = 0; n2 < B; n2++) t[n2] = a[A * n2 + k1];
+        dftR<T, S, B>(t);
+#pragma unroll
+        for (int k2 = 0; k2 < B; k2++) v[k1 + A * k2] = t[k2];
     }
 }
+template <typename T, int S, int LEN>
+__device__ __forceinline__ void dft_len(cpx<T> *v) {
+    if constexpr (LEN == 12) dft_ab<T, S, 3, 4>(v);
+    else if constexpr (LEN == 16) dft_ab<T, S, 4, 4>(v);
+    else if constexpr (LEN == 20) dft_ab<T, S, 5, 4>(v);
+    else if constexpr (LEN == 24) dft_ab<T, S, 3, 8>(v);
+    else dftR<T, S, LEN>(v);
+}
 
-// Passes IDX.. of a transform whose last pass writes the rows < rows straight
-// to global memory (row-contiguous): in the last pass NS*R = H, so output
-// t + r*NS of consecutive threads is a contiguous run.
-template <typename T, int S, int H, int ROWS, int IDX, int NS>
-__device__ __forceinline__ void passes_ct_to_global(cpx<T> *src, cpx<T> *dst, const cpx<T> *tw, cpx<T> *g,
-                                                    int rows) {
-    constexpr int R = radix_at(H, IDX);
-    if constexpr (IDX + 1 < radix_count(H)) {
-        pass_ct<T, S, H, ROWS, R, NS>(src, dst, tw);
-        __syncthreads();
-        passes_ct_to_global<T, S, H, ROWS, IDX + 1, NS * R>(dst, src, tw, g, rows);
+// FP64 sum of a grid row of 2 P Q reals held by P consecutive lanes, lane t
+// holding the complex elements t + P j (j < Q): each lane adds its values in
+// j order (real part first), then the P lanes combine by an xor butterfly, so
+// every lane ends with the same value
+template <int P, int Q>
+__device__ __forceinline__ double row_sum_fp64(const cpx<float> *v) {
+    double a = 0.0;
+#pragma unroll
+    for (int j = 0; j < Q; j++) {
+        a += (double)v[j].x;
+        a += (double)v[j].y;
+    }
+#pragma unroll
+    for (int o = 1; o < P; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
+}
+
+// Which fields of a forward set the n = 0 kernel needs row sums of: the
+// temperature and humidity tendencies and (gridpointa) the ln ps tendency
+struct RowSums {
+    double *out = nullptr;   // one per grid row; null: none
+    int L = 0, dset = 0;
+    __device__ __forceinline__ bool field(long long f) const {
+        if (!out) return false;
+        const int nfi = dset ? 4 * L : 9 * L + 1, i = (int)(f % nfi);
+        return dset ? i < L || i >= 3 * L : i < 2 * L || i == 7 * L;
+    }
+};
+
+__device__ __forceinline__ void cp_async8(void *dst_smem, const void *src_gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(tc::smem_u32(dst_smem)), "l"(src_gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void *dst_smem, const void *src_gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_u32(dst_smem)), "l"(src_gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// the Fourier coefficient X_k of a real row from Z_k and Z_{h-k} of its
+// half-length complex transform (k > 0), scaled by 1/n
+template <typename T>
+__device__ __forceinline__ cpx<T> rf_split(cpx<T> a, cpx<T> b, cpx<T> wk, T scale) {
+    const cpx<T> E{(T)0.5 * (a.x + b.x), (T)0.5 * (a.y - b.y)};
+    const cpx<T> O{(T)0.5 * (a.y + b.y), (T)0.5 * (b.x - a.x)};
+    const cpx<T> wo = cmul(wk, O);
+    return cpx<T>{(E.x + wo.x) * scale, (E.y + wo.y) * scale};
+}
+
+// Forward transform of block blk's RB rows.  FOLD: the block takes RB/2
+// latitude pairs j of one field (rows r and r + RB/2 a pair's northern and
+// southern rows) and stores E = X(j) + X(nlat-1-j) at row field*nlat + j and
+// O = X(j) - X(nlat-1-j) at row field*nlat + nlat/2 + j of the m-major side
+// (complex element (row, m) at row + m*f_ms), for the Legendre kernels; lot is
+// a multiple of nlat.  Otherwise row r's X_k goes to r*f_rs + k*f_ms.
+template <typename T, int N, bool FOLD>
+__device__ __forceinline__ void rr_fwd_body(const T *gp, T *fc, int nlat, long long lot, int kf, long long f_rs,
+                                            long long f_ms, const cpx<T> *__restrict__ w,
+                                            const cpx<T> *__restrict__ rt, RowSums rs, long long blk) {
+    using Lay = RrLayout<T, N>;
+    constexpr int P = Lay::P, Q = Lay::Q, H = Lay::H, RB = Lay::RB, QP = Lay::QP, PR = RB / 2;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cpx<T> *sm = reinterpret_cast<cpx<T> *>(smraw);
+    const int t = threadIdx.x % P, r = threadIdx.x / P;
+    const int nlath = nlat / 2, nbpf = FOLD ? (nlath + PR - 1) / PR : 1;
+    const long long field = FOLD ? blk / nbpf : 0, row0 = blk * RB;
+    const int j0 = FOLD ? (int)(blk - field * nbpf) * PR : 0;
+    long long grow;   // this thread's grid row, or -1
+    if constexpr (FOLD) {
+        const int j = j0 + (r % PR);
+        grow = j < nlath && field * nlat < lot ? field * nlat + (r < PR ? j : nlat - 1 - j) : -1;
     } else {
-        static_assert(NS * R == H, "last pass");
-        constexpr int NQ = H / R, NIT = ROWS * NQ, STEP = H / (NS * R), HP = fpad_row<H>();
-        for (int it = threadIdx.x; it < NIT; it += blockDim.x) {
-            const int row = it / NQ, t = it - row * NQ, k = t % NS;
-            if (row >= rows) continue;
-            const cpx<T> *s = src + row * HP;
-            cpx<T> v[R];
-#pragma unroll
-            for (int r = 0; r < R; r++) v[r] = s[fpad(t + r * NQ)];
-            if constexpr (NS > 1) {
-#pragma unroll
-                for (int r = 1; r < R; r++) {
-                    cpx<T> w = tw[r * k * STEP];
-                    if (S > 0) w.y = -w.y;
-                    v[r] = cmul(v[r], w);
-                }
-            }
-            dftR<T, S, R>(v);
-            cpx<T> *d = g + (size_t)row * H;
-#pragma unroll
-            for (int r = 0; r < R; r++) d[t + r * NS] = v[r];
-        }
+        grow = row0 + r < lot ? row0 + r : -1;
     }
-}
-
-template <typename T> struct vec2 { using t = float4; };
-template <> struct vec2<double> { using t = double2; };
-
-// block blk of a forward transform of lot rows (the kernels below pass blockIdx.x)
-template <typename T, int N, int ROWS>
-__device__ __forceinline__ void rfft_fwd_ct_body(const T *gp, T *fc, long long lot, int kf, long long f_rs,
-                                                 long long f_ms, const cpx<T> *__restrict__ wtab,
-                                                 const cpx<T> *__restrict__ rtab, long long blk) {
-    constexpr int H = N / 2, HP = fpad_row<H>();
-    extern __shared__ __align__(16) unsigned char smraw[];
-    cpx<T> *b0 = reinterpret_cast<cpx<T> *>(smraw);
-    cpx<T> *b1 = b0 + ROWS * HP;
-    // twiddles are read from global memory (L1-cached); shared memory holds only the rows
-    const cpx<T> *tw = wtab, *rt = rtab;
-    const long long row0 = blk * ROWS;
-    const int rows = (int)min((long long)ROWS, lot - row0);
+    cpx<T> v[Q];
     pdl_trigger();
-    pdl_wait();   // the grid rows may come from the previous kernel
-    // the first pass reads the grid rows directly (unit twiddles); the rest run in shared memory
-    constexpr int R0 = radix_at(H, 0);
-    pass_ct_first_global<T, H, ROWS, R0>(reinterpret_cast<const cpx<T> *>(gp + row0 * N), rows, b1);
-    __syncthreads();
-    const cpx<T> *Z = passes_ct<T, -1, H, ROWS, 1, R0>(b1, b0, tw);
-    const T scale = (T)1 / (T)N;
-    // X_k and X_{H-k} from Z_k and Z_{H-k} (k <= H/2), each Z read once; only
-    // k < kf are stored.  Rows fastest: consecutive threads write adjacent
-    // entries of the m-major side.
-    auto fold = [&](cpx<T> a, cpx<T> b, int k) {
-        const cpx<T> E{(T)0.5 * (a.x + b.x), (T)0.5 * (a.y - b.y)};
-        const cpx<T> O{(T)0.5 * (a.y + b.y), (T)0.5 * (b.x - a.x)};
-        const cpx<T> wo = cmul(rt[k], O);
-        return cpx<T>{(E.x + wo.x) * scale, (E.y + wo.y) * scale};
-    };
-    const int kh = min(H / 2, kf - 1);   // pairs (k, H-k) with k <= kh cover every k < kf
-    for (int it = threadIdx.x; it < ROWS * (kh + 1); it += blockDim.x) {
-        const int row = it % ROWS, k = it / ROWS, k2 = H - k;
-        if (row >= rows) continue;
-        const cpx<T> *z = Z + row * HP;
-        T *fr = fc + 2 * ((row0 + row) * f_rs);
-        const cpx<T> a = z[fpad(k)];
-        if (k == 0) {
-            *reinterpret_cast<cpx<T> *>(fr) = cpx<T>{(a.x + a.y) * scale, (T)0};
-            continue;
-        }
-        const cpx<T> b = z[fpad(k2)];
-        *reinterpret_cast<cpx<T> *>(fr + 2 * (long long)k * f_ms) = fold(a, b, k);
-        if (k2 < kf && k2 != k) *reinterpret_cast<cpx<T> *>(fr + 2 * (long long)k2 * f_ms) = fold(b, a, k2);
-    }
-}
-
-// Forward transform that writes the Fourier side folded about the equator,
-// for the tensor-core Legendre kernel: for a field of nlat grid rows (north to
-// south) and latitude pair j < nlat/2 it stores E = X(j) + X(nlat-1-j) at row
-// field*nlat + j and O = X(j) - X(nlat-1-j) at row field*nlat + nlat/2 + j of
-// the m-major side (complex element (row, m) at row + m*f_ms).  A block takes
-// ROWS/2 latitude pairs of one field: rows r and r + ROWS/2 are a pair's
-// northern and southern rows.  lot is a multiple of nlat.
-template <typename T, int N, int ROWS>
-__device__ __forceinline__ void rfft_fwd_fold_body(const T *gp, T *fc, int nlat, long long lot, int kf,
-                                                   long long f_ms, const cpx<T> *__restrict__ wtab,
-                                                   const cpx<T> *__restrict__ rtab, long long blk) {
-    constexpr int H = N / 2, HP = fpad_row<H>(), PR = ROWS / 2;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    cpx<T> *b0 = reinterpret_cast<cpx<T> *>(smraw);
-    cpx<T> *b1 = b0 + ROWS * HP;
-    // twiddles are read from global memory (L1-cached); shared memory holds only the rows
-    const cpx<T> *tw = wtab, *rt = rtab;
-    __shared__ long long rowg[ROWS];
-    const int nlath = nlat / 2, nbpf = (nlath + PR - 1) / PR;
-    const long long field = blk / nbpf;
-    const int j0 = (int)(blk - field * nbpf) * PR;
-    if (threadIdx.x < ROWS) {
-        const int r = threadIdx.x, j = j0 + (r % PR);
-        const int lat = r < PR ? j : nlat - 1 - j;
-        rowg[r] = (j < nlath && field * nlat < lot) ? field * nlat + lat : -1;
-    }
-    pdl_trigger();
-    __syncthreads();
     pdl_wait();   // the grid rows may come from the previous kernel, which may still read the output
-    constexpr int R0 = radix_at(H, 0);
-    pass_ct_first_rows<T, H, ROWS, R0>(reinterpret_cast<const cpx<T> *>(gp), rowg, b1);
-    __syncthreads();
-    const cpx<T> *Z = passes_ct<T, -1, H, ROWS, 1, R0>(b1, b0, tw);
-    const T scale = (T)1 / (T)N;
-    auto fold = [&](cpx<T> a, cpx<T> b, int k) {
-        const cpx<T> E{(T)0.5 * (a.x + b.x), (T)0.5 * (a.y - b.y)};
-        const cpx<T> O{(T)0.5 * (a.y + b.y), (T)0.5 * (b.x - a.x)};
-        const cpx<T> wo = cmul(rt[k], O);
-        return cpx<T>{(E.x + wo.x) * scale, (E.y + wo.y) * scale};
-    };
-    auto put = [&](long long row, int k, cpx<T> xn, cpx<T> xs) {
-        T *fr = fc + 2 * (row + (long long)k * f_ms);
-        *reinterpret_cast<cpx<T> *>(fr) = cpx<T>{xn.x + xs.x, xn.y + xs.y};
-        *reinterpret_cast<cpx<T> *>(fr + 2 * (long long)nlath) = cpx<T>{xn.x - xs.x, xn.y - xs.y};
-    };
-    const int kh = min(H / 2, kf - 1);   // pairs (k, H-k) with k <= kh cover every k < kf
-    for (int it = threadIdx.x; it < PR * (kh + 1); it += blockDim.x) {
-        const int pr = it % PR, k = it / PR, k2 = H - k, j = j0 + pr;
-        if (rowg[pr] < 0) continue;
-        const long long row = field * nlat + j;     // E row; O is nlath further
-        const cpx<T> *zn = Z + pr * HP, *zs = Z + (pr + PR) * HP;
-        const cpx<T> an = zn[fpad(k)], as = zs[fpad(k)];
-        if (k == 0) {
-            put(row, 0, cpx<T>{(an.x + an.y) * scale, (T)0}, cpx<T>{(as.x + as.y) * scale, (T)0});
-            continue;
+    {
+        const cpx<T> *g = reinterpret_cast<const cpx<T> *>(gp) + (grow < 0 ? 0 : grow) * H + t;
+#pragma unroll
+        for (int j = 0; j < Q; j++) v[j] = grow < 0 ? cpx<T>{0, 0} : g[P * j];
+    }
+    if constexpr (FOLD && sizeof(T) == 4) {
+        if (rs.field(field)) {   // block-uniform
+            const double a = row_sum_fp64<P, Q>(v);
+            if (grow >= 0 && t == 0) rs.out[grow] = a;
         }
-        const cpx<T> bn = zn[fpad(k2)], bs = zs[fpad(k2)];
-        put(row, k, fold(an, bn, k), fold(as, bs, k));
-        if (k2 < kf && k2 != k) put(row, k2, fold(bn, an, k2), fold(bs, as, k2));
+    }
+    dft_len<T, -1, Q>(v);
+    cpx<T> *x = sm + r * Lay::RS;
+    x[t] = v[0];
+#pragma unroll
+    for (int q = 1; q < Q; q++) x[q * (P + 1) + t] = cmul(v[q], w[t * q]);   // t q < h
+    __syncwarp();
+    cpx<T> z[QP][P];
+#pragma unroll
+    for (int i = 0; i < QP; i++) {
+        if (Q % P != 0 && t + P * i >= Q) continue;
+#pragma unroll
+        for (int u = 0; u < P; u++) z[i][u] = x[(t + P * i) * (P + 1) + u];
+        dft_len<T, -1, P>(z[i]);
+    }
+    __syncthreads();   // the spectra overwrite the transposition
+    cpx<T> *zr = sm + r * Lay::RZ;
+#pragma unroll
+    for (int i = 0; i < QP; i++) {
+        if (Q % P != 0 && t + P * i >= Q) continue;
+#pragma unroll
+        for (int m = 0; m < P; m++) zr[t + P * i + Q * m] = z[i][m];
+    }
+    __syncthreads();
+    const T scale = (T)1 / (T)N;
+    const int kh = min(H / 2, kf - 1);   // pairs (k, h-k) with k <= kh cover every k < kf
+    cpx<T> *out = reinterpret_cast<cpx<T> *>(fc);
+    if constexpr (FOLD) {
+        for (int it = threadIdx.x; it < PR * (kh + 1); it += RR_THREADS) {
+            const int pr = it % PR, k = it / PR, k2 = H - k, j = j0 + pr;
+            if (j >= nlath || field * nlat >= lot) continue;
+            cpx<T> *fr = out + field * nlat + j;   // E row; O is nlath further
+            const cpx<T> *zn = sm + pr * Lay::RZ, *zs = sm + (pr + PR) * Lay::RZ;
+            const cpx<T> an = zn[k], as = zs[k];
+            auto put = [&](int kk, cpx<T> xn, cpx<T> xs) {
+                cpx<T> *fk = fr + (long long)kk * f_ms;
+                fk[0] = cpx<T>{xn.x + xs.x, xn.y + xs.y};
+                fk[nlath] = cpx<T>{xn.x - xs.x, xn.y - xs.y};
+            };
+            if (k == 0) {
+                put(0, cpx<T>{(an.x + an.y) * scale, (T)0}, cpx<T>{(as.x + as.y) * scale, (T)0});
+                continue;
+            }
+            const cpx<T> bn = zn[k2], bs = zs[k2], wk = rt[k];
+            put(k, rf_split(an, bn, wk, scale), rf_split(as, bs, wk, scale));
+            if (k2 < kf && k2 != k) {
+                const cpx<T> wk2 = rt[k2];
+                put(k2, rf_split(bn, an, wk2, scale), rf_split(bs, as, wk2, scale));
+            }
+        }
+    } else {
+        const int rows = (int)min((long long)RB, lot - row0);
+        const bool kfast = f_ms == 1;   // row-major Fourier side: k fastest across threads
+        for (int it = threadIdx.x; it < RB * (kh + 1); it += RR_THREADS) {
+            const int rr = kfast ? it / (kh + 1) : it % RB, k = kfast ? it - rr * (kh + 1) : it / RB, k2 = H - k;
+            if (rr >= rows) continue;
+            const cpx<T> *zz = sm + rr * Lay::RZ;
+            cpx<T> *fr = out + (row0 + rr) * f_rs;
+            const cpx<T> a = zz[k];
+            if (k == 0) {
+                fr[0] = cpx<T>{(a.x + a.y) * scale, (T)0};
+                continue;
+            }
+            const cpx<T> b = zz[k2];
+            fr[(long long)k * f_ms] = rf_split(a, b, rt[k], scale);
+            if (k2 < kf && k2 != k) fr[(long long)k2 * f_ms] = rf_split(b, a, rt[k2], scale);
+        }
     }
 }
 
-template <typename T, int N, int ROWS>
-__device__ __forceinline__ void rfft_inv_ct_body(const T *fc, T *gp, long long lot, int kf, long long f_rs,
-                                                 long long f_ms, const cpx<T> *__restrict__ wtab,
-                                                 const cpx<T> *__restrict__ rtab, long long blk) {
-    constexpr int H = N / 2, HP = fpad_row<H>();
+// Inverse transform of block blk's RB rows (coefficients k < kf, zero above)
+template <typename T, int N>
+__device__ __forceinline__ void rr_inv_body(const T *fc, T *gp, long long lot, int kf, long long f_rs, long long f_ms,
+                                            const cpx<T> *__restrict__ w, const cpx<T> *__restrict__ rt, long long blk) {
+    using Lay = RrLayout<T, N>;
+    constexpr int P = Lay::P, Q = Lay::Q, H = Lay::H, RB = Lay::RB, QP = Lay::QP, RC = Lay::RC;
     extern __shared__ __align__(16) unsigned char smraw[];
-    cpx<T> *b0 = reinterpret_cast<cpx<T> *>(smraw);
-    cpx<T> *b1 = b0 + ROWS * HP;
-    // twiddles are read from global memory (L1-cached); shared memory holds only the rows
-    const cpx<T> *tw = wtab;
-    const long long row0 = blk * ROWS;
-    const int rows = (int)min((long long)ROWS, lot - row0);
+    cpx<T> *sm = reinterpret_cast<cpx<T> *>(smraw);
+    const int t = threadIdx.x % P, r = threadIdx.x / P;
+    const long long row0 = blk * RB;
+    const int rows = (int)min((long long)RB, lot - row0);
     pdl_trigger();
     pdl_wait();   // the coefficients come from the previous kernel
-    // Z_k and Z_{H-k} of the half-length complex transform from c_k and c_{H-k}
-    // (c = 0 for k >= kf, and the m = 0 imaginary part ignored), one load of
-    // each coefficient; rows fastest, so consecutive threads read adjacent
-    // entries of the m-major side
-    auto unfold = [](cpx<T> a, cpx<T> b, cpx<T> w) {
-        const cpx<T> E{a.x + b.x, a.y - b.y};
-        const cpx<T> D{a.x - b.x, a.y + b.y};
-        w.y = -w.y;
-        const cpx<T> O = cmul(D, w);
-        return cpx<T>{E.x - O.y, E.y + O.x};
-    };
-    for (int it = threadIdx.x; it < ROWS * (H / 2 + 1); it += blockDim.x) {
-        const int row = it % ROWS, k = it / ROWS, k2 = H - k;
-        cpx<T> a{0, 0}, b{0, 0};
-        if (row < rows) {
-            const T *fr = fc + 2 * ((row0 + row) * f_rs);
+    {
+        const cpx<T> *fcc = reinterpret_cast<const cpx<T> *>(fc) + row0 * f_rs;
+        const bool kfast = f_ms == 1;
+        for (int i = threadIdx.x; i < kf * RB; i += RR_THREADS) {
+            const int k = kfast ? i % kf : i / RB, rr = kfast ? i / kf : i % RB;
+            cpx<T> *dst = sm + k * RC + rr;
+            if (rr >= rows) *dst = cpx<T>{0, 0};
+            else if constexpr (sizeof(T) == 4) cp_async8(dst, fcc + rr * f_rs + (long long)k * f_ms);
+            else cp_async16(dst, fcc + rr * f_rs + (long long)k * f_ms);
+        }
+        cp_async_commit();
+        cp_async_wait_all();
+        __syncthreads();
+    }
+    cpx<T> z[QP][P];
+#pragma unroll
+    for (int i = 0; i < QP; i++) {
+        const int q = t + P * i;
+        if (Q % P != 0 && q >= Q) continue;
+#pragma unroll
+        for (int m = 0; m < P; m++) {
+            const int k = q + Q * m, k2 = H - k;
+            cpx<T> a{0, 0}, b{0, 0};
             if (k < kf) {
-                a = *reinterpret_cast<const cpx<T> *>(fr + 2 * (long long)k * f_ms);
+                a = sm[k * RC + r];
                 if (k == 0) a.y = 0;
             }
-            if (k > 0 && k2 < kf) b = *reinterpret_cast<const cpx<T> *>(fr + 2 * (long long)k2 * f_ms);
+            if (k > 0 && k2 < kf) b = sm[k2 * RC + r];
+            // Z_k of the half-length complex sequence (c = 0 for k >= kf, the m = 0 imaginary part ignored)
+            const cpx<T> E{a.x + b.x, a.y - b.y}, D{a.x - b.x, a.y + b.y};
+            cpx<T> wk = rt[k];
+            wk.y = -wk.y;
+            const cpx<T> O = cmul(D, wk);
+            z[i][m] = cpx<T>{E.x - O.y, E.y + O.x};
         }
-        b0[row * HP + fpad(k)] = unfold(a, b, rtab[k]);
-        if (k > 0 && k2 != k) b0[row * HP + fpad(k2)] = unfold(b, a, rtab[k2]);
+        dft_len<T, +1, P>(z[i]);
     }
-    __syncthreads();
-    // the last pass writes the grid rows directly
-    passes_ct_to_global<T, +1, H, ROWS, 0, 1>(b0, b1, tw, reinterpret_cast<cpx<T> *>(gp + row0 * N), rows);
+    __syncthreads();   // the staged coefficients are read; the transposition overwrites them
+    cpx<T> *x = sm + r * Lay::RS;
+#pragma unroll
+    for (int i = 0; i < QP; i++) {
+        if (Q % P != 0 && t + P * i >= Q) continue;
+#pragma unroll
+        for (int u = 0; u < P; u++) x[(t + P * i) * (P + 1) + u] = z[i][u];
+    }
+    __syncwarp();
+    cpx<T> v[Q];
+    v[0] = x[t];
+#pragma unroll
+    for (int q = 1; q < Q; q++) {
+        const cpx<T> wq = w[t * q];
+        v[q] = cmul(x[q * (P + 1) + t], cpx<T>{wq.x, -wq.y});
+    }
+    dft_len<T, +1, Q>(v);
+    if (r < rows) {
+        cpx<T> *g = reinterpret_cast<cpx<T> *>(gp) + (row0 + r) * H + t;
+#pragma unroll
+        for (int j = 0; j < Q; j++) g[P * j] = v[j];
+    }
 }
 
-template <typename T, int N, int ROWS>
-__global__ void __launch_bounds__(256) k_rfft_fwd_ct(const T *gp, T *fc, long long lot, int kf, long long f_rs,
-                                                      long long f_ms, const cpx<T> *__restrict__ wtab,
-                                                      const cpx<T> *__restrict__ rtab) {
-    rfft_fwd_ct_body<T, N, ROWS>(gp, fc, lot, kf, f_rs, f_ms, wtab, rtab, blockIdx.x);
+template <typename T, int N, bool FOLD>
+__global__ void __launch_bounds__(RR_THREADS) k_rfft_fwd_rr(const T *gp, T *fc, int nlat, long long lot, int kf,
+                                                             long long f_rs, long long f_ms, const cpx<T> *__restrict__ w,
+                                                             const cpx<T> *__restrict__ rt, RowSums rs) {
+    rr_fwd_body<T, N, FOLD>(gp, fc, nlat, lot, kf, f_rs, f_ms, w, rt, rs, blockIdx.x);
 }
-template <typename T, int N, int ROWS>
-__global__ void __launch_bounds__(256) k_rfft_inv_ct(const T *fc, T *gp, long long lot, int kf, long long f_rs,
-                                                      long long f_ms, const cpx<T> *__restrict__ wtab,
-                                                      const cpx<T> *__restrict__ rtab) {
-    rfft_inv_ct_body<T, N, ROWS>(fc, gp, lot, kf, f_rs, f_ms, wtab, rtab, blockIdx.x);
-}
-
-template <typename T> constexpr int ct_rows(int n) {
-    return (sizeof(T) == 4) ? (n <= 256 ? 16 : 8) : (n <= 256 ? 8 : 4);
+template <typename T, int N>
+__global__ void __launch_bounds__(RR_THREADS) k_rfft_inv_rr(const T *fc, T *gp, long long lot, int kf, long long f_rs,
+                                                             long long f_ms, const cpx<T> *__restrict__ w,
+                                                             const cpx<T> *__restrict__ rt) {
+    rr_inv_body<T, N>(fc, gp, lot, kf, f_rs, f_ms, w, rt, blockIdx.x);
 }
 
-template <typename T, int N, int ROWS>
-__global__ void __launch_bounds__(256) k_rfft_fwd_fold(const T *gp, T *fc, int nlat, long long lot, int kf,
-                                                        long long f_ms, const cpx<T> *__restrict__ wtab,
-                                                        const cpx<T> *__restrict__ rtab) {
-    rfft_fwd_fold_body<T, N, ROWS>(gp, fc, nlat, lot, kf, f_ms, wtab, rtab, blockIdx.x);
-}
-
-// ------------------------------------------------ register-resident transforms
-// For h = P*Q complex points with P | Q, P threads work a row:
-//   Z[q + Q m] = sum_t W_P^{t m} W_h^{t q} sum_j z[t + P j] W_Q^{j q}   (W = e^{-2 pi i/.})
-// Thread t takes the Q-point DFT of its column z[t + P j] in registers and
-// applies W_h^{t q}; one transposition through shared memory then hands it the
-// Q/P whole P-point DFTs q = (Q/P) t + i.  The inverse runs the same steps in
-// the other order.  A block of NT threads works RB = NT/P rows.  The grid
+// ------------------------------- n = 384 in FP32 (T127): bulk copies, persistent
+// The same transform with P = 8, Q = 24 for the largest throughput case: the grid
 // rows (contiguous 4n-byte runs) move between global and shared memory as bulk
 // (TMA) copies, one per row; the inverse's Fourier coefficients, runs of only
-// RB complex values per wavenumber, arrive by plain coalesced loads.  The
-// twiddles W_h^{t q} sit in a per-block table, Q contiguous values per t.
+// RB complex values per wavenumber, arrive by cp.async; the twiddles W_h^{t q}
+// sit in a per-block table, Q contiguous values per t.
 __device__ int g_fft_error;   // nonzero: a bounded wait in an FFT kernel gave up
 
 template <int N> struct RfShape { static constexpr int P = 0, Q = 0, NT = 256; };
@@ -603,66 +644,6 @@ template <int N> struct RfLayout {
     static_assert(H * RC <= R, "the staged coefficients fit region R");
     static_assert(RB <= 32 && RB % 4 == 0, "warp 0 issues one row copy per lane");
 };
-
-// cos(2 pi a / 24) for an integer a (multiples of 15 degrees)
-__host__ __device__ constexpr double cos24(int a) {
-    a = ((a % 24) + 24) % 24;
-    if (a > 12) a = 24 - a;
-    switch (a) {
-        case 0: return 1.0;
-        case 1: return 0.96592582628906828675;
-        case 2: return 0.86602540378443864676;
-        case 3: return 0.70710678118654752440;
-        case 4: return 0.5;
-        case 5: return 0.25881904510252076235;
-        case 6: return 0.0;
-        case 7: return -0.25881904510252076235;
-        case 8: return -0.5;
-        case 9: return -0.70710678118654752440;
-        case 10: return -0.86602540378443864676;
-        case 11: return -0.96592582628906828675;
-        default: return -1.0;
-    }
-}
-// v * e^{S 2 pi i a / 24} for a constant a
-template <typename T, int S>
-__device__ __forceinline__ cpx<T> cmul_w24(cpx<T> v, int a) {
-    a %= 24;
-    if (a == 0) return v;
-    if (a == 6) return rot90<T, S>(v);
-    if (a == 12) return cpx<T>{-v.x, -v.y};
-    if (a == 18) return rot90<T, -S>(v);
-    const T c = (T)cos24(a), s = (T)(S * cos24(a - 6));   // sin(x) = cos(x - pi/2)
-    return cpx<T>{v.x * c - v.y * s, v.x * s + v.y * c};
-}
-// 24-point DFT in registers, V[k] = sum_n v[n] e^{S 2 pi i nk/24}:
-// n = 8 n1 + n2, k = k1 + 3 k2; 3-point DFTs over n1, twiddles W_24^{n2 k1},
-// 8-point DFTs over n2
-template <typename T, int S>
-__device__ __forceinline__ void dft24(cpx<T> *v) {
-    cpx<T> a[24];
-#pragma unroll
-    for (int n2 = 0; n2 < 8; n2++) {
-        cpx<T> t[3] = {v[n2], v[8 + n2], v[16 + n2]};
-        dft3<T, S>(t);
-#pragma unroll
-        for (int k1 = 0; k1 < 3; k1++) a[3 * n2 + k1] = cmul_w24<T, S>(t[k1], n2 * k1);
-    }
-#pragma unroll
-    for (int k1 = 0; k1 < 3; k1++) {
-        cpx<T> t[8];
-#pragma unroll
-        for (int n2 = 0; n2 < 8; n2++) t[n2] = a[3 * n2 + k1];
-        dft8<T, S>(t);
-#pragma unroll
-        for (int k2 = 0; k2 < 8; k2++) v[k1 + 3 * k2] = t[k2];
-    }
-}
-template <typename T, int S, int Q>
-__device__ __forceinline__ void dftQ(cpx<T> *v) {
-    static_assert(Q == 24, "register DFT length");
-    dft24<T, S>(v);
-}
 
 // bulk copy shared -> global in this thread's bulk group (16-byte aligned, size % 16 == 0)
 __device__ __forceinline__ void bulk_s2g(void *dst_gmem, const void *src_smem, uint32_t bytes) {
@@ -718,24 +699,6 @@ __device__ __forceinline__ bool rf_wait_loads(uint64_t *bar, uint32_t phase = 0)
     return ok;
 }
 
-// FP64 sum of a grid row of 2 P Q reals held by P consecutive lanes, lane t
-// holding the complex elements t + P j (j < Q): each lane adds its values in
-// j order (real part first), then the P lanes combine by an xor butterfly, so
-// every lane ends with the same value.  The n = 0 kernel (legendre_tc.cu) reproduces
-// this order when it sums the rows from global memory.
-template <int P, int Q>
-__device__ __forceinline__ double row_sum_fp64(const cpx<float> *v) {
-    double a = 0.0;
-#pragma unroll
-    for (int j = 0; j < Q; j++) {
-        a += (double)v[j].x;
-        a += (double)v[j].y;
-    }
-#pragma unroll
-    for (int o = 1; o < P; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    return a;
-}
-
 // Warp 0 issues one bulk copy per row of the block into `stage` (row stride
 // RG), completing on `bar`; rows without a source (grow(r) < 0) are zeroed by
 // their own threads.  grow(r) is row r's index in g (rows of n floats).
@@ -762,9 +725,9 @@ __device__ __forceinline__ void rf_issue_rows(const float *__restrict__ g, RowOf
 // the block).  `stage` and `x` may be the same region.  after_read() runs
 // once every thread has its row values in registers (a block barrier lies
 // before it), before x is written.
-template <int N, bool RSUM = false, int RZ = RfLayout<N>::RZ, typename AfterRead>
+template <int N, int RZ = RfLayout<N>::RZ, typename AfterRead>
 __device__ __forceinline__ void rf_forward_core(const cpx<float> *stage, cpx<float> *x, const cpx<float> *tqs,
-                                                AfterRead after_read, double *rsum = nullptr) {
+                                                AfterRead after_read, bool sums = false, double *rsum = nullptr) {
     using Lay = RfLayout<N>;
     constexpr int P = Lay::P, Q = Lay::Q, QP = Q / P;
     const int t = threadIdx.x % P, r = threadIdx.x / P;
@@ -774,8 +737,8 @@ __device__ __forceinline__ void rf_forward_core(const cpx<float> *stage, cpx<flo
     for (int j = 0; j < Q; j++) v[j] = s[P * j];
     __syncthreads();   // the staged rows are read
     after_read();
-    if constexpr (RSUM) *rsum = row_sum_fp64<P, Q>(v);   // after the next loads are on their way
-    dftQ<float, -1, Q>(v);
+    if (sums) *rsum = row_sum_fp64<P, Q>(v);   // block-uniform; after the next loads are on their way
+    dft_len<float, -1, Q>(v);
     const cpx<float> *tq = tqs + t * Lay::RT;
 #pragma unroll
     for (int q = 2; q < Q; q += 2) {
@@ -809,23 +772,15 @@ __device__ __forceinline__ void rf_forward_core(const cpx<float> *stage, cpx<flo
 // sits at S.r[r * RZ + k] (visible to the block).  grow(r) is row r's index in
 // g (rows of n floats), or < 0 for a zero row.  False if the loads timed out.
 template <int N, typename RowOf>
-__device__ __forceinline__ bool rf_forward_rows(const float *__restrict__ g, RowOf grow, const RfSmem<N> &S) {
+__device__ __forceinline__ bool rf_forward_rows(const float *__restrict__ g, RowOf grow, const RfSmem<N> &S,
+                                                bool sums = false, double *rsum = nullptr) {
     rf_issue_rows<N>(g, grow, S.r, S.bar);
     if (!rf_wait_loads(S.bar)) return false;
-    rf_forward_core<N>(S.r, S.r, S.tq, [] {});
+    rf_forward_core<N>(S.r, S.r, S.tq, [] {}, sums, rsum);
     return true;
 }
 
-// the Fourier coefficient X_k of a real row from Z_k and Z_{h-k} of its
-// half-length complex transform (k > 0), scaled by 1/n
-__device__ __forceinline__ cpx<float> rf_split(cpx<float> a, cpx<float> b, cpx<float> wk, float scale) {
-    const cpx<float> E{0.5f * (a.x + b.x), 0.5f * (a.y - b.y)};
-    const cpx<float> O{0.5f * (a.y + b.y), 0.5f * (b.x - a.x)};
-    const cpx<float> wo = cmul(wk, O);
-    return cpx<float>{(E.x + wo.x) * scale, (E.y + wo.y) * scale};
-}
-
-// rfft_fwd_ct_body for the register-resident lengths: RB rows per block
+// RB rows per block, rows to r*f_rs + k*f_ms
 template <int N>
 __device__ __forceinline__ void rfft_fwd_rf_body(const float *gp, float *fc, long long lot, int kf, long long f_rs,
                                                  long long f_ms, const cpx<float> *__restrict__ w,
@@ -859,13 +814,11 @@ __device__ __forceinline__ void rfft_fwd_rf_body(const float *gp, float *fc, lon
     }
 }
 
-// rfft_fwd_fold_body for the register-resident lengths: a block takes RB/2
-// latitude pairs of one field, rows r and r + RB/2 being a pair's northern and
-// southern rows
+// rr_fwd_body's folded form: a block takes RB/2 latitude pairs of one field
 template <int N>
 __device__ __forceinline__ void rfft_fwd_fold_rf_body(const float *gp, float *fc, int nlat, long long lot, int kf,
                                                       long long f_ms, const cpx<float> *__restrict__ w,
-                                                      const cpx<float> *__restrict__ rt, long long blk) {
+                                                      const cpx<float> *__restrict__ rt, RowSums rsel, long long blk) {
     using Lay = RfLayout<N>;
     constexpr int H = Lay::H, RB = Lay::RB, PR = RB / 2;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -881,7 +834,10 @@ __device__ __forceinline__ void rfft_fwd_fold_rf_body(const float *gp, float *fc
         const int j = j0 + (r % PR);
         return (fin && j < nlath) ? field * nlat + (r < PR ? j : nlat - 1 - j) : -1ll;
     };
-    if (!rf_forward_rows<N>(gp, grow, S)) return;
+    const bool sums = rsel.field(field);
+    double rs = 0.0;
+    if (!rf_forward_rows<N>(gp, grow, S, sums, &rs)) return;
+    if (sums && threadIdx.x % Lay::P == 0 && grow(threadIdx.x / Lay::P) >= 0) rsel.out[grow(threadIdx.x / Lay::P)] = rs;
     const float scale = 1.f / (float)N;
     auto put = [&](long long row, int k, cpx<float> xn, cpx<float> xs) {
         cpx<float> *fr = reinterpret_cast<cpx<float> *>(fc) + row + (long long)k * f_ms;
@@ -927,11 +883,11 @@ template <int N> struct RfPLayout {
     static_assert(OFF_X % 16 == 0 && OFF_TQ % 16 == 0 && OFF_BAR % 16 == 0, "16-byte aligned regions");
 };
 
-template <int N, bool RSUM>
+template <int N>
 __global__ void __launch_bounds__(128) k_rfft_fwd_fold_rf_p(const float *gp, float *fc, int nlat, long long lot,
                                                              int kf, long long f_ms, long long nitems,
                                                              const cpx<float> *__restrict__ w,
-                                                             const cpx<float> *__restrict__ rt, double *rowsum) {
+                                                             const cpx<float> *__restrict__ rt, RowSums rsel) {
     using Lay = RfLayout<N>;
     using PL = RfPLayout<N>;
     constexpr int H = Lay::H, RB = Lay::RB, PR = RB / 2;
@@ -969,15 +925,16 @@ __global__ void __launch_bounds__(128) k_rfft_fwd_fold_rf_p(const float *gp, flo
     for (uint32_t phase = 0; item < nitems; phase ^= 1) {
         if (!rf_wait_loads(bar, phase)) return;
         const long long next = item + gridDim.x;
+        const bool sums = rsel.field(item / nbpf);
         double rs = 0.0;
-        const long long myrow = RSUM ? grow_of(item)(threadIdx.x / Lay::P) : -1ll;
-        rf_forward_core<N, RSUM, PL::RZF>(G, X, tqs, [&] {
+        const long long myrow = sums ? grow_of(item)(threadIdx.x / Lay::P) : -1ll;
+        rf_forward_core<N, PL::RZF>(G, X, tqs, [&] {
             if (next < nitems) {
                 tc::fence_proxy_async();   // G was read (and zero rows written) through the generic proxy
                 rf_issue_rows<N>(gp, grow_of(next), G, bar);
             }
-        }, &rs);
-        if (RSUM && myrow >= 0 && threadIdx.x % Lay::P == 0) rowsum[myrow] = rs;
+        }, sums, &rs);
+        if (myrow >= 0 && threadIdx.x % Lay::P == 0) rsel.out[myrow] = rs;
         const long long field = item / nbpf;
         const int j0 = (int)(item - field * nbpf) * PR;
         const bool fin = field * nlat < lot;
@@ -1012,7 +969,7 @@ __global__ void __launch_bounds__(128) k_rfft_fwd_fold_rf_p(const float *gp, flo
     }
 }
 
-// rfft_inv_ct_body for the register-resident lengths: the block's
+// The block's
 // coefficients c_k (k < kf) are staged k-major in shared memory by plain
 // coalesced loads (a k's RB rows are one run of the m-major side); each thread
 // forms the Z_k of its own q from c_k and c_{h-k}, takes their P-point DFTs,
@@ -1091,7 +1048,7 @@ __device__ __forceinline__ void rfft_inv_rf_body(const float *fc, float *gp, lon
         v[q] = q ? cmul(cpx<float>{f.x, f.y}, cpx<float>{wq.x, -wq.y}) : cpx<float>{f.x, f.y};
         v[q + 1] = cmul(cpx<float>{f.z, f.w}, cpx<float>{wq.z, -wq.w});
     }
-    dftQ<float, +1, Q>(v);
+    dft_len<float, +1, Q>(v);
     __syncthreads();   // the transposition is read; the grid rows are staged over it
     cpx<float> *gs = S.r + r * Lay::RG + t;
 #pragma unroll
@@ -1110,12 +1067,6 @@ __device__ __forceinline__ void rfft_inv_rf_body(const float *fc, float *gp, lon
 // 8-byte copies (cp.async), so the next item's copies are issued as soon as
 // this item's coefficients are read and arrive while it is transformed and
 // stored; the transposition and the staged grid rows use a second region.
-__device__ __forceinline__ void cp_async8(void *dst_smem, const void *src_gmem) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(tc::smem_u32(dst_smem)), "l"(src_gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
 template <int N> struct RfIPLayout {
     using Lay = RfLayout<N>;
     static constexpr int RW = Lay::RS > Lay::RG ? Lay::RS : Lay::RG;
@@ -1205,7 +1156,7 @@ __global__ void __launch_bounds__(128) k_rfft_inv_rf_p(const float *fc, float *g
             v[q] = q ? cmul(cpx<float>{f.x, f.y}, cpx<float>{wq.x, -wq.y}) : cpx<float>{f.x, f.y};
             v[q + 1] = cmul(cpx<float>{f.z, f.w}, cpx<float>{wq.z, -wq.w});
         }
-        dftQ<float, +1, Q>(v);
+        dft_len<float, +1, Q>(v);
         __syncthreads();   // the transposition is read; the grid rows are staged over it
         cpx<float> *gs = wk_s + r * Lay::RG + t;
 #pragma unroll
@@ -1231,13 +1182,6 @@ __global__ void __launch_bounds__(256) k_rfft_inv_rf(const float *fc, float *gp,
                                                       const cpx<float> *__restrict__ rt) {
     rfft_inv_rf_body<N>(fc, gp, lot, kf, f_rs, f_ms, w, rt, blockIdx.x);
 }
-template <int N>
-__global__ void __launch_bounds__(256) k_rfft_fwd_fold_rf(const float *gp, float *fc, int nlat, long long lot, int kf,
-                                                           long long f_ms, const cpx<float> *__restrict__ w,
-                                                           const cpx<float> *__restrict__ rt) {
-    rfft_fwd_fold_rf_body<N>(gp, fc, nlat, lot, kf, f_ms, w, rt, blockIdx.x);
-}
-
 // ---------------------------------------------------------------- ensembles
 // One launch transforms the rows of up to FFT_ENS_MAXSEG segments of different
 // lengths (an uneven ensemble); block b belongs to the last segment whose
@@ -1247,7 +1191,8 @@ struct FftEnsArgs {
     float *out;
     long long lot, f_rs, f_ms;
     int n, kf, block0;
-    int fold_nlat;          // forward only: > 0 writes the equator-folded layout (rfft_fwd_fold_body)
+    int fold_nlat;          // forward only: > 0 writes the equator-folded layout (rr_fwd_body)
+    RowSums rs;             // forward only
     const cpx<float> *w, *r;
 };
 struct FftEnsLaunch {
@@ -1255,127 +1200,137 @@ struct FftEnsLaunch {
     int nseg;
 };
 
-template <bool FWD>
-__global__ void __launch_bounds__(256) k_rfft_ens(const __grid_constant__ FftEnsLaunch P) {
+// LONG: the launch has segments of length 384 or 512, whose bodies take more
+// registers per thread
+template <bool FWD, bool LONG>
+__global__ void __launch_bounds__(RR_THREADS) k_rfft_ens(const __grid_constant__ FftEnsLaunch P) {
     int s = 0;
     while (s + 1 < P.nseg && P.seg[s + 1].block0 <= (int)blockIdx.x) s++;
     const FftEnsArgs &S = P.seg[s];
     const long long blk = (long long)blockIdx.x - S.block0;
-    switch (S.n) {
-#define EXOTX_FFT_ENS_CASE(NN)                                                                                 \
-    case NN:                                                                                                   \
-        if (FWD && S.fold_nlat) rfft_fwd_fold_body<float, NN, ct_rows<float>(NN)>(S.in, S.out, S.fold_nlat, S.lot, S.kf, S.f_ms, S.w, S.r, blk); \
-        else if (FWD) rfft_fwd_ct_body<float, NN, ct_rows<float>(NN)>(S.in, S.out, S.lot, S.kf, S.f_rs, S.f_ms, S.w, S.r, blk); \
-        else rfft_inv_ct_body<float, NN, ct_rows<float>(NN)>(S.in, S.out, S.lot, S.kf, S.f_rs, S.f_ms, S.w, S.r, blk);    \
+#define EXOTX_FFT_ENS_CASE(NN)                                                                                        \
+    case NN:                                                                                                          \
+        if (FWD && S.fold_nlat)                                                                                       \
+            rr_fwd_body<float, NN, true>(S.in, S.out, S.fold_nlat, S.lot, S.kf, 1, S.f_ms, S.w, S.r, S.rs, blk);      \
+        else if (FWD) rr_fwd_body<float, NN, false>(S.in, S.out, 0, S.lot, S.kf, S.f_rs, S.f_ms, S.w, S.r, S.rs, blk); \
+        else rr_inv_body<float, NN>(S.in, S.out, S.lot, S.kf, S.f_rs, S.f_ms, S.w, S.r, blk);                         \
         break;
+    switch (S.n) {
         EXOTX_FFT_ENS_CASE(64)
         EXOTX_FFT_ENS_CASE(128)
         EXOTX_FFT_ENS_CASE(192)
         EXOTX_FFT_ENS_CASE(256)
         EXOTX_FFT_ENS_CASE(320)
-        EXOTX_FFT_ENS_CASE(512)
-#undef EXOTX_FFT_ENS_CASE
         default: break;
     }
-}
-// the register-resident lengths (more registers per thread) in a launch of their own
-template <bool FWD>
-__global__ void __launch_bounds__(256) k_rfft_ens_rf(const __grid_constant__ FftEnsLaunch P) {
-    int s = 0;
-    while (s + 1 < P.nseg && P.seg[s + 1].block0 <= (int)blockIdx.x) s++;
-    const FftEnsArgs &S = P.seg[s];
-    const long long blk = (long long)blockIdx.x - S.block0;
-    if (S.n == 384) {
-        if (FWD && S.fold_nlat) rfft_fwd_fold_rf_body<384>(S.in, S.out, S.fold_nlat, S.lot, S.kf, S.f_ms, S.w, S.r, blk);
-        else if (FWD) rfft_fwd_rf_body<384>(S.in, S.out, S.lot, S.kf, S.f_rs, S.f_ms, S.w, S.r, blk);
-        else rfft_inv_rf_body<384>(S.in, S.out, S.lot, S.kf, S.f_rs, S.f_ms, S.w, S.r, blk);
-    }
-}
-
-static bool ens_len(int n) {
-    return n == 64 || n == 128 || n == 192 || n == 256 || n == 320 || n == 384 || n == 512;
-}
-static bool rf_len_host(int n) { return n == 384; }
-static bool aligned16_(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-
-// one launch over the segments whose lengths have (rf) or have not (!rf) a
-// register-resident kernel
-static exotx_status fft_ens_group(bool fwd, bool rf, const FftEnsSeg *segs, int nseg, cudaStream_t s) {
-    FftEnsLaunch P;
-    P.nseg = 0;
-    int blocks = 0;
-    size_t smem = 0;
-    for (int i = 0; i < nseg; i++) {
-        const FftEnsSeg &g = segs[i];
-        if (rf_len_host(g.n) != rf) continue;
-        exotx_status st;
-        const FftTables *t = fft_tables(g.n, &st);
-        if (!t) return st;
-        const int rows = rf ? RfLayout<384>::RB : ct_rows<float>(g.n);
-        FftEnsArgs &a = P.seg[P.nseg++];
-        a.in = g.in; a.out = g.out; a.lot = g.lot; a.f_rs = g.f_rs; a.f_ms = g.f_ms; a.n = g.n; a.kf = g.kf;
-        a.fold_nlat = fwd ? g.fold_nlat : 0;
-        a.w = reinterpret_cast<const cpx<float> *>(t->w32);
-        a.r = reinterpret_cast<const cpx<float> *>(t->r32);
-        a.block0 = blocks;
-        if (a.fold_nlat) {
-            const int nbpf = (g.fold_nlat / 2 + rows / 2 - 1) / (rows / 2);
-            blocks += (int)(g.lot / g.fold_nlat) * nbpf;
-        } else {
-            blocks += (int)((g.lot + rows - 1) / rows);
+    if constexpr (LONG) {
+        switch (S.n) {
+            EXOTX_FFT_ENS_CASE(512)
+            case 384:
+                if (FWD && S.fold_nlat) rfft_fwd_fold_rf_body<384>(S.in, S.out, S.fold_nlat, S.lot, S.kf, S.f_ms, S.w, S.r, S.rs, blk);
+                else if (FWD) rfft_fwd_rf_body<384>(S.in, S.out, S.lot, S.kf, S.f_rs, S.f_ms, S.w, S.r, blk);
+                else rfft_inv_rf_body<384>(S.in, S.out, S.lot, S.kf, S.f_rs, S.f_ms, S.w, S.r, blk);
+                break;
+            default: break;
         }
-        const int hp = g.n / 2 + 2 * (g.n / 32);   // padded row, as fpad_row
-        smem = std::max(smem, rf ? RfLayout<384>::SMEM : 2 * (size_t)rows * hp * sizeof(cpx<float>));
     }
-    if (blocks == 0) return EXOTX_OK;
-    const int kid = fwd ? EXOTX_K_FFT_FORWARD : EXOTX_K_FFT_INVERSE;
-    void (*k)(FftEnsLaunch) = rf ? (fwd ? k_rfft_ens_rf<true> : k_rfft_ens_rf<false>)
-                                 : (fwd ? k_rfft_ens<true> : k_rfft_ens<false>);
-    if (smem > 48 * 1024) EXOTX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    cudaEvent_t ev = ktimer_start(kid, s);
-    k<<<blocks, rf ? RfLayout<384>::NT : 256, smem, s>>>(P);
-    EXOTX_CHECK_LAUNCH();
-    ktimer_stop(kid, s, ev);
-    return EXOTX_OK;
+#undef EXOTX_FFT_ENS_CASE
+}
+
+static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// run fn(integral_constant N) for a length with a specialised kernel
+template <typename Fn>
+static exotx_status by_len(int n, Fn fn) {
+    switch (n) {
+        case 64: return fn(std::integral_constant<int, 64>{});
+        case 128: return fn(std::integral_constant<int, 128>{});
+        case 192: return fn(std::integral_constant<int, 192>{});
+        case 256: return fn(std::integral_constant<int, 256>{});
+        case 320: return fn(std::integral_constant<int, 320>{});
+        case 384: return fn(std::integral_constant<int, 384>{});
+        case 512: return fn(std::integral_constant<int, 512>{});
+    }
+    return EXOTX_NOT_BUILT;
+}
+bool fft_fold_rowsum(int n) {
+    return by_len(n, [](auto) { return EXOTX_OK; }) == EXOTX_OK;
 }
 
 exotx_status fft_ens(bool fwd, const FftEnsSeg *segs, int nseg, cudaStream_t s) {
     if (nseg < 1 || nseg > FFT_ENS_MAXSEG) return EXOTX_BAD_ARG;
     for (int i = 0; i < nseg; i++) {
         const FftEnsSeg &g = segs[i];
-        if (!ens_len(g.n)) return EXOTX_NOT_BUILT;
-        if (!aligned16_(g.in) || !aligned16_(g.out)) return EXOTX_BAD_ARG;
+        if (by_len(g.n, [](auto) { return EXOTX_OK; }) != EXOTX_OK) return EXOTX_NOT_BUILT;
+        if (!aligned16(g.in) || !aligned16(g.out)) return EXOTX_BAD_ARG;
         const int fold = fwd ? g.fold_nlat : 0;
         if (fold && (g.n != 2 * fold || g.lot % fold || g.f_rs != 1)) return EXOTX_BAD_ARG;
     }
-    EXOTX_TRY(fft_ens_group(fwd, false, segs, nseg, s));
-    return fft_ens_group(fwd, true, segs, nseg, s);
+    FftEnsLaunch P;
+    P.nseg = nseg;
+    int blocks = 0;
+    size_t smem = 0;
+    bool lng = false;
+    for (int i = 0; i < nseg; i++) {
+        const FftEnsSeg &g = segs[i];
+        exotx_status st;
+        const FftTables *t = fft_tables(g.n, &st);
+        if (!t) return st;
+        FftEnsArgs &a = P.seg[i];
+        a.in = g.in; a.out = g.out; a.lot = g.lot; a.f_rs = g.f_rs; a.f_ms = g.f_ms; a.n = g.n; a.kf = g.kf;
+        a.fold_nlat = fwd ? g.fold_nlat : 0;
+        a.rs = RowSums{fwd ? g.rowsum : nullptr, g.L, 0};
+        a.w = reinterpret_cast<const cpx<float> *>(t->w32);
+        a.r = reinterpret_cast<const cpx<float> *>(t->r32);
+        a.block0 = blocks;
+        int rows = 0;
+        EXOTX_TRY(by_len(g.n, [&](auto n) {
+            using Lay = RrLayout<float, decltype(n)::value>;
+            rows = n == 384 ? RfLayout<384>::RB : Lay::RB;
+            smem = std::max(smem, n == 384 ? RfLayout<384>::SMEM : fwd ? Lay::fwd_smem() : Lay::inv_smem(g.kf));
+            lng = lng || n >= 384;
+            return EXOTX_OK;
+        }));
+        if (a.fold_nlat) {
+            const int nbpf = (g.fold_nlat / 2 + rows / 2 - 1) / (rows / 2);
+            blocks += (int)(g.lot / g.fold_nlat) * nbpf;
+        } else {
+            blocks += (int)((g.lot + rows - 1) / rows);
+        }
+    }
+    if (blocks == 0) return EXOTX_OK;
+    const int kid = fwd ? EXOTX_K_FFT_FORWARD : EXOTX_K_FFT_INVERSE;
+    static_assert(RfLayout<384>::NT == RR_THREADS, "one block size");
+    void (*k)(FftEnsLaunch) = lng ? (fwd ? k_rfft_ens<true, true> : k_rfft_ens<false, true>)
+                                  : (fwd ? k_rfft_ens<true, false> : k_rfft_ens<false, false>);
+    if (smem > 48 * 1024) EXOTX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cudaEvent_t ev = ktimer_start(kid, s);
+    EXOTX_CUDA(launch_pdl(k, dim3((unsigned)blocks), dim3(RR_THREADS), smem, s, P));
+    EXOTX_CHECK_LAUNCH();
+    ktimer_stop(kid, s, ev);
+    return EXOTX_OK;
 }
 
 template <typename T, int N>
-static exotx_status launch_ct(bool fwd, const T *in, T *out, long long lot, int kf, long long f_rs, long long f_ms,
+static exotx_status launch_rr(bool fwd, const T *in, T *out, long long lot, int kf, long long f_rs, long long f_ms,
                               const cpx<T> *w, const cpx<T> *r, cudaStream_t s) {
-    constexpr int ROWS = ct_rows<T>(N);
-    const size_t smem = 2 * ROWS * fpad_row<N / 2>() * sizeof(cpx<T>);
-    const long long nb = (lot + ROWS - 1) / ROWS;
+    using Lay = RrLayout<T, N>;
+    const size_t smem = fwd ? Lay::fwd_smem() : Lay::inv_smem(kf);
+    const long long nb = (lot + Lay::RB - 1) / Lay::RB;
     const int kid = fwd ? EXOTX_K_FFT_FORWARD : EXOTX_K_FFT_INVERSE;
-    if (fwd) {
-        if (smem > 48 * 1024)
-            EXOTX_CUDA(cudaFuncSetAttribute(k_rfft_fwd_ct<T, N, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem));
-    } else {
-        if (smem > 48 * 1024)
-            EXOTX_CUDA(cudaFuncSetAttribute(k_rfft_inv_ct<T, N, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem));
+    if (smem > 48 * 1024) {
+        if (fwd)
+            EXOTX_CUDA(cudaFuncSetAttribute(k_rfft_fwd_rr<T, N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        else
+            EXOTX_CUDA(cudaFuncSetAttribute(k_rfft_inv_rr<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     }
     cudaEvent_t ev = ktimer_start(kid, s);
-    // dependent launch: the block set-up overlaps the previous kernel's tail
     if (fwd)
-        EXOTX_CUDA(launch_pdl(k_rfft_fwd_ct<T, N, ROWS>, dim3((unsigned)nb), dim3(256), smem, s, in, out, lot, kf,
-                              f_rs, f_ms, w, r));
+        EXOTX_CUDA(launch_pdl(k_rfft_fwd_rr<T, N, false>, dim3((unsigned)nb), dim3(RR_THREADS), smem, s, in, out, 0, lot,
+                              kf, f_rs, f_ms, w, r, RowSums{}));
     else
-        EXOTX_CUDA(launch_pdl(k_rfft_inv_ct<T, N, ROWS>, dim3((unsigned)nb), dim3(256), smem, s, in, out, lot, kf,
-                              f_rs, f_ms, w, r));
+        EXOTX_CUDA(launch_pdl(k_rfft_inv_rr<T, N>, dim3((unsigned)nb), dim3(RR_THREADS), smem, s, in, out, lot, kf, f_rs,
+                              f_ms, w, r));
     EXOTX_CHECK_LAUNCH();
     ktimer_stop(kid, s, ev);
     return EXOTX_OK;
@@ -1427,21 +1382,16 @@ static exotx_status launch_rf(bool fwd, const float *in, float *out, long long l
 
 // returns EXOTX_NOT_BUILT when n has no specialised kernel
 template <typename T>
-static exotx_status dispatch_ct(bool fwd, int n, const T *in, T *out, long long lot, int kf, long long f_rs,
-                                long long f_ms, const cpx<T> *w, const cpx<T> *r, cudaStream_t s) {
-    if constexpr (sizeof(T) == 4) {   // single precision: register-resident kernels where built
+static exotx_status dispatch_len(bool fwd, int n, const T *in, T *out, long long lot, int kf, long long f_rs,
+                                 long long f_ms, const cpx<T> *w, const cpx<T> *r, cudaStream_t s) {
+    if constexpr (sizeof(T) == 4) {
         if (n == 384) return launch_rf<384>(fwd, in, out, lot, kf, f_rs, f_ms, w, r, s);
     }
-    switch (n) {
-        case 64: return launch_ct<T, 64>(fwd, in, out, lot, kf, f_rs, f_ms, w, r, s);
-        case 128: return launch_ct<T, 128>(fwd, in, out, lot, kf, f_rs, f_ms, w, r, s);
-        case 192: return launch_ct<T, 192>(fwd, in, out, lot, kf, f_rs, f_ms, w, r, s);
-        case 256: return launch_ct<T, 256>(fwd, in, out, lot, kf, f_rs, f_ms, w, r, s);
-        case 320: return launch_ct<T, 320>(fwd, in, out, lot, kf, f_rs, f_ms, w, r, s);
-        case 384: return launch_ct<T, 384>(fwd, in, out, lot, kf, f_rs, f_ms, w, r, s);
-        case 512: return launch_ct<T, 512>(fwd, in, out, lot, kf, f_rs, f_ms, w, r, s);
-    }
-    return EXOTX_NOT_BUILT;
+    return by_len(n, [&](auto len) {
+        constexpr int N = decltype(len)::value;
+        if constexpr (sizeof(T) == 4 && N == 384) return EXOTX_NOT_BUILT;
+        else return launch_rr<T, N>(fwd, in, out, lot, kf, f_rs, f_ms, w, r, s);
+    });
 }
 
 // ----------------------------------------------------------------- tables
@@ -1526,8 +1476,6 @@ static FftLaunch make_launch(const FftTables *t, long long lot, int kf, long lon
     return L;
 }
 
-static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-
 template <typename T>
 static exotx_status set_smem(const void *fn, size_t smem) {
     if (smem > 48 * 1024) {
@@ -1546,7 +1494,7 @@ exotx_status fft_forward_l(const T *in, T *out, int n, long long lot, int kout, 
     if (!t) return st;
     if (lot <= 0) return EXOTX_OK;
     if (aligned16(in) && aligned16(out)) {
-        exotx_status sc = dispatch_ct<T>(true, n, in, out, lot, kout, f_rs, f_ms, wt<T>(t), rt<T>(t), s);
+        exotx_status sc = dispatch_len<T>(true, n, in, out, lot, kout, f_rs, f_ms, wt<T>(t), rt<T>(t), s);
         if (sc != EXOTX_NOT_BUILT) return sc;
     }
     size_t smem;
@@ -1568,7 +1516,7 @@ exotx_status fft_inverse_l(const T *in, T *out, int n, long long lot, int kin, l
     if (!t) return st;
     if (lot <= 0) return EXOTX_OK;
     if (aligned16(in) && aligned16(out)) {
-        exotx_status sc = dispatch_ct<T>(false, n, in, out, lot, kin, f_rs, f_ms, wt<T>(t), rt<T>(t), s);
+        exotx_status sc = dispatch_len<T>(false, n, in, out, lot, kin, f_rs, f_ms, wt<T>(t), rt<T>(t), s);
         if (sc != EXOTX_NOT_BUILT) return sc;
     }
     size_t smem;
@@ -1589,64 +1537,51 @@ template exotx_status fft_forward_l<float>(const float *, float *, int, long lon
 
 template <int N>
 static exotx_status launch_fold(const float *in, float *out, int nlat, long long lot, int kf, long long f_ms,
-                                const cpx<float> *w, const cpx<float> *r, double *rowsum, cudaStream_t s) {
-    if (rowsum && !rf_len<N>()) return EXOTX_NOT_BUILT;
-    if constexpr (rf_len<N>()) {
+                                const cpx<float> *w, const cpx<float> *r, RowSums rs, cudaStream_t s) {
+    cudaEvent_t ev = nullptr;
+    if constexpr (N == 384) {
         using Lay = RfLayout<N>;
         using PL = RfPLayout<N>;
         const int nbpf = (nlat / 2 + Lay::RB / 2 - 1) / (Lay::RB / 2);
         const long long nb = (lot / nlat) * nbpf;
-        auto kern = rowsum ? k_rfft_fwd_fold_rf_p<N, true> : k_rfft_fwd_fold_rf_p<N, false>;
+        auto kern = k_rfft_fwd_fold_rf_p<N>;
         EXOTX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL::SMEM));
         int slots = 0;
         EXOTX_TRY(resident_slots((const void *)kern, Lay::NT, PL::SMEM, &slots));
         const long long grid = std::min<long long>(nb, slots);
-        cudaEvent_t ev = ktimer_start(EXOTX_K_FFT_FORWARD, s);
+        ev = ktimer_start(EXOTX_K_FFT_FORWARD, s);
         EXOTX_CUDA(launch_pdl(kern, dim3((unsigned)grid), dim3(Lay::NT), PL::SMEM, s, in, out, nlat, lot, kf, f_ms, nb,
-                              w, r, rowsum));
-        EXOTX_CHECK_LAUNCH();
-        ktimer_stop(EXOTX_K_FFT_FORWARD, s, ev);
-        return EXOTX_OK;
+                              w, r, rs));
+    } else {
+        using Lay = RrLayout<float, N>;
+        const int nbpf = (nlat / 2 + Lay::RB / 2 - 1) / (Lay::RB / 2);
+        const long long nb = (lot / nlat) * nbpf;
+        constexpr size_t smem = Lay::fwd_smem();
+        static_assert(smem <= 48 * 1024, "default shared memory");
+        ev = ktimer_start(EXOTX_K_FFT_FORWARD, s);
+        EXOTX_CUDA(launch_pdl(k_rfft_fwd_rr<float, N, true>, dim3((unsigned)nb), dim3(RR_THREADS), smem, s, in, out, nlat,
+                              lot, kf, 1LL, f_ms, w, r, rs));
     }
-    constexpr int ROWS = ct_rows<float>(N);
-    const size_t smem = 2 * ROWS * fpad_row<N / 2>() * sizeof(cpx<float>);
-    const int nbpf = (nlat / 2 + ROWS / 2 - 1) / (ROWS / 2);
-    const long long nb = (lot / nlat) * nbpf;
-    if (smem > 48 * 1024)
-        EXOTX_CUDA(cudaFuncSetAttribute(k_rfft_fwd_fold<float, N, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem));
-    cudaEvent_t ev = ktimer_start(EXOTX_K_FFT_FORWARD, s);
-    EXOTX_CUDA(launch_pdl(k_rfft_fwd_fold<float, N, ROWS>, dim3((unsigned)nb), dim3(256), smem, s, in, out, nlat, lot,
-                          kf, f_ms, w, r));
     EXOTX_CHECK_LAUNCH();
     ktimer_stop(EXOTX_K_FFT_FORWARD, s, ev);
     return EXOTX_OK;
 }
 
 // forward transform of lot = fields x nlat grid rows of length n = 2 nlat into
-// the equator-folded m-major layout (rfft_fwd_fold_body); EXOTX_NOT_BUILT when
-// n has no specialised kernel or the buffers are not 16-byte aligned
-bool fft_fold_rowsum(int n) { return n == 384; }   // the register-resident lengths (RfShape)
-
+// the equator-folded m-major layout (rr_fwd_body); EXOTX_NOT_BUILT when n has
+// no specialised kernel or the buffers are not 16-byte aligned
 exotx_status fft_forward_fold(const float *in, float *out, int n, int nlat, long long lot, int kf, long long f_ms,
-                              double *rowsum, cudaStream_t s) {
+                              double *rowsum, int L, int dset, cudaStream_t s) {
     if (n != 2 * nlat || nlat < 2 || lot % nlat) return EXOTX_BAD_ARG;
     exotx_status st;
     const FftTables *t = fft_tables(n, &st);
     if (!t) return st;
     if (lot <= 0) return EXOTX_OK;
     if (!aligned16(in) || !aligned16(out)) return EXOTX_NOT_BUILT;
-    const cpx<float> *w = wt<float>(t), *r = rt<float>(t);
-    switch (n) {
-        case 64: return launch_fold<64>(in, out, nlat, lot, kf, f_ms, w, r, rowsum, s);
-        case 128: return launch_fold<128>(in, out, nlat, lot, kf, f_ms, w, r, rowsum, s);
-        case 192: return launch_fold<192>(in, out, nlat, lot, kf, f_ms, w, r, rowsum, s);
-        case 256: return launch_fold<256>(in, out, nlat, lot, kf, f_ms, w, r, rowsum, s);
-        case 320: return launch_fold<320>(in, out, nlat, lot, kf, f_ms, w, r, rowsum, s);
-        case 384: return launch_fold<384>(in, out, nlat, lot, kf, f_ms, w, r, rowsum, s);
-        case 512: return launch_fold<512>(in, out, nlat, lot, kf, f_ms, w, r, rowsum, s);
-    }
-    return EXOTX_NOT_BUILT;
+    return by_len(n, [&](auto len) {
+        return launch_fold<decltype(len)::value>(in, out, nlat, lot, kf, f_ms, wt<float>(t), rt<float>(t),
+                                                 RowSums{rowsum, L, dset}, s);
+    });
 }
 template exotx_status fft_inverse_l<double>(const double *, double *, int, long long, int, long long, long long,
                                             cudaStream_t);
@@ -1694,7 +1629,7 @@ exotx_status fft_forward_tw(const T *in, T *out, int n, long long lot, int kout,
     if (lot <= 0) return EXOTX_OK;
     const cpx<T> *wc = reinterpret_cast<const cpx<T> *>(w), *rc = reinterpret_cast<const cpx<T> *>(r);
     if (aligned16(in) && aligned16(out)) {
-        exotx_status sc = dispatch_ct<T>(true, n, in, out, lot, kout, f_rs, f_ms, wc, rc, s);
+        exotx_status sc = dispatch_len<T>(true, n, in, out, lot, kout, f_rs, f_ms, wc, rc, s);
         if (sc != EXOTX_NOT_BUILT) return sc;
     }
     FftTables t;  // radix schedule only

@@ -508,8 +508,8 @@ __global__ void __launch_bounds__(256) k_n0_fp64(const __grid_constant__ N0Launc
     if (S.rowsum) {
         for (int lat = threadIdx.x; lat < S.nlat; lat += blockDim.x) rs[lat] = S.rowsum[row0 + lat];
     } else {
-        // eight lanes per row in the order of the forward FFT's row sums: lane t
-        // adds the complex elements t + 8 j (real part first), then an xor butterfly
+        // eight lanes per row: lane t adds the complex elements t + 8 j (real part
+        // first), then an xor butterfly
         const int t = threadIdx.x & 7, g = threadIdx.x >> 3, ng = blockDim.x >> 3, h = S.nlon / 2;
         for (int lat0 = 0; lat0 < S.nlat; lat0 += ng) {
             const int lat = lat0 + g;
@@ -582,7 +582,7 @@ exotx_status tc_ens_n0(const EnsSeg *segs, const float *const *gpin, int nseg, c
     P.nseg = nseg;
     int nblk = 0;
     for (int i = 0; i < nseg; i++) {
-        n0_seg(P.seg[i], segs[i].p, gpin[i], nullptr, segs[i].spout, segs[i].L, 0, nblk);
+        n0_seg(P.seg[i], segs[i].p, gpin[i], segs[i].rowsum, segs[i].spout, segs[i].L, 0, nblk);
         nblk += segs[i].ninst * P.seg[i].nf;
     }
     return n0_launch(P, nblk, s);
@@ -598,7 +598,7 @@ static exotx_status tc_forward_run(exotx_plan p, const float *gpin, float *spout
     int chunk = (int)std::max<size_t>(1, p->chunk_fwd / per_inst);
     chunk = std::min(chunk, ninst);
     // the FP64 grid-row sums of the n = 0 coefficients follow the intermediate,
-    // where the folded FFT forms them (register-resident lengths)
+    // where the folded FFT forms them
     const bool with_rs = fft_fold_rowsum(p->nlon);
     const size_t rs_off = (per_inst * chunk + 255) & ~(size_t)255;
     EXOTX_TRY(ensure_work(p, with_rs ? rs_off + (size_t)chunk * nfi * p->nlat * sizeof(double) : per_inst * chunk));
@@ -611,7 +611,7 @@ static exotx_status tc_forward_run(exotx_plan p, const float *gpin, float *spout
         // a specialised FFT (and the grid is 16-byte aligned); otherwise north and south rows
         double *rowsum = with_rs ? reinterpret_cast<double *>(static_cast<char *>(p->d_work) + rs_off) : nullptr;
         const exotx_status sf = fft_forward_fold(gsrc, (float *)p->d_work, p->nlon, p->nlat, nrows, p->ntp1, nrows,
-                                                 rowsum, s);
+                                                 rowsum, L, dset, s);
         if (sf != EXOTX_OK && sf != EXOTX_NOT_BUILT) return sf;
         const bool folded = sf == EXOTX_OK;
         if (!folded) {
