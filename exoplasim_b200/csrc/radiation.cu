@@ -8,17 +8,7 @@
 #include "radiation_kernel.cuh"
 
 namespace exotx {
-exotx_status launch_radstep_fp64(const RadDev &D, int blocks, int warps, size_t smem, cudaStream_t st);
-
-static exotx_status launch_radstep_fp32(const RadDev &D, int blocks, int warps, size_t smem, cudaStream_t st) {
-    if (smem > 48 * 1024)
-        EXOTX_CUDA(cudaFuncSetAttribute(k_radstep<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    cudaEvent_t ev = ktimer_start(EXOTX_K_RADSTEP, st);
-    k_radstep<float><<<blocks, warps * 32, smem, st>>>(D);
-    EXOTX_CHECK_LAUNCH();
-    ktimer_stop(EXOTX_K_RADSTEP, st, ev);
-    return EXOTX_OK;
-}
+exotx_status launch_radstep_fp64(const RadDev &D, int maxcols, bool list, cudaStream_t st);
 }  // namespace exotx
 
 using namespace exotx;
@@ -126,30 +116,8 @@ exotx_status radstep_columns(const exotx_rad_params *p, int prec, const exotx_ra
     D.dlwfl = io->dlwfl; D.dflux = io->dflux; D.dtdt = io->dtdt; D.dtdtswr = io->dtdtswr;
     D.dtdtlwr = io->dtdtlwr; D.dconv = io->dconv;
     D.zsol = io->zsol; D.cols = cols; D.ncols = ncols;
-    int L = p->nlev, E = L + 1;
-    size_t elems = (size_t)6 * E + 7 * L + 11 * L + 8 * L + 8 * E + 2 * E + 4 * L + 2 * (E + 1) + (size_t)L * L + L +
-                   6 * E + 32;
-    size_t esz = prec == EXOTX_FP64 ? 8 : 4;
-    // warps per block limited by the column scratch (<= 200 KB of shared memory)
-    int warps = (int)((200 * 1024) / (elems * esz));
-    warps = warps < 1 ? 1 : (warps > RAD_WARPS ? RAD_WARPS : warps);
-    size_t smem = elems * esz * warps;
-    int blocks = (maxcols + warps - 1) / warps;
-    // a column list is usually short (often empty): one wave of resident blocks
-    // strides over it instead of one block per possible entry
-    if (cols) {
-        static int nsm = 0;
-        if (!nsm) {
-            int dev = 0;
-            if (cudaGetDevice(&dev) != cudaSuccess ||
-                cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm < 1)
-                nsm = 148;
-        }
-        const int per_sm = std::max(1, (int)((227 * 1024) / std::max<size_t>(smem, 1)));
-        blocks = std::min(blocks, nsm * per_sm);
-    }
-    if (prec == EXOTX_FP64) return launch_radstep_fp64(D, blocks, warps, smem, st);
-    return launch_radstep_fp32(D, blocks, warps, smem, st);
+    if (prec == EXOTX_FP64) return launch_radstep_fp64(D, maxcols, cols != nullptr, st);
+    return launch_radstep<float>(D, maxcols, cols != nullptr, st);
 }
 }  // namespace exotx
 
