@@ -102,10 +102,36 @@ __host__ __device__ inline RadScratch rad_scratch(int L) {
     s.size = p;
     return s;
 }
-// bytes: the scratch of COLS columns, the log(sigmah) ratios and the pair list
+// lwr's fit constants (:2207-2218) and mko3's, formed once per block
+enum { RK_AO30 = 0, RK_CO20, RK_H2O0A, RK_H2O0, RK_AO3C, RK_ACO2C, RK_AH2OC, RK_TH2OC, RK_ZCONST, RK_N };
+template <typename T>
+__device__ T rad_const(const exotx_rad_params &P, int i) {
+    const T zao30 = (T)0.209 * P_((T)7.e-5, (T)0.436);
+    const T zco20 = (T)0.0676 * P_((T)0.01022, (T)0.421);
+    const T zh2o0a = (T)0.846 * P_((T)3.59e-5, (T)0.243);
+    const T zh2o0 = (T)0.832 * P_((T)0.0286, (T)0.26);
+    switch (i) {
+        case RK_AO30: return zao30;
+        case RK_CO20: return zco20;
+        case RK_H2O0A: return zh2o0a;
+        case RK_H2O0: return zh2o0;
+        case RK_AO3C: return (T)0.209 * P_((T)0.01 + (T)7.e-5, (T)0.436) - zao30 - (T)0.0212 * log10((T)0.01);
+        case RK_ACO2C: return (T)0.0676 * P_((T)1.01022, (T)0.421) - zco20;
+        case RK_AH2OC: return (T)0.846 * P_((T)0.01 + (T)3.59e-5, (T)0.243) - zh2o0a - (T)0.24 * log10((T)0.02);
+        case RK_TH2OC: return (T)1. - ((T)0.832 * P_((T)2. + (T)0.0286, (T)0.26) - zh2o0) + (T)0.1196 * log((T)2. - (T)0.6931);
+        default: return exp(-(T)P.bo3 / (T)P.co3);
+    }
+}
+// byte offset of the warps' argument buffers, after the scratch of COLS columns,
+// the log(sigmah) ratios, the constants and the pair list; and the total
+template <typename T>
+__host__ __device__ inline size_t rad_args(int L, int cols) {
+    const size_t b = ((size_t)rad_scratch(L).size * cols + L + RK_N) * sizeof(T) + 8 + (size_t)(L * (L + 1) / 2) * 2;
+    return (b + 15) & ~(size_t)15;
+}
 template <typename T>
 __host__ __device__ inline size_t rad_smem(int L, int cols) {
-    return ((size_t)rad_scratch(L).size * cols + L) * sizeof(T) + (size_t)(L * (L + 1) / 2) * 2 + 16;
+    return rad_args<T>(L, cols) + (sizeof(T) == 8 ? (size_t)(RAD_THREADS / 32) * 128 * sizeof(T) : 0);
 }
 
 template <typename T, int COLS>
@@ -118,7 +144,8 @@ __global__ void __launch_bounds__(RAD_THREADS, sizeof(T) == 8 ? 3 : 4) k_radstep
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, c = tid % COLS, it0 = tid / COLS;
     T *sm = reinterpret_cast<T *>(smraw) + c;
     T *lg = reinterpret_cast<T *>(smraw) + (size_t)S.size * COLS;        // log(sigmah(j-1)/sigmah(j))
-    int *next = reinterpret_cast<int *>(lg + L);                         // pair chunks handed out
+    T *kc = lg + L;                                                      // rad_const
+    int *next = reinterpret_cast<int *>(kc + RK_N);                      // pair chunks handed out
     unsigned short *pairs = reinterpret_cast<unsigned short *>(next + 2);
 #define V(a, k) sm[(S.a + (k)) * COLS]
     const T PI = (T)3.14159265359, TWOPI = PI + PI;
@@ -141,6 +168,8 @@ __global__ void __launch_bounds__(RAD_THREADS, sizeof(T) == 8 ? 3 : 4) k_radstep
         for (int jl2 = jl; jl2 < L; jl2++) pairs[p0 + jl2 - jl] = (unsigned short)(jl << 8 | jl2);
         if (jl >= 1) lg[jl] = log((T)P.sigmah[jl - 1] / (T)P.sigmah[jl]);
     }
+    if (lane == 0)
+        for (int i = warp; i < RK_N; i += RAD_THREADS / 32) kc[i] = rad_const<T>(P, i);
     const int count = D.cols ? *D.ncols : nhor;
     for (int base = blockIdx.x * COLS; base < count; base += gridDim.x * COLS) {
         const bool valid = base + c < count;
@@ -207,8 +236,8 @@ __global__ void __launch_bounds__(RAD_THREADS, sizeof(T) == 8 ? 3 : 4) k_radstep
         }
         // mko3 (radmod.f90:1489-1522): the sums in height on one lane per column
         if (P.no3 == 1) {
-            const T zconst = exp(-(T)P.bo3 / (T)P.co3);
             __syncthreads();
+            const T zconst = kc[RK_ZCONST];
             if (it0 == 0) {
                 T sd = sid[jlat];
                 V(sc, SC_ZA) = (T)P.a0o3 + (T)P.a1o3 * fabs(sd) + (T)P.aco3 * sd * cos(TWOPI * ((T)P.zcday - (T)P.toffo3));
@@ -488,43 +517,90 @@ __global__ void __launch_bounds__(RAD_THREADS, sizeof(T) == 8 ? 3 : 4) k_radstep
         // handed out 32/COLS at a time; each sums its absorbers, and multiplies the
         // layers' cloud transmissivities (random overlap), from jlev upward
         if (P.nlwr == 1) {
-            const T zao30 = (T)0.209 * P_((T)7.e-5, (T)0.436);
-            const T zco20 = (T)0.0676 * P_((T)0.01022, (T)0.421);
-            const T zh2o0a = (T)0.846 * P_((T)3.59e-5, (T)0.243);
-            const T zh2o0 = (T)0.832 * P_((T)0.0286, (T)0.26);
-            const T zao3c = (T)0.209 * P_((T)0.01 + (T)7.e-5, (T)0.436) - zao30 - (T)0.0212 * log10((T)0.01);
-            const T zaco2c = (T)0.0676 * P_((T)1.01022, (T)0.421) - zco20;
-            const T zah2oc = (T)0.846 * P_((T)0.01 + (T)3.59e-5, (T)0.243) - zh2o0a - (T)0.24 * log10((T)0.02);
-            const T zth2oc = (T)1. - ((T)0.832 * P_((T)2. + (T)0.0286, (T)0.26) - zh2o0) + (T)0.1196 * log((T)2. - (T)0.6931);
+            const T zao30 = kc[RK_AO30], zco20 = kc[RK_CO20], zh2o0a = kc[RK_H2O0A], zh2o0 = kc[RK_H2O0];
+            const T zao3c = kc[RK_AO3C], zaco2c = kc[RK_ACO2C], zah2oc = kc[RK_AH2OC], zth2oc = kc[RK_TH2OC];
             const T th2oc = (T)P.th2oc;
             constexpr int PW = 32 / COLS;
+            // The fits' two branches (a power of a small path, a logarithm of a large
+            // one) mix within a warp.  In FP64 its 4 x 32 arguments are sorted into the
+            // powers (from the front of arg) and the logarithms (from the back), so each
+            // is evaluated once by full warps (13 levels: 89 -> 80 us for 4608 columns);
+            // in FP32 both branches cost less than the sorting (88 against 99 us)
+            constexpr bool SORT = sizeof(T) == 8;
             __syncwarp();
             while (true) {
                 int ch = lane == 0 ? atomicAdd(next, 1) : 0;
                 ch = __shfl_sync(0xffffffffu, ch, 0);
                 if (ch * PW >= npair) break;
                 const int pi = ch * PW + lane / COLS;
-                if (pi >= npair) continue;
-                const int jl = pairs[pi] >> 8, jl2 = pairs[pi] & 255;
+                const bool live = pi < npair;
+                const int jl = live ? pairs[pi] >> 8 : 0, jl2 = live ? pairs[pi] & 255 : 0;
                 T zsumwv = 0, zsumo3 = 0, zsumco2 = 0, ztaucc = 1;
                 for (int k = jl; k <= jl2; k++) {
                     zsumwv = zsumwv + V(q, k); zsumo3 = zsumo3 + V(qo3, k); zsumco2 = zsumco2 + V(qco2, k);
                     ztaucc = ztaucc * V(tcc, k);
                 }
-                T zah2o, zaco2, zth2o, zao3;
-                if (zsumwv <= (T)0.01) zah2o = (T)0.846 * P_(zsumwv + (T)3.59e-5, (T)0.243) - zh2o0a;
-                else zah2o = (T)0.24 * log10(zsumwv + (T)0.01) + zah2oc;
-                if (th2oc > (T)0.) zah2o = fmin(zah2o + ((T)1. - exp(-th2oc * zsumwv)), (T)1.);
-                if (zsumco2 <= (T)1.0) zaco2 = (T)0.0676 * P_(zsumco2 + (T)0.01022, (T)0.421) - zco20;
-                else zaco2 = (T)0.0546 * log10(zsumco2) + zaco2c;
-                if (zsumwv <= (T)2.) zth2o = (T)1. - ((T)0.832 * P_(zsumwv + (T)0.0286, (T)0.26) - zh2o0);
-                else zth2o = fmax((T)0., zth2oc - (T)0.1196 * log(zsumwv - (T)0.6931));
-                if (zsumo3 <= (T)0.01) zao3 = (T)0.209 * P_(zsumo3 + (T)7.e-5, (T)0.436) - zao30;
-                else zao3 = (T)0.0212 * log10(zsumo3) + zao3c;
-                T tcs = (T)1. - zah2o - zao3 - zaco2 * zth2o;
-                tcs = fmin((T)1. - zero, fmax(zero, tcs));
-                if (jl == 0) V(tau0, jl2) = tcs;
-                V(tau, pi) = tcs * ztaucc;
+                T zah2o = 0, zaco2 = 0, zth2o = 0, zao3 = 0;
+                if constexpr (SORT) {
+                    T *arg = reinterpret_cast<T *>(smraw + rad_args<T>(L, COLS)) + warp * 128;
+                    const T expo[4] = {(T)0.243, (T)0.421, (T)0.26, (T)0.436};
+                    const unsigned below = (1u << lane) - 1u;
+                    // evaluations 0 h2o, 1 co2, 2 h2o in the co2 overlap, 3 o3
+                    const bool pw[4] = {zsumwv <= (T)0.01, zsumco2 <= (T)1.0, zsumwv <= (T)2., zsumo3 <= (T)0.01};
+                    const T x[4] = {pw[0] ? zsumwv + (T)3.59e-5 : zsumwv + (T)0.01, pw[1] ? zsumco2 + (T)0.01022 : zsumco2,
+                                    pw[2] ? zsumwv + (T)0.0286 : zsumwv - (T)0.6931, pw[3] ? zsumo3 + (T)7.e-5 : zsumo3};
+                    int pos[4], np = 0, nl = 0, pend[4], l2a = 0, l2b = 0;
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const unsigned mp = __ballot_sync(0xffffffffu, live && pw[e]), ml = __ballot_sync(0xffffffffu, live && !pw[e]);
+                        pos[e] = pw[e] ? np + __popc(mp & below) : 127 - (nl + __popc(ml & below));
+                        if (e == 2) l2a = nl;
+                        np += __popc(mp);
+                        nl += __popc(ml);
+                        if (e == 2) l2b = nl;
+                        pend[e] = np;
+                        if (live) arg[pos[e]] = x[e];
+                    }
+                    __syncwarp();
+                    for (int i = lane; i < np; i += 32)
+                        arg[i] = P_(arg[i], i < pend[0] ? expo[0] : i < pend[1] ? expo[1] : i < pend[2] ? expo[2] : expo[3]);
+                    for (int i = lane; i < nl; i += 32) {
+                        const T v = arg[127 - i];
+                        arg[127 - i] = i >= l2a && i < l2b ? log(v) : log10(v);
+                    }
+                    __syncwarp();
+                    if (live) {
+                        T r[4];
+#pragma unroll
+                        for (int e = 0; e < 4; e++) r[e] = arg[pos[e]];
+                        if (pw[0]) zah2o = (T)0.846 * r[0] - zh2o0a;
+                        else zah2o = (T)0.24 * r[0] + zah2oc;
+                        if (th2oc > (T)0.) zah2o = fmin(zah2o + ((T)1. - exp(-th2oc * zsumwv)), (T)1.);
+                        if (pw[1]) zaco2 = (T)0.0676 * r[1] - zco20;
+                        else zaco2 = (T)0.0546 * r[1] + zaco2c;
+                        if (pw[2]) zth2o = (T)1. - ((T)0.832 * r[2] - zh2o0);
+                        else zth2o = fmax((T)0., zth2oc - (T)0.1196 * r[2]);
+                        if (pw[3]) zao3 = (T)0.209 * r[3] - zao30;
+                        else zao3 = (T)0.0212 * r[3] + zao3c;
+                    }
+                    __syncwarp();   // arg is free for the next pairs
+                } else if (live) {
+                    if (zsumwv <= (T)0.01) zah2o = (T)0.846 * P_(zsumwv + (T)3.59e-5, (T)0.243) - zh2o0a;
+                    else zah2o = (T)0.24 * log10(zsumwv + (T)0.01) + zah2oc;
+                    if (th2oc > (T)0.) zah2o = fmin(zah2o + ((T)1. - exp(-th2oc * zsumwv)), (T)1.);
+                    if (zsumco2 <= (T)1.0) zaco2 = (T)0.0676 * P_(zsumco2 + (T)0.01022, (T)0.421) - zco20;
+                    else zaco2 = (T)0.0546 * log10(zsumco2) + zaco2c;
+                    if (zsumwv <= (T)2.) zth2o = (T)1. - ((T)0.832 * P_(zsumwv + (T)0.0286, (T)0.26) - zh2o0);
+                    else zth2o = fmax((T)0., zth2oc - (T)0.1196 * log(zsumwv - (T)0.6931));
+                    if (zsumo3 <= (T)0.01) zao3 = (T)0.209 * P_(zsumo3 + (T)7.e-5, (T)0.436) - zao30;
+                    else zao3 = (T)0.0212 * log10(zsumo3) + zao3c;
+                }
+                if (live) {
+                    T tcs = (T)1. - zah2o - zao3 - zaco2 * zth2o;
+                    tcs = fmin((T)1. - zero, fmax(zero, tcs));
+                    if (jl == 0) V(tau0, jl2) = tcs;
+                    V(tau, pi) = tcs * ztaucc;
+                }
             }
         }
         __syncthreads();
