@@ -1,10 +1,10 @@
 // radmod.f90 radiation column pass on the GPU (device code).
 //
 // The reference evaluates radstep (:927-1110) with array statements over all
-// NHOR columns.  Here a block of 256 threads owns RAD_COLS columns (fewer where
-// a column's scratch is large), held in shared memory level by level with the
-// columns fastest.  A thread works one column c = tid % COLS and takes the
-// levels, or the (jlev, jlev2) pairs of lwr, i = tid / COLS, + 256/COLS, ...:
+// NHOR columns.  Here a block owns COLS = 16 columns (fewer where a column's
+// scratch is large), held in shared memory level by level with the columns
+// fastest.  A thread works one column c = tid % COLS and takes the levels, or
+// the (jlev, jlev2) pairs of lwr, i = tid / COLS, + rad_items, ...:
 // the transcendental work (cloud optics, ozone and water-vapour
 // transmissivities, the O(NLEV^2) longwave absorptivities) is spread over all
 // threads.  What is serial in height -- mko3's sums, the absorber paths, the
@@ -15,7 +15,7 @@
 // Bound by the FP64 (FP32: FP32 and special-function) instructions of pow, log
 // and exp.  One warp per column, the form before, left the serial parts to one
 // lane of 32: they were two thirds of its instructions.  8192 T42 L20 columns:
-// FP64 401 -> RADF64 us, FP32 265 -> RADF32 us.
+// FP64 401 -> 176 us, FP32 265 -> 75 us.
 #pragma once
 #include <cmath>
 #include "exotx_internal.cuh"
@@ -23,7 +23,11 @@
 namespace exotx {
 
 constexpr int RAD_MAXLEV = 64;
-constexpr int RAD_THREADS = 256;
+
+// Items (levels, pairs) in flight per column, and so threads per block: 32 in
+// FP64, 16 in FP32 (half the registers per thread, so more blocks per SM).
+template <typename T> constexpr int rad_items() { return sizeof(T) == 8 ? 32 : 16; }
+template <typename T> constexpr int rad_threads(int cols) { return cols * rad_items<T>(); }
 
 struct RadDev {
     exotx_rad_params p;
@@ -131,16 +135,17 @@ __host__ __device__ inline size_t rad_args(int L, int cols) {
 }
 template <typename T>
 __host__ __device__ inline size_t rad_smem(int L, int cols) {
-    return rad_args<T>(L, cols) + (sizeof(T) == 8 ? (size_t)(RAD_THREADS / 32) * 128 * sizeof(T) : 0);
+    return rad_args<T>(L, cols) + (sizeof(T) == 8 ? (size_t)(rad_threads<T>(cols) / 32) * 128 * sizeof(T) : 0);
 }
 
 template <typename T, int COLS>
-__global__ void __launch_bounds__(RAD_THREADS, sizeof(T) == 8 ? 3 : 4) k_radstep(const __grid_constant__ RadDev D) {
+__global__ void __launch_bounds__(rad_threads<T>(COLS), (sizeof(T) == 8 ? 512 : 768) / rad_threads<T>(COLS))
+    k_radstep(const __grid_constant__ RadDev D) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const exotx_rad_params &P = D.p;
     const int L = P.nlev, E = L + 1, nhor = P.nhor, nlon = P.nlon, npair = L * (L + 1) / 2;
     const RadScratch S = rad_scratch(L);
-    constexpr int NI = RAD_THREADS / COLS;     // items in flight per column
+    constexpr int NI = rad_items<T>(), NTHR = rad_threads<T>(COLS);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, c = tid % COLS, it0 = tid / COLS;
     T *sm = reinterpret_cast<T *>(smraw) + c;
     T *lg = reinterpret_cast<T *>(smraw) + (size_t)S.size * COLS;        // log(sigmah(j-1)/sigmah(j))
@@ -163,13 +168,13 @@ __global__ void __launch_bounds__(RAD_THREADS, sizeof(T) == 8 ? 3 : 4) k_radstep
     const T zb4 = (T)P.tswr2 * sqrt(zmu00);
     const T zb5 = (T)P.tswr3 * zmu00 * zmu00;
     // the pair list and the level constants, once per block
-    for (int jl = tid; jl < L; jl += RAD_THREADS) {
+    for (int jl = tid; jl < L; jl += NTHR) {
         const int p0 = jl * L - jl * (jl - 1) / 2;       // row jl has L - jl entries
         for (int jl2 = jl; jl2 < L; jl2++) pairs[p0 + jl2 - jl] = (unsigned short)(jl << 8 | jl2);
         if (jl >= 1) lg[jl] = log((T)P.sigmah[jl - 1] / (T)P.sigmah[jl]);
     }
     if (lane == 0)
-        for (int i = warp; i < RK_N; i += RAD_THREADS / 32) kc[i] = rad_const<T>(P, i);
+        for (int i = warp; i < RK_N; i += NTHR / 32) kc[i] = rad_const<T>(P, i);
     const int count = D.cols ? *D.ncols : nhor;
     for (int base = blockIdx.x * COLS; base < count; base += gridDim.x * COLS) {
         const bool valid = base + c < count;
@@ -214,7 +219,7 @@ __global__ void __launch_bounds__(RAD_THREADS, sizeof(T) == 8 ? 3 : 4) k_radstep
         // column of the row itself.
         if (P.ndcycle == 0) {
             __syncthreads();
-            for (int cc = warp; cc < COLS; cc += RAD_THREADS / 32) {
+            for (int cc = warp; cc < COLS; cc += NTHR / 32) {
                 const int ww = min(base + cc, count - 1), cl = D.cols ? D.cols[ww] : ww, jr = cl / nlon;
                 T zsum = 0;
                 int icnt = 0;
@@ -707,15 +712,21 @@ __global__ void __launch_bounds__(RAD_THREADS, sizeof(T) == 8 ? 3 : 4) k_radstep
 #undef V
 }
 
-// columns per block: eight, fewer where their scratch does not fit a block
+// Columns per block: 16, or fewer where the scratch of the blocks that the
+// registers allow per SM (one of 512 threads in FP64, three of 256 in FP32)
+// does not fit.  8192 columns, L20: 16 columns 176 / 76 us, eight 183 / 81
+// (FP64 / FP32); eight columns by 512 threads 238, 16 by 256 in FP64 247.
 template <typename T>
-inline int rad_cols(int L) { return rad_smem<T>(L, 8) <= 200 * 1024 ? 8 : 4; }
+inline int rad_cols(int L) {
+    const size_t room = 220 * 1024 / (sizeof(T) == 8 ? 1 : 2);
+    return rad_smem<T>(L, 16) <= room ? 16 : rad_smem<T>(L, 8) <= room ? 8 : 4;
+}
 
 template <typename T>
 inline exotx_status launch_radstep(const RadDev &D, int maxcols, bool list, cudaStream_t st) {
     const int L = D.p.nlev, cols = rad_cols<T>(L);
     const size_t smem = rad_smem<T>(L, cols);
-    auto kern = cols == 8 ? k_radstep<T, 8> : k_radstep<T, 4>;
+    auto kern = cols == 16 ? k_radstep<T, 16> : cols == 8 ? k_radstep<T, 8> : k_radstep<T, 4>;
     if (smem > 48 * 1024) EXOTX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int blocks = (maxcols + cols - 1) / cols;
     // a column list is usually short (often empty): one wave of resident blocks
@@ -731,7 +742,7 @@ inline exotx_status launch_radstep(const RadDev &D, int maxcols, bool list, cuda
         blocks = blocks < nsm ? blocks : nsm;
     }
     cudaEvent_t ev = ktimer_start(EXOTX_K_RADSTEP, st);
-    kern<<<blocks, RAD_THREADS, smem, st>>>(D);
+    kern<<<blocks, rad_threads<T>(cols), smem, st>>>(D);
     EXOTX_CHECK_LAUNCH();
     ktimer_stop(EXOTX_K_RADSTEP, st, ev);
     return EXOTX_OK;
