@@ -227,12 +227,19 @@ exotx_status tc_ens_jobs(const EnsSeg *segs, int nseg, int dir, int nc_qi_cap, i
 exotx_status tc_ens_run(const EnsSeg *segs, int nseg, int dir, const int4 *d_jobs, int njobs, size_t smem,
                         int nprod, cudaStream_t s);
 exotx_status tc_ens_n0(const EnsSeg *segs, const float *const *gpin, int nseg, cudaStream_t s);
-// FP32-accurate GEMM on the tensor cores (tc_gemm.cu): C = A B (+ bias), A(m,k) = A[m*am + k*ak],
-// B(k,n) = B[k*bk + n*bn]; work: tc_sgemm_work(M, N, K) floats (0: none needed)
-exotx_status tc_sgemm(int M, int N, int K, const float *A, long long am, long long ak, const float *B, long long bk,
-                      long long bn, float *C, long long ldc, const float *bias, float *work, size_t work_elems,
-                      cudaStream_t s);
-size_t tc_sgemm_work(int M, int N, int K);
+// FP32-accurate training GEMMs on the tensor cores (tc_gemm.cu), rows contiguous:
+// Z = X W^T + b (n x dout), and H = silu(Z) unless H is null
+constexpr int TG_MAXL = 8;
+exotx_status tc_mlp_forward(int n, int din, int dout, const float *X, const float *W, const float *bias, float *Z, float *H,
+                            cudaStream_t s);
+// Z (n x din) = (dZ W) silu'(Z)
+exotx_status tc_mlp_activation(int n, int din, int dout, const float *dZ, const float *W, float *Z, cudaStream_t s);
+// G[woff[l]] = dZ[l]^T H[l] and G[boff[l]] = column sums of dZ[l] for every layer, which together fill G's
+// nparams; work: tc_mlp_weights_work(nparams, n) floats
+exotx_status tc_mlp_weights(int nl, const int *din, const int *dout, const float *const *dZ, const float *const *H,
+                            const long long *woff, const long long *boff, long long nparams, int n, float *work, float *G,
+                            cudaStream_t s);
+size_t tc_mlp_weights_work(long long nparams, int n);
 exotx_status tc_sgemm_error(int *err, cudaStream_t s);
 exotx_status tc_error_reset(cudaStream_t s);
 exotx_status tc_error_read(int *err, cudaStream_t s);

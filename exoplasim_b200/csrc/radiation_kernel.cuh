@@ -153,6 +153,8 @@ __global__ void __launch_bounds__(rad_threads<T>(COLS), (sizeof(T) == 8 ? 512 : 
     int *next = reinterpret_cast<int *>(kc + RK_N);                      // pair chunks handed out
     unsigned short *pairs = reinterpret_cast<unsigned short *>(next + 2);
 #define V(a, k) sm[(S.a + (k)) * COLS]
+    const int count = D.cols ? *D.ncols : nhor;
+    if (blockIdx.x * COLS >= count) return;                              // an empty column list costs no more than this
     const T PI = (T)3.14159265359, TWOPI = PI + PI;
     const T ga = (T)P.ga, gascon = (T)P.gascon;
     const int nclouds = P.nclouds, newrsc = P.newrsc, nrscat = P.nrscat;
@@ -175,7 +177,6 @@ __global__ void __launch_bounds__(rad_threads<T>(COLS), (sizeof(T) == 8 ? 512 : 
     }
     if (lane == 0)
         for (int i = warp; i < RK_N; i += NTHR / 32) kc[i] = rad_const<T>(P, i);
-    const int count = D.cols ? *D.ncols : nhor;
     for (int base = blockIdx.x * COLS; base < count; base += gridDim.x * COLS) {
         const bool valid = base + c < count;
         const int w = valid ? base + c : count - 1;      // spare lanes repeat the last column and store nothing

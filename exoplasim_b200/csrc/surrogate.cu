@@ -40,8 +40,7 @@ struct exotx_mlp_s {
     bool prepared = false;
     int *fb = nullptr;       // [0] = fallback count, [1..] = column list
     int fb_cap = 0;
-    float *split = nullptr;  // split-K workspace of the weight-gradient GEMMs
-    size_t split_elems = 0;
+    float *split = nullptr;  // partial weight gradients, one set per range of the batch
 };
 
 namespace exotx {
@@ -122,14 +121,8 @@ __global__ void k_surr_targets(SurrIn<T> in, const T *dtdt, const T *dfd, const 
 
 // ------------------------------------------------------------ training (FP32)
 // The three GEMMs of a layer's forward and backward pass run on the tensor
-// cores in FP32-accurate split form (tc_sgemm, tc_gemm.cu); the element-wise
-// parts are the kernels below.
-
-__device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
-__device__ __forceinline__ float silu_grad(float z) {
-    const float sg = 1.f / (1.f + expf(-z));
-    return sg * (1.f + z * (1.f - sg));
-}
+// cores in FP32-accurate split form, with the activations and the bias
+// gradients (tc_gemm.cu); the loss and the optimiser are the kernels below.
 
 // inference activation: fast exponential and division (the result is rounded to BF16)
 // silu(z) = z sigmoid(z) = h + h tanh(h) with h = z/2: one MUFU operation (tanh.approx, max relative
@@ -144,14 +137,6 @@ __device__ __forceinline__ float silu_fast(float z) {
     return fmaf(h, tanh_approx(h), h);
 }
 
-__global__ void k_silu(const float *Z, float *H, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        H[i] = silu(Z[i]);
-}
-__global__ void k_silu_bwd(const float *dH, const float *Z, float *dZ, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        dZ[i] = dH[i] * silu_grad(Z[i]);
-}
 // mean (optionally weighted: Wt per element, may be null) squared error over
 // n x nout; dY = d(loss)/dY; loss accumulated into *loss
 __global__ void k_mse(const float *Y, const float *T, const float *Wt, float *dY, long long n, float scale,
@@ -171,22 +156,6 @@ __global__ void k_mse(const float *Y, const float *T, const float *Wt, float *dY
     }
     if (threadIdx.x == 0 && loss) atomicAdd(loss, red[0] * scale);
 }
-// db[o] = sum_b dZ[b][o]
-__global__ void k_colsum(const float *dZ, float *db, int n, int nc) {
-    const int o = blockIdx.x * 32 + (threadIdx.x & 31);
-    const int r0 = threadIdx.x >> 5, nr = blockDim.x >> 5;
-    __shared__ float red[8][33];
-    float acc = 0.f;
-    if (o < nc)
-        for (int b = r0; b < n; b += nr) acc += dZ[(size_t)b * nc + o];
-    red[r0][threadIdx.x & 31] = acc;
-    __syncthreads();
-    if (r0 == 0 && o < nc) {
-        float t = 0.f;
-        for (int r = 0; r < nr; r++) t += red[r][threadIdx.x & 31];
-        db[o] = t;
-    }
-}
 __global__ void k_adam(float *P, const float *G, float *M, float *V, long long n, float lr, float b1, float b2,
                        float eps, float c1, float c2) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -201,31 +170,18 @@ __global__ void k_adam(float *P, const float *G, float *M, float *V, long long n
 
 static unsigned grid_for(long long n) { return (unsigned)std::min<long long>((n + 255) / 256, 148 * 16); }
 
-// activations: Z_l, H_l (maxb x width) for hidden l, then Y, dY (maxb x nout), dA, dZa, dZb (maxb x width)
+// activations: Z_l, H_l (maxb x width) for hidden l, then Y, dY (maxb x nout);
+// the backward pass writes dZ_l over Z_l
 static float *ws_Z(exotx_mlp net, int l) { return net->ws + (size_t)2 * l * net->maxb * net->width; }
 static float *ws_H(exotx_mlp net, int l) { return ws_Z(net, l) + (size_t)net->maxb * net->width; }
 static float *ws_Y(exotx_mlp net) { return net->ws + (size_t)2 * net->nhid * net->maxb * net->width; }
 static float *ws_dY(exotx_mlp net) { return ws_Y(net) + (size_t)net->maxb * net->nout; }
-static float *ws_dA(exotx_mlp net) { return ws_dY(net) + (size_t)net->maxb * net->nout; }
-static float *ws_dZ(exotx_mlp net, int i) { return ws_dA(net) + (size_t)(1 + i) * net->maxb * net->width; }
 
-static exotx_status gemm(exotx_mlp net, int M, int N, int K, const float *A, long long am, long long ak,
-                         const float *B, long long bk, long long bn, float *C, long long ldc, const float *bias,
-                         cudaStream_t s) {
-    return tc_sgemm(M, N, K, A, am, ak, B, bk, bn, C, ldc, bias, net->split, net->split_elems, s);
-}
-
-static exotx_status mlp_forward(exotx_mlp net, const float *X, int n, cudaStream_t s) {
-    const float *H = X;
+static exotx_status mlp_forward(exotx_mlp net, const float *X, float *Y, int n, cudaStream_t s) {
     for (int l = 0; l < net->nl; l++) {
-        const int din = net->din[l], dout = net->dout[l];
-        float *Z = l < net->nhid ? ws_Z(net, l) : ws_Y(net);
-        EXOTX_TRY(gemm(net, n, dout, din, H, din, 1, net->P + net->woff[l], 1, din, Z, dout, net->P + net->boff[l], s));
-        if (l < net->nhid) {
-            k_silu<<<grid_for((long long)n * dout), 256, 0, s>>>(Z, ws_H(net, l), (long long)n * dout);
-            EXOTX_CHECK_LAUNCH();
-            H = ws_H(net, l);
-        }
+        const bool hid = l < net->nhid;
+        EXOTX_TRY(tc_mlp_forward(n, net->din[l], net->dout[l], l ? ws_H(net, l - 1) : X, net->P + net->woff[l],
+                                 net->P + net->boff[l], hid ? ws_Z(net, l) : Y, hid ? ws_H(net, l) : nullptr, s));
     }
     return EXOTX_OK;
 }
@@ -611,14 +567,12 @@ EXOTX_API exotx_status exotx_mlp_create(int nin, int width, int nhidden, int nou
         net->boff[l] = off; off += net->dout[l];
     }
     net->nparams = off;
-    const size_t wsf = (size_t)2 * nhidden * max_batch * width + (size_t)2 * max_batch * nout +
-                       (size_t)3 * max_batch * width;
-    net->split_elems = tc_sgemm_work(std::max(width, nout), std::max(nin, width), max_batch);
+    const size_t wsf = (size_t)2 * nhidden * max_batch * width + (size_t)2 * max_batch * nout;
     bool ok = cudaMalloc(&net->P, off * 4) == cudaSuccess && cudaMalloc(&net->G, off * 4) == cudaSuccess &&
               cudaMalloc(&net->M, off * 4) == cudaSuccess && cudaMalloc(&net->V, off * 4) == cudaSuccess &&
               cudaMalloc(&net->ws, wsf * 4) == cudaSuccess &&
               cudaMalloc(&net->norm, sizeof(float) * (4 * nin + 2 * nout)) == cudaSuccess &&
-              (net->split_elems == 0 || cudaMalloc(&net->split, net->split_elems * 4) == cudaSuccess);
+              cudaMalloc(&net->split, tc_mlp_weights_work(off, max_batch) * 4) == cudaSuccess;
     ok = ok && cudaMemset(net->P, 0, off * 4) == cudaSuccess && cudaMemset(net->G, 0, off * 4) == cudaSuccess &&
          cudaMemset(net->M, 0, off * 4) == cudaSuccess && cudaMemset(net->V, 0, off * 4) == cudaSuccess;
     if (!ok) {
@@ -666,10 +620,7 @@ EXOTX_API exotx_status exotx_mlp_set_norm(exotx_mlp net, const float *host_norm)
 EXOTX_API exotx_status exotx_mlp_forward(exotx_mlp net, const float *X, float *Y, int n, exotx_stream s) {
     if (!net || !X || !Y || n < 0 || n > net->maxb) return EXOTX_BAD_ARG;
     if (n == 0) return EXOTX_OK;
-    EXOTX_TRY(mlp_forward(net, X, n, (cudaStream_t)s));
-    EXOTX_CUDA(cudaMemcpyAsync(Y, ws_Y(net), sizeof(float) * n * net->nout, cudaMemcpyDeviceToDevice,
-                               (cudaStream_t)s));
-    return EXOTX_OK;
+    return mlp_forward(net, X, Y, n, (cudaStream_t)s);
 }
 
 EXOTX_API exotx_status exotx_mlp_backward(exotx_mlp net, const float *X, const float *Tt, int n, float *loss,
@@ -681,31 +632,19 @@ EXOTX_API exotx_status exotx_mlp_backward_weighted(exotx_mlp net, const float *X
                                                    int n, float *loss, exotx_stream sv) {
     if (!net || !X || !Tt || n < 1 || n > net->maxb) return EXOTX_BAD_ARG;
     cudaStream_t s = (cudaStream_t)sv;
-    EXOTX_TRY(mlp_forward(net, X, n, s));
+    EXOTX_TRY(mlp_forward(net, X, ws_Y(net), n, s));
     const long long ny = (long long)n * net->nout;
     k_mse<<<grid_for(ny), 256, 0, s>>>(ws_Y(net), Tt, Wt, ws_dY(net), ny, 1.f / (float)ny, loss);
     EXOTX_CHECK_LAUNCH();
-    const float *dZ = ws_dY(net);
-    int cur = 0;
+    // dZ of every layer, from the last down: dH_prev = dZ W through the SiLU of layer l-1
+    const float *dZ[MLP_MAX_LAYERS], *Hp[MLP_MAX_LAYERS];
     for (int l = net->nl - 1; l >= 0; l--) {
-        const int din = net->din[l], dout = net->dout[l];
-        const float *Hp = l > 0 ? ws_H(net, l - 1) : X;
-        // dW = dZ^T H_prev, db = column sums of dZ
-        EXOTX_TRY(gemm(net, dout, din, n, dZ, 1, dout, Hp, din, 1, net->G + net->woff[l], din, nullptr, s));
-        k_colsum<<<(dout + 31) / 32, 256, 0, s>>>(dZ, net->G + net->boff[l], n, dout);
-        EXOTX_CHECK_LAUNCH();
-        if (l > 0) {
-            // dH_prev = dZ W, then through the SiLU of layer l-1
-            EXOTX_TRY(gemm(net, n, din, dout, dZ, dout, 1, net->P + net->woff[l], din, 1, ws_dA(net), din, nullptr, s));
-            float *dZn = ws_dZ(net, cur);
-            k_silu_bwd<<<grid_for((long long)n * din), 256, 0, s>>>(ws_dA(net), ws_Z(net, l - 1), dZn,
-                                                                  (long long)n * din);
-            EXOTX_CHECK_LAUNCH();
-            dZ = dZn;
-            cur ^= 1;
-        }
+        dZ[l] = l < net->nhid ? ws_Z(net, l) : ws_dY(net);
+        Hp[l] = l > 0 ? ws_H(net, l - 1) : X;
+        if (l > 0)
+            EXOTX_TRY(tc_mlp_activation(n, net->din[l], net->dout[l], dZ[l], net->P + net->woff[l], ws_Z(net, l - 1), s));
     }
-    return EXOTX_OK;
+    return tc_mlp_weights(net->nl, net->din, net->dout, dZ, Hp, net->woff, net->boff, net->nparams, n, net->split, net->G, s);
 }
 
 EXOTX_API exotx_status exotx_mlp_check(exotx_mlp net, exotx_stream s) {
