@@ -9,12 +9,10 @@
 // the forward set's 9L+1 fields, with consecutive threads on consecutive
 // columns (every access is a coalesced row of the NHOR-fastest layout).  The
 // O(L^2) sums (the c(j,k) and g(i,k) matrices of the semi-implicit scheme)
-// need the whole column's zvgpg, zvgpg + gd and ztv1 - gt: those three
-// profiles live in shared memory, laid out level-major so that a warp's
-// accesses fall in distinct banks.  The matrices and per-level constants are
-// one small block, staged in shared memory in the step's precision once per
-// block where it fits (every thread of a warp then reads it word for word
-// alike).  The kernel is HBM-bound: (15L+4) values move per column.
+// run over zvgpg, zvgpg + gd and ztv1 - gt of the column: their partial sums
+// live in registers, or for many levels the profiles in shared memory, laid out
+// level-major so that a warp's accesses fall in distinct banks.  The kernel is
+// HBM-bound: (15L+4) values move per column.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -28,9 +26,11 @@ struct exotx_gpconst_s {
 
 namespace exotx {
 
-exotx_status launch_gridpoint_fp64(const GpArgs<double> &A, cudaStream_t s);
+exotx_status launch_gridpoint_fp64(const GpArgs<double> &A, const exotx_gp_params &h, cudaStream_t s);
 
-static exotx_status launch_gridpoint_fp32(const GpArgs<float> &A, cudaStream_t s) { return gp_launch<float>(A, s); }
+static exotx_status launch_gridpoint_fp32(const GpArgs<float> &A, const exotx_gp_params &h, cudaStream_t s) {
+    return gp_launch<float>(A, h, s);
+}
 
 }  // namespace exotx
 
@@ -139,12 +139,12 @@ EXOTX_API exotx_status exotx_gridpoint(exotx_plan p, exotx_gpconst c, int prec, 
         A.sid = p->d_sid; A.k = c->d; A.ncol = nhor * ninst;
         A.L = L; A.nhor = (int)nhor; A.nlon = p->nlon; A.nqspec = c->h.nqspec; A.g_lower = c->g_lower;
         A.akap = c->h.akap; A.rdbrv = c->h.rdbrv; A.adv = c->h.adv; A.psurf = c->h.psurf; A.ww = c->h.ww;
-        return launch_gridpoint_fp64(A, (cudaStream_t)s);
+        return launch_gridpoint_fp64(A, c->h, (cudaStream_t)s);
     }
     GpArgs<float> A;
     A.gin = (const float *)gin; A.gout = (float *)gout; A.dw = (float *)dw; A.dq = (const float *)dq;
     A.sid = p->d_sid; A.k = c->d; A.ncol = nhor * ninst;
     A.L = L; A.nhor = (int)nhor; A.nlon = p->nlon; A.nqspec = c->h.nqspec; A.g_lower = c->g_lower;
     A.akap = c->h.akap; A.rdbrv = c->h.rdbrv; A.adv = c->h.adv; A.psurf = c->h.psurf; A.ww = c->h.ww;
-    return launch_gridpoint_fp32(A, (cudaStream_t)s);
+    return launch_gridpoint_fp32(A, c->h, (cudaStream_t)s);
 }

@@ -3,5 +3,7 @@
 #include "gridpoint_kernel.cuh"
 
 namespace exotx {
-exotx_status launch_gridpoint_fp64(const GpArgs<double> &A, cudaStream_t s) { return gp_launch<double>(A, s); }
+exotx_status launch_gridpoint_fp64(const GpArgs<double> &A, const exotx_gp_params &h, cudaStream_t s) {
+    return gp_launch<double>(A, h, s);
+}
 }  // namespace exotx
