@@ -68,6 +68,9 @@ SIGNATURES = {
     "exotx_sp2fcdmu": [_P, _I, _P, _P, _I, _S],
     "exotx_fc2sp": [_P, _I, _P, _P, _I, _S],
     "exotx_dv2uv": [_P, _I, _P, _P, _P, _P, _I, _S],
+    "exotx_sp2gp_scaled": [_P, _I, _P, _P, _I, C.c_double, _I, _P, _S],
+    "exotx_dv2gp_scaled": [_P, _I, _P, _P, _P, _P, _I, _P, C.c_double, _I, _P, _S],
+    "exotx_gp2sp_scaled": [_P, _I, _P, _P, _I, C.c_double, _P, _S],
     "exotx_uv2dv": [_P, _I, _P, _P, _P, _P, _I, _S],
     "exotx_mktend": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _S],
     "exotx_qtend": [_P, _I, _P, _P, _P, _P, _I, _S],

@@ -131,13 +131,16 @@ struct FourierLayout {
 enum { OP_SP2FC = 0, OP_SP2FCDMU = 1, OP_DV2UV = 2 };
 enum { OP_FC2SP = 0, OP_UV2DV = 1, OP_QTEND = 2, OP_MKTEND = 3 };
 
-// FP64 tensor-core Legendre launchers (legendre_fp64mma.cu)
+// FP64 tensor-core Legendre launchers (legendre_fp64mma.cu).  The outputs are
+// multiplied by scale, and the inverse's by each latitude's rscale (device
+// memory, null: 1) and, with roll, by (-1)^m, which turns the grid row by half
 template <typename T>
 exotx_status leg_inverse_l(exotx_plan p, int op, const T *a, const T *b, T *oa, T *ob, int nlev,
-                           long long a_fs, long long b_fs, FourierLayout L, cudaStream_t s);
+                           long long a_fs, long long b_fs, FourierLayout L, cudaStream_t s, double scale = 1.0,
+                           const double *rscale = nullptr, bool roll = false);
 template <typename T>
 exotx_status leg_forward_l(exotx_plan p, int op, const T *const *in, T *const *out, int nlev,
-                           FourierLayout L, long long o_fs, cudaStream_t s);
+                           FourierLayout L, long long o_fs, cudaStream_t s, double scale = 1.0);
 // the Legendre half of a set in one launch over up to TC_MAXSEG segments, a
 // resolution, a level count and a run of states each (dset = 0 gridpointa, 1
 // gridpointd, one segment): inverse spectral states -> m-major intermediate,

@@ -93,6 +93,9 @@ struct LegInv {
     int wm, wn, kc;      // warps along latitudes and columns; modes staged at a time
     int L, nlat, nlath, ntl, ntp1, nrsp, dset, mz;  // ntl: tiles of 8 latitudes; single op: wavenumbers ntp1 <= m < mz are zeroed
     double plavor;
+    const double *rscale;  // single op: factor of each latitude's coefficients (null: 1) ...
+    double scale;          // ... times this,
+    int roll;              // and (-1)^m: the grid row turned by half its length
 };
 
 // One launch covers up to NSEG segments (a resolution, a level count and a run
@@ -308,7 +311,8 @@ __global__ void __launch_bounds__(192, NT == 1 ? 2 : 4) k_leg_inv(const __grid_c
             reinterpret_cast<C2<T> *>(o)[(size_t)m * A.nrows + f * nlat + lat] = C2<T>{(T)x, (T)y};
         } else {
             const size_t e = 2 * (f * A.fs + lat * A.ls + (long long)m * A.ms);
-            o[e] = (T)x; o[e + 1] = (T)y;
+            const double sc = (A.roll && (m & 1) ? -A.scale : A.scale) * (A.rscale ? A.rscale[lat] : 1.0);
+            o[e] = (T)(x * sc); o[e + 1] = (T)(y * sc);
         }
     };
     if (g < 2) {
@@ -386,6 +390,7 @@ struct LegFwd {
     long long fs, ls, ms, nrows;
     T *out[3];               // single op: spectral outputs; set: out[0] is the set's output
     long long o_fs;          // spectral field stride (reals)
+    double scale;            // single op: factor of the outputs
     int folded;              // the intermediate holds N+S, then N-S per field (rfft_fwd_fold_body)
     int nu, nt;              // units (levels x states) and unit tiles per wavenumber
     int nu1, nt1;            // gridpointa: ln ps tendencies (fc2sp) and their tiles
@@ -578,7 +583,7 @@ __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, double *sm, in
     for (int i = 0; i < MT; i++) {
         const int kk = (kt0 + i) * 8 + r, k = 2 * kk + p;
         if (kk >= kq) continue;
-        const double f = A.filt[m + k];
+        const double f = SET ? A.filt[m + k] : A.filt[m + k] * A.scale;
 #pragma unroll
         for (int x = 0; x < NOUT; x++) {
             T *d;
@@ -682,13 +687,15 @@ static exotx_status inv_launch(LegItem<LegInv<T>> *it, int n, cudaStream_t s) {
 
 template <typename T>
 exotx_status leg_inverse_l(exotx_plan p, int op, const T *a, const T *b, T *oa, T *ob, int nlev,
-                           long long a_fs, long long b_fs, FourierLayout L, cudaStream_t s) {
+                           long long a_fs, long long b_fs, FourierLayout L, cudaStream_t s, double scale,
+                           const double *rscale, bool roll) {
     if (nlev <= 0) return EXOTX_OK;
     if (op != OP_SP2FC && op != OP_SP2FCDMU && op != OP_DV2UV) return EXOTX_BAD_ARG;
     LegItem<LegInv<T>> it = {p, {}};
     LegInv<T> &A = it.a;
     A.a = a; A.b = b; A.a_fs = a_fs; A.b_fs = b_fs;
     A.oa = oa; A.ob = ob; A.fs = L.fs; A.ls = L.ls; A.ms = L.ms; A.mz = L.mz;
+    A.scale = scale; A.rscale = rscale; A.roll = roll;
     A.nu[op == OP_SP2FC ? 0 : op == OP_SP2FCDMU ? 1 : 2] = nlev;
     return inv_launch<T, false, 1>(&it, 1, s);
 }
@@ -757,7 +764,7 @@ static exotx_status fwd_launch(LegItem<LegFwd<T>> *it, int n, cudaStream_t s) {
 
 template <typename T>
 exotx_status leg_forward_l(exotx_plan p, int op, const T *const *in, T *const *out, int nlev,
-                           FourierLayout L, long long o_fs, cudaStream_t s) {
+                           FourierLayout L, long long o_fs, cudaStream_t s, double scale) {
     if (nlev <= 0) return EXOTX_OK;
     LegItem<LegFwd<T>> it = {p, {}};
     LegFwd<T> &A = it.a;
@@ -765,7 +772,7 @@ exotx_status leg_forward_l(exotx_plan p, int op, const T *const *in, T *const *o
     const int nout = op == OP_MKTEND ? 3 : op == OP_UV2DV ? 2 : 1;
     for (int i = 0; i < nin; i++) A.in[i] = in[i];
     for (int i = 0; i < nout; i++) A.out[i] = out[i];
-    A.fs = L.fs; A.ls = L.ls; A.ms = L.ms; A.o_fs = o_fs;
+    A.fs = L.fs; A.ls = L.ls; A.ms = L.ms; A.o_fs = o_fs; A.scale = scale;
     A.nu = nlev;
     switch (op) {
         case OP_FC2SP: return fwd_launch<T, OP_FC2SP, false, 1>(&it, 1, s);
@@ -803,9 +810,9 @@ exotx_status leg_forward_set(const LegSeg<T> *segs, int n, int dset, cudaStream_
 
 #define LEG_INSTANCES(T)                                                                                            \
     template exotx_status leg_inverse_l<T>(exotx_plan, int, const T *, const T *, T *, T *, int, long long,         \
-                                           long long, FourierLayout, cudaStream_t);                                 \
+                                           long long, FourierLayout, cudaStream_t, double, const double *, bool);   \
     template exotx_status leg_forward_l<T>(exotx_plan, int, const T *const *, T *const *, int, FourierLayout,       \
-                                           long long, cudaStream_t);                                                \
+                                           long long, cudaStream_t, double);                                        \
     template exotx_status leg_inverse_set<T>(const LegSeg<T> *, int, int, cudaStream_t);                            \
     template exotx_status leg_forward_set<T>(const LegSeg<T> *, int, int, cudaStream_t);
 LEG_INSTANCES(double)

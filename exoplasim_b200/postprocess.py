@@ -49,18 +49,20 @@ def transformvar(variable, nlat, nlon, nlev, ntru, mode="grid", physfilter=False
             return _out(v, isnp)
         ntimes = v.shape[0]
         nlevs = v.shape[1] if v.dim() == 3 else 1
-        sp = v.reshape(ntimes * nlevs, nrsp).t()                       # Fortran (NRSP, times*levels)
-        gp = pyfft.sp2gp(sp, nlat, nlon, ntru, nfs)                    # (nlon, nlat, times*levels)
+        p = pyfft._plan(int(nlat), nfs)
+        pyfft._check_trunc(p, nlon, ntru)
         shape = (ntimes, nlevs, nlat, nlon) if v.dim() == 3 else (ntimes, nlat, nlon)
-        gp = gp.permute(2, 1, 0).reshape(shape)
-        return _out(torch.roll(gp, nlon // 2, dims=-1), isnp)
+        # sp2gp of every time and level, the half-turn of the longitudes with it
+        gp = pyfft._sp_to_grid(p, v.reshape(ntimes * nlevs, nrsp).contiguous(), roll=True)
+        return _out(gp.reshape(shape), isnp)
     if mode == "spectral":
         if spectral:
             out = v
         elif v.dim() in (3, 4):
             lead = v.shape[:-2]
-            gp = v.reshape(-1, nlat, nlon).permute(2, 1, 0)           # (nlon, nlat, times*levels)
-            out = pyfft.gp2sp(gp, nlat, nlon, ntru, nfs).t().reshape(*lead, nrsp)
+            p = pyfft._plan(int(nlat), nfs)
+            pyfft._check_trunc(p, nlon, ntru)
+            out = pyfft._grid_to_sp(p, v.reshape(-1, nlat, nlon).contiguous()).reshape(*lead, nrsp)
         else:
             return _out(v, isnp)                                       # columns and scalars pass through
         return _out(out.reshape(*out.shape[:-1], nrsp // 2, 2), isnp)
@@ -97,13 +99,13 @@ def transformvectorvar(uvar, vvar, lats, nlon, nlev, ntru, mode="grid", physfilt
         return _out(u, isnp), _out(v, isnp)
     ntimes = u.shape[0]
     nlevs = u.shape[1] if u.dim() == 3 else 1
-    rdcostheta = radius / np.cos(rlats)
-    su = u.reshape(ntimes * nlevs, nrsp).t()
-    sv = v.reshape(ntimes * nlevs, nrsp).t()
-    gu, gv = pyfft.spvgp(su, sv, torch.as_tensor(rdcostheta, device="cuda"), nlon, ntru, int(physfilter))
+    rdcostheta = torch.from_numpy(np.ascontiguousarray(radius / np.cos(rlats)))
+    p = pyfft._plan(nlat, int(physfilter))
+    pyfft._check_trunc(p, nlon, ntru)
+    su, sv = (t.reshape(ntimes * nlevs, nrsp).contiguous() for t in (u, v))
+    gu, gv = pyfft._dv_to_grid(p, su, sv, rdcostheta.to("cuda", non_blocking=True), roll=True)
     shape = (ntimes, nlevs, nlat, nlon) if u.dim() == 3 else (ntimes, nlat, nlon)
-    f = lambda g: torch.roll(g.permute(2, 1, 0).reshape(shape), nlon // 2, dims=-1)  # noqa: E731
-    return _out(f(gu), isnp), _out(f(gv), isnp)
+    return _out(gu.reshape(shape), isnp), _out(gv.reshape(shape), isnp)
 
 
 def refactor(variable, header, ntimes=None, nlev=10):

@@ -32,7 +32,8 @@ import functools
 import numpy as np
 import torch
 
-from .transforms import Plan
+from ._lib import call
+from .transforms import FP64, Plan, _ptr, _stream
 
 SQRT2 = 1.4142135623730951
 
@@ -75,6 +76,41 @@ def _grid_levels(gp):
     if gp.dim() == 2:
         gp = gp.unsqueeze(-1)
     return gp.permute(2, 1, 0).contiguous()
+
+
+def _work(p, nfields):
+    return torch.empty(nfields * p.nlat * (p.ntru + 1) * 2, dtype=torch.float64, device="cuda")
+
+
+def _sp_to_grid(p, lev, roll=False):
+    """(nlev, NRSP) -> (nlev, nlat, nlon): sp2fc, fc2gp, times sqrt(2); roll: by half a turn of longitude."""
+    g = torch.empty((lev.shape[0], p.nlat, p.nlon), dtype=torch.float64, device="cuda")
+    call("exotx_sp2gp_scaled", p._h, FP64, _ptr(lev), _ptr(g), lev.shape[0], SQRT2, int(roll),
+         _ptr(_work(p, lev.shape[0])), _stream())
+    return g
+
+
+def _dv_to_grid(p, d, z, rowscale, roll=False):
+    """(divergence, vorticity) (nlev, NRSP) -> winds (nlev, nlat, nlon) times sqrt(2) rowscale(nlat)."""
+    if z.shape != d.shape:
+        raise ValueError(f"divergence {tuple(d.shape)} and vorticity {tuple(z.shape)} differ")
+    n = d.shape[0]
+    u, v = (torch.empty((n, p.nlat, p.nlon), dtype=torch.float64, device="cuda") for _ in range(2))
+    call("exotx_dv2gp_scaled", p._h, FP64, _ptr(d), _ptr(z), _ptr(u), _ptr(v), n, _ptr(rowscale), SQRT2, int(roll),
+         _ptr(_work(p, 2 * n)), _stream())
+    return u, v
+
+
+def _grid_to_sp(p, rows):
+    """(nlev, nlat, nlon) -> (nlev, NRSP): gp2fc of gp/sqrt(2), fc2sp."""
+    if tuple(rows.shape[1:]) != (p.nlat, p.nlon):
+        raise ValueError(f"grid levels must be {(p.nlat, p.nlon)}, got {tuple(rows.shape[1:])}")
+    if rows.data_ptr() % 16:
+        rows = rows.clone()   # a view that starts on an odd element
+    sp = torch.empty((rows.shape[0], p.nrsp), dtype=torch.float64, device="cuda")
+    call("exotx_gp2sp_scaled", p._h, FP64, _ptr(rows), _ptr(sp), rows.shape[0], 1.0 / SQRT2,
+         _ptr(_work(p, rows.shape[0])), _stream())
+    return sp
 
 
 def inigau(nlat):
@@ -171,11 +207,7 @@ def sp2gp(sp, nlat, nlon, ntru, nfs=0):
     t, isnp = _dev(sp)
     p = _plan(int(nlat), int(nfs))
     _check_trunc(p, nlon, ntru)
-    lev = _spec_levels(t, p.ntru)
-    g = p.sp2fc(lev)
-    Plan.fc2gp(g)
-    g.mul_(SQRT2)
-    return _out(g.permute(2, 1, 0), isnp)
+    return _out(_sp_to_grid(p, _spec_levels(t, p.ntru)).permute(2, 1, 0), isnp)
 
 
 def gp2sp(gp, nlat, nlon, ntru, nfs=0):
@@ -183,10 +215,7 @@ def gp2sp(gp, nlat, nlon, ntru, nfs=0):
     t, isnp = _dev(gp)
     p = _plan(int(nlat), int(nfs))
     _check_trunc(p, nlon, ntru)
-    rows = _grid_levels(t) / SQRT2
-    Plan.gp2fc(rows)
-    sp = p.fc2sp(rows)
-    return _out(sp.t(), isnp)
+    return _out(_grid_to_sp(p, _grid_levels(t)).t(), isnp)
 
 
 def dv2uv(sd, sz, nlat, nlon, ntru, nlev=None, nfs=0):
@@ -224,12 +253,7 @@ def spvgp(sd, sz, rdcostheta, nlon, ntru, nfs=0):
     nlat = rc.shape[0]
     p = _plan(int(nlat), int(nfs))
     _check_trunc(p, nlon, ntru)
-    u, v = p.dv2uv(_spec_levels(td, p.ntru), _spec_levels(tz, p.ntru))
-    Plan.fc2gp(u)
-    Plan.fc2gp(v)
-    scale = (rc * SQRT2).view(1, nlat, 1)
-    u.mul_(scale)
-    v.mul_(scale)
+    u, v = _dv_to_grid(p, _spec_levels(td, p.ntru), _spec_levels(tz, p.ntru), rc.reshape(nlat).contiguous())
     return _out(u.permute(2, 1, 0), isnp), _out(v.permute(2, 1, 0), isnp)
 
 

@@ -112,6 +112,17 @@ exotx_status exotx_mktend(exotx_plan p, int prec, void *d, void *t, void *z,
 exotx_status exotx_qtend(exotx_plan p, int prec, void *q, const void *qn,
                          const void *uq, const void *vq, int nlev, exotx_stream s);
 
+/* ---- spectral <-> grid in one call, without the reference's Fourier rows between ----
+ * gp = scale * fc2gp(sp2fc(sp)), the rows turned by NLON/2 with roll; gu, gv the same of dv2uv(pd, pz), each
+ * latitude also times rscale (device memory, NLAT doubles, may be null); sp = scale * fc2sp(gp2fc(gp)), gp kept.
+ * FP64 and FP32; gp 16-byte aligned; work: nlev (dv2gp: 2 nlev) x NLAT x (NTRU+1) complex values */
+exotx_status exotx_sp2gp_scaled(exotx_plan p, int prec, const void *sp, void *gp, int nlev, double scale, int roll,
+                                void *work, exotx_stream s);
+exotx_status exotx_dv2gp_scaled(exotx_plan p, int prec, const void *pd, const void *pz, void *gu, void *gv, int nlev,
+                                const double *rscale, double scale, int roll, void *work, exotx_stream s);
+exotx_status exotx_gp2sp_scaled(exotx_plan p, int prec, const void *gp, void *sp, int nlev, double scale, void *work,
+                                exotx_stream s);
+
 /* ---- real FFTs of lot rows of length n, in place ---- */
 /* gp2fc (fftmod.f90:29 / fft991mod.f90:32): grid rows -> (A0,0,A1,B1,...) x 1/n */
 exotx_status exotx_gp2fc(int prec, void *a, int n, int lot, exotx_stream s);
