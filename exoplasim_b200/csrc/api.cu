@@ -87,7 +87,7 @@ static exotx_status inv_api(exotx_plan p, int prec, int op, const void *a, const
     FourierLayout F = ref_layout(p);
     return by_prec(prec, [&](auto tag) {
         using T = std::remove_pointer_t<decltype(tag)>;
-        return leg_inverse_l<T>(p, op, (const T *)a, (const T *)b, (T *)oa, (T *)ob, nlev, nrsp, nrsp, F,
+        return leg_inverse_l<T>(p, op, (const T *)a, (const T *)b, (T *)oa, (T *)ob, nlev, nrsp, F,
                                 (cudaStream_t)s);
     });
 }
@@ -182,7 +182,7 @@ EXOTX_API exotx_status exotx_sp2gp_scaled(exotx_plan p, int prec, const void *sp
     const long long nrsp = 2LL * p->ncsp, rows = (long long)nlev * p->nlat;
     return by_prec(prec, [&](auto tag) {
         using T = std::remove_pointer_t<decltype(tag)>;
-        EXOTX_TRY(leg_inverse_l<T>(p, OP_SP2FC, (const T *)sp, nullptr, (T *)work, nullptr, nlev, nrsp, nrsp,
+        EXOTX_TRY(leg_inverse_l<T>(p, OP_SP2FC, (const T *)sp, nullptr, (T *)work, nullptr, nlev, nrsp,
                                    FourierLayout{p->nlat, 1, rows, p->ntp1}, (cudaStream_t)s, scale, nullptr, roll != 0));
         return fft_inverse_l<T>((const T *)work, (T *)gp, p->nlon, rows, p->ntp1, 1, rows, (cudaStream_t)s);
     });
@@ -198,7 +198,7 @@ EXOTX_API exotx_status exotx_dv2gp_scaled(exotx_plan p, int prec, const void *pd
     return by_prec(prec, [&](auto tag) {
         using T = std::remove_pointer_t<decltype(tag)>;
         T *wu = (T *)work, *wv = wu + 2 * rows * p->ntp1;
-        EXOTX_TRY(leg_inverse_l<T>(p, OP_DV2UV, (const T *)pd, (const T *)pz, wu, wv, nlev, nrsp, nrsp,
+        EXOTX_TRY(leg_inverse_l<T>(p, OP_DV2UV, (const T *)pd, (const T *)pz, wu, wv, nlev, nrsp,
                                    FourierLayout{p->nlat, 1, rows, p->ntp1}, (cudaStream_t)s, scale, rscale, roll != 0));
         EXOTX_TRY(fft_inverse_l<T>(wu, (T *)gu, p->nlon, rows, p->ntp1, 1, rows, (cudaStream_t)s));
         return fft_inverse_l<T>(wv, (T *)gv, p->nlon, rows, p->ntp1, 1, rows, (cudaStream_t)s);

@@ -136,7 +136,7 @@ enum { OP_FC2SP = 0, OP_UV2DV = 1, OP_QTEND = 2, OP_MKTEND = 3 };
 // memory, null: 1) and, with roll, by (-1)^m, which turns the grid row by half
 template <typename T>
 exotx_status leg_inverse_l(exotx_plan p, int op, const T *a, const T *b, T *oa, T *ob, int nlev,
-                           long long a_fs, long long b_fs, FourierLayout L, cudaStream_t s, double scale = 1.0,
+                           long long fs, FourierLayout L, cudaStream_t s, double scale = 1.0,
                            const double *rscale = nullptr, bool roll = false);
 template <typename T>
 exotx_status leg_forward_l(exotx_plan p, int op, const T *const *in, T *const *out, int nlev,

@@ -84,8 +84,8 @@ struct LegInv {
     size_t tsz;
     const int *woff;
     const double *filt;  // skspgp(n)
-    const T *a, *b;      // spectral inputs (re, im pairs); single op: fields a (and b) at stride a_fs (b_fs)
-    long long a_fs, b_fs;
+    const T *a;          // spectral inputs (re, im pairs); single op: fields at stride a_fs,
+    long long a_fs, b_off;   // the second input b_off bytes from the first
     T *oa, *ob;          // Fourier outputs (set: oa is the intermediate)
     long long fs, ls, ms, nrows;
     int nu[3], nt[3];    // units and column tiles of each group
@@ -184,41 +184,48 @@ __global__ void __launch_bounds__(192, NT == 1 ? 2 : 4) k_leg_inv(const __grid_c
         if (kb) __syncthreads();
         // stage the filtered coefficients, even modes then odd ones, zeros past the
         // last mode and column; a warp takes a column, lanes along its modes
-        for (int c = warp; c < cb; c += blockDim.x >> 5) {
-            const T *pa = nullptr, *pb = nullptr;
-            if (c < n) {
+        // two columns at a time, their loads together
+        const int nw = blockDim.x >> 5;
+        const long long bo = SET ? (long long)sizeof(T) * 2 * A.L * A.nrsp : A.b_off;   // bytes from a's field to b's
+        for (int cc = warp; cc < cb; cc += 2 * nw) {
+            const T *pa[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int c = cc + h * nw, u = u0 + min(c, n - 1);
                 if constexpr (SET) {
                     int inst, fin, fout;
-                    if (g == 0) inv_field(A.L, A.dset, u0 + c, &inst, &fin, &fout);
-                    else if (g == 1) { inst = u0 + c; fin = 4 * A.L; }
-                    else { inst = (u0 + c) / A.L; fin = (u0 + c) - inst * A.L; }
-                    pa = A.a + ((size_t)inst * (4 * A.L + 1) + fin) * A.nrsp;
-                    pb = pa + (size_t)2 * A.L * A.nrsp;
+                    if (g == 0) inv_field(A.L, A.dset, u, &inst, &fin, &fout);
+                    else if (g == 1) { inst = u; fin = 4 * A.L; }
+                    else { inst = u / A.L; fin = u - inst * A.L; }
+                    pa[h] = A.a + ((size_t)inst * (4 * A.L + 1) + fin) * A.nrsp;
                 } else {
-                    pa = A.a + (u0 + c) * A.a_fs;
-                    if (g == 2) pb = A.b + (u0 + c) * A.b_fs;
+                    pa[h] = A.a + u * A.a_fs;
                 }
-                pa += 2 * (w0 + kb);
-                pb += 2 * (w0 + kb);
+                pa[h] += 2 * (w0 + kb);
             }
             const double *fl = A.filt + m + kb;
-#pragma unroll 2
             for (int k = lane; k < kp; k += 32) {
-                Z2 va{0, 0}, vb{0, 0};
-                if (c < n && k < kn) {
-                    const double f = fl[k];
-                    va = ld2(pa + 2 * k);
-                    va.x *= f; va.y *= f;
+                Z2 va[2], vb[2];
+                const double f = k < kn ? fl[k] : 0.0;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const bool in = cc + h * nw < n && k < kn;
+                    va[h] = vb[h] = Z2{0, 0};
+                    if (in) va[h] = ld2(pa[h] + 2 * k);
+                    if (in && g == 2) vb[h] = ld2(reinterpret_cast<const T *>(reinterpret_cast<const char *>(pa[h] + 2 * k) + bo));
+                }
+                const int o = ((k & 1) * kh + (k >> 1)) * rs;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int c = cc + h * nw;
+                    if (c >= cb) break;
+                    *reinterpret_cast<Z2 *>(xs + o + 2 * c) = Z2{va[h].x * f, va[h].y * f};
                     if (g == 2) {
                         // vorticity; plavor leaves mode (0,1) (legmod.f90:332)
-                        vb = ld2(pb + 2 * k);
-                        if (m == 0 && kb + k == 1) vb.x -= A.plavor;
-                        vb.x *= f; vb.y *= f;
+                        if (m == 0 && kb + k == 1 && c < n) vb[h].x -= A.plavor;
+                        *reinterpret_cast<Z2 *>(xz + o + 2 * c) = Z2{vb[h].x * f, vb[h].y * f};
                     }
                 }
-                const int o = ((k & 1) * kh + (k >> 1)) * rs + 2 * c;
-                *reinterpret_cast<Z2 *>(xs + o) = va;
-                if (g == 2) *reinterpret_cast<Z2 *>(xz + o) = vb;
             }
         }
         __syncthreads();
@@ -376,7 +383,10 @@ __global__ void __launch_bounds__(192, NT == 1 ? 2 : 4) k_leg_inv(const __grid_c
 enum { OP_LEVEL_A = 4, OP_LEVEL_D = 5 };
 
 constexpr int FWD_THREADS = 192;   // least threads of a block
-constexpr int FWD_JC = 16;         // latitude pairs per staged chunk
+// latitude pairs per staged chunk (of esize-byte values).  Few inputs leave room for
+// longer chunks, fewer waits for the slowest warp: gridpointd T127 L20 x8 238 -> 222 us;
+// in FP64 the copies on their way would take a block per SM with them (T63: 31 -> 34 us)
+__host__ __device__ constexpr int fwd_jc(int nin, size_t esize) { return nin <= 4 && esize == 4 ? 32 : 16; }
 // staged (north, south) values per thread and chunk: 9 inputs x 4 units x 16 pairs over 192 threads
 constexpr int FWD_ITEMS = 3;
 
@@ -448,7 +458,8 @@ __device__ __forceinline__ void fwd_terms(double (*o)[FwdShape<OP>::nout][2], co
 template <typename T, int OP, int MT, bool SET>
 __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, double *sm, int m, int mblk, int u0, int n) {
     using S = FwdShape<OP>;
-    constexpr int NIN = S::nin, NOUT = S::nout, rs = leg_stride(8), SEL = FWD_JC * rs, BUF = NIN * 2 * SEL;
+    constexpr int NIN = S::nin, NOUT = S::nout, rs = leg_stride(8);
+    constexpr int FWD_JC = fwd_jc(NIN, sizeof(T)), SEL = FWD_JC * rs, BUF = NIN * 2 * SEL;
     static_assert(NIN * 4 * FWD_JC <= FWD_ITEMS * FWD_THREADS, "a chunk's values fit the threads' items");
     const int nlath = A.nlath, nlat = A.nlat, L = A.L;
     const int K = A.ntp1 - m, K0 = (K + 1) >> 1, K1 = K >> 1;
@@ -475,10 +486,10 @@ __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, double *sm, in
 #pragma unroll
         for (int i = 0; i < MT; i++) {
             if (i >= ntile) break;
-            const double2 *f = reinterpret_cast<const double2 *>(tb + to[i]);
-            const double2 ce = f[0];
-            t[i].c = ce.x; t[i].e = ce.y;
-            if constexpr (S::m || S::q) { const double2 mq = f[1]; t[i].m = mq.x; t[i].q = mq.y; }
+            if constexpr (S::m || S::q)
+                asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                    : "=d"(t[i].c), "=d"(t[i].e), "=d"(t[i].m), "=d"(t[i].q) : "l"(tb + to[i]));
+            else t[i].c = tb[to[i]].c;
         }
         tb += tstr;
     };
@@ -687,13 +698,13 @@ static exotx_status inv_launch(LegItem<LegInv<T>> *it, int n, cudaStream_t s) {
 
 template <typename T>
 exotx_status leg_inverse_l(exotx_plan p, int op, const T *a, const T *b, T *oa, T *ob, int nlev,
-                           long long a_fs, long long b_fs, FourierLayout L, cudaStream_t s, double scale,
+                           long long fs, FourierLayout L, cudaStream_t s, double scale,
                            const double *rscale, bool roll) {
     if (nlev <= 0) return EXOTX_OK;
     if (op != OP_SP2FC && op != OP_SP2FCDMU && op != OP_DV2UV) return EXOTX_BAD_ARG;
     LegItem<LegInv<T>> it = {p, {}};
     LegInv<T> &A = it.a;
-    A.a = a; A.b = b; A.a_fs = a_fs; A.b_fs = b_fs;
+    A.a = a; A.a_fs = fs; A.b_off = b ? reinterpret_cast<const char *>(b) - reinterpret_cast<const char *>(a) : 0;
     A.oa = oa; A.ob = ob; A.fs = L.fs; A.ls = L.ls; A.ms = L.ms; A.mz = L.mz;
     A.scale = scale; A.rscale = rscale; A.roll = roll;
     A.nu[op == OP_SP2FC ? 0 : op == OP_SP2FCDMU ? 1 : 2] = nlev;
@@ -744,7 +755,7 @@ static exotx_status fwd_launch_t(LegItem<LegFwd<T>> *it, int n, cudaStream_t s) 
         if (blocks > 0x7fffffffLL) return EXOTX_BAD_DIM;
     }
     // one operand chunk and two chunks of copies on their way
-    const size_t smem = (size_t)FwdShape<OP>::nin * 2 * FWD_JC * leg_stride(8) * sizeof(double) +
+    const size_t smem = (size_t)FwdShape<OP>::nin * 2 * fwd_jc(FwdShape<OP>::nin, sizeof(T)) * leg_stride(8) * sizeof(double) +
                         (size_t)FWD_ITEMS * 4 * threads * sizeof(C2<T>);
     if (smem > LEG_MAXSMEM) return EXOTX_BAD_DIM;
     auto kern = k_leg_fwd<T, OP, MT, SET, NSEG>;
@@ -810,7 +821,7 @@ exotx_status leg_forward_set(const LegSeg<T> *segs, int n, int dset, cudaStream_
 
 #define LEG_INSTANCES(T)                                                                                            \
     template exotx_status leg_inverse_l<T>(exotx_plan, int, const T *, const T *, T *, T *, int, long long,         \
-                                           long long, FourierLayout, cudaStream_t, double, const double *, bool);   \
+                                           FourierLayout, cudaStream_t, double, const double *, bool);              \
     template exotx_status leg_forward_l<T>(exotx_plan, int, const T *const *, T *const *, int, FourierLayout,       \
                                            long long, cudaStream_t, double);                                        \
     template exotx_status leg_inverse_set<T>(const LegSeg<T> *, int, int, cudaStream_t);                            \
