@@ -16,8 +16,19 @@ static bool prec_ok(int prec) { return prec == EXOTX_FP64 || prec == EXOTX_FP32 
 // (at least one state), so that it is still in L2 when the next kernel reads it
 // and the plan's work buffer stays small.
 constexpr size_t PLAIN_CHUNK = (size_t)96 << 20;
-static int plain_chunk(size_t per_inst, int ninst) {
-    return (int)std::min<size_t>((size_t)ninst, std::max<size_t>(1, PLAIN_CHUNK / per_inst));
+// Under capture, where nothing can be allocated, a chunk is what the buffer at
+// hand takes; where memory is short it is one state.
+static exotx_status plain_work(exotx_plan p, size_t per_inst, int ninst, cudaStream_t s, int *chunk) {
+    int c = (int)std::min<size_t>((size_t)ninst, std::max<size_t>(1, PLAIN_CHUNK / per_inst));
+    if (p->work_bytes < per_inst * c) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+        else if (cap != cudaStreamCaptureStatusNone) c = (int)std::max<size_t>(1, p->work_bytes / per_inst);
+    }
+    exotx_status st = ensure_work(p, per_inst * c);
+    if (st == EXOTX_NO_MEM && c > 1) st = ensure_work(p, per_inst * (c = 1));
+    *chunk = c;
+    return st;
 }
 
 // invlega / invlegd (legmod.f90:635-677) and fc2gp of every field: gridpointa
@@ -29,8 +40,8 @@ static exotx_status inverse_set_plain(exotx_plan p, const T *spin, T *gpout, int
     const size_t nrsp = 2 * (size_t)p->ncsp, nhor = (size_t)p->nlat * p->nlon;
     const int nfo = dset ? 4 * L + 1 : 6 * L + 3;
     const size_t per_inst = sizeof(T) * 2 * (size_t)nfo * p->nlat * p->ntp1;
-    const int chunk = plain_chunk(per_inst, ninst);
-    EXOTX_TRY(ensure_work(p, per_inst * chunk));
+    int chunk;
+    EXOTX_TRY(plain_work(p, per_inst, ninst, s, &chunk));
     T *w = (T *)p->d_work;
     for (int i0 = 0; i0 < ninst; i0 += chunk) {
         const int ni = std::min(chunk, ninst - i0);
@@ -50,8 +61,8 @@ static exotx_status forward_set_plain(exotx_plan p, const T *gpin, T *spout, int
     const size_t nrsp = 2 * (size_t)p->ncsp, nhor = (size_t)p->nlat * p->nlon;
     const int nfi = dset ? 4 * L : 9 * L + 1, nfo = dset ? 4 * L : 4 * L + 1;
     const size_t per_inst = sizeof(T) * 2 * (size_t)nfi * p->nlat * p->ntp1;
-    const int chunk = plain_chunk(per_inst, ninst);
-    EXOTX_TRY(ensure_work(p, per_inst * chunk));
+    int chunk;
+    EXOTX_TRY(plain_work(p, per_inst, ninst, s, &chunk));
     T *w = (T *)p->d_work;
     for (int i0 = 0; i0 < ninst; i0 += chunk) {
         const int ni = std::min(chunk, ninst - i0);

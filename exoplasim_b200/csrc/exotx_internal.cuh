@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstddef>
+#include <vector>
 #include "exotx.h"
 
 #define EXOTX_API extern "C" __attribute__((visibility("default")))
@@ -101,6 +102,7 @@ struct exotx_plan_s {
     // work buffer for the forward transform set (Fourier rows of gpin)
     void *d_work = nullptr;
     size_t work_bytes = 0;
+    std::vector<void *> old_work;   // outgrown ones, which captured graphs may still use
     exotx::TcTables *tc = nullptr;
     exotx::HostPipe *hpipe = nullptr;  // device slots and streams of exotx_sets_host
     // bytes of m-major Fourier intermediate one tensor-core launch covers

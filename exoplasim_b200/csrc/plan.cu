@@ -3,6 +3,7 @@
 //
 // This file is compiled with -fmad=false so every product and sum is rounded
 // separately, in the order the reference's 8-byte build evaluates them.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -137,7 +138,7 @@ __global__ void k_legini(int nlat, int ntru, int ncsp, const int *woff, const do
 }
 
 // Both layouts hold the tables as the 8x4 operand fragments that the Legendre
-// kernels' FP64 tensor-core instructions read (legendre_simt.cu): 32 lanes,
+// kernels' FP64 tensor-core instructions read (legendre_fp64mma.cu): 32 lanes,
 // lane = 4 r + q for row r and column q, zeros past the last latitude or mode.
 // One block per wavenumber (and parity).
 
@@ -214,16 +215,30 @@ static void host_filters(const exotx_grid_desc &d, int ntru, std::vector<double>
     }
 }
 
+// A captured graph of an earlier call may hold the buffer that no longer
+// suffices, so that one stays until the plan goes, unless memory is short; each
+// is at least half as large again as the one before, which bounds their sum by
+// twice the last.
 exotx_status ensure_work(exotx_plan p, size_t bytes) {
     if (p->work_bytes >= bytes) return EXOTX_OK;
-    if (p->d_work) {
+    void *q = nullptr;
+    size_t size = std::max(bytes, p->work_bytes + p->work_bytes / 2);
+    cudaError_t e = cudaMalloc(&q, size);
+    if (e == cudaErrorMemoryAllocation && p->d_work) {
+        cudaGetLastError();
         cudaDeviceSynchronize();
         cudaFree(p->d_work);
+    for (void *q : p->old_work) cudaFree(q);
         p->d_work = nullptr;
         p->work_bytes = 0;
+        size = bytes;
+        e = cudaMalloc(&q, size);
     }
-    EXOTX_CUDA(cudaMalloc(&p->d_work, bytes));
-    p->work_bytes = bytes;
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();   // reported by the status alone
+    EXOTX_CUDA(e);
+    if (p->d_work) p->old_work.push_back(p->d_work);
+    p->d_work = q;
+    p->work_bytes = size;
     return EXOTX_OK;
 }
 
