@@ -118,6 +118,8 @@ static const int kFwdRef[4] = {2, 3, 4, 5};
 // columns; T170 forward: another tcgen05 kernel, no longer built.)
 static bool tc_inv(exotx_plan p) { return p->ntp1 > 96; }
 static bool tc_fwd(exotx_plan p) { return p->ntp1 > 112 && p->ntp1 <= 128; }
+// the tcgen05 kernels move spectral coefficients as complex values; the FP64 ones ask for aligned reals only
+static bool aligned8(const void *q) { return (reinterpret_cast<uintptr_t>(q) & 7) == 0; }
 
 struct TcTables {
     int nj8;                          // inverse rows: latitude pairs rounded up to 8
@@ -398,7 +400,7 @@ static exotx_status tc_inverse_run(exotx_plan p, const float *spin, float *gpout
     int chunk = (int)std::max<size_t>(1, p->chunk_inv / per_inst);
     chunk = std::min(chunk, ninst);
     EXOTX_TRY(ensure_work(p, per_inst * chunk));
-    if (!tc_inv(p)) {
+    if (!tc_inv(p) || !aligned8(spin)) {
         for (int i0 = 0; i0 < ninst; i0 += chunk) {
             const int ni = std::min(chunk, ninst - i0);
             const long long nrows = (long long)ni * nfo * p->nlat;
@@ -618,7 +620,7 @@ static exotx_status tc_forward_run(exotx_plan p, const float *gpin, float *spout
             rowsum = nullptr;
             EXOTX_TRY(fft_forward_l<float>(gsrc, (float *)p->d_work, p->nlon, nrows, p->ntp1, 1, nrows, s));
         }
-        if (folded && !dset && tc_fwd(p)) {
+        if (folded && !dset && tc_fwd(p) && aligned8(spout)) {
             const int4 *jl;
             int nj;
             EXOTX_TRY(tc_jobs(p, T, 1, L, ni, &jl, &nj));
@@ -704,6 +706,7 @@ exotx_status tc_ens_jobs(const EnsSeg *segs, int nseg, int dir, int nc_qi_cap, i
 exotx_status tc_ens_run(const EnsSeg *segs, int nseg, int dir, const int4 *d_jobs, int njobs, size_t smem,
                         int nprod, cudaStream_t s) {
     if (nseg < 1 || nseg > TC_MAXSEG || (nprod != 3 && nprod != 6)) return EXOTX_BAD_ARG;
+    if (njobs && !aligned8(dir == 0 ? (const void *)segs[0].spin : segs[0].spout)) return EXOTX_BAD_ARG;
     LegSeg<float> f64[TC_MAXSEG];
     int n64 = 0;
     for (int i = nseg - 1; i >= 0; i--) {   // the longest contractions first
