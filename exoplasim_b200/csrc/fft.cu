@@ -1186,6 +1186,7 @@ __global__ void __launch_bounds__(256) k_rfft_inv_rf(const float *fc, float *gp,
 // One launch transforms the rows of up to FFT_ENS_MAXSEG segments of different
 // lengths (an uneven ensemble); block b belongs to the last segment whose
 // first block is <= b.
+constexpr int FFT_ENS_MAXSMEM = 160 * 1024;   // one limit for every mix of lengths
 struct FftEnsArgs {
     const float *in;
     float *out;
@@ -1303,7 +1304,7 @@ exotx_status fft_ens(bool fwd, const FftEnsSeg *segs, int nseg, cudaStream_t s) 
     static_assert(RfLayout<384>::NT == RR_THREADS, "one block size");
     void (*k)(FftEnsLaunch) = lng ? (fwd ? k_rfft_ens<true, true> : k_rfft_ens<false, true>)
                                   : (fwd ? k_rfft_ens<true, false> : k_rfft_ens<false, false>);
-    if (smem > 48 * 1024) EXOTX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) EXOTX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, FFT_ENS_MAXSMEM));
     cudaEvent_t ev = ktimer_start(kid, s);
     EXOTX_CUDA(launch_pdl(k, dim3((unsigned)blocks), dim3(RR_THREADS), smem, s, P));
     EXOTX_CHECK_LAUNCH();
@@ -1318,11 +1319,13 @@ static exotx_status launch_rr(bool fwd, const T *in, T *out, long long lot, int 
     const size_t smem = fwd ? Lay::fwd_smem() : Lay::inv_smem(kf);
     const long long nb = (lot + Lay::RB - 1) / Lay::RB;
     const int kid = fwd ? EXOTX_K_FFT_FORWARD : EXOTX_K_FFT_INVERSE;
+    // the limit is the kernel's, whatever kf: another thread may be between its own call and its launch
     if (smem > 48 * 1024) {
         if (fwd)
             EXOTX_CUDA(cudaFuncSetAttribute(k_rfft_fwd_rr<T, N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         else
-            EXOTX_CUDA(cudaFuncSetAttribute(k_rfft_inv_rr<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            EXOTX_CUDA(cudaFuncSetAttribute(k_rfft_inv_rr<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)Lay::inv_smem(Lay::H)));
     }
     cudaEvent_t ev = ktimer_start(kid, s);
     if (fwd)

@@ -25,8 +25,8 @@
 // float but whose sums run in FP64 with the FP64 tables and are rounded once.
 // Factors i and -i read the partner column (re <-> im) and flip its sign.
 //
-// One T127 L20 state, FP64: INV_A_US inverse and FWD_A_US forward against 147
-// and 180 us for register-tiled FP64 FMA kernels (4 x 4 tiles: 240 registers,
+// One T127 L20 state, FP64: 52 us inverse and 62 forward against 147 and 180 for
+// register-tiled FP64 FMA kernels (4 x 4 tiles: 240 registers,
 // 6 warps per SM, the FP64 pipe 16% busy: two of three instructions were loads
 // and addresses).  Eight DMMAs need six loads here, and the FP64 tensor cores
 // were measured at 36.7 TFLOP/s (FMA: 30.8).

@@ -192,6 +192,7 @@ __global__ void __launch_bounds__(TG_THREADS, 2) k_tc_gemm(const __grid_constant
     };
     float cs[4] = {0.f, 0.f, 0.f, 0.f};              // TG_WEIGHTS: this thread's share of db
     const uint32_t idesc = tc::idesc_bf16(TG_M, NT);
+    int issued = 0;                                  // chunks whose MMAs are on their way
     // stage chunk c, issue the loads of chunk c + 2 in its place, then the MMAs
     auto step = [&](TgChunk<AKC, BKC> &t, int c) {
         const int b = c & 1;
@@ -226,6 +227,7 @@ __global__ void __launch_bounds__(TG_THREADS, 2) k_tc_gemm(const __grid_constant
             }
             tc::mma_commit(bar + b);
         }
+        issued = c + 1;
         return true;
     };
     load(cur, 0);
@@ -235,8 +237,9 @@ __global__ void __launch_bounds__(TG_THREADS, 2) k_tc_gemm(const __grid_constant
         ok = step(cur, c);
         if (ok && c + 1 < nchunk) ok = step(nxt, c + 1);
     }
-    // every MMA has completed once the last chunk's commit has arrived
-    if (ok) ok = tc::mbar_wait(bar + ((nchunk - 1) & 1), ((nchunk - 1) >> 1) & 1);
+    // every MMA has completed once the last issued chunk's commit has arrived; waited
+    // for after a timeout too, before the accumulators are given back
+    if (issued && !tc::mbar_wait(bar + ((issued - 1) & 1), ((issued - 1) >> 1) & 1)) ok = false;
     ok = __syncthreads_and(ok) != 0;
     if (!ok && tid == 0) atomicExch(&g_tg_error, 1);
     tc::fence_after_sync();
