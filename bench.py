@@ -461,7 +461,7 @@ def run_ours(a, rank, world, local_rank):
             ach, pk, unit = rate / 1e9, hbm, "GB/s"
         elif bound == "tensor":
             ach, pk, unit = rate / 1e12, tc, "TFLOP/s"
-        else:  # SIMT FMA path: no measured peak to divide by
+        else:  # FP64 tensor-core path: no measured peak to divide by
             ach, pk, unit = rate / 1e12, None, "TFLOP/s"
         kernels[name] = {"bound": bound, "ms_total": kms, "launches": nl, "ms_per_launch": kms / nl,
                          "achieved": ach, "peak": pk, "unit": unit, "frac": ach / pk if pk else None,

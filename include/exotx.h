@@ -17,8 +17,9 @@
  * Latitudes run north to south (sid(1) > 0), as inigau returns them.
  *
  * Precision: EXOTX_FP64 arrays are double; EXOTX_FP32 and EXOTX_MIXED arrays
- * are float.  EXOTX_MIXED runs the Legendre contractions on the tensor cores
- * with 3-term BF16 splits of both operands and FP32 accumulation.
+ * are float.  EXOTX_MIXED runs the long Legendre contractions on the tensor
+ * cores with 3-term BF16 splits of both operands and FP32 accumulation, the
+ * others on the FP64 tensor cores.
  */
 #ifndef EXOTX_H
 #define EXOTX_H
