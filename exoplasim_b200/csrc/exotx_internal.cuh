@@ -154,6 +154,7 @@ template <typename T> struct LegSeg {
     const T *in;
     T *out;
     bool folded;
+    const double *rowsum = nullptr;   // forward, one segment of float: also the n = 0 coefficients from these sums
 };
 template <typename T>
 exotx_status leg_inverse_set(const LegSeg<T> *segs, int n, int dset, cudaStream_t s);

@@ -406,6 +406,10 @@ struct LegFwd {
     int nu1, nt1;            // gridpointa: ln ps tendencies (fc2sp) and their tiles
     int wb, nmb;             // warps along the modes of a block; mode blocks per wavenumber
     int L, nlat, nlath, ntp1;
+    // float sets: the FP64 sums of the grid rows (null: none), whose zonal means give
+    // the n = 0 coefficients of n0 fields, a warp each in the launch's last blocks
+    const double *rowsum, *qc00;   // qc(0, lat) at stride qstride
+    int qstride, nlon, n0;
 };
 
 template <int OP> struct FwdShape;
@@ -597,6 +601,7 @@ __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, double *sm, in
         const double f = SET ? A.filt[m + k] : A.filt[m + k] * A.scale;
 #pragma unroll
         for (int x = 0; x < NOUT; x++) {
+            if (SET && sizeof(T) == 4 && m + k == 0 && (OP == OP_FC2SP || (x & 1)) && A.rowsum) continue;   // leg_fwd_n0
             T *d;
             if constexpr (SET) {
                 // sdf[L] stf[L] szf[L] sqf[L] (gridpointa: spf)
@@ -612,6 +617,27 @@ __device__ __forceinline__ void leg_fwd_block(const LegFwd<T> &A, double *sm, in
     }
 }
 
+// The global means of a mixed set (k_n0_fp64, whose order of sums this is, does the
+// same where the rows' sums come from elsewhere).  As warps of the forward launch
+// they cost nothing; the launch of their own took 5 us of the 57 of T42 L20.
+template <int OP>
+__device__ __forceinline__ void leg_fwd_n0(const LegFwd<float> &A, int w) {
+    constexpr bool D = OP == OP_LEVEL_D;
+    const int L = A.L, nf = D ? 2 * L : 2 * L + 1, lane = threadIdx.x & 31;
+    if (w >= A.n0) return;
+    const int inst = w / nf, f = w - inst * nf;
+    const int fin = f < L ? f : f < 2 * L ? (D ? 2 * L + f : f) : 7 * L, fout = f < L ? L + f : f < 2 * L ? 2 * L + f : 4 * L;
+    const double *rs = A.rowsum + ((long long)inst * (D ? 4 * L : 9 * L + 1) + fin) * A.nlat;
+    double acc = 0.0;
+    for (int lat = lane; lat < A.nlat; lat += 32) acc += A.qc00[(size_t)lat * A.qstride] * (rs[lat] / (double)A.nlon);
+    for (int o = 1; o < 32; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) {
+        float *o = A.out[0] + ((size_t)inst * (D ? 4 * L : 4 * L + 1) + fout) * A.o_fs;
+        o[0] = (float)(acc * A.filt[0]);
+        o[1] = 0.0f;
+    }
+}
+
 template <typename T, int OP, int MT, bool SET, int NSEG>
 __global__ void __launch_bounds__(384, MT == 1 ? 1 : 2) k_leg_fwd(const __grid_constant__ LegLaunch<LegFwd<T>, NSEG> P) {
     const int seg = P.find(blockIdx.x), blk = blockIdx.x - P.blk0[seg];
@@ -622,6 +648,12 @@ __global__ void __launch_bounds__(384, MT == 1 ? 1 : 2) k_leg_fwd(const __grid_c
     const int m = mb / A.nmb, mblk = mb - m * A.nmb;
     pdl_trigger();
     pdl_wait();
+    if constexpr (SET && sizeof(T) == 4) {
+        if (m >= A.ntp1) {
+            leg_fwd_n0<OP>(A, (blk - A.ntp1 * A.nmb * nt) * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5));
+            return;
+        }
+    }
     if (ti < A.nt) {
         // where one tile per warp suffices (the larger half of the wavenumbers) every warp of the block works
         const int K = A.ntp1 - m, tiles = (((K + 1) >> 1) + 7) / 8 + ((K >> 1) + 7) / 8;
@@ -752,6 +784,11 @@ static exotx_status fwd_launch_t(LegItem<LegFwd<T>> *it, int n, cudaStream_t s) 
         A.nt1 = (A.nu1 + 3) / 4;
         P.blk0[i] = (int)blocks;
         blocks += (long long)p->ntp1 * A.nmb * (A.nt + A.nt1);
+        if (A.rowsum) {   // one segment, so threads is its own
+            A.qc00 = p->d_qref + (size_t)2 * p->nlat * p->ncsp;   // qc(w = 0, lat) of the reference tables [t][lat][w]
+            A.qstride = p->ncsp; A.nlon = p->nlon;
+            blocks += (A.n0 + threads / 32 - 1) / (threads / 32);
+        }
         if (blocks > 0x7fffffffLL) return EXOTX_BAD_DIM;
     }
     // one operand chunk and two chunks of copies on their way
@@ -810,6 +847,8 @@ exotx_status leg_forward_set(const LegSeg<T> *segs, int n, int dset, cudaStream_
         A.nrows = (long long)g.ninst * (dset ? 4 * g.L : 9 * g.L + 1) * g.p->nlat;
         A.nu = g.ninst * g.L;
         A.nu1 = dset ? 0 : g.ninst;
+        A.rowsum = n == 1 ? g.rowsum : nullptr;
+        A.n0 = g.ninst * (dset ? 2 * g.L : 2 * g.L + 1);
     }
     if (n > 1) {
         if constexpr (sizeof(T) == 4)

@@ -477,7 +477,8 @@ exotx_status tc_inverse_batch_d(exotx_plan p, const float *spin, float *gpout, i
 // energy budgets then close in FP64 (the reference keeps spp(1:2) conserved,
 // plasim.f90:2937-2938).  Field f of an instance: 0..L-1 temperature, L..2L-1
 // humidity, 2L the ln ps tendency (gridpointa only).  One launch covers the
-// segments of an ensemble as well.
+// segments of an ensemble as well.  Sets whose contraction and row sums come from
+// the FP64 kernels have the same sums in that launch (leg_fwd_n0).
 struct N0Seg {
     const float *gpin;
     const double *rowsum; // FP64 grid-row sums from the forward FFT (may be null: summed here)
@@ -630,8 +631,9 @@ static exotx_status tc_forward_run(exotx_plan p, const float *gpin, float *spout
             fwd3_args(P3.seg[0], p, T, L, (const float2 *)p->d_work, nrows, sdst);
             EXOTX_TRY(launch_fwd_pipe(P3, nj, T->njc, s));
         } else {
-            const LegSeg<float> g = {p, L, ni, (const float *)p->d_work, sdst, folded};
+            const LegSeg<float> g = {p, L, ni, (const float *)p->d_work, sdst, folded, rowsum};
             EXOTX_TRY(leg_forward_set<float>(&g, 1, dset, s));
+            if (rowsum) continue;   // the global means are in that launch
         }
         EXOTX_TRY(n0_fp64(p, gsrc, rowsum, sdst, L, ni, dset, s));
     }

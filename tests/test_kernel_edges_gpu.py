@@ -96,6 +96,27 @@ def test_sets_at_tile_edges(oracle, nlat, nlev, ninst, prec):
     assert tc_error() == 0
 
 
+# T21 and T42: the global means are warps of the forward launch in both sets; T127: in the gridpointd one
+@pytest.mark.parametrize("nlat,nlev,ninst", [(32, 1, 1), (32, 5, 3), (64, 13, 2), (192, 2, 2)])
+def test_mixed_global_means_are_rounded_once(oracle, nlat, nlev, ninst):
+    # FP64 sums rounded once to float32: half an ulp, and 1e-14 for the order of the sums
+    P = Plan(nlat)
+    O = Oracle(oracle, nlat)
+    gin = np.stack([S.grid_tendencies(nlat, nlev, seed=70 + i) for i in range(ninst)])
+    gin[:, :2 * nlev] += 0.3
+    gin[:, 3 * nlev:4 * nlev] += 0.2
+    g = _cuda(gin, torch.float32)
+    sa = P.forward_set_batch(g, nlev, precision="mixed").double().cpu().numpy()
+    sd = P.forward_set_d_batch(g[:, :4 * nlev].contiguous(), nlev, precision="mixed").double().cpu().numpy()
+    for i in range(ninst):
+        rows = g[i].double().cpu().numpy().reshape(9 * nlev + 1, -1)
+        for out, ref, top in ((sa[i], O.forward("forward_set", rows, nlev), [4 * nlev]),
+                              (sd[i], O.forward("forward_set_d", rows[:4 * nlev], nlev), [])):
+            for f in list(range(nlev, 2 * nlev)) + list(range(3 * nlev, 4 * nlev)) + top:
+                half = 0.5 * float(np.spacing(np.float32(abs(ref[f][0]))))
+                assert abs(out[f][0] - ref[f][0]) <= half + 1e-14 * abs(ref[f][0]) and out[f][1] == 0.0, (i, f)
+
+
 @pytest.mark.parametrize("nlat,prec", [(32, "fp64"), (64, "fp32"), (64, "mixed"), (192, "mixed")])
 def test_sets_on_arrays_aligned_to_their_reals(nlat, prec):
     # a grid that starts on an odd element takes the general FFT, a state the FP64 kernels
