@@ -242,10 +242,11 @@ __global__ void __launch_bounds__(256) k_rfft_inverse(const T *fc, T *gp, FftLau
 // works RB = RR_THREADS/P rows.  The m-major Fourier side is reached rows
 // fastest: through the spectra in shared memory (forward) or the staged
 // coefficients (inverse), which take the transposition's place in turn.
-// T42 L20 FP64, one state (181 fields): forward RRF64 us, inverse RRI64 us,
-// against 11.3 and 10.1 us for the three-pass shared-memory (Stockham) kernels
-// before, which moved every value through shared memory six times and were
-// bound by instruction issue; T85 L13 x3 FP32 RRF32 and RRI32 against 39.8 and 32.9.
+// Per launch (CUDA events), against the three-pass shared-memory (Stockham)
+// kernels before, which moved every value through shared memory six times and
+// were bound by instruction issue: T127 L20 FP64 forward 53 us against 66,
+// inverse 38 against 49; T85 L13 x3 FP32 31 against 40 and 19 against 33; T42 L20
+// FP64, one state, where latency bounds both, 11.2 against 11.3 and 9.7 against 10.1.
 constexpr int RR_THREADS = 128;
 // P: 16 where Q would need over 64 registers in FP64 (n = 384 with P = 8: 132
 // registers, 3 blocks per SM, forward 67 us per T127 L20 state)
