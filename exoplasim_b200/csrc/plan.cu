@@ -228,7 +228,8 @@ exotx_status ensure_work(exotx_plan p, size_t bytes) {
         cudaGetLastError();
         cudaDeviceSynchronize();
         cudaFree(p->d_work);
-    for (void *q : p->old_work) cudaFree(q);
+        for (void *w : p->old_work) cudaFree(w);
+        p->old_work.clear();
         p->d_work = nullptr;
         p->work_bytes = 0;
         size = bytes;
@@ -259,6 +260,7 @@ static void plan_free(exotx_plan p) {
     cudaFree(p->d_fs32);
     cudaFree(p->d_fg32);
     cudaFree(p->d_work);
+    for (void *w : p->old_work) cudaFree(w);
     delete p;
 }
 
