@@ -20,13 +20,9 @@ constexpr size_t PLAIN_CHUNK = (size_t)96 << 20;
 // hand takes; where memory is short it is one state.
 static exotx_status plain_work(exotx_plan p, size_t per_inst, int ninst, cudaStream_t s, int *chunk) {
     int c = (int)std::min<size_t>((size_t)ninst, std::max<size_t>(1, PLAIN_CHUNK / per_inst));
-    if (p->work_bytes < per_inst * c) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
-        else if (cap != cudaStreamCaptureStatusNone) c = (int)std::max<size_t>(1, p->work_bytes / per_inst);
-    }
-    exotx_status st = ensure_work(p, per_inst * c);
-    if (st == EXOTX_NO_MEM && c > 1) st = ensure_work(p, per_inst * (c = 1));
+    if (p->work_bytes < per_inst * c && capturing(s)) c = (int)std::max<size_t>(1, p->work_bytes / per_inst);
+    exotx_status st = ensure_work(p, per_inst * c, s);
+    if (st == EXOTX_NO_MEM && c > 1) st = ensure_work(p, per_inst * (c = 1), s);
     *chunk = c;
     return st;
 }

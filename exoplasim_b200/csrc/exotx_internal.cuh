@@ -102,7 +102,8 @@ struct exotx_plan_s {
     // work buffer for the forward transform set (Fourier rows of gpin)
     void *d_work = nullptr;
     size_t work_bytes = 0;
-    std::vector<void *> old_work;   // outgrown ones, which captured graphs may still use
+    bool work_held = false;         // a captured graph uses the buffer
+    std::vector<void *> old_work;   // outgrown ones that captured graphs use
     exotx::TcTables *tc = nullptr;
     exotx::HostPipe *hpipe = nullptr;  // device slots and streams of exotx_sets_host
     // bytes of m-major Fourier intermediate one tensor-core launch covers
@@ -120,7 +121,13 @@ namespace exotx {
 enum { INV_QI = 0, INV_QJ = 1, INV_QU = 2, INV_QV = 3 };
 enum { FWD_QC = 0, FWD_QE = 1, FWD_QM = 2, FWD_QQ = 3 };
 
-exotx_status ensure_work(exotx_plan p, size_t bytes);
+exotx_status ensure_work(exotx_plan p, size_t bytes, cudaStream_t s);
+inline bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+    cudaGetLastError();   // the legacy stream while another one captures
+    return true;
+}
 
 // Fourier-side addressing: complex element (field f, latitude l, wavenumber m)
 // at base + f*fs + l*ls + m*ms (complex units); m < mz are produced.

@@ -12,12 +12,6 @@ static std::mutex g_kt_mu;
 static bool g_kt_on = false;
 static std::vector<std::pair<cudaEvent_t, cudaEvent_t>> g_kt_rec[EXOTX_K_COUNT];
 
-static bool capturing(cudaStream_t s) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) return true;
-    return st != cudaStreamCaptureStatusNone;
-}
-
 cudaEvent_t ktimer_start(int k, cudaStream_t s) {
     {
         std::lock_guard<std::mutex> lk(g_kt_mu);

@@ -399,7 +399,7 @@ static exotx_status tc_inverse_run(exotx_plan p, const float *spin, float *gpout
     const size_t per_inst = (size_t)nfo * p->nlat * p->ntp1 * sizeof(float2);
     int chunk = (int)std::max<size_t>(1, p->chunk_inv / per_inst);
     chunk = std::min(chunk, ninst);
-    EXOTX_TRY(ensure_work(p, per_inst * chunk));
+    EXOTX_TRY(ensure_work(p, per_inst * chunk, s));
     if (!tc_inv(p) || !aligned8(spin)) {
         for (int i0 = 0; i0 < ninst; i0 += chunk) {
             const int ni = std::min(chunk, ninst - i0);
@@ -604,7 +604,7 @@ static exotx_status tc_forward_run(exotx_plan p, const float *gpin, float *spout
     // where the folded FFT forms them
     const bool with_rs = fft_fold_rowsum(p->nlon);
     const size_t rs_off = (per_inst * chunk + 255) & ~(size_t)255;
-    EXOTX_TRY(ensure_work(p, with_rs ? rs_off + (size_t)chunk * nfi * p->nlat * sizeof(double) : per_inst * chunk));
+    EXOTX_TRY(ensure_work(p, with_rs ? rs_off + (size_t)chunk * nfi * p->nlat * sizeof(double) : per_inst * chunk, s));
     for (int i0 = 0; i0 < ninst; i0 += chunk) {
         const int ni = std::min(chunk, ninst - i0);
         const long long nrows = (long long)ni * nfi * p->nlat;

@@ -215,31 +215,35 @@ static void host_filters(const exotx_grid_desc &d, int ntru, std::vector<double>
     }
 }
 
-// A captured graph of an earlier call may hold the buffer that no longer
-// suffices, so that one stays until the plan goes, unless memory is short; each
-// is at least half as large again as the one before, which bounds their sum by
-// twice the last.
-exotx_status ensure_work(exotx_plan p, size_t bytes) {
-    if (p->work_bytes >= bytes) return EXOTX_OK;
-    void *q = nullptr;
-    size_t size = std::max(bytes, p->work_bytes + p->work_bytes / 2);
-    cudaError_t e = cudaMalloc(&q, size);
-    if (e == cudaErrorMemoryAllocation && p->d_work) {
-        cudaGetLastError();
-        cudaDeviceSynchronize();
-        cudaFree(p->d_work);
-        for (void *w : p->old_work) cudaFree(w);
-        p->old_work.clear();
-        p->d_work = nullptr;
-        p->work_bytes = 0;
-        size = bytes;
-        e = cudaMalloc(&q, size);
+// A buffer of at least `bytes` for a call on stream s.  One that no longer
+// suffices goes back first, unless a captured graph uses it: that one stays until
+// the plan goes, and the next is at least half as large again, where memory allows,
+// so that such buffers together take at most twice the last one's bytes.
+exotx_status ensure_work(exotx_plan p, size_t bytes, cudaStream_t s) {
+    const bool cap = capturing(s);
+    if (p->work_bytes < bytes) {
+        const bool keep = p->d_work && (cap || p->work_held);
+        if (p->d_work && !keep) {
+            cudaDeviceSynchronize();
+            cudaFree(p->d_work);
+            p->d_work = nullptr;
+            p->work_bytes = 0;
+        }
+        void *q = nullptr;
+        size_t size = std::max(bytes, p->work_bytes + p->work_bytes / 2);
+        cudaError_t e = cudaMalloc(&q, size);
+        if (e == cudaErrorMemoryAllocation && size > bytes) {
+            cudaGetLastError();
+            e = cudaMalloc(&q, size = bytes);
+        }
+        if (e == cudaErrorMemoryAllocation) cudaGetLastError();   // reported by the status alone
+        EXOTX_CUDA(e);
+        if (keep) p->old_work.push_back(p->d_work);
+        p->d_work = q;
+        p->work_bytes = size;
+        p->work_held = false;
     }
-    if (e == cudaErrorMemoryAllocation) cudaGetLastError();   // reported by the status alone
-    EXOTX_CUDA(e);
-    if (p->d_work) p->old_work.push_back(p->d_work);
-    p->d_work = q;
-    p->work_bytes = size;
+    p->work_held = p->work_held || cap;
     return EXOTX_OK;
 }
 

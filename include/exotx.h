@@ -65,7 +65,10 @@ exotx_status exotx_grid_desc_default(int nlat, exotx_grid_desc *d);
 /* Plan = device tables for one resolution, built on the GPU in FP64: the
  * Gaussian Newton iteration (replaces inigau, gaussmod.f90:5-40) and the
  * associated-Legendre recurrence with its eight derived tables (replaces
- * legini, legmod.f90:30-171), plus FP32 and BF16-split copies. */
+ * legini, legmod.f90:30-171), plus FP32 and BF16-split copies.  The sets also
+ * keep a device work buffer in the plan, as large as the largest call so far
+ * needs; buffers of captured calls stay until the plan is destroyed, so that
+ * their graphs may run again. */
 exotx_status exotx_plan_create(const exotx_grid_desc *d, exotx_plan *out);
 exotx_status exotx_plan_destroy(exotx_plan p);
 exotx_status exotx_plan_dims(exotx_plan p, int *nlat, int *nlon, int *ntru, int *ncsp);

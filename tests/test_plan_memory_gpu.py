@@ -69,3 +69,41 @@ def test_requests_beyond_memory_leave_the_plan_usable():
         s.gp.zero_(), s.so.zero_()
         assert torch.equal(s.inverse(), ref[0]) and torch.equal(s.forward(), ref[1])
     torch.cuda.synchronize()
+
+
+def test_outgrown_buffer_is_given_back_at_once():
+    # where no captured graph uses it, a plan holds what its largest call needs
+    s = Sets()
+    s.inverse(), s.forward()
+    s.p = None
+    s.p = Plan(NLAT)
+    tables = _used()
+    s.inverse()
+    s.forward()
+    assert _used() - tables < NINST * (9 * NLEV + 1) * FIELDS + BLOCK
+
+
+def test_captured_graphs_keep_their_buffers():
+    s = Sets()
+    ref = s.inverse(2).clone()
+    torch.cuda.synchronize()
+    s.p = None
+    s.p = Plan(NLAT)
+    s.inverse(2)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        s.inverse(2)
+    held = _used()
+    full = s.forward().clone()             # outgrows the graph's buffer
+    s.beyond_memory()                      # and gives its own back in vain
+    other = torch.full((NINST * (9 * NLEV + 1) * FIELDS // 8,), 7.0, device="cuda", dtype=torch.float64)
+    s.gp.zero_()
+    graph.replay()                         # writes to no memory but the graph's
+    torch.cuda.synchronize()
+    assert torch.equal(s.gp[:2], ref) and bool((other == 7.0).all())
+    assert torch.equal(s.forward(), full)
+    del graph, other, full, ref
+    s.p = None
+    torch.cuda.empty_cache()
+    assert _used() <= held
