@@ -65,6 +65,16 @@ inline cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t
     return cudaLaunchKernelEx(&cfg, k, static_cast<Args &&>(args)...);
 }
 
+// Lets kernel k take `limit` bytes of dynamic shared memory where a launch of it takes
+// more than the default 48 KB.  The limit belongs to the kernel, not to the launch: it
+// is the same at every call, because another thread may stand between its own call
+// here and its launch.
+constexpr size_t SMEM_MAX = 227 * 1024;   // all that a block may have
+template <typename K>
+inline cudaError_t allow_smem(K *k, size_t smem, size_t limit = SMEM_MAX) {
+    return smem > 48 * 1024 ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit) : cudaSuccess;
+}
+
 // Real FFT twiddle tables for one length n, owned by a process-wide cache.
 struct FftTables {
     int n = 0, h = 0;            // h = n/2 complex points

@@ -268,7 +268,7 @@ template <typename T, int N> struct RrLayout {
     static constexpr int QP = (Q + P - 1) / P;
     static_assert(P * Q == H && 32 % P == 0, "a row's threads are in one warp");
     static constexpr size_t fwd_smem() { return (size_t)RB * (RS > RZ ? RS : RZ) * 2 * sizeof(T); }
-    static size_t inv_smem(int kf) {
+    static constexpr size_t inv_smem(int kf) {
         const size_t c = (size_t)kf * RC, x = (size_t)RB * RS;
         return (c > x ? c : x) * 2 * sizeof(T);
     }
@@ -1320,14 +1320,7 @@ static exotx_status launch_rr(bool fwd, const T *in, T *out, long long lot, int 
     const size_t smem = fwd ? Lay::fwd_smem() : Lay::inv_smem(kf);
     const long long nb = (lot + Lay::RB - 1) / Lay::RB;
     const int kid = fwd ? EXOTX_K_FFT_FORWARD : EXOTX_K_FFT_INVERSE;
-    // the limit is the kernel's, whatever kf: another thread may be between its own call and its launch
-    if (smem > 48 * 1024) {
-        if (fwd)
-            EXOTX_CUDA(cudaFuncSetAttribute(k_rfft_fwd_rr<T, N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        else
-            EXOTX_CUDA(cudaFuncSetAttribute(k_rfft_inv_rr<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)Lay::inv_smem(Lay::H)));
-    }
+    static_assert(Lay::fwd_smem() <= 48 * 1024 && Lay::inv_smem(Lay::H) <= 48 * 1024, "default shared memory");
     cudaEvent_t ev = ktimer_start(kid, s);
     if (fwd)
         EXOTX_CUDA(launch_pdl(k_rfft_fwd_rr<T, N, false>, dim3((unsigned)nb), dim3(RR_THREADS), smem, s, in, out, 0, lot,
@@ -1364,7 +1357,7 @@ static exotx_status launch_rf(bool fwd, const float *in, float *out, long long l
     size_t smem_p = 0;
     if (!fwd && kf <= Lay::H) {   // persistent form: one block per resident slot
         smem_p = RfIPLayout<N>::smem(kf);
-        EXOTX_CUDA(cudaFuncSetAttribute(k_rfft_inv_rf_p<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p));
+        EXOTX_CUDA(allow_smem(k_rfft_inv_rf_p<N>, RfIPLayout<N>::smem(Lay::H), RfIPLayout<N>::smem(Lay::H)));
         int slots = 0;
         EXOTX_TRY(resident_slots((const void *)k_rfft_inv_rf_p<N>, Lay::NT, smem_p, &slots));
         grid = std::min<long long>(nb, slots);
@@ -1480,15 +1473,6 @@ static FftLaunch make_launch(const FftTables *t, long long lot, int kf, long lon
     return L;
 }
 
-template <typename T>
-static exotx_status set_smem(const void *fn, size_t smem) {
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return cuda_status(e);
-    }
-    return EXOTX_OK;
-}
-
 // Fourier layout helper: row-major reference layout (row stride n/2, m stride 1)
 template <typename T>
 exotx_status fft_forward_l(const T *in, T *out, int n, long long lot, int kout, long long f_rs, long long f_ms,
@@ -1503,7 +1487,7 @@ exotx_status fft_forward_l(const T *in, T *out, int n, long long lot, int kout, 
     }
     size_t smem;
     FftLaunch L = make_launch<T>(t, lot, kout, f_rs, f_ms, &smem);
-    EXOTX_TRY(set_smem<T>((const void *)k_rfft_forward<T>, smem));
+    EXOTX_CUDA(allow_smem(k_rfft_forward<T>, smem));
     long long nb = (lot + L.rows_per_block - 1) / L.rows_per_block;
     cudaEvent_t ev = ktimer_start(EXOTX_K_FFT_FORWARD, s);
     k_rfft_forward<T><<<(unsigned)nb, 256, smem, s>>>(in, out, L, wt<T>(t), rt<T>(t));
@@ -1525,7 +1509,7 @@ exotx_status fft_inverse_l(const T *in, T *out, int n, long long lot, int kin, l
     }
     size_t smem;
     FftLaunch L = make_launch<T>(t, lot, kin, f_rs, f_ms, &smem);
-    EXOTX_TRY(set_smem<T>((const void *)k_rfft_inverse<T>, smem));
+    EXOTX_CUDA(allow_smem(k_rfft_inverse<T>, smem));
     long long nb = (lot + L.rows_per_block - 1) / L.rows_per_block;
     cudaEvent_t ev = ktimer_start(EXOTX_K_FFT_INVERSE, s);
     k_rfft_inverse<T><<<(unsigned)nb, 256, smem, s>>>(in, out, L, wt<T>(t), rt<T>(t));
@@ -1642,7 +1626,7 @@ exotx_status fft_forward_tw(const T *in, T *out, int n, long long lot, int kout,
     factor_h(t.h, t.fac, &t.nfac);
     size_t smem;
     FftLaunch L = make_launch<T>(&t, lot, kout, f_rs, f_ms, &smem);
-    EXOTX_TRY(set_smem<T>((const void *)k_rfft_forward<T>, smem));
+    EXOTX_CUDA(allow_smem(k_rfft_forward<T>, smem));
     long long nb = (lot + L.rows_per_block - 1) / L.rows_per_block;
     cudaEvent_t ev = ktimer_start(EXOTX_K_FFT_FORWARD, s);
     k_rfft_forward<T><<<(unsigned)nb, 256, smem, s>>>(in, out, L, wc, rc);

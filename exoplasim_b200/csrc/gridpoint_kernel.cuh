@@ -412,8 +412,7 @@ inline exotx_status gp_launch_async(const GpArgs<T> &A, const exotx_gp_params &h
 template <typename T, bool SK, int LC>
 inline exotx_status gp_launch_k(const GpArgs<T> &A, size_t smem, cudaStream_t s) {
     const long long nb = (A.ncol + GP_THREADS - 1) / GP_THREADS;
-    if (smem > 48 * 1024)
-        EXOTX_CUDA(cudaFuncSetAttribute(k_gridpoint<T, SK, LC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EXOTX_CUDA(allow_smem(k_gridpoint<T, SK, LC>, smem));
     k_gridpoint<T, SK, LC><<<(unsigned)nb, GP_THREADS, smem, s>>>(A);
     EXOTX_CHECK_LAUNCH();
     return EXOTX_OK;

@@ -791,8 +791,7 @@ EXOTX_API exotx_status exotx_tc_selftest(const float *A, const float *B, float *
     int zero = 0;
     EXOTX_CUDA(cudaMemcpyToSymbolAsync(g_tc_error, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, (cudaStream_t)s));
     size_t smem = (size_t)3 * (128 + N) * K * 2 + 16;
-    if (smem > 48 * 1024)
-        EXOTX_CUDA(cudaFuncSetAttribute(k_tc_selftest, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EXOTX_CUDA(allow_smem(k_tc_selftest, smem));
     k_tc_selftest<<<1, 128, smem, (cudaStream_t)s>>>(A, B, C, N, K, nprod);
     EXOTX_CHECK_LAUNCH();
     int err = 0;

@@ -728,7 +728,7 @@ inline exotx_status launch_radstep(const RadDev &D, int maxcols, bool list, cuda
     const int L = D.p.nlev, cols = rad_cols<T>(L);
     const size_t smem = rad_smem<T>(L, cols);
     auto kern = cols == 16 ? k_radstep<T, 16> : cols == 8 ? k_radstep<T, 8> : k_radstep<T, 4>;
-    if (smem > 48 * 1024) EXOTX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EXOTX_CUDA(allow_smem(kern, smem));
     int blocks = (maxcols + cols - 1) / cols;
     // a column list is usually short (often empty): one wave of resident blocks
     // strides over it instead of one block per possible entries

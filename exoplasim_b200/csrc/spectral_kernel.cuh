@@ -233,8 +233,7 @@ inline exotx_status spec_launch(const SpecBatch<T> &P, int n, bool d_part, cudaS
         k_spectrald<T><<<grid, block, 0, s>>>(P);
     } else {
         const size_t smem = spec_smem_a<T>(A.L);
-        if (smem > 48 * 1024)
-            EXOTX_CUDA(cudaFuncSetAttribute(k_spectrala<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXOTX_CUDA(allow_smem(k_spectrala<T>, smem));
         k_spectrala<T><<<grid, block, smem, s>>>(P);
     }
     EXOTX_CHECK_LAUNCH();
