@@ -28,6 +28,8 @@ constexpr int RAD_MAXLEV = 64;
 // FP64, 16 in FP32 (half the registers per thread, so more blocks per SM).
 template <typename T> constexpr int rad_items() { return sizeof(T) == 8 ? 32 : 16; }
 template <typename T> constexpr int rad_threads(int cols) { return cols * rad_items<T>(); }
+// threads per SM that the registers are shared out among
+template <typename T> constexpr int RAD_SM_THREADS = sizeof(T) == 8 ? 512 : 768;
 
 struct RadDev {
     exotx_rad_params p;
@@ -139,7 +141,7 @@ __host__ __device__ inline size_t rad_smem(int L, int cols) {
 }
 
 template <typename T, int COLS>
-__global__ void __launch_bounds__(rad_threads<T>(COLS), (sizeof(T) == 8 ? 512 : 768) / rad_threads<T>(COLS))
+__global__ void __launch_bounds__(rad_threads<T>(COLS), RAD_SM_THREADS<T> / rad_threads<T>(COLS))
     k_radstep(const __grid_constant__ RadDev D) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const exotx_rad_params &P = D.p;
@@ -713,10 +715,12 @@ __global__ void __launch_bounds__(rad_threads<T>(COLS), (sizeof(T) == 8 ? 512 : 
 #undef V
 }
 
-// Columns per block: 16, or fewer where the scratch of the blocks that the
-// registers allow per SM (one of 512 threads in FP64, three of 256 in FP32)
-// does not fit.  8192 columns, L20: 16 columns 176 / 76 us, eight 183 / 81
-// (FP64 / FP32); eight columns by 512 threads 238, 16 by 256 in FP64 247.
+// Columns per block: 16, or fewer where the scratch of one block per SM in FP64,
+// of two in FP32, does not fit.  (The registers allow one of 512 threads and three
+// of 256, but two blocks of 16 columns, from 27 levels on, beat the blocks of eight
+// that fit as many columns: L30 160 us against 173.)  8192 columns, L20: 16 columns
+// 176 / 78 us, eight 183 / 81 (FP64 / FP32); eight columns by 512 threads 238, 16 by
+// 256 in FP64 247.
 template <typename T>
 inline int rad_cols(int L) {
     const size_t room = 220 * 1024 / (sizeof(T) == 8 ? 1 : 2);
@@ -731,7 +735,8 @@ inline exotx_status launch_radstep(const RadDev &D, int maxcols, bool list, cuda
     EXOTX_CUDA(allow_smem(kern, smem));
     int blocks = (maxcols + cols - 1) / cols;
     // a column list is usually short (often empty): one wave of resident blocks
-    // strides over it instead of one block per possible entries
+    // strides over it instead of one block per possible entry (FP32, 32768 columns all
+    // listed: 549 us with one block per SM, 311 with the three that fit)
     if (list) {
         static int nsm = 0;
         if (!nsm) {
@@ -740,7 +745,9 @@ inline exotx_status launch_radstep(const RadDev &D, int maxcols, bool list, cuda
                 cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm < 1)
                 nsm = 148;
         }
-        blocks = blocks < nsm ? blocks : nsm;
+        const int regs = RAD_SM_THREADS<T> / rad_threads<T>(cols), fit = (int)((SMEM_MAX + 1024) / (smem + 1024));
+        const int wave = nsm * (regs < fit ? regs : fit);
+        blocks = blocks < wave ? blocks : wave;
     }
     cudaEvent_t ev = ktimer_start(EXOTX_K_RADSTEP, st);
     kern<<<blocks, rad_threads<T>(cols), smem, st>>>(D);
