@@ -343,6 +343,7 @@ template <int EPI>
 static exotx_status tg_launch(const TgArgs &g, dim3 grid, cudaStream_t s) {
     EXOTX_CUDA(cudaFuncSetAttribute(k_tc_gemm<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TG_SMEM));
     EXOTX_CUDA(launch_pdl(k_tc_gemm<EPI>, grid, dim3(TG_THREADS), TG_SMEM, s, g));
+    EXOTX_CHECK_LAUNCH();
     return EXOTX_OK;
 }
 static dim3 tg_grid(const TgArgs &g) {
@@ -381,6 +382,7 @@ exotx_status tc_mlp_weights(int nl, const int *din, const int *dout, const float
     EXOTX_TRY(tg_launch<TG_WEIGHTS>(g, dim3((unsigned)g.tile0[nl], (unsigned)nz), s));
     EXOTX_CUDA(launch_pdl(k_tg_reduce, dim3((unsigned)std::min<long long>((nparams + 255) / 256, 1184)), dim3(256), 0, s,
                           (const float *)work, nz, nparams, G));
+    EXOTX_CHECK_LAUNCH();
     return EXOTX_OK;
 }
 

@@ -1,4 +1,4 @@
-"""Launches: the grid of a launch over a column list."""
+"""Launches: their count, and the grid of a launch over a column list."""
 import numpy as np
 import pytest
 import torch
@@ -6,6 +6,7 @@ import torch
 from exoplasim_b200 import radiation as R
 from exoplasim_b200 import surrogate as SG
 from exoplasim_b200 import synthetic as S
+from exoplasim_b200.transforms import launch_count
 
 pytestmark = pytest.mark.gpu
 
@@ -16,6 +17,24 @@ def _columns(nlat, nlev, dt):
     dev = {k: torch.as_tensor(np.ascontiguousarray(v), dtype=dt, device="cuda") for k, v in dict(cols, zsol=zsol).items()}
     params = R.default_params(nlev, g["nhor"], g["nlon"], nsol=0)
     return params, dev, R.alloc_outputs(params, dt)
+
+
+@pytest.mark.parametrize("nhid,n", [(1, 5), (6, 300)])
+def test_training_launches_are_counted(nhid, n):
+    net = SG.Mlp(SG.nin_for(10), SG.nout_for(10), width=64, nhidden=nhid, max_batch=n)
+    net.init(seed=1)
+    x, t = torch.randn((n, net.nin), device="cuda"), torch.randn((n, net.nout), device="cuda")
+    loss, nl = torch.zeros(1, device="cuda"), nhid + 1
+    c0 = launch_count()
+    net.forward(x)
+    c1 = launch_count()
+    assert c1 - c0 == nl                 # one GEMM per layer
+    net.backward(x, t, loss)
+    c2 = launch_count()
+    # a GEMM per layer forward, the loss, a GEMM per layer below the last, all layers' weights and their sum
+    assert c2 - c1 == nl + 1 + (nl - 1) + 2
+    net.adam(1e-4, 1)
+    assert launch_count() - c2 == 1
 
 
 def _time(f, reps=5):
