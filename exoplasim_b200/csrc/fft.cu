@@ -4,11 +4,12 @@
 //            k < n/2 (the Nyquist term is not stored)
 //   inverse  x_j = A0 + 2 sum_{k=1}^{n/2-1} Re(c_k e^{+2 pi i jk/n}), B0 ignored.
 // A length-n real row is transformed as a length-h = n/2 complex sequence
-// z_j = x_{2j} + i x_{2j+1} with a self-sorting (Stockham) mixed-radix FFT in
-// shared memory, plus the usual even/odd split twiddle e^{-2 pi i k/n}.
-// One block transforms R rows; loads and stores of the grid side are
-// row-contiguous and coalesced.  The Fourier side may be row-major (the
-// reference layout) or m-major (the transform sets' intermediate).
+// z_j = x_{2j} + i x_{2j+1}, plus the usual even/odd split twiddle e^{-2 pi i k/n}.
+// Any length has a self-sorting (Stockham) mixed-radix form in shared memory; the
+// model's grid lengths have the same form with its schedule fixed at compile time,
+// for few rows, and a register-resident form, for many; n = 384 in FP32 has a
+// persistent one.  The Fourier side may be row-major (the reference layout) or
+// m-major (the transform sets' intermediate).
 #include <algorithm>
 #include <cmath>
 #include <map>
@@ -231,6 +232,228 @@ __global__ void __launch_bounds__(256) k_rfft_inverse(const T *fc, T *gp, FftLau
     for (int i = threadIdx.x; i < rows * n; i += blockDim.x) dst[i] = zr[i];
 }
 
+// the Fourier coefficient X_k of a real row from Z_k and Z_{h-k} of its
+// half-length complex transform (k > 0), scaled by 1/n
+template <typename T>
+__device__ __forceinline__ cpx<T> rf_split(cpx<T> a, cpx<T> b, cpx<T> wk, T scale) {
+    const cpx<T> E{(T)0.5 * (a.x + b.x), (T)0.5 * (a.y - b.y)};
+    const cpx<T> O{(T)0.5 * (a.y + b.y), (T)0.5 * (b.x - a.x)};
+    const cpx<T> wo = cmul(wk, O);
+    return cpx<T>{(E.x + wo.x) * scale, (E.y + wo.y) * scale};
+}
+
+// ---------------------------------------- Stockham passes at fixed lengths
+// For the model's grid lengths: the radix schedule, loop trip counts and index
+// divisions are compile-time constants; a block of 256 threads transforms ROWS
+// rows, most of its threads a point or a butterfly each.  Few rows (rr_from) take
+// this form, which has eight or more threads to a row for one of the
+// register-resident form below and so a short serial chain; many rows take that
+// one, which moves every value through shared memory fewer times.
+__host__ __device__ constexpr int radix_count(int h) {
+    int r = h, k = 0;
+    while (r % 8 == 0 && r > 8) { k++; r /= 8; }
+    while (r % 4 == 0) { k++; r /= 4; }
+    while (r % 2 == 0) { k++; r /= 2; }
+    while (r % 3 == 0) { k++; r /= 3; }
+    while (r % 5 == 0) { k++; r /= 5; }
+    if (r == 8) k++;
+    return k;
+}
+__host__ __device__ constexpr int radix_at(int h, int idx) {
+    int r = h, k = 0;
+    while (r % 8 == 0 && r > 8) { if (k++ == idx) return 8; r /= 8; }
+    while (r % 4 == 0) { if (k++ == idx) return 4; r /= 4; }
+    while (r % 2 == 0) { if (k++ == idx) return 2; r /= 2; }
+    while (r % 3 == 0) { if (k++ == idx) return 3; r /= 3; }
+    while (r % 5 == 0) { if (k++ == idx) return 5; r /= 5; }
+    return 8;
+}
+
+// Rows in shared memory keep 2 spare complex slots after every 16 elements:
+// the passes' strided reads and writes then spread over the banks (about half
+// the wavefronts of a dense row), and even indices stay 16-byte aligned for the
+// vector copies.  H is a multiple of 16 for every specialised length.
+__host__ __device__ constexpr int fpad(int j) { return j + 2 * (j >> 4); }
+template <int H> __host__ __device__ constexpr int fpad_row() { return H + 2 * (H / 16); }
+
+template <typename T, int S, int H, int ROWS, int R, int NS>
+__device__ __forceinline__ void pass_ct(const cpx<T> *src, cpx<T> *dst, const cpx<T> *tw) {
+    constexpr int NQ = H / R, STEP = H / (NS * R), NIT = ROWS * NQ, HP = fpad_row<H>();
+    for (int it = threadIdx.x; it < NIT; it += blockDim.x) {
+        const int row = it / NQ, t = it - row * NQ, k = t % NS;
+        const cpx<T> *s = src + row * HP;
+        cpx<T> *d = dst + row * HP;
+        cpx<T> v[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) v[r] = s[fpad(t + r * NQ)];
+        if constexpr (NS > 1) {  // the first pass has unit twiddles only
+#pragma unroll
+            for (int r = 1; r < R; r++) {
+                cpx<T> w = tw[r * k * STEP];
+                if (S > 0) w.y = -w.y;
+                v[r] = cmul(v[r], w);
+            }
+        }
+        dftR<T, S, R>(v);
+        const int base = (t / NS) * NS * R + k;
+#pragma unroll
+        for (int r = 0; r < R; r++) d[fpad(base + r * NS)] = v[r];
+    }
+}
+
+template <typename T, int S, int H, int ROWS, int IDX, int NS>
+__device__ __forceinline__ const cpx<T> *passes_ct(cpx<T> *src, cpx<T> *dst, const cpx<T> *tw) {
+    if constexpr (IDX >= radix_count(H)) {
+        return src;
+    } else {
+        constexpr int R = radix_at(H, IDX);
+        pass_ct<T, S, H, ROWS, R, NS>(src, dst, tw);
+        __syncthreads();
+        return passes_ct<T, S, H, ROWS, IDX + 1, NS * R>(dst, src, tw);
+    }
+}
+
+// First pass of a forward transform (unit twiddles), reading its inputs straight
+// from the grid rows in global memory: consecutive threads take consecutive
+// butterflies of a row, so each of the R loads is a contiguous run per row.
+template <typename T, int H, int ROWS, int R>
+__device__ __forceinline__ void pass_ct_first_global(const cpx<T> *g, int rows, cpx<T> *dst) {
+    constexpr int NQ = H / R, NIT = ROWS * NQ, HP = fpad_row<H>();
+    for (int it = threadIdx.x; it < NIT; it += blockDim.x) {
+        const int row = it / NQ, t = it - row * NQ;
+        cpx<T> v[R];
+        if (row < rows) {
+            const cpx<T> *s = g + (size_t)row * H;
+#pragma unroll
+            for (int r = 0; r < R; r++) v[r] = s[t + r * NQ];
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; r++) v[r] = cpx<T>{0, 0};
+        }
+        dftR<T, -1, R>(v);
+        cpx<T> *d = dst + row * HP;
+#pragma unroll
+        for (int r = 0; r < R; r++) d[fpad(t * R + r)] = v[r];
+    }
+}
+
+// Passes IDX.. of a transform whose last pass writes the rows < rows straight
+// to global memory (row-contiguous): in the last pass NS*R = H, so output
+// t + r*NS of consecutive threads is a contiguous run.
+template <typename T, int S, int H, int ROWS, int IDX, int NS>
+__device__ __forceinline__ void passes_ct_to_global(cpx<T> *src, cpx<T> *dst, const cpx<T> *tw, cpx<T> *g,
+                                                    int rows) {
+    constexpr int R = radix_at(H, IDX);
+    if constexpr (IDX + 1 < radix_count(H)) {
+        pass_ct<T, S, H, ROWS, R, NS>(src, dst, tw);
+        __syncthreads();
+        passes_ct_to_global<T, S, H, ROWS, IDX + 1, NS * R>(dst, src, tw, g, rows);
+    } else {
+        static_assert(NS * R == H, "last pass");
+        constexpr int NQ = H / R, NIT = ROWS * NQ, STEP = H / (NS * R), HP = fpad_row<H>();
+        for (int it = threadIdx.x; it < NIT; it += blockDim.x) {
+            const int row = it / NQ, t = it - row * NQ, k = t % NS;
+            if (row >= rows) continue;
+            const cpx<T> *s = src + row * HP;
+            cpx<T> v[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) v[r] = s[fpad(t + r * NQ)];
+            if constexpr (NS > 1) {
+#pragma unroll
+                for (int r = 1; r < R; r++) {
+                    cpx<T> w = tw[r * k * STEP];
+                    if (S > 0) w.y = -w.y;
+                    v[r] = cmul(v[r], w);
+                }
+            }
+            dftR<T, S, R>(v);
+            cpx<T> *d = g + (size_t)row * H;
+#pragma unroll
+            for (int r = 0; r < R; r++) d[t + r * NS] = v[r];
+        }
+    }
+}
+
+template <typename T> constexpr int ct_rows(int n) {
+    return (sizeof(T) == 4) ? (n <= 256 ? 16 : 8) : (n <= 256 ? 8 : 4);
+}
+
+template <typename T, int N, int ROWS>
+__global__ void __launch_bounds__(256) k_rfft_fwd_ct(const T *gp, T *fc, long long lot, int kf, long long f_rs,
+                                                      long long f_ms, const cpx<T> *__restrict__ w,
+                                                      const cpx<T> *__restrict__ rt) {
+    constexpr int H = N / 2, HP = fpad_row<H>();
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cpx<T> *b0 = reinterpret_cast<cpx<T> *>(smraw), *b1 = b0 + ROWS * HP;
+    const long long row0 = (long long)blockIdx.x * ROWS;
+    const int rows = (int)min((long long)ROWS, lot - row0);
+    pdl_trigger();
+    pdl_wait();   // the grid rows may come from the previous kernel
+    // the first pass reads the grid rows directly (unit twiddles); the rest run in shared memory
+    constexpr int R0 = radix_at(H, 0);
+    pass_ct_first_global<T, H, ROWS, R0>(reinterpret_cast<const cpx<T> *>(gp + row0 * N), rows, b1);
+    __syncthreads();
+    const cpx<T> *Z = passes_ct<T, -1, H, ROWS, 1, R0>(b1, b0, w);
+    const T scale = (T)1 / (T)N;
+    // X_k and X_{H-k} from Z_k and Z_{H-k} (k <= H/2), each Z read once; only
+    // k < kf are stored.  Rows fastest: consecutive threads write adjacent
+    // entries of the m-major side.
+    const int kh = min(H / 2, kf - 1);   // pairs (k, H-k) with k <= kh cover every k < kf
+    for (int it = threadIdx.x; it < ROWS * (kh + 1); it += blockDim.x) {
+        const int row = it % ROWS, k = it / ROWS, k2 = H - k;
+        if (row >= rows) continue;
+        const cpx<T> *z = Z + row * HP;
+        cpx<T> *fr = reinterpret_cast<cpx<T> *>(fc) + (row0 + row) * f_rs;
+        const cpx<T> a = z[fpad(k)];
+        if (k == 0) {
+            fr[0] = cpx<T>{(a.x + a.y) * scale, (T)0};
+            continue;
+        }
+        const cpx<T> b = z[fpad(k2)];
+        fr[(long long)k * f_ms] = rf_split(a, b, rt[k], scale);
+        if (k2 < kf && k2 != k) fr[(long long)k2 * f_ms] = rf_split(b, a, rt[k2], scale);
+    }
+}
+
+template <typename T, int N, int ROWS>
+__global__ void __launch_bounds__(256) k_rfft_inv_ct(const T *fc, T *gp, long long lot, int kf, long long f_rs,
+                                                      long long f_ms, const cpx<T> *__restrict__ w,
+                                                      const cpx<T> *__restrict__ rt) {
+    constexpr int H = N / 2, HP = fpad_row<H>();
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cpx<T> *b0 = reinterpret_cast<cpx<T> *>(smraw), *b1 = b0 + ROWS * HP;
+    const long long row0 = (long long)blockIdx.x * ROWS;
+    const int rows = (int)min((long long)ROWS, lot - row0);
+    pdl_trigger();
+    pdl_wait();   // the coefficients come from the previous kernel
+    // Z_k and Z_{H-k} of the half-length complex transform from c_k and c_{H-k}
+    // (c = 0 for k >= kf, and the m = 0 imaginary part ignored), one load of
+    // each coefficient; rows fastest, so consecutive threads read adjacent
+    // entries of the m-major side
+    auto unfold = [](cpx<T> a, cpx<T> b, cpx<T> wk) {
+        const cpx<T> E{a.x + b.x, a.y - b.y}, D{a.x - b.x, a.y + b.y};
+        const cpx<T> O = cmul(D, cpx<T>{wk.x, -wk.y});
+        return cpx<T>{E.x - O.y, E.y + O.x};
+    };
+    for (int it = threadIdx.x; it < ROWS * (H / 2 + 1); it += blockDim.x) {
+        const int row = it % ROWS, k = it / ROWS, k2 = H - k;
+        cpx<T> a{0, 0}, b{0, 0};
+        if (row < rows) {
+            const cpx<T> *fr = reinterpret_cast<const cpx<T> *>(fc) + (row0 + row) * f_rs;
+            if (k < kf) {
+                a = fr[(long long)k * f_ms];
+                if (k == 0) a.y = 0;
+            }
+            if (k > 0 && k2 < kf) b = fr[(long long)k2 * f_ms];
+        }
+        b0[row * HP + fpad(k)] = unfold(a, b, rt[k]);
+        if (k > 0 && k2 != k) b0[row * HP + fpad(k2)] = unfold(b, a, rt[k2]);
+    }
+    __syncthreads();
+    // the last pass writes the grid rows directly
+    passes_ct_to_global<T, +1, H, ROWS, 0, 1>(b0, b1, w, reinterpret_cast<cpx<T> *>(gp + row0 * N), rows);
+}
+
 // ------------------------------------------------ register-resident transforms
 // For the model's grid lengths (h = n/2 = P*Q complex points) P threads of a
 // warp work a row:
@@ -242,11 +465,10 @@ __global__ void __launch_bounds__(256) k_rfft_inverse(const T *fc, T *gp, FftLau
 // works RB = RR_THREADS/P rows.  The m-major Fourier side is reached rows
 // fastest: through the spectra in shared memory (forward) or the staged
 // coefficients (inverse), which take the transposition's place in turn.
-// Per launch (CUDA events), against the three-pass shared-memory (Stockham)
-// kernels before, which moved every value through shared memory six times and
-// were bound by instruction issue: T127 L20 FP64 forward 53 us against 66,
-// inverse 38 against 49; T85 L13 x3 FP32 31 against 40 and 19 against 33; T42 L20
-// FP64, one state, where latency bounds both, 11.2 against 11.3 and 9.7 against 10.1.
+// Per launch (CUDA events), against the Stockham form above, which moves every
+// value through shared memory six times and is bound by instruction issue: T127 L20
+// FP64 forward 53 us against 66, inverse 38 against 49; T85 L13 x3 FP32 31 against 40
+// and 19 against 33.  With few rows its serial chain is the longer one: see rr_from.
 constexpr int RR_THREADS = 128;
 // P: 16 where Q would need over 64 registers in FP64 (n = 384 with P = 8: 132
 // registers, 3 blocks per SM, forward 67 us per T127 L20 state)
@@ -405,16 +627,6 @@ __device__ __forceinline__ void cp_async16(void *dst_smem, const void *src_gmem)
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-// the Fourier coefficient X_k of a real row from Z_k and Z_{h-k} of its
-// half-length complex transform (k > 0), scaled by 1/n
-template <typename T>
-__device__ __forceinline__ cpx<T> rf_split(cpx<T> a, cpx<T> b, cpx<T> wk, T scale) {
-    const cpx<T> E{(T)0.5 * (a.x + b.x), (T)0.5 * (a.y - b.y)};
-    const cpx<T> O{(T)0.5 * (a.y + b.y), (T)0.5 * (b.x - a.x)};
-    const cpx<T> wo = cmul(wk, O);
-    return cpx<T>{(E.x + wo.x) * scale, (E.y + wo.y) * scale};
-}
 
 // Forward transform of block blk's RB rows.  FOLD: the block takes RB/2
 // latitude pairs j of one field (rows r and r + RB/2 a pair's northern and
@@ -1333,6 +1545,22 @@ static exotx_status launch_rr(bool fwd, const T *in, T *out, long long lot, int 
     return EXOTX_OK;
 }
 
+template <typename T, int N>
+static exotx_status launch_ct(bool fwd, const T *in, T *out, long long lot, int kf, long long f_rs, long long f_ms,
+                              const cpx<T> *w, const cpx<T> *r, cudaStream_t s) {
+    constexpr int ROWS = ct_rows<T>(N);
+    constexpr size_t smem = 2 * ROWS * fpad_row<N / 2>() * sizeof(cpx<T>);
+    static_assert(smem <= 48 * 1024, "default shared memory");
+    const long long nb = (lot + ROWS - 1) / ROWS;
+    const int kid = fwd ? EXOTX_K_FFT_FORWARD : EXOTX_K_FFT_INVERSE;
+    auto kern = fwd ? k_rfft_fwd_ct<T, N, ROWS> : k_rfft_inv_ct<T, N, ROWS>;
+    cudaEvent_t ev = ktimer_start(kid, s);
+    EXOTX_CUDA(launch_pdl(kern, dim3((unsigned)nb), dim3(256), smem, s, in, out, lot, kf, f_rs, f_ms, w, r));
+    EXOTX_CHECK_LAUNCH();
+    ktimer_stop(kid, s, ev);
+    return EXOTX_OK;
+}
+
 // blocks of a kernel resident on the whole device at once (SMs x blocks per SM)
 static exotx_status resident_slots(const void *kernel, int threads, size_t smem, int *slots) {
     int dev = 0, occ = 0, nsm = 0;
@@ -1377,6 +1605,35 @@ static exotx_status launch_rf(bool fwd, const float *in, float *out, long long l
     return EXOTX_OK;
 }
 
+// The rows from which on a transform is faster in the register-resident form than in
+// the Stockham form.  Between a row-major Fourier side and the grid (gp2fc, fc2gp)
+// the line was measured for each length at 2^11 to 2^23 points (rows x n) in steps of
+// two; in us, Stockham / register-resident:
+//   FP64 n=64  2^17 fwd 2.8/4.2 inv 2.7/3.6, 2^21 13.2/10.5 11.8/10.1
+//       n=256  2^16 4.4/8.5 4.3/6.5, 2^21 17.4/14.7 18.2/13.8
+//       n=320  2^16 3.4/9.0 3.3/7.7, 2^20 8.6/12.6 8.2/13.7, 2^23 41.7/35.8 39.7/40.3
+//       n=512  2^16 3.9/8.6 4.1/6.4, 2^22 27.6/23.6 27.6/21.6
+//   FP32 n=192 2^16 4.6/5.9 4.7/4.3, n=320 3.9/8.2 3.9/6.0, n=512 5.0/6.2 5.0/4.9
+// The sets' m-major side favours the register-resident form (its rows are runs there),
+// but at n = 320, whose 20 points a thread make its longest chain and where eight
+// threads share 20 eight-point transforms: one mixed T106 state, inverse sets of L5
+// 25.7/30.7 us, L10 32.7/34.8, L15 37.3/35.8; gridpointd L5 21.9/26.8, L20 35.6/36.0.
+template <typename T>
+static long long rr_from(bool fwd, int n, bool row_major) {
+    constexpr bool D = sizeof(T) == 8;
+    if (n == 320) return row_major ? 16384 : D && !fwd ? 6400 : 13000;
+    if (!row_major) return 0;
+    switch (n) {
+        case 64: return D ? 32768 : 4096;
+        case 128: return D ? (fwd ? 2048 : 1024) : 0;
+        case 192: return D ? (fwd ? 5120 : 10240) : fwd ? 2560 : 0;
+        case 256: return D ? (fwd ? 4608 : 1152) : fwd ? 2048 : 0;
+        case 384: return D ? (fwd ? 2560 : 5120) : 0;
+        case 512: return D ? 4096 : fwd ? 2048 : 0;
+    }
+    return 0;
+}
+
 // returns EXOTX_NOT_BUILT when n has no specialised kernel
 template <typename T>
 static exotx_status dispatch_len(bool fwd, int n, const T *in, T *out, long long lot, int kf, long long f_rs,
@@ -1387,7 +1644,9 @@ static exotx_status dispatch_len(bool fwd, int n, const T *in, T *out, long long
     return by_len(n, [&](auto len) {
         constexpr int N = decltype(len)::value;
         if constexpr (sizeof(T) == 4 && N == 384) return EXOTX_NOT_BUILT;
-        else return launch_rr<T, N>(fwd, in, out, lot, kf, f_rs, f_ms, w, r, s);
+        else {
+            return (lot < rr_from<T>(fwd, n, f_ms == 1) ? launch_ct<T, N> : launch_rr<T, N>)(fwd, in, out, lot, kf, f_rs, f_ms, w, r, s);
+        }
     });
 }
 
