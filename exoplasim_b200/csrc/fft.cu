@@ -489,11 +489,14 @@ template <typename T, int N> struct RrLayout {
     static constexpr int RC = GR > 1 ? rr_pad(RB, GR, G) : RB + 1;
     static constexpr int QP = (Q + P - 1) / P;
     static_assert(P * Q == H && 32 % P == 0, "a row's threads are in one warp");
-    static constexpr size_t fwd_smem() { return (size_t)RB * (RS > RZ ? RS : RZ) * 2 * sizeof(T); }
-    static constexpr size_t inv_smem(int kf) {
+    static constexpr size_t fwd_x() { return (size_t)RB * (RS > RZ ? RS : RZ); }   // complex values
+    static __host__ __device__ constexpr size_t inv_x(int kf) {
         const size_t c = (size_t)kf * RC, x = (size_t)RB * RS;
-        return (c > x ? c : x) * 2 * sizeof(T);
+        return c > x ? c : x;
     }
+    // early: the split twiddles behind
+    static constexpr size_t fwd_smem(bool early = false) { return (fwd_x() + (early ? H : 0)) * 2 * sizeof(T); }
+    static constexpr size_t inv_smem(int kf, bool early = false) { return (inv_x(kf) + (early ? H : 0)) * 2 * sizeof(T); }
 };
 
 // cos(2 pi a / n) for n = 12, 16, 20, 24
@@ -628,13 +631,24 @@ __device__ __forceinline__ void cp_async16(void *dst_smem, const void *src_gmem)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
+// EARLY: the twiddles are fetched before the wait for the previous kernel, a thread's
+// column twiddles into registers and the split twiddles into shared memory
+template <typename T, int N, int Q>
+__device__ __forceinline__ void rr_early(const cpx<T> *w, const cpx<T> *rt, cpx<T> (&wt)[Q], cpx<T> *rts) {
+    using Lay = RrLayout<T, N>;
+    static_assert(Q == Lay::Q, "a column");
+#pragma unroll
+    for (int q = 0; q < Q; q++) wt[q] = w[(threadIdx.x % Lay::P) * q];   // t q < h
+    for (int k = threadIdx.x; k < Lay::H; k += RR_THREADS) rts[k] = rt[k];   // block barriers lie before their use
+}
+
 // Forward transform of block blk's RB rows.  FOLD: the block takes RB/2
 // latitude pairs j of one field (rows r and r + RB/2 a pair's northern and
 // southern rows) and stores E = X(j) + X(nlat-1-j) at row field*nlat + j and
 // O = X(j) - X(nlat-1-j) at row field*nlat + nlat/2 + j of the m-major side
 // (complex element (row, m) at row + m*f_ms), for the Legendre kernels; lot is
 // a multiple of nlat.  Otherwise row r's X_k goes to r*f_rs + k*f_ms.
-template <typename T, int N, bool FOLD>
+template <typename T, int N, bool FOLD, bool EARLY = false>
 __device__ __forceinline__ void rr_fwd_body(const T *gp, T *fc, int nlat, long long lot, int kf, long long f_rs,
                                             long long f_ms, const cpx<T> *__restrict__ w,
                                             const cpx<T> *__restrict__ rt, RowSums rs, long long blk) {
@@ -655,6 +669,9 @@ __device__ __forceinline__ void rr_fwd_body(const T *gp, T *fc, int nlat, long l
     }
     cpx<T> v[Q];
     pdl_trigger();
+    cpx<T> wt[EARLY ? Q : 1];
+    if constexpr (EARLY) rr_early<T, N>(w, rt, wt, sm + Lay::fwd_x());
+    auto split = [&](int k) { return EARLY ? sm[Lay::fwd_x() + k] : rt[k]; };
     pdl_wait();   // the grid rows may come from the previous kernel, which may still read the output
     {
         const cpx<T> *g = reinterpret_cast<const cpx<T> *>(gp) + (grow < 0 ? 0 : grow) * H + t;
@@ -671,14 +688,15 @@ __device__ __forceinline__ void rr_fwd_body(const T *gp, T *fc, int nlat, long l
     cpx<T> *x = sm + r * Lay::RS;
     x[t] = v[0];
 #pragma unroll
-    for (int q = 1; q < Q; q++) x[q * (P + 1) + t] = cmul(v[q], w[t * q]);   // t q < h
+    for (int q = 1; q < Q; q++) x[q * (P + 1) + t] = cmul(v[q], EARLY ? wt[EARLY ? q : 0] : w[t * q]);   // t q < h
     __syncwarp();
     cpx<T> z[QP][P];
 #pragma unroll
     for (int i = 0; i < QP; i++) {
-        if (Q % P != 0 && t + P * i >= Q) continue;
+        if (!EARLY && Q % P != 0 && t + P * i >= Q) continue;
+        const int q = EARLY && Q % P != 0 ? min(t + P * i, Q - 1) : t + P * i;   // without a branch: the last again
 #pragma unroll
-        for (int u = 0; u < P; u++) z[i][u] = x[(t + P * i) * (P + 1) + u];
+        for (int u = 0; u < P; u++) z[i][u] = x[q * (P + 1) + u];
         dft_len<T, -1, P>(z[i]);
     }
     __syncthreads();   // the spectra overwrite the transposition
@@ -709,10 +727,10 @@ __device__ __forceinline__ void rr_fwd_body(const T *gp, T *fc, int nlat, long l
                 put(0, cpx<T>{(an.x + an.y) * scale, (T)0}, cpx<T>{(as.x + as.y) * scale, (T)0});
                 continue;
             }
-            const cpx<T> bn = zn[k2], bs = zs[k2], wk = rt[k];
+            const cpx<T> bn = zn[k2], bs = zs[k2], wk = split(k);
             put(k, rf_split(an, bn, wk, scale), rf_split(as, bs, wk, scale));
             if (k2 < kf && k2 != k) {
-                const cpx<T> wk2 = rt[k2];
+                const cpx<T> wk2 = split(k2);
                 put(k2, rf_split(bn, an, wk2, scale), rf_split(bs, as, wk2, scale));
             }
         }
@@ -730,14 +748,14 @@ __device__ __forceinline__ void rr_fwd_body(const T *gp, T *fc, int nlat, long l
                 continue;
             }
             const cpx<T> b = zz[k2];
-            fr[(long long)k * f_ms] = rf_split(a, b, rt[k], scale);
-            if (k2 < kf && k2 != k) fr[(long long)k2 * f_ms] = rf_split(b, a, rt[k2], scale);
+            fr[(long long)k * f_ms] = rf_split(a, b, split(k), scale);
+            if (k2 < kf && k2 != k) fr[(long long)k2 * f_ms] = rf_split(b, a, split(k2), scale);
         }
     }
 }
 
 // Inverse transform of block blk's RB rows (coefficients k < kf, zero above)
-template <typename T, int N>
+template <typename T, int N, bool EARLY = false>
 __device__ __forceinline__ void rr_inv_body(const T *fc, T *gp, long long lot, int kf, long long f_rs, long long f_ms,
                                             const cpx<T> *__restrict__ w, const cpx<T> *__restrict__ rt, long long blk) {
     using Lay = RrLayout<T, N>;
@@ -748,6 +766,8 @@ __device__ __forceinline__ void rr_inv_body(const T *fc, T *gp, long long lot, i
     const long long row0 = blk * RB;
     const int rows = (int)min((long long)RB, lot - row0);
     pdl_trigger();
+    cpx<T> wt[EARLY ? Q : 1];
+    if constexpr (EARLY) rr_early<T, N>(w, rt, wt, sm + Lay::inv_x(kf));
     pdl_wait();   // the coefficients come from the previous kernel
     {
         const cpx<T> *fcc = reinterpret_cast<const cpx<T> *>(fc) + row0 * f_rs;
@@ -766,8 +786,8 @@ __device__ __forceinline__ void rr_inv_body(const T *fc, T *gp, long long lot, i
     cpx<T> z[QP][P];
 #pragma unroll
     for (int i = 0; i < QP; i++) {
-        const int q = t + P * i;
-        if (Q % P != 0 && q >= Q) continue;
+        if (!EARLY && Q % P != 0 && t + P * i >= Q) continue;
+        const int q = EARLY && Q % P != 0 ? min(t + P * i, Q - 1) : t + P * i;   // without a branch: the last again
 #pragma unroll
         for (int m = 0; m < P; m++) {
             const int k = q + Q * m, k2 = H - k;
@@ -779,7 +799,7 @@ __device__ __forceinline__ void rr_inv_body(const T *fc, T *gp, long long lot, i
             if (k > 0 && k2 < kf) b = sm[k2 * RC + r];
             // Z_k of the half-length complex sequence (c = 0 for k >= kf, the m = 0 imaginary part ignored)
             const cpx<T> E{a.x + b.x, a.y - b.y}, D{a.x - b.x, a.y + b.y};
-            cpx<T> wk = rt[k];
+            cpx<T> wk = EARLY ? sm[Lay::inv_x(kf) + k] : rt[k];
             wk.y = -wk.y;
             const cpx<T> O = cmul(D, wk);
             z[i][m] = cpx<T>{E.x - O.y, E.y + O.x};
@@ -799,7 +819,7 @@ __device__ __forceinline__ void rr_inv_body(const T *fc, T *gp, long long lot, i
     v[0] = x[t];
 #pragma unroll
     for (int q = 1; q < Q; q++) {
-        const cpx<T> wq = w[t * q];
+        const cpx<T> wq = EARLY ? wt[EARLY ? q : 0] : w[t * q];
         v[q] = cmul(x[q * (P + 1) + t], cpx<T>{wq.x, -wq.y});
     }
     dft_len<T, +1, Q>(v);
@@ -810,17 +830,17 @@ __device__ __forceinline__ void rr_inv_body(const T *fc, T *gp, long long lot, i
     }
 }
 
-template <typename T, int N, bool FOLD>
+template <typename T, int N, bool FOLD, bool EARLY>
 __global__ void __launch_bounds__(RR_THREADS) k_rfft_fwd_rr(const T *gp, T *fc, int nlat, long long lot, int kf,
                                                              long long f_rs, long long f_ms, const cpx<T> *__restrict__ w,
                                                              const cpx<T> *__restrict__ rt, RowSums rs) {
-    rr_fwd_body<T, N, FOLD>(gp, fc, nlat, lot, kf, f_rs, f_ms, w, rt, rs, blockIdx.x);
+    rr_fwd_body<T, N, FOLD, EARLY>(gp, fc, nlat, lot, kf, f_rs, f_ms, w, rt, rs, blockIdx.x);
 }
-template <typename T, int N>
+template <typename T, int N, bool EARLY>
 __global__ void __launch_bounds__(RR_THREADS) k_rfft_inv_rr(const T *fc, T *gp, long long lot, int kf, long long f_rs,
                                                              long long f_ms, const cpx<T> *__restrict__ w,
                                                              const cpx<T> *__restrict__ rt) {
-    rr_inv_body<T, N>(fc, gp, lot, kf, f_rs, f_ms, w, rt, blockIdx.x);
+    rr_inv_body<T, N, EARLY>(fc, gp, lot, kf, f_rs, f_ms, w, rt, blockIdx.x);
 }
 
 // ------------------------------- n = 384 in FP32 (T127): bulk copies, persistent
@@ -1529,17 +1549,23 @@ template <typename T, int N>
 static exotx_status launch_rr(bool fwd, const T *in, T *out, long long lot, int kf, long long f_rs, long long f_ms,
                               const cpx<T> *w, const cpx<T> *r, cudaStream_t s) {
     using Lay = RrLayout<T, N>;
-    const size_t smem = fwd ? Lay::fwd_smem() : Lay::inv_smem(kf);
+    // n = 320 has the longest chain, 20 points a thread: with few rows (one T106 state of
+    // up to 12 levels) the inverse fetches its twiddles early.  Mixed sets of L5 31.5 us
+    // without, 25.7 with, L10 34.8 and 31.4; with many the registers cost more (nine states
+    // of L20 256 and 277)
+    constexpr bool MAY = sizeof(T) == 4 && N == 320;
+    const bool early = MAY && !fwd && lot < 13000;
+    const size_t smem = fwd ? Lay::fwd_smem() : Lay::inv_smem(kf, early);
     const long long nb = (lot + Lay::RB - 1) / Lay::RB;
     const int kid = fwd ? EXOTX_K_FFT_FORWARD : EXOTX_K_FFT_INVERSE;
-    static_assert(Lay::fwd_smem() <= 48 * 1024 && Lay::inv_smem(Lay::H) <= 48 * 1024, "default shared memory");
+    static_assert(Lay::fwd_smem() <= 48 * 1024 && Lay::inv_smem(Lay::H, MAY) <= 48 * 1024, "default shared memory");
     cudaEvent_t ev = ktimer_start(kid, s);
     if (fwd)
-        EXOTX_CUDA(launch_pdl(k_rfft_fwd_rr<T, N, false>, dim3((unsigned)nb), dim3(RR_THREADS), smem, s, in, out, 0, lot,
+        EXOTX_CUDA(launch_pdl(k_rfft_fwd_rr<T, N, false, false>, dim3((unsigned)nb), dim3(RR_THREADS), smem, s, in, out, 0, lot,
                               kf, f_rs, f_ms, w, r, RowSums{}));
     else
-        EXOTX_CUDA(launch_pdl(k_rfft_inv_rr<T, N>, dim3((unsigned)nb), dim3(RR_THREADS), smem, s, in, out, lot, kf, f_rs,
-                              f_ms, w, r));
+        EXOTX_CUDA(launch_pdl(early ? k_rfft_inv_rr<T, N, MAY> : k_rfft_inv_rr<T, N, false>, dim3((unsigned)nb),
+                              dim3(RR_THREADS), smem, s, in, out, lot, kf, f_rs, f_ms, w, r));
     EXOTX_CHECK_LAUNCH();
     ktimer_stop(kid, s, ev);
     return EXOTX_OK;
@@ -1614,20 +1640,18 @@ static exotx_status launch_rf(bool fwd, const float *in, float *out, long long l
 //       n=320  2^16 3.4/9.0 3.3/7.7, 2^20 8.6/12.6 8.2/13.7, 2^23 41.7/35.8 39.7/40.3
 //       n=512  2^16 3.9/8.6 4.1/6.4, 2^22 27.6/23.6 27.6/21.6
 //   FP32 n=192 2^16 4.6/5.9 4.7/4.3, n=320 3.9/8.2 3.9/6.0, n=512 5.0/6.2 5.0/4.9
-// The sets' m-major side favours the register-resident form (its rows are runs there),
-// but at n = 320, whose 20 points a thread make its longest chain and where eight
-// threads share 20 eight-point transforms: one mixed T106 state, inverse sets of L5
-// 25.7/30.7 us, L10 32.7/34.8, L15 37.3/35.8; gridpointd L5 21.9/26.8, L20 35.6/36.0.
+// The sets' m-major side, whose rows are runs in the register-resident form, takes it
+// at every row count, and so a state has the same bits in any batch or ensemble.
 template <typename T>
 static long long rr_from(bool fwd, int n, bool row_major) {
     constexpr bool D = sizeof(T) == 8;
-    if (n == 320) return row_major ? 16384 : D && !fwd ? 6400 : 13000;
     if (!row_major) return 0;
     switch (n) {
         case 64: return D ? 32768 : 4096;
         case 128: return D ? (fwd ? 2048 : 1024) : 0;
         case 192: return D ? (fwd ? 5120 : 10240) : fwd ? 2560 : 0;
         case 256: return D ? (fwd ? 4608 : 1152) : fwd ? 2048 : 0;
+        case 320: return 16384;
         case 384: return D ? (fwd ? 2560 : 5120) : 0;
         case 512: return D ? 4096 : fwd ? 2048 : 0;
     }
@@ -1803,10 +1827,13 @@ static exotx_status launch_fold(const float *in, float *out, int nlat, long long
         using Lay = RrLayout<float, N>;
         const int nbpf = (nlat / 2 + Lay::RB / 2 - 1) / (Lay::RB / 2);
         const long long nb = (lot / nlat) * nbpf;
-        constexpr size_t smem = Lay::fwd_smem();
+        // n = 320: twiddles early (launch_rr); mixed forward sets of one T106 state, L5 32.8
+        // us without, 29.1 with, L10 44.3 and 41.0, nine of L20 372 and 365
+        constexpr bool EARLY = N == 320;
+        constexpr size_t smem = Lay::fwd_smem(EARLY);
         static_assert(smem <= 48 * 1024, "default shared memory");
         ev = ktimer_start(EXOTX_K_FFT_FORWARD, s);
-        EXOTX_CUDA(launch_pdl(k_rfft_fwd_rr<float, N, true>, dim3((unsigned)nb), dim3(RR_THREADS), smem, s, in, out, nlat,
+        EXOTX_CUDA(launch_pdl(k_rfft_fwd_rr<float, N, true, EARLY>, dim3((unsigned)nb), dim3(RR_THREADS), smem, s, in, out, nlat,
                               lot, kf, 1LL, f_ms, w, r, rs));
     }
     EXOTX_CHECK_LAUNCH();

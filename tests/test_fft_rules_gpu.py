@@ -1,12 +1,13 @@
 """The FFT forms on either side of the row counts where the dispatch changes between them.
 
 Tolerances, fixed beforehand: a double transform 1e-13, a float one 2e-6 (2 log2(n) roundings of 6e-8 are 1.1e-6 at
-n = 512); sets FP64 1e-12, FP32 2e-5, mixed 5e-6, the bars those paths have elsewhere."""
+n = 512)."""
 import numpy as np
 import pytest
 import torch
 
 from exoplasim_b200 import synthetic as S
+from exoplasim_b200.ensemble import Ensemble
 from exoplasim_b200.transforms import Plan, fc2gp, gp2fc
 from tests._util import relerr
 
@@ -39,17 +40,27 @@ def test_rows_about_the_line(dt, tol, n, lines):
             assert relerr(a.double().cpu().numpy(), np.fft.irfft(c * n, n=n, axis=-1)) < tol
 
 
-@pytest.mark.parametrize("prec,tol", [("fp64", 1e-12), ("fp32", 2e-5), ("mixed", 5e-6)])
-def test_t106_batch_and_states(prec, tol):
-    # eight states of 320-point rows take the many-row form, one the other
+@pytest.mark.parametrize("prec", ["fp64", "fp32", "mixed"])
+def test_t106_states_have_their_bits_in_any_batch(prec):
+    # eight states of 320-point rows and one take two forms of the inverse; an ensemble a third, and its own forward one
     nlat, nlev, ninst = 160, 6, 8
     P, dt = Plan(nlat), torch.float64 if prec == "fp64" else torch.float32
     sp = torch.as_tensor(np.stack([S.transform_state(P.ntru, nlev, seed=i, kind="steep") for i in range(ninst)]), dtype=dt).cuda()
     gi = torch.as_tensor(np.stack([S.grid_tendencies(nlat, nlev, seed=i) for i in range(ninst)]), dtype=dt).cuda()
     td = gi[:, :4 * nlev].contiguous()
+    one = {}
     for f, x in ((P.inverse_set_batch, sp), (P.forward_set_batch, gi), (P.inverse_set_d_batch, sp), (P.forward_set_d_batch, td)):
-        many = f(x, nlev, precision=prec).double().cpu().numpy()
+        many = f(x, nlev, precision=prec)
         for i in (0, ninst - 1):
-            one = f(x[i:i + 1].contiguous(), nlev, precision=prec).double().cpu().numpy()[0]
-            for a, b in zip(many[i].reshape(len(one), -1), one.reshape(len(one), -1)):
-                assert relerr(a, b) < tol
+            one[f.__name__] = f(x[i:i + 1].contiguous(), nlev, precision=prec)[0]
+            assert torch.equal(many[i], one[f.__name__])
+    if prec == "mixed":
+        E = Ensemble([nlat, 32], [nlev, 5])
+        spin, gout, gin, spout = E.buffers()
+        spin.zero_(), gin.zero_()
+        spin[int(E.spec_off[0]):][:sp[0].numel()] = sp[-1].reshape(-1)
+        gin[int(E.gin_off[0]):][:gi[0].numel()] = gi[-1].reshape(-1)
+        E.inverse(spin, gout)
+        E.forward(gin, spout)
+        assert torch.equal(E.unpack("gout", gout)[0].reshape(-1), one["inverse_set_batch"].reshape(-1))
+        assert torch.equal(E.unpack("spec", spout)[0].reshape(-1), one["forward_set_batch"].reshape(-1))
