@@ -127,9 +127,8 @@ struct exotx_plan_s {
 };
 
 namespace exotx {
-// table indices inside d_inv* and d_fwd*
+// table indices inside d_inv64
 enum { INV_QI = 0, INV_QJ = 1, INV_QU = 2, INV_QV = 3 };
-enum { FWD_QC = 0, FWD_QE = 1, FWD_QM = 2, FWD_QQ = 3 };
 
 exotx_status ensure_work(exotx_plan p, size_t bytes, cudaStream_t s);
 inline bool capturing(cudaStream_t s) {
@@ -229,8 +228,6 @@ cudaEvent_t ktimer_start(int kernel, cudaStream_t s);
 void ktimer_stop(int kernel, cudaStream_t s, cudaEvent_t e0);
 
 // tensor-core Legendre (legendre_tc.cu)
-exotx_status tc_inverse_set(exotx_plan p, const float *spin, float *four, int nlev, cudaStream_t s);
-exotx_status tc_forward_set(exotx_plan p, const float *four, float *spout, int nlev, cudaStream_t s);
 exotx_status tc_inverse_batch(exotx_plan p, const float *spin, float *gpout, int L, int ninst, cudaStream_t s);
 exotx_status tc_forward_batch(exotx_plan p, const float *gpin, float *spout, int L, int ninst, cudaStream_t s);
 // the gridpointd sets (plasim.f90:3142-3149, :3415-3428) on the same kernels
@@ -269,6 +266,5 @@ exotx_status tc_error_read(int *err, cudaStream_t s);
 // the same for the FFT kernels' bounded waits (fft.cu)
 exotx_status fft_error_reset(cudaStream_t s);
 exotx_status fft_error_read(int *err, cudaStream_t s);
-exotx_status tc_available();
 void tc_free(exotx_plan p);
 }  // namespace exotx

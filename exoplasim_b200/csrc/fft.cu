@@ -853,7 +853,6 @@ __device__ int g_fft_error;   // nonzero: a bounded wait in an FFT kernel gave u
 
 template <int N> struct RfShape { static constexpr int P = 0, Q = 0, NT = 256; };
 template <> struct RfShape<384> { static constexpr int P = 8, Q = 24, NT = 128; };
-template <int N> constexpr bool rf_len() { return RfShape<N>::P > 0; }
 // Shared memory (complex units unless noted), P = 8:
 //   region R, reused in turn for the staged grid rows (row stride RG = 8 mod 16:
 //   the two rows of a half-warp on different banks), the transposition (a
@@ -1409,12 +1408,6 @@ __global__ void __launch_bounds__(256) k_rfft_fwd_rf(const float *gp, float *fc,
                                                       const cpx<float> *__restrict__ rt) {
     rfft_fwd_rf_body<N>(gp, fc, lot, kf, f_rs, f_ms, w, rt, blockIdx.x);
 }
-template <int N>
-__global__ void __launch_bounds__(256) k_rfft_inv_rf(const float *fc, float *gp, long long lot, int kf, long long f_rs,
-                                                      long long f_ms, const cpx<float> *__restrict__ w,
-                                                      const cpx<float> *__restrict__ rt) {
-    rfft_inv_rf_body<N>(fc, gp, lot, kf, f_rs, f_ms, w, rt, blockIdx.x);
-}
 // ---------------------------------------------------------------- ensembles
 // One launch transforms the rows of up to FFT_ENS_MAXSEG segments of different
 // lengths (an uneven ensemble); block b belongs to the last segment whose
@@ -1602,32 +1595,25 @@ static exotx_status launch_rf(bool fwd, const float *in, float *out, long long l
                               long long f_ms, const cpx<float> *w, const cpx<float> *r, cudaStream_t s) {
     using Lay = RfLayout<N>;
     const long long nb = (lot + Lay::RB - 1) / Lay::RB;
-    const int kid = fwd ? EXOTX_K_FFT_FORWARD : EXOTX_K_FFT_INVERSE;
-    if (fwd)
+    if (fwd) {
         EXOTX_CUDA(cudaFuncSetAttribute(k_rfft_fwd_rf<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::SMEM));
-    else if (kf > Lay::H)
-        EXOTX_CUDA(cudaFuncSetAttribute(k_rfft_inv_rf<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::SMEM));
-    long long grid = nb;
-    size_t smem_p = 0;
-    if (!fwd && kf <= Lay::H) {   // persistent form: one block per resident slot
-        smem_p = RfIPLayout<N>::smem(kf);
-        EXOTX_CUDA(allow_smem(k_rfft_inv_rf_p<N>, RfIPLayout<N>::smem(Lay::H), RfIPLayout<N>::smem(Lay::H)));
-        int slots = 0;
-        EXOTX_TRY(resident_slots((const void *)k_rfft_inv_rf_p<N>, Lay::NT, smem_p, &slots));
-        grid = std::min<long long>(nb, slots);
-    }
-    cudaEvent_t ev = ktimer_start(kid, s);
-    if (fwd)
+        cudaEvent_t ev = ktimer_start(EXOTX_K_FFT_FORWARD, s);
         EXOTX_CUDA(launch_pdl(k_rfft_fwd_rf<N>, dim3((unsigned)nb), dim3(Lay::NT), Lay::SMEM, s, in, out, lot, kf, f_rs,
                               f_ms, w, r));
-    else if (smem_p)
-        EXOTX_CUDA(launch_pdl(k_rfft_inv_rf_p<N>, dim3((unsigned)grid), dim3(Lay::NT), smem_p, s, in, out, lot, kf,
-                              f_rs, f_ms, nb, w, r));
-    else
-        EXOTX_CUDA(launch_pdl(k_rfft_inv_rf<N>, dim3((unsigned)nb), dim3(Lay::NT), Lay::SMEM, s, in, out, lot, kf, f_rs,
-                              f_ms, w, r));
+        EXOTX_CHECK_LAUNCH();
+        ktimer_stop(EXOTX_K_FFT_FORWARD, s, ev);
+        return EXOTX_OK;
+    }
+    // persistent: one block per resident slot
+    const size_t smem = RfIPLayout<N>::smem(kf), most = RfIPLayout<N>::smem(Lay::H);
+    EXOTX_CUDA(allow_smem(k_rfft_inv_rf_p<N>, most, most));
+    int slots = 0;
+    EXOTX_TRY(resident_slots((const void *)k_rfft_inv_rf_p<N>, Lay::NT, smem, &slots));
+    cudaEvent_t ev = ktimer_start(EXOTX_K_FFT_INVERSE, s);
+    EXOTX_CUDA(launch_pdl(k_rfft_inv_rf_p<N>, dim3((unsigned)std::min<long long>(nb, slots)), dim3(Lay::NT), smem, s, in, out,
+                          lot, kf, f_rs, f_ms, nb, w, r));
     EXOTX_CHECK_LAUNCH();
-    ktimer_stop(kid, s, ev);
+    ktimer_stop(EXOTX_K_FFT_INVERSE, s, ev);
     return EXOTX_OK;
 }
 

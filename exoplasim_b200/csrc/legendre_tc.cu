@@ -267,7 +267,6 @@ void tc_free(exotx_plan p) {
     delete p->tc;
     p->tc = nullptr;
 }
-exotx_status tc_available() { return EXOTX_OK; }
 
 // ------------------------------------------------------------------ jobs
 // inverse groups: 0 = qi on sd,st,sz,sq,sp; 1 = qj on sp; 2 = qu,qv on (D,Z)
@@ -761,13 +760,6 @@ exotx_status tc_ens_run(const EnsSeg *segs, int nseg, int dir, const int4 *d_job
         EXOTX_TRY(launch_fwd_pipe(P3, njobs, njmax, s));
     }
     return EXOTX_OK;
-}
-
-exotx_status tc_inverse_set(exotx_plan p, const float *spin, float *gpout, int L, cudaStream_t s) {
-    return tc_inverse_batch(p, spin, gpout, L, 1, s);
-}
-exotx_status tc_forward_set(exotx_plan p, const float *gpin, float *spout, int L, cudaStream_t s) {
-    return tc_forward_batch(p, gpin, spout, L, 1, s);
 }
 
 exotx_status tc_error_reset(cudaStream_t s) {
