@@ -179,7 +179,7 @@ EXOTX_API exotx_status exotx_fc2gp(int prec, void *a, int n, int lot, exotx_stre
 // are factors of the Fourier coefficients (sqrt(2), (-1)^m), where separate calls
 // made the reference's row-major Fourier layout with its zero tails and passed
 // over the grid for each: a T42 L10 file's temperature, wind and cloud cover took
-// 25 launches and 280 us, now 8 and 118, bound by the calls on the host.
+// 25 launches and 280 us, now 7 and 118, bound by the calls on the host.
 EXOTX_API exotx_status exotx_sp2gp_scaled(exotx_plan p, int prec, const void *sp, void *gp, int nlev, double scale,
                                           int roll, void *work, exotx_stream s) {
     if (!p || (prec != EXOTX_FP64 && prec != EXOTX_FP32) || nlev < 0) return EXOTX_BAD_ARG;

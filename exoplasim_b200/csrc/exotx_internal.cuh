@@ -116,12 +116,11 @@ struct exotx_plan_s {
     std::vector<void *> old_work;   // outgrown ones that captured graphs use
     exotx::TcTables *tc = nullptr;
     exotx::HostPipe *hpipe = nullptr;  // device slots and streams of exotx_sets_host
-    // bytes of m-major Fourier intermediate one tensor-core launch covers
-    // (instances are grouped up to this, at least one): the intermediate is
-    // written by one kernel and read by the next, so it should stay in L2
-    // 512 MB: up to 21 T127 L20 instances per inverse launch, 14 per forward;
-    // fewer, larger launches measured faster than L2-sized ones (T127 L20,
-    // 8 instances: 10.2K round trips/s with one launch per half, 9.5K with 80 MB)
+    // bytes of m-major Fourier intermediate one launch of a mixed set covers
+    // (instances are grouped up to this, at least one).  512 MB: up to 21 T127
+    // L20 instances per inverse launch, 14 per forward; fewer, larger launches
+    // measured faster than L2-sized ones (T127 L20, 8 instances: 10.2K round
+    // trips/s with one launch per half, 9.5K with 80 MB)
     size_t chunk_inv = (size_t)512 << 20, chunk_fwd = (size_t)512 << 20;
     int inv_half_ok = 0;   // the inverse kernel may run two CTAs per SM where they fit
 };

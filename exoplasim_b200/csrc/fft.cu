@@ -1201,7 +1201,7 @@ __global__ void __launch_bounds__(128) k_rfft_fwd_fold_rf_p(const float *gp, flo
     }
 }
 
-// The block's
+// Inverse transform of block blk's RB rows of n = 384 (the ensembles' form).  The
 // coefficients c_k (k < kf) are staged k-major in shared memory by plain
 // coalesced loads (a k's RB rows are one run of the m-major side); each thread
 // forms the Z_k of its own q from c_k and c_{h-k}, takes their P-point DFTs,

@@ -231,7 +231,8 @@ __device__ __forceinline__ void gp_copy(T *s, const T *g) {
 
 // x / d from r = 1 / d rounded: one correction by the exact residual gives the
 // correctly rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990); where the
-// residual is not finite the product stands, as the quotient itself would
+// residual is not finite the product stands, as the quotient itself would for a zero
+// or infinite operand (1 / d overflows for d below 2^-128, surface pressures of e^-88)
 __device__ __forceinline__ float gp_div(float x, float d, float r) {
     const float q = x * r, e = fmaf(-q, d, x);
     return fabsf(e) <= 3.402823466e38f ? fmaf(e, r, q) : q;
@@ -419,9 +420,9 @@ inline exotx_status gp_launch_k(const GpArgs<T> &A, size_t smem, cudaStream_t s)
 }
 // The asynchronous form takes initsi's triangular g up to 25 levels in FP32 and 20
 // in FP64: its code is unrolled over the levels, and beyond 128 KB of it the
-// instruction cache no longer holds it (FP64 T85 x5: 20 levels 159 against 224 us
-// at T127 x3, 25 levels 376 against 290).  The rest runs in the general form, its
-// constants in shared memory where they fit beside the profiles.
+// instruction cache no longer holds it (FP64, asynchronous / general form: T127 x3
+// with 20 levels 160 / 224 us, T85 x5 with 25 levels 376 / 290).  The rest runs in the
+// general form, its constants in shared memory where they fit beside the profiles.
 template <typename T>
 inline exotx_status gp_launch(const GpArgs<T> &A, const exotx_gp_params &h, cudaStream_t s) {
     const int L = A.L;
@@ -436,7 +437,9 @@ inline exotx_status gp_launch(const GpArgs<T> &A, const exotx_gp_params &h, cuda
     const bool sk = gp_smem<T>(L, true) <= 227 * 1024;
     const size_t smem = gp_smem<T>(L, sk);
     if (!sk) return gp_launch_k<T, false, 0>(A, smem, s);
-    switch (L) {   // the level counts of the standard configurations
+    // the level counts of the standard configurations, for other than initsi's g and for
+    // FP64's 25 (T85 x3, any count / its own: FP32 L10 31 / 23 us, L20 90 / 55; FP64 alike)
+    switch (L) {
         case 10: return gp_launch_k<T, true, 10>(A, smem, s);
         case 20: return gp_launch_k<T, true, 20>(A, smem, s);
         case 25: return gp_launch_k<T, true, 25>(A, smem, s);

@@ -401,7 +401,7 @@ struct LegFwd {
     T *out[3];               // single op: spectral outputs; set: out[0] is the set's output
     long long o_fs;          // spectral field stride (reals)
     double scale;            // single op: factor of the outputs
-    int folded;              // the intermediate holds N+S, then N-S per field (rfft_fwd_fold_body)
+    int folded;              // the intermediate holds N+S, then N-S per field (rr_fwd_body)
     int nu, nt;              // units (levels x states) and unit tiles per wavenumber
     int nu1, nt1;            // gridpointa: ln ps tendencies (fc2sp) and their tiles
     int wb, nmb;             // warps along the modes of a block; mode blocks per wavenumber

@@ -108,14 +108,24 @@ static const int kFwdRef[4] = {2, 3, 4, 5};
 // tiles of 128 rows and six split products per term, so they need long
 // contractions: at T42 their forward tile is 37% full.  The FP64 tensor cores
 // (legendre_fp64mma.cu, 8-row tiles, one product, the float arrays' values exact
-// in FP64) take the rest.  Microseconds per launch, tcgen05 / FP64, L20 (T170:
-// L25) with 8 states (T170: one):
-//            T42       T63       T85       T106      T127      T170
-//   inverse  54 / 27   77 / 58   108 / 93  142 / 218 180 / 299 73 / 95
-//   forward  85 / 29   131 / 62  172 / 121 244 / 224 312 / 365 541 / 147
-//   d-set    87 / 23   131 / 50  170 / 81  238 / 155 305 / 235 522 / 110
-// (d-set: the gridpointd forward half, whose tcgen05 jobs would carry empty
-// columns; T170 forward: another tcgen05 kernel, no longer built.)
+// in FP64) take the rest.  The lines lie by truncation alone, whatever the levels and
+// states, so that a state has the same bits in any batch.  Microseconds per launch,
+// tcgen05 / FP64, event overheads of 5 to 8 us included (a tcgen05 forward half also
+// takes k_n0_fp64, 5 us):
+//   8 states   T42      T63       T85        T106       T127       T170 (one, L25)
+//    inverse   54 / 27  80 / 58   109 / 95   142 / 213  178 / 290   78 / 103
+//    forward   84 / 31  130 / 64  170 / 113  239 / 207  304 / 312  539 / 146
+//    d-set     87 / 23  130 / 52  167 / 81   236 / 154  300 / 210  522 / 109
+//   one, L20
+//    inverse   21 / 12  27 / 15   29 / 19    35 / 35    44 / 52     68 / 84
+//    forward   21 / 11  27 / 19   31 / 29    39 / 39    47 / 53    432 / 113
+//    d-set     21 / 11  27 / 17   31 / 17    39 / 25    47 / 35    416 / 80
+//   one, L5
+//    inverse   13 / 9   17 / 11   19 / 13    25 / 21    25 / 23     35 / 35
+//    forward   13 / 11  14 / 14   19 / 21    19 / 27    21 / 34    144 / 58
+//    d-set     13 / 9   14 / 11   19 / 17    19 / 22    21 / 25    131 / 39
+// (d-set: the gridpointd forward half, whose tcgen05 jobs would carry empty columns;
+// T170 forward: another tcgen05 kernel, no longer built.)
 static bool tc_inv(exotx_plan p) { return p->ntp1 > 96; }
 static bool tc_fwd(exotx_plan p) { return p->ntp1 > 112 && p->ntp1 <= 128; }
 // the tcgen05 kernels move spectral coefficients as complex values; the FP64 ones ask for aligned reals only
@@ -394,7 +404,7 @@ static exotx_status tc_inverse_run(exotx_plan p, const float *spin, float *gpout
     EXOTX_TRY(tc_tables(p, &T));
     const long long nrsp = 2LL * p->ncsp, nhor = (long long)p->nlat * p->nlon;
     const int nfo = dset ? 4 * L + 1 : 6 * L + 3;
-    // chunk instances so the m-major Fourier intermediate stays L2-resident
+    // instances a launch covers: as many as the m-major Fourier intermediate may hold (chunk_inv)
     const size_t per_inst = (size_t)nfo * p->nlat * p->ntp1 * sizeof(float2);
     int chunk = (int)std::max<size_t>(1, p->chunk_inv / per_inst);
     chunk = std::min(chunk, ninst);

@@ -623,7 +623,7 @@ __device__ __forceinline__ long long f3_row(const TcFwd3Args &A, int inst, int l
 }
 
 // Operand staging works on slots.  The intermediate is folded about the equator
-// (rfft_fwd_fold_body): each field row holds E = N + S for the latitude pairs,
+// (rr_fwd_body, fft.cu): each field row holds E = N + S for the latitude pairs,
 // then O = N - S, so a parity reads only the half it needs.  A slot is one
 // column pair q (a field level, re and im) and eight latitude pairs j = 8jg ..
 // 8jg+7 of one row (n[] the first four, s[] the next four), stored as one

@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(rad_threads<T>(COLS), RAD_SM_THREADS<T> / rad_
 // of two in FP32, does not fit.  (The registers allow one of 512 threads and three
 // of 256, but two blocks of 16 columns, from 27 levels on, beat the blocks of eight
 // that fit as many columns: L30 160 us against 173.)  8192 columns, L20: 16 columns
-// 176 / 78 us, eight 183 / 81 (FP64 / FP32); eight columns by 512 threads 238, 16 by
+// 176 / 76 us, eight 183 / 81 (FP64 / FP32); eight columns by 512 threads 238, 16 by
 // 256 in FP64 247.
 template <typename T>
 inline int rad_cols(int L) {

@@ -80,10 +80,9 @@ exotx_status exotx_plan_table(exotx_plan p, int which, double *out);
 
 /* Tunables of a plan's tensor-core sets (no counterpart in the reference):
  * the bytes of m-major Fourier intermediate one inverse (forward) launch
- * covers -- instances are grouped up to it, at least one per launch -- so that
- * the intermediate one kernel writes is still in L2 when the next reads it.
- * Default 512 MB each: fewer, larger launches measured faster than L2-sized
- * ones at T127 L20. */
+ * covers; instances are grouped up to it, at least one per launch, and the
+ * plan's work buffer is as large.  Default 512 MB each: fewer, larger launches
+ * measured faster at T127 L20 than ones whose intermediate stays in L2. */
 /* EXOTX_TUNE_INV_HALF: 1 lets the inverse kernel run two CTAs per SM, each
  * holding one parity half of a table, where they fit shared memory; 0 (the
  * default: the two measured alike at T127 L20) keeps one CTA per SM with both
