@@ -126,7 +126,9 @@ exotx_status exotx_dv2gp_scaled(exotx_plan p, int prec, const void *pd, const vo
 exotx_status exotx_gp2sp_scaled(exotx_plan p, int prec, const void *gp, void *sp, int nlev, double scale, void *work,
                                 exotx_stream s);
 
-/* ---- real FFTs of lot rows of length n, in place ---- */
+/* ---- real FFTs of lot rows of length n, in place ----
+ * Few and many rows may take kernels of different order of operations, so a
+ * row's last bits may depend on lot (the transform sets' do not). */
 /* gp2fc (fftmod.f90:29 / fft991mod.f90:32): grid rows -> (A0,0,A1,B1,...) x 1/n */
 exotx_status exotx_gp2fc(int prec, void *a, int n, int lot, exotx_stream s);
 /* fc2gp (fftmod.f90:64 / fft991mod.f90:60): inverse, m=0 imaginary slot ignored */
